@@ -154,6 +154,13 @@ struct P1Args {
     ScoreConsts sc;
     float* bot;             // strip-boundary rows: per warp slot 2 x 5 x Lmax
     long long botstride;    // floats per warp slot
+    // phase-1 pairs whose strips are work items of their own (the first nsplit of order)
+    int nsplit;
+    const long long* sboff; // sum of the lengths (rounded up to 4) before each pair of order
+    float* sbnd;            // per split pair at 10 x sboff: two last-row buffers of 5 floats a column
+    int* sprog;             // [nstrips][nsplit] finished columns per strip
+    int* sdone;             // [nsplit] finished strips
+    unsigned long long* skey;  // [nsplit] maximum so far and its cell, packed
     // phase-1 outputs (indexed by profile)
     float* best;
     unsigned* coords;

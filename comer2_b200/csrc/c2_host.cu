@@ -104,8 +104,10 @@ struct DevBuf {
 struct DbStore {
     DevBuf<float> d_drec, d_pbkg, d_dtrn, d_peno;
     DevBuf<int> d_plen, d_order;
-    DevBuf<long long> d_poff;
+    DevBuf<long long> d_poff, d_soff;
     DevBuf<unsigned char> d_daa, d_dss;
+    std::vector<int> slen;             // lengths in processing order (longest first)
+    std::vector<long long> soff;       // sums of the lengths (rounded up to 4) before each, and the total (d_soff)
     // tensor-core score operands, packed on first use (under tc_mu)
     DevBuf<unsigned> d_tcdb;
     DevBuf<long long> d_ttile;
@@ -172,6 +174,8 @@ struct c2_handle {
     DevBuf<int> d_counter;
     DevBuf<float> d_bot;
     long long botstride = 0;
+    DevBuf<float> d_splitbnd;                  // phase-1 pairs split into strip items (split_pairs)
+    DevBuf<unsigned long long> d_splitsync;    // their maxima, done counts and strip progress
     // finalisation
     int ncand = 0;
     std::vector<int> h_cand;
@@ -246,7 +250,7 @@ static const char* status_text(int st)
 {
     switch (st) {
     case 2: return "traceback DP disagrees with phase 1";
-    case PIPE_ERR_TIMEOUT: return "a strip wait in a phase-2 sweep timed out";
+    case PIPE_ERR_TIMEOUT: return "a strip wait timed out";
     default: return "unknown device error";
     }
 }
@@ -704,8 +708,15 @@ extern "C" c2_status c2_upload_db(c2_handle* h, const c2_profiles* d, uint64_t t
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return d->lengths[a] > d->lengths[b]; });
     std::vector<long long> poff(d->offsets, d->offsets + P);
+    h->db->slen.resize(P);
+    h->db->soff.assign((size_t)P + 1, 0);
+    for (int i = 0; i < P; i++) {
+        h->db->slen[i] = d->lengths[order[i]];
+        h->db->soff[i + 1] = h->db->soff[i] + ((h->db->slen[i] + 3) & ~3);
+    }
     if (h->db->d_drec.ensure((size_t)N * DR_STRIDE, h->budget) || h->db->d_pbkg.ensure(bkg.size(), h->budget) || h->db->d_plen.ensure(P, h->budget) ||
-        h->db->d_order.ensure(P, h->budget) || h->db->d_poff.ensure(P, h->budget) || h->d_best.ensure(P, h->budget) || h->d_coords.ensure(P, h->budget))
+        h->db->d_order.ensure(P, h->budget) || h->db->d_poff.ensure(P, h->budget) ||
+        h->db->d_soff.ensure(P, h->budget) || h->d_best.ensure(P, h->budget) || h->d_coords.ensure(P, h->budget))
         return fail(h, C2_ERR_NOMEM, "device allocation for %d profiles / %lld positions failed", P, (long long)N);
     if (h->db->d_dtrn.ensure((size_t)(N + P) * 7, h->budget))
         return fail(h, C2_ERR_NOMEM, "device allocation of db transitions failed");
@@ -714,6 +725,7 @@ extern "C" c2_status c2_upload_db(c2_handle* h, const c2_profiles* d, uint64_t t
     CK(cudaMemcpy(h->db->d_plen.p, d->lengths, (size_t)P * 4, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->db->d_order.p, order.data(), (size_t)P * 4, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->db->d_poff.p, poff.data(), (size_t)P * 8, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(h->db->d_soff.p, h->db->soff.data(), (size_t)P * 8, cudaMemcpyHostToDevice));
     // raw transitions, residues, SS states and ENOs for the statistics and MAP stages
     if (h->db->d_daa.ensure((size_t)N, h->budget) || h->db->d_dss.ensure((size_t)N, h->budget) ||
         h->db->d_peno.ensure((size_t)P, h->budget))
@@ -1083,6 +1095,48 @@ static void fill_p1(c2_handle* h, P1Args& a)
     a.spin = h->spin;
 }
 
+// Phase-1 pairs whose strips become work items of their own (p1_take): those
+// that one of the nwarps warps would sweep in more than SPLIT_SHARE of the
+// time all pairs together take on all warps (both grow with the number of
+// strips alike, so the query length does not enter).  Pairs below that even
+// out over the warps by the longest-first order; pairs above it would be the
+// tail of the search.  Phase-1 times with shares of infinity (none split) / 1 /
+// 0.5 / 0.25 / 0.1: 1 x 3,000 vs 4,000 profiles 41.9 / 23.2 / 23.8 / 26.7 / 25.7
+// ms, 1 x 1,237 vs 4,999 16.2 / 9.7 / 10.4 / 10.8 / 11.3, 1 x 250 vs 3,000 (FP32)
+// 4.5 / 2.3 / 2.1 / 2.3 / 2.3, 7 queries vs 1,000 (FP32) 32 / 11 / 8.4 / 8.6 /
+// 8.6, 1 x 150 vs 2,000 0.70 / 0.66 / 0.60 / 0.57 / 0.55; no pair is split (and
+// nothing changes) against 50,000 profiles.  0 without the scratch (it is small: the two boundary
+// rows of the split pairs) -- the pairs then run whole, with the same results.
+constexpr double SPLIT_SHARE = 0.5;
+
+static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
+{
+    const int P = h->nprof, ns = (h->Lq + 31) / 32;
+    a.nsplit = 0;
+    if (ns < 2) return 0;
+    const double mean = ((double)h->npos + 31.0 * P) / std::max(1, nwarps);
+    const std::vector<int>& sl = h->db->slen;
+    const int n = (int)(std::partition_point(sl.begin(), sl.end(),
+                                             [&](int L) { return (double)L + 31.0 > SPLIT_SHARE * mean; }) - sl.begin());
+    if (n == 0 || (long long)n * ns > 0x7fffffff) return 0;
+    const size_t words = (size_t)n * 8 + (size_t)n * 4 + (size_t)n * ns * 4;
+    if (h->d_splitbnd.ensure((size_t)h->db->soff[n] * 10, h->budget) != cudaSuccess ||
+        h->d_splitsync.ensure((words + 7) / 8, h->budget) != cudaSuccess ||
+        cudaMemsetAsync(h->d_splitsync.p, 0, words, h->stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        h->d_splitbnd.release();
+        h->d_splitsync.release();
+        return 0;
+    }
+    a.nsplit = n;
+    a.sboff = h->db->d_soff.p;
+    a.sbnd = h->d_splitbnd.p;
+    a.skey = h->d_splitsync.p;
+    a.sdone = reinterpret_cast<int*>(h->d_splitsync.p + n);
+    a.sprog = a.sdone + n;
+    return n;
+}
+
 extern "C" c2_status c2_run_phase1(c2_handle* h)
 {
     if (!h) return C2_ERR_ARG;
@@ -1108,6 +1162,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
             return fail(h, C2_ERR_CUDA, "tensor-core phase-1 kernel does not fit on an SM (%s)",
                         cudaGetErrorString(oe));
         gt = std::min(gt, h->grid * P1_WARPS / P1T_WARPS);
+        split_pairs(h, gt * P1T_WARPS, a);
         CK(launch_p1(a, h->d_qbkg.p, P1K_TENSOR, gt, h->stream));
         h->launches++;
         return C2_OK;
@@ -1117,6 +1172,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     int gc = (h->nsm - h->p1_reserve) * p1c_blocks_per_sm(h->sc.cvcard);
     if (gc < 1) return fail(h, C2_ERR_CUDA, "phase-1 kernel does not fit on an SM");
     gc = std::min(gc, h->grid * P1_WARPS / P1C_WARPS);
+    split_pairs(h, gc * P1C_WARPS, a);
     CK(launch_p1(a, h->d_qbkg.p, P1K_CHUNKED, gc, h->stream));
     h->launches++;
     return C2_OK;
@@ -1180,7 +1236,7 @@ extern "C" c2_status c2_db_device_bytes(const c2_handle* h, int64_t npositions, 
     const uint64_t N = (uint64_t)npositions, P = (uint64_t)nprofiles;
     uint64_t b = N * DR_STRIDE * sizeof(float)                 // d_drec
                  + P * NAA * sizeof(float)                     // d_pbkg
-                 + P * (sizeof(int) * 2 + sizeof(long long))   // d_plen, d_order, d_poff
+                 + P * (sizeof(int) * 2 + sizeof(long long) * 2)   // d_plen, d_order, d_poff, d_soff
                  + P * (sizeof(float) + sizeof(unsigned))      // d_best, d_coords
                  + (N + P) * 7 * sizeof(float)                 // d_dtrn
                  + N * 2                                        // d_daa, d_dss

@@ -130,6 +130,7 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Stage the records of columns [REC_CHUNK*m, REC_CHUNK*(m+1)) (clipped to L)
@@ -390,7 +391,6 @@ struct WfLane {
     float qMM, qMI, qII;
     float2 XB, YB;                // diagonal sums of the column -1 boundary state
     float zB, lbMM, lbIM, lbND;   // and the column -1 left state
-    float bnxt[5];                // row above the strip: columns [32m+32, 32m+64) (lane i: column 32m+32+i)
     float best;
     int kbest;
 };
@@ -539,6 +539,156 @@ __device__ __forceinline__ void bot_flush(const float* __restrict__ bnd, float* 
 __device__ __forceinline__ int corner_a(int r, int Lq, int edge) { return (Lq <= r + edge) ? edge + r - Lq : -1; }
 __device__ __forceinline__ int corner_b(int r, int L, int edge) { return (r < edge) ? L - edge + r : 0x7fffffff; }
 
+// Phase-1 work items.  A pair is swept by one warp, strip after strip, with
+// the rows between the strips in the warp's own boundary buffer -- except the
+// nsplit longest pairs, whose strips are items of their own (any warp may take
+// them): those hand the rows on through per-pair buffers with published
+// progress, as the phase-2 sweeps do (c2_device.cuh).  Without that a search
+// with few pairs, or with pairs much longer than the mean, ends in a tail where
+// a few warps walk all strips of a long pair alone: 1 x 1,237 against 4,999
+// profiles took 16.3 ms, the time of its longest pair (39 strips x 2,031 steps).
+// Which pairs are split: split_pairs (c2_host.cu).
+// Order: strip 0 of all split pairs, then strip 1 and so on, then the whole
+// pairs, all from one counter: strip s is taken after strip s - 1, by a running
+// warp, and the whole pairs, the shortest last, even out the end.  (Warps that
+// look whether the next strip is ready and exchange the counter only then,
+// taking a whole pair otherwise, serialise on the counter: 5 times slower on
+// 10,000 items.)
+struct P1Item {
+    int p, L;        // profile, its length
+    int s0, s1;      // strips [s0, s1)
+    int pi;          // split pair (index in the longest-first order), -1: whole pair
+};
+
+__device__ __forceinline__ bool p1_take(const P1Args& a, int nstrips, int lane, P1Item& it)
+{
+    int item = 0;
+    if (lane == 0) item = atomicAdd(a.counter, 1);
+    item = __shfl_sync(FULL, item, 0);
+    const int nsi = a.nsplit * nstrips;
+    int code = item - nsi + a.nsplit, strip = -1;   // index in the longest-first order; strip (-1: all)
+    if (item < nsi) {
+        strip = item / a.nsplit;
+        code = item - strip * a.nsplit;
+    } else if (code >= a.nwork) {
+        return false;
+    }
+    it.p = a.order[code];
+    it.L = a.plen[it.p];
+    it.pi = strip < 0 ? -1 : code;
+    it.s0 = strip < 0 ? 0 : strip;
+    it.s1 = strip < 0 ? nstrips : strip + 1;
+    return true;
+}
+
+// The rows between the strips of a pair, in the layout of the shared-memory
+// row (bnd_put): states MM MI IM DN per column, then the ND values from
+// 4 ldb on; ldb a multiple of 4 columns, the buffer 16-byte aligned.  Each
+// half is thus one wide store or asynchronous copy per chunk.
+
+// Wait (split pairs only) until columns [c0, c0 + 32) of the row above strip s
+// are there; false: no such row
+__device__ __forceinline__ bool p1_row_ready(const P1Args& a, const P1Item& it, int s, int c0, int lane, bool& broken)
+{
+    const bool have = s > 0 && c0 < it.L;
+    if (have && it.pi >= 0)
+        pipe_wait(a.sprog + (long long)(s - 1) * a.nsplit + it.pi, min(c0 + 32, it.L), lane, a.status, broken, a.spin);
+    return have;
+}
+
+// The row above strip s, columns [c0, c0 + 32), into the warp's shared row by
+// asynchronous copies through L2 (a split pair's row comes from another SM);
+// zeros where there is none.  Commits one group.  Columns past the matrix hold
+// whatever the buffer does: no cell inside the matrix reads them.
+__device__ __forceinline__ void p1_row_async(const P1Args& a, const P1Item& it, int s, float* bnd,
+                                             const float* __restrict__ botr, int ldb, int c0, int lane, bool& broken)
+{
+    if (p1_row_ready(a, it, s, c0, lane, broken)) {
+        const int c = c0 + lane, c4 = c0 + 4 * lane;
+        if (c < it.L) cp_async16(bnd + 4 * lane, botr + 4 * c);
+        if (lane < 8 && c4 < it.L) cp_async16(bnd + BND_ND + 4 * lane, botr + 4 * ldb + c4);
+    } else {
+        bnd_put(bnd, lane, 0.f, 0.f, 0.f, 0.f, 0.f);
+    }
+    cp_async_commit();
+}
+
+// The same into registers (lane i: column c0 + i)
+__device__ __forceinline__ void p1_row_load(const P1Args& a, const P1Item& it, int s, const float* __restrict__ botr,
+                                            int ldb, int c0, int lane, bool& broken, float4& v, float& nd)
+{
+    const int c = c0 + lane;
+    v = make_float4(0.f, 0.f, 0.f, 0.f);
+    nd = 0.f;
+    if (p1_row_ready(a, it, s, c0, lane, broken) && c < it.L) {
+        v = __ldcg(reinterpret_cast<const float4*>(botr) + c);
+        nd = __ldcg(botr + 4 * ldb + c);
+    }
+}
+
+// The strip's last row after a DP stage over [k0, k0 + 32) (as bot_flush)
+__device__ __forceinline__ void p1_row_flush(const float* __restrict__ bnd, float* __restrict__ botw, int ldb, int k0,
+                                             int L, int lane)
+{
+    const int c = k0 - 31 + lane;
+    if (c >= 0 && c < L) {
+        reinterpret_cast<float4*>(botw)[c] = *reinterpret_cast<const float4*>(bnd + lane * 4);
+        botw[4 * ldb + c] = bnd[BND_ND + lane];
+    }
+}
+
+// Strip s of a split pair has stored the columns [0, n) of its last row
+__device__ __forceinline__ void p1_publish(const P1Args& a, const P1Item& it, int s, int n, int lane)
+{
+    __syncwarp();
+    if (lane == 0) {
+        __threadfence();
+        pipe_st_release(a.sprog + (long long)s * a.nsplit + it.pi, n);
+    }
+}
+
+// The item's maximum over its lanes (largest score, then smallest row, then
+// smallest column) to the pair's result.  Strips of a split pair combine theirs
+// as a 64-bit key (score bits, complement of the cell); the strip that
+// completes the pair writes the result.
+__device__ __forceinline__ void p1_result(const P1Args& a, const P1Item& it, int nstrips, int lane, float b, int row,
+                                          int col)
+{
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        const float ob = __shfl_xor_sync(FULL, b, o);
+        const int orr = __shfl_xor_sync(FULL, row, o);
+        const int oc = __shfl_xor_sync(FULL, col, o);
+        if (ob > b || (ob == b && (orr < row || (orr == row && oc < col)))) {
+            b = ob; row = orr; col = oc;
+        }
+    }
+    if (lane == 0) {
+        bool wr = true;
+        if (it.pi >= 0) {
+            const unsigned cell = ((unsigned)row << 16) | ((unsigned)col & 0xffffu);
+            if (b > 0.f)
+                atomicMax(a.skey + it.pi,
+                          ((unsigned long long)__float_as_uint(b) << 32) | (unsigned long long)(0xffffffffu - cell));
+            __threadfence();
+            wr = atomicAdd(a.sdone + it.pi, 1) == nstrips - 1;
+            if (wr) {
+                __threadfence();
+                const unsigned long long key = atomicMax(a.skey + it.pi, 0ull);
+                const unsigned c = 0xffffffffu - (unsigned)(key & 0xffffffffu);
+                b = __uint_as_float((unsigned)(key >> 32));
+                row = (int)(c >> 16);
+                col = (int)(c & 0xffffu);
+            }
+        }
+        if (wr) {
+            a.best[it.p] = b;
+            a.coords[it.p] = (b > 0.f) ? (((unsigned)col << 16) | ((unsigned)row & 0xffffu)) : 0u;
+        }
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(P1C_WARPS * 32, 1)
 p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 {
@@ -563,23 +713,24 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
     const int nstrips = (Lq + 31) >> 5;
     const ScoreConsts sc = a.sc;
 
+    bool broken = false;   // a strip wait gave up
     for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(a.counter, 1);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= a.nwork) break;
-        const int p = a.order[item];
-        const int L = a.plen[p];
+        P1Item it;
+        if (!p1_take(a, nstrips, lane, it)) break;
+        const int p = it.p, L = it.L;
         const long long off = a.poff[p];
         const float* __restrict__ dr = a.drec + off * DR_STRIDE;
         const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
         const int edge = corner_edge(Lq, L);
-        float* botr = bot0;
-        float* botw = bot0 + 5 * Lmax;
+        // rows between the strips: the warp's own buffer, or the split pair's
+        const int ldb = it.pi < 0 ? Lmax : (L + 3) & ~3;
+        float* botr = it.pi < 0 ? bot0 : a.sbnd + 10 * a.sboff[it.pi];
+        float* botw = botr + 5 * ldb;
+        if (it.s0 & 1) { float* t = botr; botr = botw; botw = t; }
         float pbest = 0.f;
         int prow = 0x7fffffff, pcol = 0x7fffffff;
 
-        for (int s = 0; s < nstrips; s++) {
+        for (int s = it.s0; s < it.s1; s++) {
             const int r = s * 32 + lane;
             const bool act = r < Lq;
             const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
@@ -613,25 +764,17 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
             const int cA = corner_a(r, Lq, edge);
             const int cB = corner_b(r, L, edge);
             wf_init(D, q7, LB, DB);
-            float bc[5];
-#pragma unroll
-            for (int f = 0; f < 5; f++) {
-                bc[f] = 0.f;
-                D.bnxt[f] = 0.f;
-                if (s > 0) {
-                    if (lane < L) bc[f] = botr[f * Lmax + lane];
-                    if (32 + lane < L) D.bnxt[f] = botr[f * Lmax + 32 + lane];
-                }
-            }
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             __syncwarp();
-            // columns [0, 32) of the row above, lane i holding column i
-            bnd_put(bnd, lane, bc[0], bc[1], bc[2], bc[3], bc[4]);
             stage_chunk(rec, dr, 0, L, lane);
             stage_chunk(rec, dr, 1, L, lane);
             const int nch = (L + 31) >> 5;        // chunks holding columns
             const int kend = L + 31;              // wavefront steps of the strip
             for (int m = 0; 32 * m < kend; m++) {
+                // the row above for this chunk's steps, loaded during the score stage
+                float4 row;
+                float rownd;
+                p1_row_load(a, it, s, botr, ldb, 32 * m, lane, broken, row, rownd);
                 // ---- score stage: columns [32m, min(32m + 32, L))
                 if (m < nch) {
                     const int c0 = 32 * m, c1 = min(c0 + 32, L);
@@ -656,6 +799,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
                         }
                     }
                 }
+                bnd_put(bnd, lane, row.x, row.y, row.z, row.w, rownd);
                 __syncwarp();
                 // ---- DP stage: wavefront steps [32m, 32m + 32)
                 const int k0 = 32 * m, k1 = min(k0 + 32, kend);
@@ -664,14 +808,9 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
                 else
                     wf_steps<true, 32, false, P1C_RING - 1>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot);
                 __syncwarp();
-                if (s + 1 < nstrips) bot_flush(bnd, botw, k0, L, Lmax, lane);
-                __syncwarp();
-                // next 32 columns of the row above the strip
-                bnd_put(bnd, lane, D.bnxt[0], D.bnxt[1], D.bnxt[2], D.bnxt[3], D.bnxt[4]);
-#pragma unroll
-                for (int f = 0; f < 5; f++) {
-                    const int cc = k0 + 64 + lane;
-                    D.bnxt[f] = (s > 0 && cc < L) ? botr[f * Lmax + cc] : 0.f;
+                if (s + 1 < nstrips) {
+                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
+                    if (it.pi >= 0) p1_publish(a, it, s, min(k1 - 31, L), lane);
                 }
                 __syncwarp();
             }
@@ -688,21 +827,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
             float* t = botr; botr = botw; botw = t;
             __syncwarp();
         }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            const float ob = __shfl_xor_sync(FULL, pbest, o);
-            const int orr = __shfl_xor_sync(FULL, prow, o);
-            const int oc = __shfl_xor_sync(FULL, pcol, o);
-            if (ob > pbest || (ob == pbest && (orr < prow || (orr == prow && oc < pcol)))) {
-                pbest = ob; prow = orr; pcol = oc;
-            }
-        }
-        if (lane == 0) {
-            const unsigned xy = (pbest > 0.f) ? (((unsigned)pcol << 16) | ((unsigned)prow & 0xffffu)) : 0u;
-            a.best[p] = pbest;
-            a.coords[p] = xy;
-        }
-        __syncwarp();
+        p1_result(a, it, nstrips, lane, pbest, prow, pcol);
     }
 }
 
@@ -861,14 +986,11 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
         }
         const int cA = corner_a(r, Lq, edge);
         const int cB = corner_b(r, L, edge);
-        // columns [0, 32) of the row above, lane i holding column i
-        float bc[5];
+        // columns [0, 32) of the row above, lane i holding column i; bnxt: the next 32
+        float bc[5], bnxt[5];
         if (s > 0) pipe_wait(pf + s - 1, min(32, L), lane, a.status, broken, a.spin);
 #pragma unroll
-        for (int f = 0; f < 5; f++) {
-            bc[f] = (s > 0 && lane < L) ? __ldcg(botr + f * L + lane) : 0.f;
-            D.bnxt[f] = 0.f;
-        }
+        for (int f = 0; f < 5; f++) bc[f] = (s > 0 && lane < L) ? __ldcg(botr + f * L + lane) : 0.f;
         const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
         __syncwarp();
         bnd_put(bnd, lane, bc[0], bc[1], bc[2], bc[3], bc[4]);
@@ -897,11 +1019,11 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
 #pragma unroll
                 for (int f = 0; f < 5; f++) {
                     const int cc = k0 + 32 + lane;
-                    D.bnxt[f] = (cc < L) ? __ldcg(botr + f * L + cc) : 0.f;
+                    bnxt[f] = (cc < L) ? __ldcg(botr + f * L + cc) : 0.f;
                 }
             } else {
 #pragma unroll
-                for (int f = 0; f < 5; f++) D.bnxt[f] = 0.f;
+                for (int f = 0; f < 5; f++) bnxt[f] = 0.f;
             }
             __syncwarp();
             // ---- DP stage: wavefront steps [32m, 32m + 32), traceback codes stored
@@ -922,7 +1044,7 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
                 }
             }
             __syncwarp();
-            bnd_put(bnd, lane, D.bnxt[0], D.bnxt[1], D.bnxt[2], D.bnxt[3], D.bnxt[4]);
+            bnd_put(bnd, lane, bnxt[0], bnxt[1], bnxt[2], bnxt[3], bnxt[4]);
             __syncwarp();
         }
         // the strip's maximum: largest score, then smallest row, then smallest column
@@ -1240,24 +1362,25 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
     // this lane's CV table replica, offset so that index 0 is the table's key 0
     const float* __restrict__ cvl = cvtab + a.sc.cvshift * P1T_CVREP + (lane & (P1T_CVREP - 1));
 
+    bool broken = false;   // a strip wait gave up
     for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(a.counter, 1);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= a.nwork) break;
-        const int p = a.order[item];
-        const int L = a.plen[p];
+        P1Item it;
+        if (!p1_take(a, nstrips, lane, it)) break;
+        const int p = it.p, L = it.L;
         const long long off = a.poff[p];
         const float* __restrict__ cold = a.cold + off * P1C_TRS;
         const unsigned* __restrict__ tb0 = a.tcdb + a.ttile[p] * (long long)TC_TILE_WORDS;
         const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
         const int edge = corner_edge(Lq, L);
-        float* botr = bot0;
-        float* botw = bot0 + 5 * Lmax;
+        // rows between the strips: the warp's own buffer, or the split pair's
+        const int ldb = it.pi < 0 ? Lmax : (L + 3) & ~3;
+        float* botr = it.pi < 0 ? bot0 : a.sbnd + 10 * a.sboff[it.pi];
+        float* botw = botr + 5 * ldb;
+        if (it.s0 & 1) { float* t = botr; botr = botw; botw = t; }
         float pbest = 0.f;
         int prow = 0x7fffffff, pcol = 0x7fffffff;
 
-        for (int s = 0; s < nstrips; s++) {
+        for (int s = it.s0; s < it.s1; s++) {
             const int r = s * 32 + lane;
             const bool act = r < Lq;
             const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
@@ -1335,19 +1458,8 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             }
             const int cA = corner_a(r, Lq, edge);
             const int cB = corner_b(r, L, edge);
-            float bc[5];
-#pragma unroll
-            for (int f = 0; f < 5; f++) {
-                bc[f] = 0.f;
-                D.bnxt[f] = 0.f;
-                if (s > 0) {
-                    if (lane < L) bc[f] = botr[f * Lmax + lane];
-                    if (32 + lane < L) D.bnxt[f] = botr[f * Lmax + 32 + lane];
-                }
-            }
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             __syncwarp();
-            bnd_put(bnd, lane, bc[0], bc[1], bc[2], bc[3], bc[4]);
             stage_cols(cring, cold, 0, L, lane);
             stage_cols(cring, cold, 1, L, lane);
             const int nch = (L + 31) >> 5;
@@ -1358,8 +1470,10 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             const int ntile = 4 * nch;
             if (lane == 0 && !tbroken) bulk_load(btile, tb0, TC_TILE_WORDS * 4, tbar);
             for (int m = 0; 32 * m < kend; m++) {
+                // the row above for this chunk's steps, copied during the score stage
+                p1_row_async(a, it, s, bnd, botr, ldb, 32 * m, lane, broken);
                 if (m < nch) {
-                    cp_async_wait_1();   // column records of chunk m have landed
+                    cp_async_wait_2();   // column records of chunk m have landed
                     __syncwarp();
                     // the next chunk's db operands (12 KB) towards L2 while this one is used
                     if (m + 1 < nch) {
@@ -1449,6 +1563,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                         }
                     }
                 }
+                cp_async_wait_all();
                 __syncwarp();
                 // ---- DP stage: wavefront steps [32m, 32m + 32).  A full stage
                 // after the first runs without bounds checks also where it passes
@@ -1462,13 +1577,9 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                 else
                     wf_steps<true, P1T_RLD, true, 0>(D, k0, k1 - k0, lane, L, act, ring, tcol, bnd, wr_bot);
                 __syncwarp();
-                if (s + 1 < nstrips) bot_flush(bnd, botw, k0, L, Lmax, lane);
-                __syncwarp();
-                bnd_put(bnd, lane, D.bnxt[0], D.bnxt[1], D.bnxt[2], D.bnxt[3], D.bnxt[4]);
-#pragma unroll
-                for (int f = 0; f < 5; f++) {
-                    const int cc = k0 + 64 + lane;
-                    D.bnxt[f] = (s > 0 && cc < L) ? botr[f * Lmax + cc] : 0.f;
+                if (s + 1 < nstrips) {
+                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
+                    if (it.pi >= 0) p1_publish(a, it, s, min(k1 - 31, L), lane);
                 }
                 // chunk m - 1's records are no longer read: chunk m + 2 into its slots
                 stage_cols(cring, cold, m + 2, L, lane);
@@ -1486,21 +1597,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             float* t = botr; botr = botw; botw = t;
             __syncwarp();
         }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            const float ob = __shfl_xor_sync(FULL, pbest, o);
-            const int orr = __shfl_xor_sync(FULL, prow, o);
-            const int oc = __shfl_xor_sync(FULL, pcol, o);
-            if (ob > pbest || (ob == pbest && (orr < prow || (orr == prow && oc < pcol)))) {
-                pbest = ob; prow = orr; pcol = oc;
-            }
-        }
-        if (lane == 0) {
-            const unsigned xy = (pbest > 0.f) ? (((unsigned)pcol << 16) | ((unsigned)prow & 0xffffu)) : 0u;
-            a.best[p] = pbest;
-            a.coords[p] = xy;
-        }
-        __syncwarp();
+        p1_result(a, it, nstrips, lane, pbest, prow, pcol);
     }
     if (tbroken) (void)mbar_wait(tbar, tpend);
     // every warp is past its last TMEM access: the allocating warp frees it
