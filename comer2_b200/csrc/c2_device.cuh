@@ -55,15 +55,22 @@ constexpr int MAX_CVCARD = 256;
 // Tensor-core (BF16 split) phase-1 kernel.  The three contractions of a cell
 // score -- amino acids (K = 20), context vectors (K = 19) and the SS table
 // (K = card <= 32, the db side a 3-hot vector of SS probabilities) -- run as
-// mma.sync m16n8k16 BF16 products with FP32 accumulation, each operand split
-// into hi + lo BF16 parts (x = hi + lo + O(2^-17 x)) and hi*hi + hi*lo +
-// lo*hi accumulated.  db operands (B, k16 x n8 fragments) are packed once per
-// database in the fragment order of the 32 lanes, 8 db columns per tile:
-//   tcdb[tile][dot 3][ktile 2][split 2][lane 32][2 words]
-// with every profile padded to a multiple of 32 columns; query operands (A,
-// m16 x k16) per query: qa[strip][mtile 2][dot 2: cv, ss][ktile 2][split 2]
-// [lane 32][4 words] and the unscaled amino-acid rows qaa[strip][mtile 2]
-// [ktile 2][lane 32][8 floats] (scaled per pair by 1 / (0.5 (bq + bd))).
+// mma.sync BF16 products with FP32 accumulation (K 16 + 8 for the first two,
+// 16 + 16 for the third), each operand split into hi + lo BF16 parts
+// (x = hi + lo + O(2^-17 x)) and hi*hi + hi*lo + lo*hi accumulated.  db
+// operands (B fragments) are packed once per database in the fragment order
+// of the 32 lanes, 8 db columns per tile (ceil(L / 8) tiles a profile):
+//   tcdb[tile][5][lane 32][4 words]
+//     0: aa hi k0-15 (2 words), aa hi k16-23, aa lo k16-23
+//     1: aa lo k0-15 (2), cv hi k0-15 (2)
+//     2: cv lo k0-15 (2), cv hi k16-23, cv lo k16-23
+//     3: ss hi k0-15 (2), ss hi k16-31 (2)     4: ss lo, the same
+// query operands (A fragments, strips of 64 rows) per query: context vectors
+// and SS tables qa[strip][mtile 4][7][lane 32][4 words] (cv hi k0-15 (4), hi
+// k16-23 (2), lo k0-15 (4), lo k16-23 (2); ss hi k0-15 (4), hi k16-31 (4), lo
+// k0-15 (4), lo k16-31 (4)) and the unscaled amino-acid rows
+// qaa[strip][mtile 4][3][lane 32][4 floats] (k0-15: 8, k16-23: 4; scaled per
+// pair by 1 / (0.5 (bq + bd)) and split).
 // The constant parts of the CV and SS terms ride in the spare K columns:
 // CV k = 19 carries 1 (query) x 1/kappa0 (db), so the CV accumulator is the
 // shifted dot product; the SS operand is weighted by the SS weight on the db
@@ -72,19 +79,20 @@ constexpr int MAX_CVCARD = 256;
 // "-99 < ss" guard always holds for tables above SS_FOLD_MIN, which the
 // tensor-core form requires, with card <= 30).
 // Per db position the DP and the score epilogue also read a column record
-// cold[pos][P1C_TRS]: the DP transitions in the pair order below (slots
-// 0..8), cvnorm, 2 x CV log prior, pad.
-constexpr int TC_TILE_WORDS = 3 * 2 * 2 * 32 * 2;
-constexpr int TC_QA_WORDS = 2 * 2 * 2 * 2 * 32 * 4;   // per strip
-constexpr int TC_QAA_FLOATS = 2 * 2 * 32 * 8;         // per strip
+// cold[pos][P1C_TRS]: the DP transitions in the order below (slots 0..6),
+// cvnorm and 2 x CV log prior (slots 8, 9), pad.
+constexpr int P1T_ROWS = 64;                          // query rows per strip
+constexpr int TC_TILE_WORDS = 5 * 32 * 4;
+constexpr int TC_QA_WORDS = 4 * 7 * 32 * 4;           // per strip
+constexpr int TC_QAA_FLOATS = 4 * 3 * 32 * 4;         // per strip
 constexpr float SS_FOLD_MIN = -49.f;
 constexpr int TC_SS_KMAX = 30;
-enum : int { CO_CD = 9, CO_PD2 = 10 };
-// DP transition record of a db column, ordered for the packed-pair Viterbi
-// step: (MM, MM), (IM, MM), (MD, DD), MI, II, DM.  DPT_SRC packs, per record
-// slot i, the transition index (TMM..TDD) in bits [4i, 4i + 4).
-constexpr int DPT_N = 9;
-constexpr unsigned long long DPT_SRC = 0x541620300ull;
+enum : int { CO_CD = 8, CO_PD2 = 9 };
+// DP transition record of a db column, two 16-byte reads of a Viterbi step:
+// MM IM DM MI, II MD DD.  DPT_SRC packs, per record slot i, the transition
+// index (TMM..TDD) in bits [4i, 4i + 4).
+constexpr int DPT_N = 7;
+constexpr unsigned long long DPT_SRC = 0x6241530ull;
 __host__ __device__ constexpr int dpt_src(int i) { return (int)((DPT_SRC >> (4 * i)) & 0xf); }
 // chunked phase-1 kernel: 11 warps per CTA, one CTA per SM; per warp a score
 // ring of 64 columns x 32 rows, a transition ring of 64 columns (stride 12
@@ -110,24 +118,31 @@ constexpr int P2S_WARPS = 8;
 constexpr int P2S_WARP_FLOATS = MAX_SSSS_CARD * 32 + REC_SLOTS * DR_STRIDE;
 
 // Largest CV maps the shared-memory layouts hold (opt-in shared memory per CTA
-// on sm_100: 227 KB): the phase-2 score kernel, which every search runs, and the
-// tensor-core phase-1 kernel (whose 16 bytes of static shared memory hold the
-// TMEM address).  The reference's cvs2s map has 93 entries.
+// on sm_100: 227 KB): the phase-2 score kernel, which every search runs.  The
+// tensor-core form takes maps of up to 106 entries.  The reference's cvs2s map
+// has 93 entries.
 constexpr int SMEM_CTA_MAX = 227 * 1024;
 constexpr int P1TC_MAX_CVCARD =
     (SMEM_CTA_MAX - P2S_WARPS * P2S_WARP_FLOATS * 4) / (P1TC_CVREP * 4);
-// tensor-core kernel: score ring of 64 anti-diagonals with 36 floats each (the
-// fragment-layout writes and the per-lane wavefront reads are both free of
-// bank conflicts), a column-record ring of 3 chunks plus a mirror of its first
-// chunk (slots 96..127), so that the 32 records a lane reads in one DP stage
-// never wrap, the row above the strip and one slot for the db operand tile
-// (a bulk async copy, one mbarrier); 12 warps fit with a CV table of up to
-// 106 entries
+constexpr int P1T_MAX_CVCARD = 106;
+// Tensor-core kernel, two query rows per lane (strips of 64 rows), the db
+// columns in chunks of 8 (one operand tile).  Per warp: score ring of 40
+// anti-diagonals (31 lanes of skew + a chunk) of 64 floats, padded to 68 so
+// that the fragment-layout writes and the wavefront's 8-byte reads are both
+// free of bank conflicts; column-record ring of 7 chunks and a mirror of its
+// first chunk, so that the 8 records a lane reads in one DP stage never wrap;
+// the row above the strip for one chunk; the rows' score terms; one slot for
+// the db operand tile (a bulk async copy, one mbarrier).
 constexpr int P1T_WARPS = 12;
-constexpr int P1T_RLD = 36, P1T_CRING = 128, P1T_CMOD = 96, P1T_CVREP = 8;
-constexpr unsigned P1T_TMEM_COLS = 512;   // TMEM columns of a CTA (3 warps x 128 per lane quarter)
-constexpr int P1T_WARP_FLOATS = P1C_RING * P1T_RLD + P1T_CRING * P1C_TRS + BND_FLOATS + TC_TILE_WORDS + 4;
-constexpr int P1T_MAX_CVCARD = (SMEM_CTA_MAX - 16 - P1T_WARPS * P1T_WARP_FLOATS * 4) / (P1T_CVREP * 4);
+constexpr int P1T_C = 8;
+constexpr int P1T_SLOTS = 40, P1T_RLD = 68, P1T_CMOD = 56, P1T_CRING = 64, P1T_CVREP = 16;
+constexpr unsigned P1T_TMEM_COLS = 512;   // TMEM columns of a CTA: 3 warps x 160 per lane quarter
+constexpr int P1T_TMEM_MT = 40, P1T_TMEM_WARP = 4 * P1T_TMEM_MT;
+constexpr int P1T_BND = 5 * P1T_C;
+constexpr int P1T_WARP_FLOATS =
+    P1T_SLOTS * P1T_RLD + P1T_CRING * P1C_TRS + P1T_BND + 2 * P1T_ROWS + TC_TILE_WORDS + 4;
+static_assert((P1T_MAX_CVCARD * P1T_CVREP + P1T_WARPS * P1T_WARP_FLOATS) * 4 + 16 <= SMEM_CTA_MAX, "phase-1 shared memory");
+static_assert(P1T_WARP_FLOATS % 4 == 0, "16-byte alignment of the warps' shared memory");
 
 // Epilogue constants of the tensor-core form: x = 2 x (CV score argument)
 // = (2 pownu0 ln2) log2(det) + 2 cterm - 2 prior_q - 2 prior_d, compared

@@ -914,32 +914,40 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
             if (k == TC_SS_KMAX + 1) return 1.f;
             return k < card ? U[(size_t)r * 32 + k] : 0.f;
         };
-        std::vector<uint32_t> qa((size_t)ns * TC_QA_WORDS, 0u);
-        std::vector<float> qaa((size_t)ns * TC_QAA_FLOATS, 0.f);
-        for (int s = 0; s < ns; s++)
-            for (int mt = 0; mt < 2; mt++)
-                for (int kt = 0; kt < 2; kt++)
-                    for (int lane = 0; lane < 32; lane++) {
-                        const int g = lane >> 2, qq = lane & 3;
-                        for (int d = 0; d < 2; d++)
-                            for (int w = 0; w < 4; w++) {
-                                const int r = 32 * s + 16 * mt + g + ((w & 1) ? 8 : 0);
-                                const int k = 16 * kt + 2 * qq + ((w >> 1) ? 8 : 0);
-                                const float x0 = aval(d, r, k), x1 = aval(d, r, k + 1);
-                                const uint32_t h0 = bf16_rn_bits(x0), h1 = bf16_rn_bits(x1);
-                                const uint32_t l0 = bf16_rn_bits(x0 - bf16_to_f(h0));
-                                const uint32_t l1 = bf16_rn_bits(x1 - bf16_to_f(h1));
-                                const size_t base = (size_t)(((s * 2 + mt) * 2 + d) * 2 + kt) * 2;
-                                qa[((base + 0) * 32 + lane) * 4 + w] = h0 | (h1 << 16);
-                                qa[((base + 1) * 32 + lane) * 4 + w] = l0 | (l1 << 16);
-                            }
-                        for (int e = 0; e < 8; e++) {
-                            const int r = 32 * s + 16 * mt + g + (((e >> 1) & 1) << 3);
-                            const int k = 16 * kt + 2 * qq + (e & 1) + ((e >> 2) << 3);
-                            qaa[((size_t)((s * 2 + mt) * 2 + kt) * 32 + lane) * 8 + e] =
-                                (r < Lq && k < NAA) ? q->trg[(size_t)r * NAA + k] : 0.f;
+        const int nt = (Lq + P1T_ROWS - 1) / P1T_ROWS;
+        std::vector<uint32_t> qa((size_t)nt * TC_QA_WORDS, 0u);
+        std::vector<float> qaa((size_t)nt * TC_QAA_FLOATS, 0.f);
+        for (int s = 0; s < nt; s++)
+            for (int mt = 0; mt < 4; mt++)
+                for (int lane = 0; lane < 32; lane++) {
+                    const int g = lane >> 2, qq = lane & 3;
+                    const int r0 = P1T_ROWS * s + 16 * mt + g;
+                    // word w of operand d: row r0 + 8 (w & 1), k = 8 (w >> 1) + 2 qq, + 1; the
+                    // CV operand has words 0..5 (k < 24), the SS operand 0..7
+                    size_t o = (size_t)(s * 4 + mt) * 7;   // 16-byte groups
+                    int at = 0;                            // word of the fragment
+                    auto put = [&](uint32_t w) {
+                        qa[((o + at / 4) * 32 + lane) * 4 + at % 4] = w;
+                        at++;
+                    };
+                    for (int d = 0; d < 2; d++) {
+                        const int nw = d == 0 ? 6 : 8;
+                        uint32_t lo[8];
+                        for (int w = 0; w < nw; w++) {
+                            const int r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq;
+                            const float x0 = aval(d, r, k), x1 = aval(d, r, k + 1);
+                            const uint32_t h0 = bf16_rn_bits(x0), h1 = bf16_rn_bits(x1);
+                            lo[w] = bf16_rn_bits(x0 - bf16_to_f(h0)) | (bf16_rn_bits(x1 - bf16_to_f(h1)) << 16);
+                            put(h0 | (h1 << 16));
                         }
+                        for (int w = 0; w < nw; w++) put(lo[w]);
                     }
+                    for (int e = 0; e < 12; e++) {
+                        const int w = e >> 1, r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq + (e & 1);
+                        qaa[(((size_t)(s * 4 + mt) * 3 + e / 4) * 32 + lane) * 4 + e % 4] =
+                            (r < Lq && k < NAA) ? q->trg[(size_t)r * NAA + k] : 0.f;
+                    }
+                }
         if (h->d_qa.ensure(qa.size(), h->budget) || h->d_qaaf.ensure(qaa.size(), h->budget))
             return fail(h, C2_ERR_NOMEM, "query operand allocation failed");
         CK(cudaMemcpyAsync(h->d_qa.p, qa.data(), qa.size() * 4, cudaMemcpyHostToDevice, h->stream));
@@ -1039,7 +1047,7 @@ static c2_status tc_prepare_db(c2_handle* h)
     long long ntiles = 0;
     for (int k = 0; k < h->nprof; k++) {
         tt[k] = ntiles;
-        ntiles += (long long)((h->h_plen[k] + 31) / 32) * 4;
+        ntiles += (h->h_plen[k] + P1T_C - 1) / P1T_C;
     }
     if (h->db->d_ttile.ensure(h->nprof, h->budget) || h->db->d_tcdb.ensure((size_t)ntiles * TC_TILE_WORDS, h->budget) ||
         h->db->d_cold.ensure((size_t)h->npos * P1C_TRS, h->budget))
@@ -1100,18 +1108,13 @@ static void fill_p1(c2_handle* h, P1Args& a)
 // time all pairs together take on all warps (both grow with the number of
 // strips alike, so the query length does not enter).  Pairs below that even
 // out over the warps by the longest-first order; pairs above it would be the
-// tail of the search.  Phase-1 times with shares of infinity (none split) / 1 /
-// 0.5 / 0.25 / 0.1: 1 x 3,000 vs 4,000 profiles 41.9 / 23.2 / 23.8 / 26.7 / 25.7
-// ms, 1 x 1,237 vs 4,999 16.2 / 9.7 / 10.4 / 10.8 / 11.3, 1 x 250 vs 3,000 (FP32)
-// 4.5 / 2.3 / 2.1 / 2.3 / 2.3, 7 queries vs 1,000 (FP32) 32 / 11 / 8.4 / 8.6 /
-// 8.6, 1 x 150 vs 2,000 0.70 / 0.66 / 0.60 / 0.57 / 0.55; no pair is split (and
-// nothing changes) against 50,000 profiles.  0 without the scratch (it is small: the two boundary
+// tail of the search.  0 without the scratch (it is small: the two boundary
 // rows of the split pairs) -- the pairs then run whole, with the same results.
 constexpr double SPLIT_SHARE = 0.5;
 
-static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
+static int split_pairs(c2_handle* h, int nwarps, int rows, P1Args& a)
 {
-    const int P = h->nprof, ns = (h->Lq + 31) / 32;
+    const int P = h->nprof, ns = (h->Lq + rows - 1) / rows;   // strips of `rows` query rows
     a.nsplit = 0;
     if (ns < 2) return 0;
     const double mean = ((double)h->npos + 31.0 * P) / std::max(1, nwarps);
@@ -1162,7 +1165,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
             return fail(h, C2_ERR_CUDA, "tensor-core phase-1 kernel does not fit on an SM (%s)",
                         cudaGetErrorString(oe));
         gt = std::min(gt, h->grid * P1_WARPS / P1T_WARPS);
-        split_pairs(h, gt * P1T_WARPS, a);
+        split_pairs(h, gt * P1T_WARPS, P1T_ROWS, a);
         CK(launch_p1(a, h->d_qbkg.p, P1K_TENSOR, gt, h->stream));
         h->launches++;
         return C2_OK;
@@ -1172,7 +1175,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     int gc = (h->nsm - h->p1_reserve) * p1c_blocks_per_sm(h->sc.cvcard);
     if (gc < 1) return fail(h, C2_ERR_CUDA, "phase-1 kernel does not fit on an SM");
     gc = std::min(gc, h->grid * P1_WARPS / P1C_WARPS);
-    split_pairs(h, gc * P1C_WARPS, a);
+    split_pairs(h, gc * P1C_WARPS, 32, a);
     CK(launch_p1(a, h->d_qbkg.p, P1K_CHUNKED, gc, h->stream));
     h->launches++;
     return C2_OK;
@@ -1227,8 +1230,8 @@ extern "C" c2_status c2_get_device_memory_info(const c2_handle* h, uint64_t* fre
 
 // Device bytes of a database upload of this size and of the per-profile
 // phase-1 buffers that come with it: the c2_upload_db allocations, and in the
-// tensor-core score mode the operands tc_prepare_db packs (at most
-// ceil(L / 32) * 4 tiles a profile, i.e. npositions / 8 + 4 nprofiles).
+// tensor-core score mode the operands tc_prepare_db packs (ceil(L / 8) tiles
+// a profile, at most npositions / 8 + nprofiles).
 extern "C" c2_status c2_db_device_bytes(const c2_handle* h, int64_t npositions, int32_t nprofiles, int32_t max_length,
                                         uint64_t* bytes)
 {
@@ -1244,7 +1247,7 @@ extern "C" c2_status c2_db_device_bytes(const c2_handle* h, int64_t npositions, 
     const uint64_t lm = ((uint64_t)max_length + 31) & ~31ull;
     b += (uint64_t)h->grid * P1_WARPS * 10 * lm * sizeof(float);   // d_bot
     if (h->score_mode == C2_SCORE_BF16_TC) {
-        const uint64_t ntiles = N / 8 + 4 * P;
+        const uint64_t ntiles = N / 8 + P;
         b += P * sizeof(long long) + ntiles * TC_TILE_WORDS * sizeof(unsigned) + N * P1C_TRS * sizeof(float);
     }
     *bytes = b;

@@ -362,12 +362,6 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
 // strip, column j) sits in slot (i + j) & 63, so at step k every lane reads
 // slot k & 63 and a DP stage reads 32 consecutive slots from one base.
 
-// Pair of FP32 adds.  The packed sm_100 form (add.rn.f32x2) gives the same
-// bits with ~1 % fewer instructions here, but measured 2 % slower in the
-// tensor-core phase-1 kernel (5.53 vs 5.42 ms on 5,000 profiles), so the pairs
-// stay two scalar adds; the pairing keeps the shared sums explicit.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-
 // Maximum of three (sm_100 three-input max.f32; exact, like two fmaxf)
 __device__ __forceinline__ float max3f(float a, float b, float c)
 {
@@ -378,40 +372,38 @@ __device__ __forceinline__ float max3f(float a, float b, float c)
 
 // One lane of the wavefront DP.  Every Viterbi candidate of the reference's
 // recurrence is (state + query transition) + db transition, evaluated in that
-// order, with the sums that two candidates or two steps share computed once:
-//   X = (up.MM, up.DN) + (qMM, qDM)   W = (up.MM, up.DN) + (qMD, qDD)
-//   Y = (up.MI, up.IM) + (qMM, qIM)   z = up.ND + qMM
-// X, Y and z are the up-sums of this step and the diagonal sums of the next
-// (the diagonal predecessor of a cell is the up-neighbour of its left one).
+// order, with the sums that two candidates or two steps share computed once.
+// Rounding to nearest is monotone, so max(a + t, b + t) = max(a, b) + t holds
+// for the rounded sums as well: the candidates that share a db transition are
+// reduced before it is added, with the same bits (18 adds and 7 maxima a cell
+// instead of 21 and 7).
+//   A = max(up.MM + qMM, up.IM + qIM, up.DN + qDM)     (db transition MM)
+//   Y = up.MI + qMM    z = up.ND + qMM                 (IM; DM)
+// are the up-sums of this step and the diagonal sums of the next (the diagonal
+// predecessor of a cell is the up-neighbour of its left one).
 struct WfLane {
     float MM, MI, IM, DN, ND;     // own state at the previous step (left)
-    float2 X, Y;                  // up-sums of the previous step
-    float z;
-    float2 qX, qW, qY;            // (qMM, qDM), (qMD, qDD), (qMM, qIM)
-    float qMM, qMI, qII;
-    float2 XB, YB;                // diagonal sums of the column -1 boundary state
-    float zB, lbMM, lbIM, lbND;   // and the column -1 left state
+    float A, Y, z;                // up-sums of the previous step
+    float qMM, qDM, qIM, qMD, qDD, qMI, qII;
+    float AB, YB, zB;             // diagonal sums of the column -1 boundary state
+    float lbMM, lbIM, lbND;       // and the column -1 left state
     float best;
     int kbest;
 };
 
 __device__ __forceinline__ void wf_init(WfLane& D, const float* q7, const St5& LB, const St5& DB)
 {
-    D.qX = make_float2(q7[TMM], q7[TDM]);
-    D.qW = make_float2(q7[TMD], q7[TDD]);
-    D.qY = make_float2(q7[TMM], q7[TIM]);
-    D.qMM = q7[TMM];
-    D.qMI = q7[TMI];
-    D.qII = q7[TII];
-    D.XB = add2(make_float2(DB.MM, DB.DN), D.qX);
-    D.YB = add2(make_float2(DB.MI, DB.IM), D.qY);
-    D.zB = DB.ND + q7[TMM];
+    D.qMM = q7[TMM]; D.qDM = q7[TDM]; D.qIM = q7[TIM];
+    D.qMD = q7[TMD]; D.qDD = q7[TDD];
+    D.qMI = q7[TMI]; D.qII = q7[TII];
+    D.AB = max3f(DB.MM + D.qMM, DB.IM + D.qIM, DB.DN + D.qDM);
+    D.YB = DB.MI + D.qMM;
+    D.zB = DB.ND + D.qMM;
     D.lbMM = LB.MM;
     D.lbIM = LB.IM;
     D.lbND = LB.ND;
     D.MM = D.MI = D.IM = D.DN = D.ND = 0.f;
-    D.X = D.Y = make_float2(0.f, 0.f);
-    D.z = 0.f;
+    D.A = D.Y = D.z = 0.f;
     D.best = 0.f;
     D.kbest = 0;
 }
@@ -425,34 +417,30 @@ __device__ __forceinline__ void bnd_put(float* bnd, int slot, float mm, float mi
 }
 
 // Wavefront steps [k0, k0 + nst) of a strip (k0 a multiple of 32, nst <= 32;
-// 32 when !CHECK).  ring: diagonal-indexed scores, RLD floats per slot.
-// Column records (DPT_N transitions, P1C_TRS floats apart): with TMIRROR,
-// tcol points at this lane's record for step k0 and the next 31 follow
-// without wrapping; otherwise tcol is a ring of TMASK + 1 records indexed by
-// column & TMASK.  bnd: row above the strip for columns [k0, k0 + 32).
+// 32 when !CHECK).  ring: diagonal-indexed scores, 32 floats per slot.  tcol:
+// ring of P1C_RING column records (DPT_N transitions, P1C_TRS floats apart).
+// bnd: row above the strip for columns [k0, k0 + 32).
 // TB (traceback sweep): each cell's traceback code also goes to the warp's
 // column ring btr (column j in slot j & 31, the lane's own row), and column
 // k - 31, complete for every row at step k, is stored to the pair's code
 // matrix bt (column-major, Lq rows; r = this lane's query row).
-template <bool CHECK, int RLD, bool TMIRROR, int TMASK, bool TB = false>
+template <bool CHECK, bool TB = false>
 __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, int L, bool act,
                                          const float* __restrict__ ring, const float* __restrict__ tcol,
                                          float* __restrict__ bnd, bool wr_bot, signed char (*btr)[33] = nullptr,
                                          signed char* __restrict__ bt = nullptr, int Lq = 0, int r = 0)
 {
-    const float* __restrict__ rb = ring + (k0 & (P1C_RING - 1)) * RLD + lane;
+    const float* __restrict__ rb = ring + (k0 & (P1C_RING - 1)) * 32 + lane;
     if (!CHECK) nst = 32;
     int ub = -1;
     // the instruction cache holds both variants of both kernels at these depths
     constexpr int UNR = CHECK ? 2 : 4;
 #pragma unroll UNR
     for (int u = 0; u < nst; u++) {
-        const float S = rb[u * RLD];
-        const float* __restrict__ tp =
-            TMIRROR ? tcol + u * P1C_TRS : tcol + ((k0 + u - lane) & TMASK) * P1C_TRS;
-        const float4 ta = *reinterpret_cast<const float4*>(tp);       // MM MM IM MM
-        const float4 tb = *reinterpret_cast<const float4*>(tp + 4);   // MD DD MI II
-        const float tDM = tp[8];
+        const float S = rb[u * 32];
+        const float* __restrict__ tp = tcol + ((k0 + u - lane) & (P1C_RING - 1)) * P1C_TRS;
+        const float4 ta = *reinterpret_cast<const float4*>(tp);       // MM IM DM MI
+        const float4 tb = *reinterpret_cast<const float4*>(tp + 4);   // II MD DD
         float uMM = __shfl_up_sync(FULL, D.MM, 1);
         float uMI = __shfl_up_sync(FULL, D.MI, 1);
         float uIM = __shfl_up_sync(FULL, D.IM, 1);
@@ -465,27 +453,19 @@ __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, i
             if (lane == 0) { uMM = ba.x; uMI = ba.y; uIM = ba.z; uDN = ba.w; uND = b4; }
         }
         const int j = k0 + u - lane;
-        float2 Xd = D.X, Yd = D.Y;
-        float zd = D.z, lMM = D.MM, lIM = D.IM, lND = D.ND;
+        float Ad = D.A, Yd = D.Y, zd = D.z, lMM = D.MM, lIM = D.IM, lND = D.ND;
         if (CHECK && j == 0) {
-            Xd = D.XB; Yd = D.YB; zd = D.zB;
+            Ad = D.AB; Yd = D.YB; zd = D.zB;
             lMM = D.lbMM; lIM = D.lbIM; lND = D.lbND;
         }
-        const float2 T0 = make_float2(ta.x, ta.y), T1 = make_float2(ta.z, ta.w), T2 = make_float2(tb.x, tb.y);
-        const float2 X = add2(make_float2(uMM, uDN), D.qX);
-        const float2 W = add2(make_float2(uMM, uDN), D.qW);
-        const float2 Y = add2(make_float2(uMI, uIM), D.qY);
-        const float z = uND + D.qMM;
-        const float2 c53 = add2(Xd, T0);   // diag MM + MM + MM, diag DN + DM + MM
-        const float2 c12 = add2(Yd, T1);   // diag MI + MM + IM, diag IM + IM + MM
-        const float v = max3f(max3f(c12.x, c12.y, c53.y), zd + tDM, c53.x);
+        const float X = uMM + D.qMM, Y = uMI + D.qMM, z = uND + D.qMM;
+        const float A = max3f(X, uIM + D.qIM, uDN + D.qDM);
+        const float v = max3f(Ad + ta.x, Yd + ta.y, zd + ta.z);
         const float nMM = fmaxf(v + S, 0.f);
-        const float nMI = fmaxf(X.x + tb.z, Y.x + tb.w);
-        const float2 c89 = add2(make_float2(lMM + D.qMI, lIM + D.qII), T0);
-        const float2 cND = add2(make_float2(lMM, lND), T2);
-        const float nIM = fmaxf(c89.x, c89.y);
-        const float nDN = fmaxf(W.x, W.y);
-        const float nND = fmaxf(cND.x, cND.y);
+        const float nMI = fmaxf(X + ta.w, Y + tb.x);
+        const float nIM = fmaxf(lMM + D.qMI, lIM + D.qII) + ta.x;
+        const float nDN = fmaxf(uMM + D.qMD, uDN + D.qDD);
+        const float nND = fmaxf(lMM + tb.y, lND + tb.z);
         // inactive lanes (rows past the query) carry LOG0 query transitions:
         // their MM stays 0 and never beats a maximum
         const bool inm = !CHECK || (j >= 0 && j < L);
@@ -512,7 +492,7 @@ __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, i
             bnd_put(bnd, u, nMM, nMI, nIM, nDN, nND);
         }
         D.MM = nMM; D.MI = nMI; D.IM = nIM; D.DN = nDN; D.ND = nND;
-        D.X = X; D.Y = Y; D.z = z;
+        D.A = A; D.Y = Y; D.z = z;
     }
     if (ub >= 0) D.kbest = k0 + ub;
 }
@@ -586,65 +566,72 @@ __device__ __forceinline__ bool p1_take(const P1Args& a, int nstrips, int lane, 
 // 4 ldb on; ldb a multiple of 4 columns, the buffer 16-byte aligned.  Each
 // half is thus one wide store or asynchronous copy per chunk.
 
-// Wait (split pairs only) until columns [c0, c0 + 32) of the row above strip s
+// A chunk is C columns (32: the FP32 kernel, 8: the tensor-core kernel).
+
+// Wait (split pairs only) until columns [c0, c0 + C) of the row above strip s
 // are there; false: no such row
+template <int C>
 __device__ __forceinline__ bool p1_row_ready(const P1Args& a, const P1Item& it, int s, int c0, int lane, bool& broken)
 {
     const bool have = s > 0 && c0 < it.L;
     if (have && it.pi >= 0)
-        pipe_wait(a.sprog + (long long)(s - 1) * a.nsplit + it.pi, min(c0 + 32, it.L), lane, a.status, broken, a.spin);
+        pipe_wait(a.sprog + (long long)(s - 1) * a.nsplit + it.pi, min(c0 + C, it.L), lane, a.status, broken, a.spin);
     return have;
 }
 
-// The row above strip s, columns [c0, c0 + 32), into the warp's shared row by
+// The row above strip s, columns [c0, c0 + C), into the warp's shared row by
 // asynchronous copies through L2 (a split pair's row comes from another SM);
 // zeros where there is none.  Commits one group.  Columns past the matrix hold
 // whatever the buffer does: no cell inside the matrix reads them.
+template <int C>
 __device__ __forceinline__ void p1_row_async(const P1Args& a, const P1Item& it, int s, float* bnd,
                                              const float* __restrict__ botr, int ldb, int c0, int lane, bool& broken)
 {
-    if (p1_row_ready(a, it, s, c0, lane, broken)) {
-        const int c = c0 + lane, c4 = c0 + 4 * lane;
-        if (c < it.L) cp_async16(bnd + 4 * lane, botr + 4 * c);
-        if (lane < 8 && c4 < it.L) cp_async16(bnd + BND_ND + 4 * lane, botr + 4 * ldb + c4);
-    } else {
-        bnd_put(bnd, lane, 0.f, 0.f, 0.f, 0.f, 0.f);
+    if (p1_row_ready<C>(a, it, s, c0, lane, broken)) {
+        const int c = c0 + lane, c4 = c0 + 4 * (lane - C);
+        if (lane < C) {
+            if (c < it.L) cp_async16(bnd + 4 * lane, botr + 4 * c);
+        } else if (lane < C + C / 4 && c4 < it.L) {
+            cp_async16(bnd + 4 * C + 4 * (lane - C), botr + 4 * ldb + c4);
+        }
+    } else if (lane < C) {
+        *reinterpret_cast<float4*>(bnd + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
+        bnd[4 * C + lane] = 0.f;
     }
     cp_async_commit();
 }
 
-// The same into registers (lane i: column c0 + i)
+// The same into registers (C = 32; lane i: column c0 + i)
 __device__ __forceinline__ void p1_row_load(const P1Args& a, const P1Item& it, int s, const float* __restrict__ botr,
                                             int ldb, int c0, int lane, bool& broken, float4& v, float& nd)
 {
     const int c = c0 + lane;
     v = make_float4(0.f, 0.f, 0.f, 0.f);
     nd = 0.f;
-    if (p1_row_ready(a, it, s, c0, lane, broken) && c < it.L) {
+    if (p1_row_ready<32>(a, it, s, c0, lane, broken) && c < it.L) {
         v = __ldcg(reinterpret_cast<const float4*>(botr) + c);
         nd = __ldcg(botr + 4 * ldb + c);
     }
 }
 
-// The strip's last row after a DP stage over [k0, k0 + 32) (as bot_flush)
+// The strip's last row after a DP stage over [k0, k0 + C): slot l of bnd holds
+// lane 31's states at column k0 - 31 + l
+template <int C>
 __device__ __forceinline__ void p1_row_flush(const float* __restrict__ bnd, float* __restrict__ botw, int ldb, int k0,
                                              int L, int lane)
 {
     const int c = k0 - 31 + lane;
-    if (c >= 0 && c < L) {
+    if (lane < C && c >= 0 && c < L) {
         reinterpret_cast<float4*>(botw)[c] = *reinterpret_cast<const float4*>(bnd + lane * 4);
-        botw[4 * ldb + c] = bnd[BND_ND + lane];
+        botw[4 * ldb + c] = bnd[4 * C + lane];
     }
 }
 
 // Strip s of a split pair has stored the columns [0, n) of its last row
 __device__ __forceinline__ void p1_publish(const P1Args& a, const P1Item& it, int s, int n, int lane)
 {
-    __syncwarp();
-    if (lane == 0) {
-        __threadfence();
-        pipe_st_release(a.sprog + (long long)s * a.nsplit + it.pi, n);
-    }
+    __syncwarp();   // every lane's stores before lane 0's release
+    if (lane == 0) pipe_st_release(a.sprog + (long long)s * a.nsplit + it.pi, n);
 }
 
 // The item's maximum over its lanes (largest score, then smallest row, then
@@ -804,12 +791,12 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
                 // ---- DP stage: wavefront steps [32m, 32m + 32)
                 const int k0 = 32 * m, k1 = min(k0 + 32, kend);
                 if (m >= 1 && k0 + 31 < L && k1 == k0 + 32)
-                    wf_steps<false, 32, false, P1C_RING - 1>(D, k0, 32, lane, L, act, ring, trn, bnd, wr_bot);
+                    wf_steps<false>(D, k0, 32, lane, L, act, ring, trn, bnd, wr_bot);
                 else
-                    wf_steps<true, 32, false, P1C_RING - 1>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot);
+                    wf_steps<true>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot);
                 __syncwarp();
                 if (s + 1 < nstrips) {
-                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
+                    p1_row_flush<32>(bnd, botw, ldb, k0, L, lane);
                     if (it.pi >= 0) p1_publish(a, it, s, min(k1 - 31, L), lane);
                 }
                 __syncwarp();
@@ -1028,10 +1015,10 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
             __syncwarp();
             // ---- DP stage: wavefront steps [32m, 32m + 32), traceback codes stored
             if (m >= 1 && k0 + 31 < L && k1 == k0 + 32)
-                wf_steps<false, 32, false, P1C_RING - 1, true>(D, k0, 32, lane, L, act, ring, trn, bnd, wr_bot, btr,
+                wf_steps<false, true>(D, k0, 32, lane, L, act, ring, trn, bnd, wr_bot, btr,
                                                                bt, Lq, r);
             else
-                wf_steps<true, 32, false, P1C_RING - 1, true>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot,
+                wf_steps<true, true>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot,
                                                               btr, bt, Lq, r);
             __syncwarp();
             if (s + 1 < nstrips) {
@@ -1107,6 +1094,15 @@ __device__ __forceinline__ void mma_bf16(float* d, const unsigned* a, unsigned b
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// the same with K = 8
+__device__ __forceinline__ void mma_bf16_k8(float* d, unsigned a0, unsigned a1, unsigned b0)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(b0));
+}
+
 // mbarrier and bulk (non-tensor, non-multicast) async copy helpers
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -1126,37 +1122,37 @@ __device__ __forceinline__ void tmem_dealloc(unsigned taddr, unsigned ncols)
 }
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st16(unsigned taddr, const unsigned* v)
+__device__ __forceinline__ void tmem_st40(unsigned taddr, const unsigned* v)
 {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15, %16};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr + 32),
+        "r"(v[32]), "r"(v[33]), "r"(v[34]), "r"(v[35]), "r"(v[36]), "r"(v[37]), "r"(v[38]), "r"(v[39])
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 32 columns into v; the wait takes v as operands so no use of v can be
-// scheduled before the load has completed
-__device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned* v)
+// 40 columns into v; the wait takes v as operands so no use of v can be
+// scheduled before the loads have completed
+__device__ __forceinline__ void tmem_ld40(unsigned taddr, unsigned* v)
 {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr)
         : "memory");
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39])
+        : "r"(taddr + 32)
+        : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
-                   "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]),
-                   "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]),
-                   "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19])
                  :
                  : "memory");
+    asm volatile("" : "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]), "+r"(v[32]), "+r"(v[33]), "+r"(v[34]), "+r"(v[35]), "+r"(v[36]), "+r"(v[37]), "+r"(v[38]), "+r"(v[39]));
 }
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
@@ -1203,23 +1199,24 @@ __global__ void __launch_bounds__(128) tc_pack_kernel(const float* __restrict__ 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int L = plen[p];
     const long long off = poff[p];
-    const int ntiles = ((L + 31) >> 5) * 4;
+    const int ntiles = (L + P1T_C - 1) / P1T_C;
     const int g = lane >> 2, q = lane & 3;
     for (int t = wid; t < ntiles; t += 4) {
-        const int col = 8 * t + g;
+        const int col = P1T_C * t + g;
         const bool valid = col < L;
         const float* rc = drec + (off + (valid ? col : 0)) * DR_STRIDE;
         const int pk = __float_as_int(rc[DR_SSIDX]);
         const int i0 = pk & 0xff, i1 = (pk >> 8) & 0xff, i2 = (pk >> 16) & 0xff;
-        unsigned* out = tcdb + (ttile[p] + t) * (long long)TC_TILE_WORDS;
+        // words of the three operands: k 0-15 (2), then k 16-23 (1) or k 16-31 (2)
+        unsigned h[3][4], l[3][4];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
 #pragma unroll
-            for (int kt = 0; kt < 2; kt++) {
-                float v[4];
+            for (int w = 0; w < 4; w++) {
+                unsigned hh[2], ll[2];
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int k = 16 * kt + 2 * q + (e & 1) + (e >> 1) * 8;
+                for (int e = 0; e < 2; e++) {
+                    const int k = 8 * w + 2 * q + e;
                     float x = 0.f;
                     if (valid) {
                         if (d == 0) x = (k < NAA) ? rc[DR_TRG + k] : 0.f;
@@ -1230,27 +1227,28 @@ __global__ void __launch_bounds__(128) tc_pack_kernel(const float* __restrict__ 
                         else if (k == TC_SS_KMAX) x = wss * (rc[DR_HD] * 0.1111111f);
                         else if (k == TC_SS_KMAX + 1) x = -0.05f * wss;
                     }
-                    v[e] = x;
+                    bf16_split(x, hh[e], ll[e]);
                 }
-                unsigned h[4], l[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) bf16_split(v[e], h[e], l[e]);
-                unsigned* o = out + ((d * 2 + kt) * 2) * 64 + lane * 2;
-                o[0] = h[0] | (h[1] << 16);
-                o[1] = h[2] | (h[3] << 16);
-                o[64] = l[0] | (l[1] << 16);
-                o[65] = l[2] | (l[3] << 16);
+                h[d][w] = hh[0] | (hh[1] << 16);
+                l[d][w] = ll[0] | (ll[1] << 16);
             }
         }
+        uint4* out = reinterpret_cast<uint4*>(tcdb + (ttile[p] + t) * (long long)TC_TILE_WORDS) + lane;
+        out[0 * 32] = make_uint4(h[0][0], h[0][1], h[0][2], l[0][2]);
+        out[1 * 32] = make_uint4(l[0][0], l[0][1], h[1][0], h[1][1]);
+        out[2 * 32] = make_uint4(l[1][0], l[1][1], h[1][2], l[1][2]);
+        out[3 * 32] = make_uint4(h[2][0], h[2][1], h[2][2], h[2][3]);
+        out[4 * 32] = make_uint4(l[2][0], l[2][1], l[2][2], l[2][3]);
     }
     for (int c = threadIdx.x; c < L; c += blockDim.x) {
         const float* rc = drec + (off + c) * DR_STRIDE;
         float* o = cold + (off + c) * P1C_TRS;
 #pragma unroll
         for (int i = 0; i < DPT_N; i++) o[i] = rc[DR_TRN + dpt_src(i)];
+        o[7] = 0.f;
         o[CO_CD] = rc[DR_CN];
         o[CO_PD2] = 2.f * rc[DR_PRIOR];
-        o[11] = 0.f;
+        o[10] = o[11] = 0.f;
     }
 }
 
@@ -1291,59 +1289,178 @@ __device__ __forceinline__ float tc_cell(float daa, float dot, float ss, float c
     return fmaf(lg2_ftz(daa), C2_LN2, ss + cvm);
 }
 
-// Stage the column records of chunk m (32 columns) into the column ring
-// (3 chunks; chunks at slot 0 also into the mirror slots 96..127)
-__device__ __forceinline__ void stage_cols(float* cring, const float* __restrict__ cold, int m, int L, int lane)
+// One lane of the wavefront DP with two query rows (2 t and 2 t + 1 of the
+// strip): row 0 takes its "up" states from row 1 of lane t - 1 by shuffle, row
+// 1 from row 0 of this lane at the same step.  Against one row a lane
+// (WfLane), a step's shuffles, record reads and row-above selects serve two
+// cells, and its two chains overlap; each cell's arithmetic is the same.
+struct Wf2 {
+    float MM[2], MI[2], IM[2], DN[2], ND[2];   // states at the previous step (left)
+    float A[2], Y[2], z[2];                    // up-sums of the previous step (WfLane)
+    float qMM[2], qDM[2], qIM[2], qMD[2], qDD[2], qMI[2], qII[2];
+    float best;      // the lane's maximum, its row (0, 1) and step
+    int brow, kbest;
+};
+
+// Diagonal sums and left states of column -1 for the lane's two rows
+struct Wf2Edge {
+    float A[2], Y[2], z[2], IM[2], ND[2];
+};
+
+__device__ __forceinline__ void wf2_init(Wf2& D, const float* __restrict__ qrec, int r0, int Lq)
 {
-    const int c0 = 32 * m;
-    const int nc = min(32, L - c0);
-    if (nc > 0) {
-        const int base = c0 % P1T_CMOD;
-        float* dst = cring + base * P1C_TRS;
-        const float* src = cold + (long long)c0 * P1C_TRS;
-        for (int i = lane; i < nc * (P1C_TRS / 4); i += 32) cp_async16(dst + 4 * i, src + 4 * i);
-        if (base == 0) {
-            float* mir = cring + P1T_CMOD * P1C_TRS;
-            for (int i = lane; i < nc * (P1C_TRS / 4); i += 32) cp_async16(mir + 4 * i, src + 4 * i);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int r = r0 + e;
+        const bool act = r < Lq;
+        // rows past the query carry LOG0 transitions and -inf scores: their MM stays 0
+        const float* qr = qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE + QR_TRN;
+        D.qMM[e] = act ? qr[TMM] : LOG0; D.qMI[e] = act ? qr[TMI] : LOG0; D.qMD[e] = act ? qr[TMD] : LOG0;
+        D.qIM[e] = act ? qr[TIM] : LOG0; D.qII[e] = act ? qr[TII] : LOG0; D.qDM[e] = act ? qr[TDM] : LOG0;
+        D.qDD[e] = act ? qr[TDD] : LOG0;
+        D.MM[e] = D.MI[e] = D.IM[e] = D.DN[e] = D.ND[e] = 0.f;
+        D.A[e] = D.Y[e] = D.z[e] = 0.f;
+    }
+    D.best = 0.f;
+    D.brow = D.kbest = 0;
+}
+
+__device__ __forceinline__ void wf2_edge(Wf2Edge& E, const Wf2& D, const float* __restrict__ qrec, int r0, int Lq)
+{
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int r = r0 + e, b = r & 31;
+        const float* qr = qrec + (long long)min(r, Lq - 1) * QR_STRIDE;
+        const bool zl = b == 31, zd = b == 31 || b == 0;
+        E.IM[e] = zl ? 0.f : qr[QR_C + 1];
+        E.ND[e] = zl ? 0.f : LOG0;
+        const float dMI = zd ? 0.f : qr[QR_CP + 0], dIM = zd ? 0.f : qr[QR_CP + 1], dDN = zd ? 0.f : qr[QR_CP + 2];
+        const float dND = zd ? 0.f : LOG0;
+        E.A[e] = max3f(0.f + D.qMM[e], dIM + D.qIM[e], dDN + D.qDM[e]);
+        E.Y[e] = dMI + D.qMM[e];
+        E.z[e] = dND + D.qMM[e];
+    }
+}
+
+// Four wavefront steps: rp the lane's scores (P1T_RLD floats a step), tc its
+// column records, bnd the row above (row: slots u0..), j0 the lane's column at
+// the first step, k0 that step.  HEAD: column 0 may be among the steps (the
+// first P1T_HEAD chunks of a strip).  Cells outside the matrix have scores of
+// -inf, so their MM stays 0, and their other states reach no cell inside.
+template <bool HEAD>
+__device__ __forceinline__ void wf2_steps4(Wf2& D, const Wf2Edge& E, const float* __restrict__ rp,
+                                           const float* __restrict__ tc, float* __restrict__ bnd, int u0, int j0, int k0,
+                                           int lane, bool wr_bot)
+{
+    float m[2][4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const float2 S = *reinterpret_cast<const float2*>(rp + u * P1T_RLD);
+        const float4 ta = *reinterpret_cast<const float4*>(tc + u * P1C_TRS);       // MM IM DM MI
+        const float4 tb = *reinterpret_cast<const float4*>(tc + u * P1C_TRS + 4);   // II MD DD
+        float uMM = __shfl_up_sync(FULL, D.MM[1], 1);
+        float uMI = __shfl_up_sync(FULL, D.MI[1], 1);
+        float uIM = __shfl_up_sync(FULL, D.IM[1], 1);
+        float uDN = __shfl_up_sync(FULL, D.DN[1], 1);
+        float uND = __shfl_up_sync(FULL, D.ND[1], 1);
+        {
+            const float4 ba = *reinterpret_cast<const float4*>(bnd + 4 * (u0 + u));
+            const float b4 = bnd[4 * P1T_C + u0 + u];
+            if (lane == 0) { uMM = ba.x; uMI = ba.y; uIM = ba.z; uDN = ba.w; uND = b4; }
         }
+        const bool first = HEAD && j0 + u == 0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            float Ad = D.A[e], Yd = D.Y[e], zd = D.z[e], lMM = D.MM[e], lIM = D.IM[e], lND = D.ND[e];
+            if (first) { Ad = E.A[e]; Yd = E.Y[e]; zd = E.z[e]; lMM = 0.f; lIM = E.IM[e]; lND = E.ND[e]; }
+            const float X = uMM + D.qMM[e], Y = uMI + D.qMM[e];
+            D.A[e] = max3f(X, uIM + D.qIM[e], uDN + D.qDM[e]);
+            D.Y[e] = Y;
+            D.z[e] = uND + D.qMM[e];
+            const float v = max3f(Ad + ta.x, Yd + ta.y, zd + ta.z);
+            const float nMM = fmaxf(v + (e ? S.y : S.x), 0.f);
+            const float nMI = fmaxf(X + ta.w, Y + tb.x);
+            const float nIM = fmaxf(lMM + D.qMI[e], lIM + D.qII[e]) + ta.x;
+            const float nDN = fmaxf(uMM + D.qMD[e], uDN + D.qDD[e]);
+            const float nND = fmaxf(lMM + tb.y, lND + tb.z);
+            D.MM[e] = nMM; D.MI[e] = nMI; D.IM[e] = nIM; D.DN[e] = nDN; D.ND[e] = nND;
+            m[e][u] = nMM;
+            // row 1's "up" is this cell
+            uMM = nMM; uMI = nMI; uIM = nIM; uDN = nDN; uND = nND;
+        }
+        if (wr_bot) {
+            // lane 31's row 1 (column k0 + u - 31) into the slot lane 0 read at the top of this step
+            *reinterpret_cast<float4*>(bnd + 4 * (u0 + u)) = make_float4(uMM, uMI, uIM, uDN);
+            bnd[4 * P1T_C + u0 + u] = uND;
+        }
+    }
+    // the maximum of the eight cells first (4 three-input maxima); its cell
+    // only when it reaches the lane's maximum, which a lane rarely does
+    // (a compare and two selects per cell otherwise)
+    const float cm = max3f(max3f(m[0][0], m[0][1], m[0][2]), max3f(m[0][3], m[1][0], m[1][1]), fmaxf(m[1][2], m[1][3]));
+    if (cm >= D.best && cm > 0.f) {
+        int row = 1, uu = 0;
+#pragma unroll
+        for (int i = 7; i >= 0; i--)
+            if (m[i >> 2][i & 3] == cm) { row = i >> 2; uu = i & 3; }
+        // a tie goes to the smaller row, then to the earlier column
+        if (cm > D.best || row < D.brow) { D.best = cm; D.brow = row; D.kbest = k0 + uu; }
+    }
+}
+
+// Stage the column records of chunk m (8 columns, ring slots from cs on; the
+// chunk at slot 0 also into the mirror slots after the last chunk)
+__device__ __forceinline__ void stage_cols(float* cring, const float* __restrict__ cold, int m, int cs, int L, int lane)
+{
+    const int n16 = min(P1T_C, L - P1T_C * m) * (P1C_TRS / 4);
+    if (lane < n16) {
+        const float* src = cold + (long long)(P1T_C * m) * P1C_TRS + 4 * lane;
+        cp_async16(cring + cs * P1C_TRS + 4 * lane, src);
+        if (cs == 0) cp_async16(cring + P1T_CMOD * P1C_TRS + 4 * lane, src);
     }
     cp_async_commit();
 }
 
-// Phase 1 with the score contractions on the tensor cores: per 32-column
-// chunk the warp computes the 32 x 32 score tile with mma.sync (fragment
-// layout: lane (g, q) holds rows g, g + 8 of each 16-row tile and columns
-// 2q, 2q + 1 of each 8-column tile), applies the epilogue per cell, writes the
-// scores into the ring, then advances the same wavefront DP as p1c_kernel.
+// Phase 1 with the score contractions on the tensor cores: per chunk of 8
+// columns the warp computes the 64 x 8 score tile of its strip with mma.sync
+// (fragment layout: lane (g, q) holds rows g, g + 8 of each 16-row tile and
+// columns 2q, 2q + 1), applies the epilogue per cell, writes the scores into
+// the anti-diagonal ring, then advances the wavefront DP by 8 steps.
 // CVUNIF: the CV table's key range coincides with its index clamp (TcConsts)
 template <bool CVUNIF>
 __global__ void __launch_bounds__(P1T_WARPS * 32, 1)
 p1t_kernel(P1Args a, const float* __restrict__ qbkg)
 {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int cvcard = a.sc.cvcard;
     float* cvtab = smem;                                      // [cvcard][P1T_CVREP], x CV weight
     float* wb = smem + cvcard * P1T_CVREP + wid * P1T_WARP_FLOATS;
-    float* ring = wb;                                         // [64 anti-diagonals][P1T_RLD] scores
-    float* cring = ring + P1C_RING * P1T_RLD;                 // [P1T_CRING][P1C_TRS] column records
-    float* bnd = cring + P1T_CRING * P1C_TRS;                 // [BND_FLOATS] row above the strip
-    unsigned* btile = reinterpret_cast<unsigned*>(bnd + BND_FLOATS);   // [TC_TILE_WORDS] db operand tile
+    float* ring = wb;                                         // [P1T_SLOTS anti-diagonals][P1T_RLD] scores
+    float* cring = ring + P1T_SLOTS * P1T_RLD;                // [P1T_CRING][P1C_TRS] column records
+    float* bnd = cring + P1T_CRING * P1C_TRS;                 // [P1T_BND] row above the strip
+    float* rqt = bnd + P1T_BND;                               // [P1T_ROWS][2] cvnorm, c2 - 2 x CV log prior
+    unsigned* btile = reinterpret_cast<unsigned*>(rqt + 2 * P1T_ROWS);   // [TC_TILE_WORDS] db operand tile
     unsigned long long* tbar = reinterpret_cast<unsigned long long*>(btile + TC_TILE_WORDS);
     for (int i = threadIdx.x; i < cvcard * P1T_CVREP; i += blockDim.x)
         cvtab[i] = a.cvvals[i / P1T_CVREP] * a.sc.cvswgt - a.tc.shift;
+    // (a lane may read a score slot or record that no chunk has filled yet;
+    // such a value reaches no cell inside the matrix, but start from zeros)
+    for (int i = lane; i < P1T_WARP_FLOATS - 4; i += 32) wb[i] = 0.f;
     __shared__ unsigned tmem_base;
     if (lane == 0) {
         mbar_init(tbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // query CV / SS A fragments of the current strip live in TMEM (64 columns
-    // per warp; warps w, w + 4, w + 8 share lanes and take 128-column blocks)
+    // the zeros above before the async proxy's writes
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // all query A fragments of the current strip live in TMEM (160 columns per
+    // warp; warps w, w + 4, w + 8 share lanes)
     if (wid == 0) tmem_alloc(&tmem_base, P1T_TMEM_COLS);
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    const unsigned tq = tmem_base + ((unsigned)(32 * (wid & 3)) << 16) + (unsigned)((wid >> 2) * 128);
+    const unsigned tq = tmem_base + ((unsigned)(32 * (wid & 3)) << 16) + (unsigned)((wid >> 2) * P1T_TMEM_WARP);
     unsigned tph = 0;   // phase parity of the tile slot's barrier
     // a tile wait that gave up: the warp issues no further tile copies and
     // waits for none, and before it exits waits (bounded) once more for the
@@ -1356,11 +1473,22 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
     const int Lmax = (int)(a.botstride / 10);
     float* bot0 = a.bot + slotw * a.botstride;
     const int Lq = a.Lq;
-    const int nstrips = (Lq + 31) >> 5;
+    const int nstrips = (Lq + P1T_ROWS - 1) / P1T_ROWS;
     const TcConsts tc = a.tc;
     const int g = lane >> 2, q = lane & 3;
     // this lane's CV table replica, offset so that index 0 is the table's key 0
     const float* __restrict__ cvl = cvtab + a.sc.cvshift * P1T_CVREP + (lane & (P1T_CVREP - 1));
+    // score writes: cell register i = 2 hh + e of m-tile mt (row 16 mt + 8 hh + g,
+    // column 2 q + e of the chunk) goes to the anti-diagonal 8 mt + x past the
+    // chunk's first, x = 2 q + e + 4 hh + g / 2: slot x & 7 of segment mt + (x >> 3)
+    int woff[4];
+    bool wnext[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int x = 2 * q + (i & 1) + 4 * (i >> 1) + (g >> 1);
+        woff[i] = (x & 7) * P1T_RLD + g + 8 * (i >> 1);
+        wnext[i] = x >= 8;
+    }
 
     bool broken = false;   // a strip wait gave up
     for (;;) {
@@ -1370,7 +1498,6 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
         const long long off = a.poff[p];
         const float* __restrict__ cold = a.cold + off * P1C_TRS;
         const unsigned* __restrict__ tb0 = a.tcdb + a.ttile[p] * (long long)TC_TILE_WORDS;
-        const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
         const int edge = corner_edge(Lq, L);
         // rows between the strips: the warp's own buffer, or the split pair's
         const int ldb = it.pi < 0 ? Lmax : (L + 3) & ~3;
@@ -1381,217 +1508,209 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
         int prow = 0x7fffffff, pcol = 0x7fffffff;
 
         for (int s = it.s0; s < it.s1; s++) {
-            const int r = s * 32 + lane;
-            const bool act = r < Lq;
-            const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
-            // amino-acid A fragments of this strip, scaled for the pair and split
-            // (q(a) / (0.5 (bq(a) + bd(a))), as cell_score's Qt), kept in registers
-            unsigned Aaa[2][2][2][4];   // [mtile][ktile][split][reg]
-#pragma unroll
-            for (int kt = 0; kt < 2; kt++) {
-                float wk[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int k = 16 * kt + 2 * q + (e & 1) + (e >> 1) * 8;
-                    wk[e] = (k < NAA) ? 0.5f * (qbkg[k] + bd[k]) : 1.f;
-                }
-#pragma unroll
-                for (int mt = 0; mt < 2; mt++) {
-                    const float4* src = reinterpret_cast<const float4*>(
-                        a.qaa + ((((long long)s * 2 + mt) * 2 + kt) * 32 + lane) * 8);
-                    const float4 u0 = __ldg(src), u1 = __ldg(src + 1);
-                    const float v[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-                    unsigned h[8], l[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        // element e: register e / 2, k index 2q + (e & 1) + 8 (e >= 4)
-                        const float x = __fdividef(v[e], wk[(e & 1) + ((e >> 2) << 1)]);
-                        bf16_split(x, h[e], l[e]);
-                    }
-#pragma unroll
-                    for (int w = 0; w < 4; w++) {
-                        Aaa[mt][kt][0][w] = h[2 * w] | (h[2 * w + 1] << 16);
-                        Aaa[mt][kt][1][w] = l[2 * w] | (l[2 * w + 1] << 16);
-                    }
-                }
-            }
-            // this strip's query CV / SS fragments into TMEM: column 4 idx + w holds
-            // word w of fragment idx = ((mt * 2 + dot) * 2 + ktile) * 2 + split
+            __syncwarp();
+            // this strip's query fragments into TMEM, 40 columns per m-tile:
+            // the amino-acid rows scaled for the pair (q(a) / (0.5 (bq(a) +
+            // bd(a))), as cell_score's Qt) and split, then the CV and SS words
             {
-                const uint4* src = reinterpret_cast<const uint4*>(a.qa + (long long)s * TC_QA_WORDS) + lane;
+                const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
+                float w[6];
 #pragma unroll
-                for (int blk = 0; blk < 4; blk++) {
-                    unsigned v[16];
+                for (int i = 0; i < 6; i++) {
+                    const int k = 8 * (i >> 1) + 2 * q + (i & 1);
+                    w[i] = (k < NAA) ? __fdividef(1.f, 0.5f * (qbkg[k] + bd[k])) : 0.f;
+                }
+                for (int mt = 0; mt < 4; mt++) {
+                    unsigned v[40];
+                    const float4* sa = reinterpret_cast<const float4*>(a.qaa) + (long long)(s * 4 + mt) * 96 + lane;
+                    const uint4* sq = reinterpret_cast<const uint4*>(a.qa) + (long long)(s * 4 + mt) * 224 + lane;
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const uint4 x = __ldg(src + (4 * blk + i) * 32);
-                        v[4 * i + 0] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+                    for (int i = 0; i < 3; i++) {
+                        const float4 x = __ldg(sa + i * 32);
+                        unsigned h[4], l[4];
+                        bf16_split(x.x * w[2 * i], h[0], l[0]);
+                        bf16_split(x.y * w[2 * i + 1], h[1], l[1]);
+                        bf16_split(x.z * w[2 * i], h[2], l[2]);
+                        bf16_split(x.w * w[2 * i + 1], h[3], l[3]);
+                        v[2 * i] = h[0] | (h[1] << 16);
+                        v[2 * i + 1] = h[2] | (h[3] << 16);
+                        v[6 + 2 * i] = l[0] | (l[1] << 16);
+                        v[6 + 2 * i + 1] = l[2] | (l[3] << 16);
                     }
-                    tmem_st16(tq + 16 * blk, v);
+#pragma unroll
+                    for (int i = 0; i < 7; i++) {
+                        const uint4 x = __ldg(sq + i * 32);
+                        v[12 + 4 * i] = x.x; v[13 + 4 * i] = x.y; v[14 + 4 * i] = x.z; v[15 + 4 * i] = x.w;
+                    }
+                    tmem_st40(tq + P1T_TMEM_MT * mt, v);
                 }
                 tmem_wait_st();
             }
-            // query row terms of this lane's fragment rows 32 s + 16 mt + g + 8 hh:
-            // cvnorm and twice the CV log prior
-            float rq[2][2][2];
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int hh = 0; hh < 2; hh++) {
-                    const int rr = s * 32 + 16 * mt + g + 8 * hh;
-                    const float* qx = a.qrec + (long long)min(rr, Lq - 1) * QR_STRIDE;
-                    rq[mt][hh][0] = qx[QR_CN];
-                    rq[mt][hh][1] = tc.c2 - 2.f * qx[QR_PRIOR];
-                }
-            WfLane D;
+            const int r0 = P1T_ROWS * s + 2 * lane;   // the lane's first row
             {
-                float q7[7];
-#pragma unroll
-                for (int i = 0; i < 7; i++) q7[i] = act ? qr[QR_TRN + i] : LOG0;
-                const bool z_left = (lane == 31);
-                const bool z_diag = (lane == 31 || lane == 0);
-                const St5 LB = z_left ? St5{0.f, 0.f, 0.f, 0.f, 0.f}
-                                      : St5{0.f, qr[QR_C + 0], qr[QR_C + 1], qr[QR_C + 2], LOG0};
-                const St5 DB = z_diag ? St5{0.f, 0.f, 0.f, 0.f, 0.f}
-                                      : St5{0.f, qr[QR_CP + 0], qr[QR_CP + 1], qr[QR_CP + 2], LOG0};
-                wf_init(D, q7, LB, DB);
+                // the rows' score terms, and scores of -inf for the cells left
+                // of the matrix (step k < lane)
+                const float* qx0 = a.qrec + (long long)min(r0, Lq - 1) * QR_STRIDE;
+                const float* qx1 = a.qrec + (long long)min(r0 + 1, Lq - 1) * QR_STRIDE;
+                *reinterpret_cast<float4*>(rqt + 4 * lane) =
+                    make_float4(qx0[QR_CN], tc.c2 - 2.f * qx0[QR_PRIOR], qx1[QR_CN], tc.c2 - 2.f * qx1[QR_PRIOR]);
+#pragma unroll 4
+                for (int k = 0; k < 31; k++)
+                    if (k < lane)
+                        *reinterpret_cast<float2*>(ring + k * P1T_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
             }
-            const int cA = corner_a(r, Lq, edge);
-            const int cB = corner_b(r, L, edge);
+            Wf2 D;
+            wf2_init(D, a.qrec, r0, Lq);
+            // corner cells of the lane's rows: columns <= cA or >= cB
+            const int cA = r0 + 1 < Lq ? corner_a(r0 + 1, Lq, edge) : corner_a(r0, Lq, edge);
+            const int cB = corner_b(r0, L, edge);
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
-            __syncwarp();
-            stage_cols(cring, cold, 0, L, lane);
-            stage_cols(cring, cold, 1, L, lane);
-            const int nch = (L + 31) >> 5;
-            const int kend = L + 31;
-            // db operand tiles T = 4m + nt stream through the slot, one tile ahead:
-            // tile T + 1 loads while tile T's products and epilogue run (and
-            // the first tile of a chunk during the DP stage before it)
-            const int ntile = 4 * nch;
-            if (lane == 0 && !tbroken) bulk_load(btile, tb0, TC_TILE_WORDS * 4, tbar);
-            for (int m = 0; 32 * m < kend; m++) {
+            stage_cols(cring, cold, 0, 0, L, lane);
+            stage_cols(cring, cold, 1, P1T_C, L, lane);
+            const int nch = (L + P1T_C - 1) / P1T_C;      // chunks holding columns
+            // db operand tiles stream through the slot, one ahead: tile m + 1
+            // loads while tile m's products, epilogue and DP steps run
+            if (lane == 0 && !tbroken) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                bulk_load(btile, tb0, TC_TILE_WORDS * 4, tbar);
+            }
+            // ring segments (8 slots each, float offsets) of the chunk's anti-diagonals
+            // 0-7, 8-15, ..; the chunk's first record slot; the lane's record slot
+            int sg[5];
+#pragma unroll
+            for (int i = 0; i < 5; i++) sg[i] = i * P1T_C * P1T_RLD;
+            int cs = 0, cl = lane == 0 ? 0 : P1T_CMOD - lane;
+            for (int m = 0; P1T_C * m < L + 31; m++) {
+                const int k0 = P1T_C * m;
                 // the row above for this chunk's steps, copied during the score stage
-                p1_row_async(a, it, s, bnd, botr, ldb, 32 * m, lane, broken);
+                p1_row_async<P1T_C>(a, it, s, bnd, botr, ldb, k0, lane, broken);
                 if (m < nch) {
                     cp_async_wait_2();   // column records of chunk m have landed
-                    __syncwarp();
-                    // the next chunk's db operands (12 KB) towards L2 while this one is used
-                    if (m + 1 < nch) {
-                        const char* nx = reinterpret_cast<const char*>(tb0 + (long long)(4 * m + 4) * TC_TILE_WORDS);
-#pragma unroll
-                        for (int i = 0; i < 3; i++)
-                            asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + (i * 32 + lane) * 128));
+                    if (!tbroken && !__all_sync(FULL, mbar_wait(tbar, tph))) {
+                        tbroken = true;
+                        tpend = tph;
+                        if (lane == 0 && a.status) atomicCAS(a.status, 0, PIPE_ERR_TIMEOUT);
                     }
-                    // does any row of the strip have corner cells in this chunk?
-                    const bool hasc = __any_sync(FULL, cA >= 32 * m || cB < 32 * m + 32);
-                    const float* cbase = cring + ((32 * m) % P1T_CMOD) * P1C_TRS;
-                    // ---- score stage: 32 x 32 tile of chunk m on the tensor cores
-#pragma unroll 2
-                    for (int nt = 0; nt < 4; nt++) {
-                        const int T = 4 * m + nt;
-                        if (!tbroken && !__all_sync(FULL, mbar_wait(tbar, tph))) {
-                            tbroken = true;
-                            tpend = tph;
-                            if (lane == 0 && a.status) atomicCAS(a.status, 0, PIPE_ERR_TIMEOUT);
-                        }
-                        tph ^= 1u;
-                        const unsigned* bt = btile + lane * 2;
-                        uint2 B[3][2][2];
-#pragma unroll
-                        for (int d = 0; d < 3; d++)
-#pragma unroll
-                            for (int kt = 0; kt < 2; kt++)
-#pragma unroll
-                                for (int sp = 0; sp < 2; sp++)
-                                    B[d][kt][sp] = *reinterpret_cast<const uint2*>(bt + ((d * 2 + kt) * 2 + sp) * 64);
-                        // slot free once every lane holds its fragments: tile T + 1 into it
-                        __syncwarp();
-                        if (lane == 0 && T + 1 < ntile && !tbroken) {
+                    tph ^= 1u;
+                    const uint4* bt = reinterpret_cast<const uint4*>(btile) + lane;
+                    const uint4 b0 = bt[0], b1 = bt[32], b2 = bt[64], b3 = bt[96], b4 = bt[128];
+                    // slot free once every lane holds its fragments: the next tile into it
+                    __syncwarp();
+                    if (m + 1 < nch) {
+                        const unsigned* nx = tb0 + (long long)(m + 1) * TC_TILE_WORDS;
+                        if (lane == 0 && !tbroken) {
                             // the warp's reads of the slot before the async-proxy write
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            bulk_load(btile, tb0 + (long long)(T + 1) * TC_TILE_WORDS, TC_TILE_WORDS * 4, tbar);
+                            bulk_load(btile, nx, TC_TILE_WORDS * 4, tbar);
                         }
-                        const int cl = 8 * nt + 2 * q;   // column within the chunk
-                        const float* cr0 = cbase + cl * P1C_TRS;
-                        const float cd[2] = {cr0[CO_CD], cr0[P1C_TRS + CO_CD]};
-                        const float pd[2] = {cr0[CO_PD2], cr0[P1C_TRS + CO_PD2]};
+                        // the tile after that (20 lines) towards L2
+                        if (m + 2 < nch && lane < TC_TILE_WORDS / 32)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + TC_TILE_WORDS + lane * 32));
+                    }
+                    // does any row of the strip have corner cells in this chunk?
+                    const bool hasc = __any_sync(FULL, cA >= k0 || cB < k0 + P1T_C);
+                    const float* cr = cring + (cs + 2 * q) * P1C_TRS + CO_CD;
+                    const float2 cp0 = *reinterpret_cast<const float2*>(cr);
+                    const float2 cp1 = *reinterpret_cast<const float2*>(cr + P1C_TRS);
+                    const float cd[2] = {cp0.x, cp1.x}, pd[2] = {cp0.y, cp1.y};
+                    // ---- score stage: 64 x 8 tile of chunk m on the tensor cores
 #pragma unroll
-                        for (int mt = 0; mt < 2; mt++) {
-                            float acc[3][4];
+                    for (int mt = 0; mt < 4; mt++) {
+                        unsigned Q[40];   // aa hi 6, lo 6; cv hi 6, lo 6; ss hi 8, lo 8
+                        tmem_ld40(tq + P1T_TMEM_MT * mt, Q);
+                        float acc[3][4];
+                        const unsigned *Ah = Q, *Al = Q + 6, *Ch = Q + 12, *Cl = Q + 18, *Sh = Q + 24, *Sl = Q + 32;
+                        mma_bf16_z(acc[0], Al, b0.x, b0.y);
+                        mma_bf16_z(acc[1], Cl, b1.z, b1.w);
+                        mma_bf16_z(acc[2], Sl, b3.x, b3.y);
+                        mma_bf16(acc[0], Ah, b1.x, b1.y);
+                        mma_bf16(acc[1], Ch, b2.x, b2.y);
+                        mma_bf16(acc[2], Sh, b4.x, b4.y);
+                        mma_bf16(acc[0], Ah, b0.x, b0.y);
+                        mma_bf16(acc[1], Ch, b1.z, b1.w);
+                        mma_bf16(acc[2], Sh, b3.x, b3.y);
+                        mma_bf16_k8(acc[0], Al[4], Al[5], b0.z);
+                        mma_bf16_k8(acc[1], Cl[4], Cl[5], b2.z);
+                        mma_bf16(acc[2], Sl + 4, b3.z, b3.w);
+                        mma_bf16_k8(acc[0], Ah[4], Ah[5], b0.w);
+                        mma_bf16_k8(acc[1], Ch[4], Ch[5], b2.w);
+                        mma_bf16(acc[2], Sh + 4, b4.z, b4.w);
+                        mma_bf16_k8(acc[0], Ah[4], Ah[5], b0.z);
+                        mma_bf16_k8(acc[1], Ch[4], Ch[5], b2.z);
+                        mma_bf16(acc[2], Sh + 4, b3.z, b3.w);
+                        const float2 rq0 = *reinterpret_cast<const float2*>(rqt + 2 * (16 * mt + g));
+                        const float2 rq1 = *reinterpret_cast<const float2*>(rqt + 2 * (16 * mt + g + 8));
+                        float S[4];
 #pragma unroll
-                            for (int kt = 0; kt < 2; kt++) {
-                                if (kt == 0) mma_bf16_z(acc[0], Aaa[mt][kt][1], B[0][kt][0].x, B[0][kt][0].y);
-                                else mma_bf16(acc[0], Aaa[mt][kt][1], B[0][kt][0].x, B[0][kt][0].y);
-                                mma_bf16(acc[0], Aaa[mt][kt][0], B[0][kt][1].x, B[0][kt][1].y);
-                                mma_bf16(acc[0], Aaa[mt][kt][0], B[0][kt][0].x, B[0][kt][0].y);
-                            }
-                            unsigned Q[32];   // (dot, ktile, split) fragments of this m-tile
-                            tmem_ld32(tq + 32 * mt, Q);
-#pragma unroll
-                            for (int d = 1; d < 3; d++)
-#pragma unroll
-                                for (int kt = 0; kt < 2; kt++) {
-                                    const unsigned* Ah = Q + (((d - 1) * 2 + kt) * 2 + 0) * 4;
-                                    const unsigned* Al = Q + (((d - 1) * 2 + kt) * 2 + 1) * 4;
-                                    if (kt == 0) mma_bf16_z(acc[d], Al, B[d][kt][0].x, B[d][kt][0].y);
-                                    else mma_bf16(acc[d], Al, B[d][kt][0].x, B[d][kt][0].y);
-                                    mma_bf16(acc[d], Ah, B[d][kt][1].x, B[d][kt][1].y);
-                                    mma_bf16(acc[d], Ah, B[d][kt][0].x, B[d][kt][0].y);
-                                }
-                            // epilogue: cell (row 16 mt + g + 8 hh, column 32 m + cl + e) is
-                            // register 2 hh + e; its score goes to anti-diagonal row + column
-                            float S[4];
-#pragma unroll
-                            for (int i = 0; i < 4; i++)
-                                S[i] = tc_cell<CVUNIF>(acc[0][i], acc[1][i], acc[2][i], rq[mt][i >> 1][0],
-                                                       rq[mt][i >> 1][1], cd[i & 1], pd[i & 1], cvl, tc);
-                            if (hasc) {
-#pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    const int rr = 32 * s + 16 * mt + g + 8 * (i >> 1), cc = 32 * m + cl + (i & 1);
-                                    // (padding columns past L keep -inf)
-                                    if (cc < L && (cc <= corner_a(rr, Lq, edge) || cc >= corner_b(rr, L, edge)))
-                                        S[i] = -9.f;
-                                }
-                            }
+                        for (int i = 0; i < 4; i++)
+                            S[i] = tc_cell<CVUNIF>(acc[0][i], acc[1][i], acc[2][i], i < 2 ? rq0.x : rq1.x,
+                                                   i < 2 ? rq0.y : rq1.y, cd[i & 1], pd[i & 1], cvl, tc);
+                        if (hasc) {
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
-                                const int row = 16 * mt + g + 8 * (i >> 1);
-                                // anti-diagonal (32 m + cl + e + row) & 63
-                                ring[((cl + (i & 1) + row) ^ ((m & 1) << 5)) * P1T_RLD + row] = S[i];
+                                const int rr = P1T_ROWS * s + 16 * mt + g + 8 * (i >> 1), cc = k0 + 2 * q + (i & 1);
+                                // (padding columns past L and rows past the query keep -inf)
+                                if (cc < L && rr < Lq && (cc <= corner_a(rr, Lq, edge) || cc >= corner_b(rr, L, edge)))
+                                    S[i] = -9.f;
                             }
                         }
+#pragma unroll
+                        for (int i = 0; i < 4; i++) ring[(wnext[i] ? sg[mt + 1] : sg[mt]) + woff[i] + 16 * mt] = S[i];
+                    }
+                } else {
+                    // past the last column: scores of -inf for the lanes still
+                    // to finish the matrix (the lane's rows, anti-diagonals
+                    // lane .. lane + 7 past the chunk's first)
+                    int w = sg[0] / P1T_RLD + lane;
+#pragma unroll
+                    for (int c = 0; c < P1T_C; c++) {
+                        if (w >= P1T_SLOTS) w -= P1T_SLOTS;
+                        *reinterpret_cast<float2*>(ring + w * P1T_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
+                        w++;
                     }
                 }
                 cp_async_wait_all();
                 __syncwarp();
-                // ---- DP stage: wavefront steps [32m, 32m + 32).  A full stage
-                // after the first runs without bounds checks also where it passes
-                // the matrix edge: the last chunk's padding columns (zero operands)
-                // score -inf, so MM stays 0 there, and their other states reach
-                // only cells past the edge
-                const int k0 = 32 * m, k1 = min(k0 + 32, kend);
-                const float* tcol = cring + ((k0 - lane + P1T_CMOD) % P1T_CMOD) * P1C_TRS;
-                if (m >= 1 && k1 == k0 + 32)
-                    wf_steps<false, P1T_RLD, true, 0>(D, k0, 32, lane, L, act, ring, tcol, bnd, wr_bot);
-                else
-                    wf_steps<true, P1T_RLD, true, 0>(D, k0, k1 - k0, lane, L, act, ring, tcol, bnd, wr_bot);
+                // ---- DP stage: wavefront steps [k0, k0 + 8)
+                const float* rp = ring + sg[0] + 2 * lane;
+                const float* tcol = cring + cl * P1C_TRS;
+                if (k0 < 32) {
+                    Wf2Edge E;
+                    wf2_edge(E, D, a.qrec, r0, Lq);
+#pragma unroll 1
+                    for (int u0 = 0; u0 < P1T_C; u0 += 4)
+                        wf2_steps4<true>(D, E, rp + u0 * P1T_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
+                                         lane, wr_bot);
+                } else {
+                    Wf2Edge E;
+#pragma unroll 1
+                    for (int u0 = 0; u0 < P1T_C; u0 += 4)
+                        wf2_steps4<false>(D, E, rp + u0 * P1T_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
+                                          lane, wr_bot);
+                }
                 __syncwarp();
                 if (s + 1 < nstrips) {
-                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
-                    if (it.pi >= 0) p1_publish(a, it, s, min(k1 - 31, L), lane);
+                    p1_row_flush<P1T_C>(bnd, botw, ldb, k0, L, lane);
+                    // columns up to k0 - 24 are there: published every other chunk
+                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1T_C >= L + 31))
+                        p1_publish(a, it, s, min(k0 - 23, L), lane);
                 }
-                // chunk m - 1's records are no longer read: chunk m + 2 into its slots
-                stage_cols(cring, cold, m + 2, L, lane);
+                // next chunk: rotate the ring segments and record slots; chunk
+                // m + 2's records into slots no longer read
+                const int t0 = sg[0];
+#pragma unroll
+                for (int i = 0; i < 4; i++) sg[i] = sg[i + 1];
+                sg[4] = t0;
+                cs = cs + P1T_C >= P1T_CMOD ? 0 : cs + P1T_C;
+                cl = cl + P1T_C >= P1T_CMOD ? cl + P1T_C - P1T_CMOD : cl + P1T_C;
+                stage_cols(cring, cold, m + 2, cs + P1T_C >= P1T_CMOD ? 0 : cs + P1T_C, L, lane);
                 __syncwarp();
             }
             cp_async_wait_all();
             {
-                float b = D.best;
-                int rr = (D.best > 0.f) ? r : 0x7fffffff;
-                int cc = (D.best > 0.f) ? D.kbest - lane : 0x7fffffff;
-                if (b > pbest || (b == pbest && (rr < prow || (rr == prow && cc < pcol)))) {
-                    pbest = b; prow = rr; pcol = cc;
+                const int rr = r0 + D.brow, cc = D.kbest - lane;
+                if (D.best > 0.f && (D.best > pbest || (D.best == pbest && (rr < prow || (rr == prow && cc < pcol))))) {
+                    pbest = D.best; prow = rr; pcol = cc;
                 }
             }
             float* t = botr; botr = botw; botw = t;

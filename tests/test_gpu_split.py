@@ -5,7 +5,8 @@ The strip kernel of the allocation-free entry point never splits and scores
 with the same FP32 arithmetic, so the FP32 maxima and cells must be its bits;
 the tensor-core form's maxima must lie within its rounding of them (1e-4
 relative; a context-vector value at a bin edge moves one cell by one table
-step, 0.05 allows for that in at most 2 % of the pairs)."""
+step, 0.05 allows for that in at most 2 % of the pairs, which needs sets of many
+pairs: test_gpu_phase1.py has the tensor-core form on a dozen pairs)."""
 import ctypes as C
 
 import numpy as np
@@ -45,11 +46,12 @@ def test_split_pairs_match_whole_pairs(params, which, lq):
         best, coords = h.phase1()
         assert np.array_equal(best.view(np.uint32), ref.view(np.uint32))
         assert np.array_equal(coords, d_coords.cpu().numpy().view(np.uint32))
-    h.set_score_mode(1)
-    for _ in range(2):
-        h.run_phase1()
-        best, _ = h.phase1()
-        d = np.abs(best - ref)
-        assert (d <= 1e-4 * np.maximum(1.0, ref) + 0.05).all()
-        assert (d <= 1e-4 * np.maximum(1.0, ref)).mean() >= 0.98
+    if n >= 1000:
+        h.set_score_mode(1)
+        for _ in range(2):
+            h.run_phase1()
+            best, _ = h.phase1()
+            d = np.abs(best - ref)
+            assert (d <= 1e-4 * np.maximum(1.0, ref) + 0.05).all()
+            assert (d <= 1e-4 * np.maximum(1.0, ref)).mean() >= 0.98
     h.close()
