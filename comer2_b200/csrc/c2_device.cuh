@@ -79,34 +79,22 @@ constexpr int MAX_CVCARD = 256;
 // "-99 < ss" guard always holds for tables above SS_FOLD_MIN, which the
 // tensor-core form requires, with card <= 30).
 // Per db position the DP and the score epilogue also read a column record
-// cold[pos][P1C_TRS]: the DP transitions in the order below (slots 0..6),
-// cvnorm and 2 x CV log prior (slots 8, 9), pad.
-constexpr int P1T_ROWS = 64;                          // query rows per strip
+// cold[pos][P1C_TRS]: the DP transitions (TMM .. TDD, slots 0..6), cvnorm and
+// 2 x CV log prior (slots 8, 9), pad.
+constexpr int P1_ROWS = 64;                           // query rows per strip of the phase-1 kernels
 constexpr int TC_TILE_WORDS = 5 * 32 * 4;
 constexpr int TC_QA_WORDS = 4 * 7 * 32 * 4;           // per strip
 constexpr int TC_QAA_FLOATS = 4 * 3 * 32 * 4;         // per strip
 constexpr float SS_FOLD_MIN = -49.f;
 constexpr int TC_SS_KMAX = 30;
 enum : int { CO_CD = 8, CO_PD2 = 9 };
-// DP transition record of a db column, two 16-byte reads of a Viterbi step:
-// MM IM DM MI, II MD DD.  DPT_SRC packs, per record slot i, the transition
-// index (TMM..TDD) in bits [4i, 4i + 4).
-constexpr int DPT_N = 7;
-constexpr unsigned long long DPT_SRC = 0x6241530ull;
-__host__ __device__ constexpr int dpt_src(int i) { return (int)((DPT_SRC >> (4 * i)) & 0xf); }
-// chunked phase-1 kernel: 11 warps per CTA, one CTA per SM; per warp a score
-// ring of 64 columns x 32 rows, a transition ring of 64 columns (stride 12
-// floats: the two 16-byte reads of 8 lanes at consecutive columns cover 32
-// distinct banks), the SS row table, the record staging ring and the row
-// above the strip for the current chunk
-constexpr int P1C_WARPS = 11;
 // phase-1 kernel variants of launch_p1
 enum : int { P1K_STRIP = 0, P1K_CHUNKED = 1, P1K_TRACEBACK = 2, P1K_TENSOR = 3 };
-constexpr int P1C_RING = 64, P1C_TRS = 12, P1C_CVREP = 16;
-// row above the strip in the shared-memory DP kernels: [32][4] + [32] floats
+// column records in shared memory, 12 floats apart (the two 16-byte reads of 8
+// lanes at consecutive columns cover 32 distinct banks)
+constexpr int P1C_RING = 64, P1C_TRS = 12;
+// row above the strip in the traceback sweep: [32][4] + [32] floats
 constexpr int BND_ND = 32 * 4, BND_FLOATS = 32 * 5;
-constexpr int P1C_WARP_FLOATS =
-    P1C_RING * 32 + P1C_RING * P1C_TRS + MAX_SSSS_CARD * 32 + REC_SLOTS * DR_STRIDE + BND_FLOATS;
 // traceback sweep over the stored score matrices: per warp the score ring, the
 // transition ring, the row above and a [32][33]-byte traceback column ring;
 // 17 warps per SM.  P1TC_CVREP: CV table replicas of the phase-2 score kernel
@@ -125,24 +113,30 @@ constexpr int SMEM_CTA_MAX = 227 * 1024;
 constexpr int P1TC_MAX_CVCARD =
     (SMEM_CTA_MAX - P2S_WARPS * P2S_WARP_FLOATS * 4) / (P1TC_CVREP * 4);
 constexpr int P1T_MAX_CVCARD = 106;
-// Tensor-core kernel, two query rows per lane (strips of 64 rows), the db
-// columns in chunks of 8 (one operand tile).  Per warp: score ring of 40
-// anti-diagonals (31 lanes of skew + a chunk) of 64 floats, padded to 68 so
-// that the fragment-layout writes and the wavefront's 8-byte reads are both
-// free of bank conflicts; column-record ring of 7 chunks and a mirror of its
-// first chunk, so that the 8 records a lane reads in one DP stage never wrap;
-// the row above the strip for one chunk; the rows' score terms; one slot for
-// the db operand tile (a bulk async copy, one mbarrier).
-constexpr int P1T_WARPS = 12;
-constexpr int P1T_C = 8;
-constexpr int P1T_SLOTS = 40, P1T_RLD = 68, P1T_CMOD = 56, P1T_CRING = 64, P1T_CVREP = 16;
+// Phase-1 kernels, two query rows per lane (strips of 64 rows), the db columns
+// in chunks of 8.  Per warp: score ring of 40 anti-diagonals (31 lanes of skew
+// + a chunk) of 64 floats, padded to 68 so that the score writes (a lane's two
+// rows, or the tensor fragments) and the wavefront's 8-byte reads are free of
+// bank conflicts; column-record ring of 7 chunks and a mirror of its first
+// chunk, so that the 8 records a lane reads in one DP stage never wrap; the row
+// above the strip for one chunk.
+constexpr int P1_C = 8;
+constexpr int P1_SLOTS = 40, P1_RLD = 68, P1_CMOD = 56, P1_CRING = 64;
+constexpr int P1_BND = 5 * P1_C;
+constexpr int P1_WF_FLOATS = P1_SLOTS * P1_RLD + P1_CRING * P1C_TRS + P1_BND;
+// FP32 kernel: also the SS row table of the strip and the record staging ring
+constexpr int P1C_WARPS = 8, P1C_CVREP = 16;
+constexpr int P1C_WARP_FLOATS = P1_WF_FLOATS + MAX_SSSS_CARD * P1_ROWS + REC_SLOTS * DR_STRIDE;
+static_assert((MAX_CVCARD * P1C_CVREP + P1C_WARPS * P1C_WARP_FLOATS) * 4 <= SMEM_CTA_MAX, "FP32 phase-1 shared memory");
+// tensor-core kernel: also the rows' score terms and one slot for the db
+// operand tile (a bulk async copy, one mbarrier)
+constexpr int P1T_WARPS = 12, P1T_CVREP = 16;
 constexpr unsigned P1T_TMEM_COLS = 512;   // TMEM columns of a CTA: 3 warps x 160 per lane quarter
 constexpr int P1T_TMEM_MT = 40, P1T_TMEM_WARP = 4 * P1T_TMEM_MT;
-constexpr int P1T_BND = 5 * P1T_C;
-constexpr int P1T_WARP_FLOATS =
-    P1T_SLOTS * P1T_RLD + P1T_CRING * P1C_TRS + P1T_BND + 2 * P1T_ROWS + TC_TILE_WORDS + 4;
-static_assert((P1T_MAX_CVCARD * P1T_CVREP + P1T_WARPS * P1T_WARP_FLOATS) * 4 + 16 <= SMEM_CTA_MAX, "phase-1 shared memory");
-static_assert(P1T_WARP_FLOATS % 4 == 0, "16-byte alignment of the warps' shared memory");
+constexpr int P1T_WARP_FLOATS = P1_WF_FLOATS + 2 * P1_ROWS + TC_TILE_WORDS + 4;
+static_assert((P1T_MAX_CVCARD * P1T_CVREP + P1T_WARPS * P1T_WARP_FLOATS) * 4 + 16 <= SMEM_CTA_MAX,
+              "tensor-core phase-1 shared memory");
+static_assert(P1T_WARP_FLOATS % 4 == 0 && P1C_WARP_FLOATS % 4 == 0, "16-byte alignment of the warps' shared memory");
 
 // Epilogue constants of the tensor-core form: x = 2 x (CV score argument)
 // = (2 pownu0 ln2) log2(det) + 2 cterm - 2 prior_q - 2 prior_d, compared

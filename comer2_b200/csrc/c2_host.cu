@@ -914,14 +914,14 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
             if (k == TC_SS_KMAX + 1) return 1.f;
             return k < card ? U[(size_t)r * 32 + k] : 0.f;
         };
-        const int nt = (Lq + P1T_ROWS - 1) / P1T_ROWS;
+        const int nt = (Lq + P1_ROWS - 1) / P1_ROWS;
         std::vector<uint32_t> qa((size_t)nt * TC_QA_WORDS, 0u);
         std::vector<float> qaa((size_t)nt * TC_QAA_FLOATS, 0.f);
         for (int s = 0; s < nt; s++)
             for (int mt = 0; mt < 4; mt++)
                 for (int lane = 0; lane < 32; lane++) {
                     const int g = lane >> 2, qq = lane & 3;
-                    const int r0 = P1T_ROWS * s + 16 * mt + g;
+                    const int r0 = P1_ROWS * s + 16 * mt + g;
                     // word w of operand d: row r0 + 8 (w & 1), k = 8 (w >> 1) + 2 qq, + 1; the
                     // CV operand has words 0..5 (k < 24), the SS operand 0..7
                     size_t o = (size_t)(s * 4 + mt) * 7;   // 16-byte groups
@@ -1047,7 +1047,7 @@ static c2_status tc_prepare_db(c2_handle* h)
     long long ntiles = 0;
     for (int k = 0; k < h->nprof; k++) {
         tt[k] = ntiles;
-        ntiles += (h->h_plen[k] + P1T_C - 1) / P1T_C;
+        ntiles += (h->h_plen[k] + P1_C - 1) / P1_C;
     }
     if (h->db->d_ttile.ensure(h->nprof, h->budget) || h->db->d_tcdb.ensure((size_t)ntiles * TC_TILE_WORDS, h->budget) ||
         h->db->d_cold.ensure((size_t)h->npos * P1C_TRS, h->budget))
@@ -1112,9 +1112,9 @@ static void fill_p1(c2_handle* h, P1Args& a)
 // rows of the split pairs) -- the pairs then run whole, with the same results.
 constexpr double SPLIT_SHARE = 0.5;
 
-static int split_pairs(c2_handle* h, int nwarps, int rows, P1Args& a)
+static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
 {
-    const int P = h->nprof, ns = (h->Lq + rows - 1) / rows;   // strips of `rows` query rows
+    const int P = h->nprof, ns = (h->Lq + P1_ROWS - 1) / P1_ROWS;
     a.nsplit = 0;
     if (ns < 2) return 0;
     const double mean = ((double)h->npos + 31.0 * P) / std::max(1, nwarps);
@@ -1165,7 +1165,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
             return fail(h, C2_ERR_CUDA, "tensor-core phase-1 kernel does not fit on an SM (%s)",
                         cudaGetErrorString(oe));
         gt = std::min(gt, h->grid * P1_WARPS / P1T_WARPS);
-        split_pairs(h, gt * P1T_WARPS, P1T_ROWS, a);
+        split_pairs(h, gt * P1T_WARPS, a);
         CK(launch_p1(a, h->d_qbkg.p, P1K_TENSOR, gt, h->stream));
         h->launches++;
         return C2_OK;
@@ -1175,7 +1175,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     int gc = (h->nsm - h->p1_reserve) * p1c_blocks_per_sm(h->sc.cvcard);
     if (gc < 1) return fail(h, C2_ERR_CUDA, "phase-1 kernel does not fit on an SM");
     gc = std::min(gc, h->grid * P1_WARPS / P1C_WARPS);
-    split_pairs(h, gc * P1C_WARPS, 32, a);
+    split_pairs(h, gc * P1C_WARPS, a);
     CK(launch_p1(a, h->d_qbkg.p, P1K_CHUNKED, gc, h->stream));
     h->launches++;
     return C2_OK;

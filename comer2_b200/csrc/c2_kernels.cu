@@ -50,74 +50,115 @@ __device__ __forceinline__ bool in_corner(int lq, int ld, int e, int y, int x)
 // _ssss.cuh:48-131, _cvs2s.cuh:47-136.  The aa term uses the per-pair row
 // factors Qt[a] = q(a) / (0.5 (bq(a) + bd(a))); the SS term uses the per-row
 // table U[c] = sum_s p_q(s) T[idx_q(s)][c].
+// The two dot products run in packed pairs of FP32 (fma.rn.f32x2: two IEEE
+// multiply-adds per instruction, the two accumulators of each chain).  NR rows
+// share the record's reads.
 struct RowOps {
-    float Qt[NAA];
-    float qcv[NCV];
+    unsigned long long Qt[NAA / 2];        // pairs (2 i, 2 i + 1)
+    unsigned long long qcv[(NCV + 1) / 2]; // the last entry's partner is 0
     float cq, pq, hq;
 };
 
-// cvtab holds each CV map value CVREP times ([cvcard][CVREP]); a lane reads
-// replica lane % CVREP so that lanes reading different entries rarely share a bank.
-template <int CVREP>
-__device__ __forceinline__ float cell_score(const RowOps& R, const float4* __restrict__ rp,
-                                            const float* __restrict__ U, const float* __restrict__ cvtab,
-                                            const ScoreConsts& sc, int lane, float& mod_out)
+__device__ __forceinline__ unsigned long long pack2(float x, float y)
 {
-    float4 v;
+    return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float lo2(unsigned long long a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi2(unsigned long long a) { return __uint_as_float((unsigned)(a >> 32)); }
+
+// query row qr against a profile with background bd
+__device__ __forceinline__ void row_ops(RowOps& R, const float* __restrict__ qr, const float* __restrict__ qbkg,
+                                        const float* __restrict__ bd)
+{
+#pragma unroll
+    for (int i = 0; i < NAA; i += 2)
+        R.Qt[i / 2] = pack2(__fdividef(qr[QR_TRG + i], 0.5f * (qbkg[i] + bd[i])),
+                            __fdividef(qr[QR_TRG + i + 1], 0.5f * (qbkg[i + 1] + bd[i + 1])));
+#pragma unroll
+    for (int i = 0; i < NCV; i += 2) R.qcv[i / 2] = pack2(qr[QR_CV + i], i + 1 < NCV ? qr[QR_CV + i + 1] : 0.f);
+    R.cq = qr[QR_CN];
+    R.pq = qr[QR_PRIOR];
+    R.hq = qr[QR_HQ];
+}
+
+// Scores of NR consecutive rows; the SS row table U has USTR floats a column,
+// the lane's first row at U[urow].  cvtab holds each CV map value CVREP times
+// ([cvcard][CVREP]); a lane reads replica lane % CVREP so that lanes reading
+// different entries rarely share a bank.
+template <int CVREP, int NR, int USTR>
+__device__ __forceinline__ void cell_scores(const RowOps* R, const float* __restrict__ rec,
+                                            const float* __restrict__ U, int urow, const float* __restrict__ cvtab,
+                                            const ScoreConsts& sc, int lane, float* S, float* mod_out)
+{
+    const ulonglong2* rp = reinterpret_cast<const ulonglong2*>(rec);
+    unsigned long long s[NR], dot[NR];
+#pragma unroll
+    for (int e = 0; e < NR; e++) s[e] = dot[e] = 0ull;
     // aa term (two accumulators shorten the dependent FMA chain)
-    float s = 0.f, s2 = 0.f;
 #pragma unroll
     for (int i = 0; i < 5; i++) {
-        v = rp[i];
-        s = fmaf(R.Qt[4 * i + 0], v.x, s);
-        s2 = fmaf(R.Qt[4 * i + 1], v.y, s2);
-        s = fmaf(R.Qt[4 * i + 2], v.z, s);
-        s2 = fmaf(R.Qt[4 * i + 3], v.w, s2);
-    }
-    s += s2;
-    const float s0 = __logf(s) - sc.shift;
-    // CV term: dot product over [20,39), then (cq)(cd) - (dot+1/kappa0)^2
-    float dot = 0.f, dot2 = 0.f;
+        const ulonglong2 v = rp[i];
 #pragma unroll
-    for (int i = 5; i < 10; i++) {
-        v = rp[i];
-        const int b = 4 * i - DR_CV;
-        dot = fmaf(R.qcv[b + 0], v.x, dot);
-        dot2 = fmaf(R.qcv[b + 1], v.y, dot2);
-        dot = fmaf(R.qcv[b + 2], v.z, dot);
-        if (b + 3 < NCV) dot2 = fmaf(R.qcv[b + 3], v.w, dot2);
+        for (int e = 0; e < NR; e++) s[e] = fma2(R[e].Qt[2 * i + 1], v.y, fma2(R[e].Qt[2 * i], v.x, s[e]));
     }
-    dot += dot2;
-    const float cd = v.w;  // DR_CN = 39
-    v = rp[10];            // 40 prior, 41..43 ss
-    const float pd = v.x;
-    const float ds0 = v.y, ds1 = v.z, ds2 = v.w;
-    const float4 v11 = rp[11];  // 44 ss idx, 45 hd
-    dot += sc.lokappa0;
-    float det = R.cq * cd - dot * dot;
-    float cvs = sc.cterm + sc.pownu0 * __logf(det) - R.pq - pd;
-    float cvm;
-    if (cvs <= sc.cvkey_first) cvm = sc.cvval_first;
-    else if (sc.cvkey_last <= cvs) cvm = sc.cvval_last;
-    else {
-        // clamp keeps the shared-memory read in bounds for any table/argument
-        const int ix = min(max(sc.cvshift + (int)rintf(2.f * cvs), 0), sc.cvcard - 1);
-        cvm = cvtab[ix * CVREP + (lane & (CVREP - 1))];
+    // CV term: dot product over [20,39) (39, the CV norm, meets a 0), then
+    // (cq)(cd) - (dot+1/kappa0)^2
+    float cd = 0.f;
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        const ulonglong2 v = rp[5 + i];
+#pragma unroll
+        for (int e = 0; e < NR; e++) dot[e] = fma2(R[e].qcv[2 * i + 1], v.y, fma2(R[e].qcv[2 * i], v.x, dot[e]));
+        if (i == 4) cd = hi2(v.y);   // DR_CN = 39
     }
-    cvm *= sc.cvswgt;
-    // SS term
+    const float4 v10 = *reinterpret_cast<const float4*>(rec + DR_PRIOR);   // 40 prior, 41..43 ss
+    const float2 v11 = *reinterpret_cast<const float2*>(rec + DR_SSIDX);   // 44 ss idx, 45 hd
     const int pk = __float_as_int(v11.x);
-    float ss = ds0 * U[(pk & 0xff) * 32 + lane];
-    ss = fmaf(ds1, U[((pk >> 8) & 0xff) * 32 + lane], ss);
-    ss = fmaf(ds2, U[((pk >> 16) & 0xff) * 32 + lane], ss);
-    if (-99.f < ss) {
-        ss += R.hq * v11.y * 0.1111111f;
-        ss -= 0.05f;
-        ss *= sc.ssswgt;
+    const float* __restrict__ u0 = U + (pk & 0xff) * USTR + urow;
+    const float* __restrict__ u1 = U + ((pk >> 8) & 0xff) * USTR + urow;
+    const float* __restrict__ u2 = U + ((pk >> 16) & 0xff) * USTR + urow;
+    float w[3][NR];
+    if (NR == 2) {
+        const float2 a = *reinterpret_cast<const float2*>(u0), b = *reinterpret_cast<const float2*>(u1),
+                     c = *reinterpret_cast<const float2*>(u2);
+        w[0][0] = a.x; w[0][NR - 1] = a.y; w[1][0] = b.x; w[1][NR - 1] = b.y; w[2][0] = c.x; w[2][NR - 1] = c.y;
+    } else {
+        w[0][0] = *u0; w[1][0] = *u1; w[2][0] = *u2;
     }
-    const float add = ss + cvm;
-    mod_out = add - 0.5f * sc.cvswgt;   // modular score of the MAP stage
-    return s0 + add;
+#pragma unroll
+    for (int e = 0; e < NR; e++) {
+        const float s0 = __logf(lo2(s[e]) + hi2(s[e])) - sc.shift;
+        const float dt = (lo2(dot[e]) + hi2(dot[e])) + sc.lokappa0;
+        const float det = R[e].cq * cd - dt * dt;
+        const float cvs = sc.cterm + sc.pownu0 * __logf(det) - R[e].pq - v10.x;
+        float cvm;
+        if (cvs <= sc.cvkey_first) cvm = sc.cvval_first;
+        else if (sc.cvkey_last <= cvs) cvm = sc.cvval_last;
+        else {
+            // clamp keeps the shared-memory read in bounds for any table/argument
+            const int ix = min(max(sc.cvshift + (int)rintf(2.f * cvs), 0), sc.cvcard - 1);
+            cvm = cvtab[ix * CVREP + (lane & (CVREP - 1))];
+        }
+        cvm *= sc.cvswgt;
+        // SS term
+        float ss = v10.y * w[0][e];
+        ss = fmaf(v10.z, w[1][e], ss);
+        ss = fmaf(v10.w, w[2][e], ss);
+        if (-99.f < ss) {
+            ss += R[e].hq * v11.y * 0.1111111f;
+            ss -= 0.05f;
+            ss *= sc.ssswgt;
+        }
+        const float add = ss + cvm;
+        mod_out[e] = add - 0.5f * sc.cvswgt;   // modular score of the MAP stage
+        S[e] = s0 + add;
+    }
 }
 
 struct St5 { float MM, MI, IM, DN, ND; };
@@ -135,8 +176,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Stage the records of columns [REC_CHUNK*m, REC_CHUNK*(m+1)) (clipped to L)
 // into ring slots; records of consecutive columns are contiguous in HBM, so a
-// chunk is one contiguous range copied by all lanes in 16-byte pieces.  Every
-// call commits one group (possibly empty) so that wait_group counts stay aligned.
+// chunk is one contiguous range copied by all lanes in 16-byte pieces.  The
+// caller commits the group (possibly empty, so that wait_group counts stay aligned).
 __device__ __forceinline__ void stage_chunk(float* rec, const float* __restrict__ dr, int m, int L, int lane)
 {
     const int c0 = m * REC_CHUNK;
@@ -147,7 +188,20 @@ __device__ __forceinline__ void stage_chunk(float* rec, const float* __restrict_
         const float* src = dr + (long long)c0 * DR_STRIDE;
         for (int i = lane; i < n16; i += 32) cp_async16(dst + 4 * i, src + 4 * i);
     }
-    cp_async_commit();
+}
+
+// Transitions of the columns of chunk m (8 columns) from their records into
+// the column ring (slots from cs on; the chunk at slot 0 also into the mirror
+// slots after the last chunk)
+__device__ __forceinline__ void stage_trn(float* cring, const float* __restrict__ dr, int m, int cs, int L, int lane)
+{
+    const int c = P1_C * m + (lane >> 1);
+    if (lane < 2 * P1_C && c < L) {
+        const float* src = dr + (long long)c * DR_STRIDE + DR_TRN + 4 * (lane & 1);
+        float* dst = cring + (cs + (lane >> 1)) * P1C_TRS + 4 * (lane & 1);
+        cp_async16(dst, src);
+        if (cs == 0) cp_async16(dst + P1_CMOD * P1C_TRS, src);
+    }
 }
 
 __global__ void __launch_bounds__(P1_WARPS * 32, 2)
@@ -193,14 +247,7 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
             const bool act = r < Lq;
             const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
             RowOps R;
-#pragma unroll
-            for (int i = 0; i < NAA; i++)
-                R.Qt[i] = __fdividef(qr[QR_TRG + i], 0.5f * (qbkg[i] + bd[i]));
-#pragma unroll
-            for (int i = 0; i < NCV; i++) R.qcv[i] = qr[QR_CV + i];
-            R.cq = qr[QR_CN];
-            R.pq = qr[QR_PRIOR];
-            R.hq = qr[QR_HQ];
+            row_ops(R, qr, qbkg, bd);
             {
                 // this strip's SS row tables (built once per query, c2_set_query)
                 const float* __restrict__ us = a.qU + (long long)s * MAX_SSSS_CARD * 32 + lane;
@@ -239,7 +286,9 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
             const int nsteps = L + 31;
             // db column records are staged into shared memory one chunk ahead
             stage_chunk(rec, dr, 0, L, lane);
+            cp_async_commit();
             stage_chunk(rec, dr, 1, L, lane);
+            cp_async_commit();
             for (int k = 0; k < nsteps; k++) {
                 if ((k & (REC_CHUNK - 1)) == 0 && k < L) {
                     cp_async_wait_1();
@@ -249,8 +298,8 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
                 float tc[7];
                 if (k < L) {
                     const float4* rp = reinterpret_cast<const float4*>(rec + (k & (REC_SLOTS - 1)) * DR_STRIDE);
-                    float mod;
-                    float S = cell_score<32>(R, rp, U, cvtab, sc, lane, mod);
+                    float mod, S;
+                    cell_scores<32, 1, 32>(&R, reinterpret_cast<const float*>(rp), U, lane, cvtab, sc, lane, &S, &mod);
                     if (!act) S = -9.f;
                     ring[(k & 31) * 32 + lane] = S;
                     const float4 ta = rp[12], tb = rp[13];
@@ -260,6 +309,7 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
                         // chunk fully read by every lane: refill its slots two chunks ahead
                         __syncwarp();
                         stage_chunk(rec, dr, (k >> REC_CHUNK_LOG) + 2, L, lane);
+                        cp_async_commit();
                     }
                 } else {
 #pragma unroll
@@ -350,17 +400,15 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
 }
 
 // ---------------------------------------------------------------------------
-// Phase 1, chunked: the same arithmetic as p1_kernel, scheduled in chunks of
-// 32 db columns.  Per chunk, every lane first scores its query row against
-// the 32 columns (independent cells: the FMA chains of consecutive columns
-// overlap), writing scores and the columns' DP transitions to shared-memory
-// rings; then the warp advances the anti-diagonal wavefront by 32 steps.
-// Wavefront steps whose 32 cells all lie inside the matrix (every chunk but
-// the first and the last ones of a strip) run without bounds checks.
+// Phase 1, chunked: the arithmetic of p1_kernel, scheduled in chunks of 8 db
+// columns and strips of 64 query rows, two to a lane.  Per chunk the scores go
+// to a shared-memory ring, then the warp advances the anti-diagonal wavefront by
+// 8 steps.  Lane t holds rows 2 t and 2 t + 1 of the strip and processes column
+// k - t at step k.
 //
-// Score rings are indexed by anti-diagonal: the score of cell (row i of the
-// strip, column j) sits in slot (i + j) & 63, so at step k every lane reads
-// slot k & 63 and a DP stage reads 32 consecutive slots from one base.
+// The score ring is indexed by anti-diagonal: the scores of rows 2 t, 2 t + 1 at
+// column j sit in slot (t + j) mod 40, so at step k every lane reads slot k mod
+// 40 and a DP stage reads 8 consecutive slots from one base.
 
 // Maximum of three (sm_100 three-input max.f32; exact, like two fmaxf)
 __device__ __forceinline__ float max3f(float a, float b, float c)
@@ -418,7 +466,7 @@ __device__ __forceinline__ void bnd_put(float* bnd, int slot, float mm, float mi
 
 // Wavefront steps [k0, k0 + nst) of a strip (k0 a multiple of 32, nst <= 32;
 // 32 when !CHECK).  ring: diagonal-indexed scores, 32 floats per slot.  tcol:
-// ring of P1C_RING column records (DPT_N transitions, P1C_TRS floats apart).
+// ring of P1C_RING column records (TMM .. TDD, P1C_TRS floats apart).
 // bnd: row above the strip for columns [k0, k0 + 32).
 // TB (traceback sweep): each cell's traceback code also goes to the warp's
 // column ring btr (column j in slot j & 31, the lane's own row), and column
@@ -439,8 +487,8 @@ __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, i
     for (int u = 0; u < nst; u++) {
         const float S = rb[u * 32];
         const float* __restrict__ tp = tcol + ((k0 + u - lane) & (P1C_RING - 1)) * P1C_TRS;
-        const float4 ta = *reinterpret_cast<const float4*>(tp);       // MM IM DM MI
-        const float4 tb = *reinterpret_cast<const float4*>(tp + 4);   // II MD DD
+        const float4 ta = *reinterpret_cast<const float4*>(tp);       // MM MI MD IM
+        const float4 tb = *reinterpret_cast<const float4*>(tp + 4);   // II DM DD
         float uMM = __shfl_up_sync(FULL, D.MM, 1);
         float uMI = __shfl_up_sync(FULL, D.MI, 1);
         float uIM = __shfl_up_sync(FULL, D.IM, 1);
@@ -460,12 +508,12 @@ __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, i
         }
         const float X = uMM + D.qMM, Y = uMI + D.qMM, z = uND + D.qMM;
         const float A = max3f(X, uIM + D.qIM, uDN + D.qDM);
-        const float v = max3f(Ad + ta.x, Yd + ta.y, zd + ta.z);
+        const float v = max3f(Ad + ta.x, Yd + ta.w, zd + tb.y);
         const float nMM = fmaxf(v + S, 0.f);
-        const float nMI = fmaxf(X + ta.w, Y + tb.x);
+        const float nMI = fmaxf(X + ta.y, Y + tb.x);
         const float nIM = fmaxf(lMM + D.qMI, lIM + D.qII) + ta.x;
         const float nDN = fmaxf(uMM + D.qMD, uDN + D.qDD);
-        const float nND = fmaxf(lMM + tb.y, lND + tb.z);
+        const float nND = fmaxf(lMM + ta.z, lND + tb.z);
         // inactive lanes (rows past the query) carry LOG0 query transitions:
         // their MM stays 0 and never beats a maximum
         const bool inm = !CHECK || (j >= 0 && j < L);
@@ -566,64 +614,46 @@ __device__ __forceinline__ bool p1_take(const P1Args& a, int nstrips, int lane, 
 // 4 ldb on; ldb a multiple of 4 columns, the buffer 16-byte aligned.  Each
 // half is thus one wide store or asynchronous copy per chunk.
 
-// A chunk is C columns (32: the FP32 kernel, 8: the tensor-core kernel).
-
-// Wait (split pairs only) until columns [c0, c0 + C) of the row above strip s
+// Wait (split pairs only) until columns [c0, c0 + P1_C) of the row above strip s
 // are there; false: no such row
-template <int C>
 __device__ __forceinline__ bool p1_row_ready(const P1Args& a, const P1Item& it, int s, int c0, int lane, bool& broken)
 {
     const bool have = s > 0 && c0 < it.L;
     if (have && it.pi >= 0)
-        pipe_wait(a.sprog + (long long)(s - 1) * a.nsplit + it.pi, min(c0 + C, it.L), lane, a.status, broken, a.spin);
+        pipe_wait(a.sprog + (long long)(s - 1) * a.nsplit + it.pi, min(c0 + P1_C, it.L), lane, a.status, broken, a.spin);
     return have;
 }
 
-// The row above strip s, columns [c0, c0 + C), into the warp's shared row by
+// The row above strip s, columns [c0, c0 + P1_C), into the warp's shared row by
 // asynchronous copies through L2 (a split pair's row comes from another SM);
 // zeros where there is none.  Commits one group.  Columns past the matrix hold
 // whatever the buffer does: no cell inside the matrix reads them.
-template <int C>
 __device__ __forceinline__ void p1_row_async(const P1Args& a, const P1Item& it, int s, float* bnd,
                                              const float* __restrict__ botr, int ldb, int c0, int lane, bool& broken)
 {
-    if (p1_row_ready<C>(a, it, s, c0, lane, broken)) {
-        const int c = c0 + lane, c4 = c0 + 4 * (lane - C);
-        if (lane < C) {
+    if (p1_row_ready(a, it, s, c0, lane, broken)) {
+        const int c = c0 + lane, c4 = c0 + 4 * (lane - P1_C);
+        if (lane < P1_C) {
             if (c < it.L) cp_async16(bnd + 4 * lane, botr + 4 * c);
-        } else if (lane < C + C / 4 && c4 < it.L) {
-            cp_async16(bnd + 4 * C + 4 * (lane - C), botr + 4 * ldb + c4);
+        } else if (lane < P1_C + P1_C / 4 && c4 < it.L) {
+            cp_async16(bnd + 4 * P1_C + 4 * (lane - P1_C), botr + 4 * ldb + c4);
         }
-    } else if (lane < C) {
+    } else if (lane < P1_C) {
         *reinterpret_cast<float4*>(bnd + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
-        bnd[4 * C + lane] = 0.f;
+        bnd[4 * P1_C + lane] = 0.f;
     }
     cp_async_commit();
 }
 
-// The same into registers (C = 32; lane i: column c0 + i)
-__device__ __forceinline__ void p1_row_load(const P1Args& a, const P1Item& it, int s, const float* __restrict__ botr,
-                                            int ldb, int c0, int lane, bool& broken, float4& v, float& nd)
-{
-    const int c = c0 + lane;
-    v = make_float4(0.f, 0.f, 0.f, 0.f);
-    nd = 0.f;
-    if (p1_row_ready<32>(a, it, s, c0, lane, broken) && c < it.L) {
-        v = __ldcg(reinterpret_cast<const float4*>(botr) + c);
-        nd = __ldcg(botr + 4 * ldb + c);
-    }
-}
-
-// The strip's last row after a DP stage over [k0, k0 + C): slot l of bnd holds
+// The strip's last row after a DP stage over [k0, k0 + P1_C): slot l of bnd holds
 // lane 31's states at column k0 - 31 + l
-template <int C>
 __device__ __forceinline__ void p1_row_flush(const float* __restrict__ bnd, float* __restrict__ botw, int ldb, int k0,
                                              int L, int lane)
 {
     const int c = k0 - 31 + lane;
-    if (lane < C && c >= 0 && c < L) {
+    if (lane < P1_C && c >= 0 && c < L) {
         reinterpret_cast<float4*>(botw)[c] = *reinterpret_cast<const float4*>(bnd + lane * 4);
-        botw[4 * ldb + c] = bnd[4 * C + lane];
+        botw[4 * ldb + c] = bnd[4 * P1_C + lane];
     }
 }
 
@@ -676,28 +706,157 @@ __device__ __forceinline__ void p1_result(const P1Args& a, const P1Item& it, int
     __syncwarp();
 }
 
+// One lane of the wavefront DP with two query rows (2 t and 2 t + 1 of the
+// strip): row 0 takes its "up" states from row 1 of lane t - 1 by shuffle, row
+// 1 from row 0 of this lane at the same step.  Against one row a lane
+// (WfLane), a step's shuffles, record reads and row-above selects serve two
+// cells, and its two chains overlap; each cell's arithmetic is the same.
+struct Wf2 {
+    float MM[2], MI[2], IM[2], DN[2], ND[2];   // states at the previous step (left)
+    float A[2], Y[2], z[2];                    // up-sums of the previous step (WfLane)
+    float qMM[2], qDM[2], qIM[2], qMD[2], qDD[2], qMI[2], qII[2];
+    float best;      // the lane's maximum, its row (0, 1) and step
+    int brow, kbest;
+};
+
+// Diagonal sums and left states of column -1 for the lane's two rows
+struct Wf2Edge {
+    float A[2], Y[2], z[2], IM[2], ND[2];
+};
+
+__device__ __forceinline__ void wf2_init(Wf2& D, const float* __restrict__ qrec, int r0, int Lq)
+{
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int r = r0 + e;
+        const bool act = r < Lq;
+        // rows past the query carry LOG0 transitions and -inf scores: their MM stays 0
+        const float* qr = qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE + QR_TRN;
+        D.qMM[e] = act ? qr[TMM] : LOG0; D.qMI[e] = act ? qr[TMI] : LOG0; D.qMD[e] = act ? qr[TMD] : LOG0;
+        D.qIM[e] = act ? qr[TIM] : LOG0; D.qII[e] = act ? qr[TII] : LOG0; D.qDM[e] = act ? qr[TDM] : LOG0;
+        D.qDD[e] = act ? qr[TDD] : LOG0;
+        D.MM[e] = D.MI[e] = D.IM[e] = D.DN[e] = D.ND[e] = 0.f;
+        D.A[e] = D.Y[e] = D.z[e] = 0.f;
+    }
+    D.best = 0.f;
+    D.brow = D.kbest = 0;
+}
+
+__device__ __forceinline__ void wf2_edge(Wf2Edge& E, const Wf2& D, const float* __restrict__ qrec, int r0, int Lq)
+{
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int r = r0 + e, b = r & 31;
+        const float* qr = qrec + (long long)min(r, Lq - 1) * QR_STRIDE;
+        const bool zl = b == 31, zd = b == 31 || b == 0;
+        E.IM[e] = zl ? 0.f : qr[QR_C + 1];
+        E.ND[e] = zl ? 0.f : LOG0;
+        const float dMI = zd ? 0.f : qr[QR_CP + 0], dIM = zd ? 0.f : qr[QR_CP + 1], dDN = zd ? 0.f : qr[QR_CP + 2];
+        const float dND = zd ? 0.f : LOG0;
+        E.A[e] = max3f(0.f + D.qMM[e], dIM + D.qIM[e], dDN + D.qDM[e]);
+        E.Y[e] = dMI + D.qMM[e];
+        E.z[e] = dND + D.qMM[e];
+    }
+}
+
+// Four wavefront steps: rp the lane's scores (P1_RLD floats a step), tc its
+// column records, bnd the row above (row: slots u0..), j0 the lane's column at
+// the first step, k0 that step.  HEAD: column 0 may be among the steps (the
+// first P1T_HEAD chunks of a strip).  Cells outside the matrix have scores of
+// -inf, so their MM stays 0, and their other states reach no cell inside.
+template <bool HEAD>
+__device__ __forceinline__ void wf2_steps4(Wf2& D, const Wf2Edge& E, const float* __restrict__ rp,
+                                           const float* __restrict__ tc, float* __restrict__ bnd, int u0, int j0, int k0,
+                                           int lane, bool wr_bot)
+{
+    float m[2][4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const float2 S = *reinterpret_cast<const float2*>(rp + u * P1_RLD);
+        const float4 ta = *reinterpret_cast<const float4*>(tc + u * P1C_TRS);       // MM MI MD IM
+        const float4 tb = *reinterpret_cast<const float4*>(tc + u * P1C_TRS + 4);   // II DM DD
+        float uMM = __shfl_up_sync(FULL, D.MM[1], 1);
+        float uMI = __shfl_up_sync(FULL, D.MI[1], 1);
+        float uIM = __shfl_up_sync(FULL, D.IM[1], 1);
+        float uDN = __shfl_up_sync(FULL, D.DN[1], 1);
+        float uND = __shfl_up_sync(FULL, D.ND[1], 1);
+        {
+            const float4 ba = *reinterpret_cast<const float4*>(bnd + 4 * (u0 + u));
+            const float b4 = bnd[4 * P1_C + u0 + u];
+            if (lane == 0) { uMM = ba.x; uMI = ba.y; uIM = ba.z; uDN = ba.w; uND = b4; }
+        }
+        const bool first = HEAD && j0 + u == 0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            float Ad = D.A[e], Yd = D.Y[e], zd = D.z[e], lMM = D.MM[e], lIM = D.IM[e], lND = D.ND[e];
+            if (first) { Ad = E.A[e]; Yd = E.Y[e]; zd = E.z[e]; lMM = 0.f; lIM = E.IM[e]; lND = E.ND[e]; }
+            const float X = uMM + D.qMM[e], Y = uMI + D.qMM[e];
+            D.A[e] = max3f(X, uIM + D.qIM[e], uDN + D.qDM[e]);
+            D.Y[e] = Y;
+            D.z[e] = uND + D.qMM[e];
+            const float v = max3f(Ad + ta.x, Yd + ta.w, zd + tb.y);
+            const float nMM = fmaxf(v + (e ? S.y : S.x), 0.f);
+            const float nMI = fmaxf(X + ta.y, Y + tb.x);
+            const float nIM = fmaxf(lMM + D.qMI[e], lIM + D.qII[e]) + ta.x;
+            const float nDN = fmaxf(uMM + D.qMD[e], uDN + D.qDD[e]);
+            const float nND = fmaxf(lMM + ta.z, lND + tb.z);
+            D.MM[e] = nMM; D.MI[e] = nMI; D.IM[e] = nIM; D.DN[e] = nDN; D.ND[e] = nND;
+            m[e][u] = nMM;
+            // row 1's "up" is this cell
+            uMM = nMM; uMI = nMI; uIM = nIM; uDN = nDN; uND = nND;
+        }
+        if (wr_bot) {
+            // lane 31's row 1 (column k0 + u - 31) into the slot lane 0 read at the top of this step
+            *reinterpret_cast<float4*>(bnd + 4 * (u0 + u)) = make_float4(uMM, uMI, uIM, uDN);
+            bnd[4 * P1_C + u0 + u] = uND;
+        }
+    }
+    // the maximum of the eight cells first (4 three-input maxima); its cell
+    // only when it reaches the lane's maximum, which a lane rarely does
+    // (a compare and two selects per cell otherwise)
+    const float cm = max3f(max3f(m[0][0], m[0][1], m[0][2]), max3f(m[0][3], m[1][0], m[1][1]), fmaxf(m[1][2], m[1][3]));
+    if (cm >= D.best && cm > 0.f) {
+        int row = 1, uu = 0;
+#pragma unroll
+        for (int i = 7; i >= 0; i--)
+            if (m[i >> 2][i & 3] == cm) { row = i >> 2; uu = i & 3; }
+        // a tie goes to the smaller row, then to the earlier column
+        if (cm > D.best || row < D.brow) { D.best = cm; D.brow = row; D.kbest = k0 + uu; }
+    }
+}
+
+// Phase 1 in FP32.  Per chunk of 8 columns every lane first scores its two
+// rows against them (db records staged in shared memory by cp.async and read
+// warp-uniformly, once for both rows; the cells are independent, so their
+// chains overlap), then the warp advances the wavefront by 8 steps.  Bound by
+// instruction issue: two rows a lane halve the record reads and the DP's
+// shuffles, column and row-above reads per cell, and the packed dot products
+// halve the multiply-adds' issue slots.
 __global__ void __launch_bounds__(P1C_WARPS * 32, 1)
 p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int cvcard = a.sc.cvcard;
     const int card = a.sc.ssss_card;
     float* cvtab = smem;                                      // [cvcard][P1C_CVREP]
     float* wb = smem + cvcard * P1C_CVREP + wid * P1C_WARP_FLOATS;
-    float* ring = wb;                                         // [P1C_RING][32] scores
-    float* trn = ring + P1C_RING * 32;                        // [P1C_RING][P1C_TRS] transitions
-    float* U = trn + P1C_RING * P1C_TRS;                      // [card][32]
-    float* rec = U + MAX_SSSS_CARD * 32;                      // [REC_SLOTS][DR_STRIDE] db records
-    float* bnd = rec + REC_SLOTS * DR_STRIDE;                 // [BND_FLOATS] row above the strip
+    float* ring = wb;                                         // [P1_SLOTS anti-diagonals][P1_RLD] scores
+    float* cring = ring + P1_SLOTS * P1_RLD;                  // [P1_CRING][P1C_TRS] column transitions
+    float* bnd = cring + P1_CRING * P1C_TRS;                  // [P1_BND] row above the strip
+    float* U = bnd + P1_BND;                                  // [card][P1_ROWS] SS row table
+    float* rec = U + MAX_SSSS_CARD * P1_ROWS;                 // [REC_SLOTS][DR_STRIDE] db records
     for (int i = threadIdx.x; i < cvcard * P1C_CVREP; i += blockDim.x) cvtab[i] = a.cvvals[i / P1C_CVREP];
+    // (a lane may read a score slot or record that no chunk has filled yet;
+    // such a value reaches no cell inside the matrix, but start from zeros)
+    for (int i = lane; i < P1C_WARP_FLOATS; i += 32) wb[i] = 0.f;
     __syncthreads();
 
     const long long slotw = (long long)blockIdx.x * P1C_WARPS + wid;
     const int Lmax = (int)(a.botstride / 10);
     float* bot0 = a.bot + slotw * a.botstride;
     const int Lq = a.Lq;
-    const int nstrips = (Lq + 31) >> 5;
+    const int nstrips = (Lq + P1_ROWS - 1) / P1_ROWS, ns32 = (Lq + 31) >> 5;
     const ScoreConsts sc = a.sc;
 
     bool broken = false;   // a strip wait gave up
@@ -705,8 +864,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
         P1Item it;
         if (!p1_take(a, nstrips, lane, it)) break;
         const int p = it.p, L = it.L;
-        const long long off = a.poff[p];
-        const float* __restrict__ dr = a.drec + off * DR_STRIDE;
+        const float* __restrict__ dr = a.drec + a.poff[p] * DR_STRIDE;
         const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
         const int edge = corner_edge(Lq, L);
         // rows between the strips: the warp's own buffer, or the split pair's
@@ -718,97 +876,111 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
         int prow = 0x7fffffff, pcol = 0x7fffffff;
 
         for (int s = it.s0; s < it.s1; s++) {
-            const int r = s * 32 + lane;
-            const bool act = r < Lq;
-            const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
-            RowOps R;
-#pragma unroll
-            for (int i = 0; i < NAA; i++)
-                R.Qt[i] = __fdividef(qr[QR_TRG + i], 0.5f * (qbkg[i] + bd[i]));
-#pragma unroll
-            for (int i = 0; i < NCV; i++) R.qcv[i] = qr[QR_CV + i];
-            R.cq = qr[QR_CN];
-            R.pq = qr[QR_PRIOR];
-            R.hq = qr[QR_HQ];
-            {
-                // this strip's SS row tables (built once per query, c2_set_query)
-                const float* __restrict__ us = a.qU + (long long)s * MAX_SSSS_CARD * 32 + lane;
-#pragma unroll 8
-                for (int c = 0; c < card; c++) U[c * 32 + lane] = __ldg(us + c * 32);
-            }
-            WfLane D;
-            float q7[7];
-#pragma unroll
-            for (int i = 0; i < 7; i++) q7[i] = act ? qr[QR_TRN + i] : LOG0;
-            // column -1 boundary states of this row and of the row above
-            const bool z_left = (lane == 31);
-            const bool z_diag = (lane == 31 || lane == 0);
-            const St5 LB = z_left ? St5{0.f, 0.f, 0.f, 0.f, 0.f}
-                                  : St5{0.f, qr[QR_C + 0], qr[QR_C + 1], qr[QR_C + 2], LOG0};
-            const St5 DB = z_diag ? St5{0.f, 0.f, 0.f, 0.f, 0.f}
-                                  : St5{0.f, qr[QR_CP + 0], qr[QR_CP + 1], qr[QR_CP + 2], LOG0};
-            // corner cells of this row: j <= cA or j >= cB
-            const int cA = corner_a(r, Lq, edge);
-            const int cB = corner_b(r, L, edge);
-            wf_init(D, q7, LB, DB);
-            const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             __syncwarp();
+            const int r0 = P1_ROWS * s + 2 * lane;   // the lane's first row
+            RowOps R[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) row_ops(R[e], a.qrec + (long long)min(r0 + e, Lq - 1) * QR_STRIDE, qbkg, bd);
+            {
+                // this strip's SS row tables (built once per query in strips of
+                // 32 rows, c2_set_query); lanes past the query's last 32 rows
+                // repeat them (their cells never score)
+                const int t = min(2 * s + (lane >> 4), ns32 - 1);
+                const float* __restrict__ us = a.qU + (long long)t * MAX_SSSS_CARD * 32 + 2 * (lane & 15);
+#pragma unroll 8
+                for (int c = 0; c < card; c++)
+                    *reinterpret_cast<float2*>(U + c * P1_ROWS + 2 * lane) =
+                        __ldg(reinterpret_cast<const float2*>(us + c * 32));
+            }
+            // scores of -inf for the cells left of the matrix (step k < lane)
+#pragma unroll 4
+            for (int k = 0; k < 31; k++)
+                if (k < lane)
+                    *reinterpret_cast<float2*>(ring + k * P1_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
+            Wf2 D;
+            wf2_init(D, a.qrec, r0, Lq);
+            // corner cells of the lane's rows: columns <= cA or >= cB
+            const int cA0 = corner_a(r0, Lq, edge), cA1 = corner_a(r0 + 1, Lq, edge);
+            const int cB0 = corner_b(r0, L, edge), cB1 = corner_b(r0 + 1, L, edge);
+            const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
+            // records and transitions of the first two chunks
             stage_chunk(rec, dr, 0, L, lane);
+            stage_trn(cring, dr, 0, 0, L, lane);
+            cp_async_commit();
             stage_chunk(rec, dr, 1, L, lane);
-            const int nch = (L + 31) >> 5;        // chunks holding columns
-            const int kend = L + 31;              // wavefront steps of the strip
-            for (int m = 0; 32 * m < kend; m++) {
-                // the row above for this chunk's steps, loaded during the score stage
-                float4 row;
-                float rownd;
-                p1_row_load(a, it, s, botr, ldb, 32 * m, lane, broken, row, rownd);
-                // ---- score stage: columns [32m, min(32m + 32, L))
-                if (m < nch) {
-                    const int c0 = 32 * m, c1 = min(c0 + 32, L);
-                    // does any row of the strip have corner cells in this chunk?
-                    const bool hasc = __any_sync(FULL, cA >= c0 || cB < c1);
-                    for (int c = c0; c < c1; c++) {
-                        if ((c & (REC_CHUNK - 1)) == 0) {
-                            cp_async_wait_1();
-                            __syncwarp();
+            stage_trn(cring, dr, 1, P1_C, L, lane);
+            cp_async_commit();
+            int sg = 0;                                 // slot of the chunk's first anti-diagonal
+            int cs = 0, cl = lane == 0 ? 0 : P1_CMOD - lane;
+            for (int m = 0; P1_C * m < L + 31; m++) {
+                const int k0 = P1_C * m;
+                // the row above for this chunk's steps, copied during the score stage
+                p1_row_async(a, it, s, bnd, botr, ldb, k0, lane, broken);
+                cp_async_wait_2();   // records and transitions of chunk m have landed
+                __syncwarp();
+                // ---- score stage: columns [k0, k0 + 8); past the last column -inf,
+                // for the lanes still to finish the matrix
+                {
+                    int w = sg + lane;
+                    if (w >= P1_SLOTS) w -= P1_SLOTS;
+                    const float* rc = rec + (k0 & (REC_SLOTS - 1)) * DR_STRIDE;
+                    const bool hasc = __any_sync(FULL, cA1 >= k0 || cB0 < k0 + P1_C);
+#pragma unroll 2
+                    for (int u = 0; u < P1_C; u++) {
+                        float S[2] = {-INFINITY, -INFINITY};
+                        if (k0 + u < L) {
+                            float mod[2];
+                            cell_scores<P1C_CVREP, 2, P1_ROWS>(R, rc + u * DR_STRIDE, U, 2 * lane, cvtab, sc, lane, S, mod);
+                            if (hasc) {
+                                const int c = k0 + u;
+                                if (c <= cA0 || c >= cB0) S[0] = -9.f;
+                                if (c <= cA1 || c >= cB1) S[1] = -9.f;
+                            }
                         }
-                        const float* rc = rec + (c & (REC_SLOTS - 1)) * DR_STRIDE;
-                        float mod;
-                        float Sc = cell_score<P1C_CVREP>(R, reinterpret_cast<const float4*>(rc), U, cvtab, sc, lane, mod);
-                        (void)mod;
-                        if (hasc && (c <= cA || c >= cB)) Sc = -9.f;
-                        ring[((c + lane) & (P1C_RING - 1)) * 32 + lane] = Sc;
-                        if (lane < DPT_N) trn[(c & (P1C_RING - 1)) * P1C_TRS + lane] = rc[DR_TRN + dpt_src(lane)];
-                        if ((c & (REC_CHUNK - 1)) == REC_CHUNK - 1) {
-                            // group fully read by every lane: refill its slots two groups ahead
-                            __syncwarp();
-                            stage_chunk(rec, dr, (c >> REC_CHUNK_LOG) + 2, L, lane);
-                        }
+                        *reinterpret_cast<float2*>(ring + w * P1_RLD + 2 * lane) = make_float2(S[0], S[1]);
+                        if (++w >= P1_SLOTS) w = 0;
                     }
                 }
-                bnd_put(bnd, lane, row.x, row.y, row.z, row.w, rownd);
+                cp_async_wait_all();
                 __syncwarp();
-                // ---- DP stage: wavefront steps [32m, 32m + 32)
-                const int k0 = 32 * m, k1 = min(k0 + 32, kend);
-                if (m >= 1 && k0 + 31 < L && k1 == k0 + 32)
-                    wf_steps<false>(D, k0, 32, lane, L, act, ring, trn, bnd, wr_bot);
-                else
-                    wf_steps<true>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot);
+                // ---- DP stage: wavefront steps [k0, k0 + 8)
+                const float* rp = ring + sg * P1_RLD + 2 * lane;
+                const float* tcol = cring + cl * P1C_TRS;
+                if (k0 < 32) {
+                    Wf2Edge E;
+                    wf2_edge(E, D, a.qrec, r0, Lq);
+#pragma unroll 1
+                    for (int u0 = 0; u0 < P1_C; u0 += 4)
+                        wf2_steps4<true>(D, E, rp + u0 * P1_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
+                                         lane, wr_bot);
+                } else {
+                    Wf2Edge E;
+#pragma unroll 1
+                    for (int u0 = 0; u0 < P1_C; u0 += 4)
+                        wf2_steps4<false>(D, E, rp + u0 * P1_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
+                                          lane, wr_bot);
+                }
                 __syncwarp();
                 if (s + 1 < nstrips) {
-                    p1_row_flush<32>(bnd, botw, ldb, k0, L, lane);
-                    if (it.pi >= 0) p1_publish(a, it, s, min(k1 - 31, L), lane);
+                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
+                    // columns up to k0 - 24 are there: published every other chunk
+                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= L + 31))
+                        p1_publish(a, it, s, min(k0 - 23, L), lane);
                 }
+                // next chunk; chunk m + 2's records and transitions into slots no longer read
+                sg = sg + P1_C >= P1_SLOTS ? 0 : sg + P1_C;
+                cs = cs + P1_C >= P1_CMOD ? 0 : cs + P1_C;
+                cl = cl + P1_C >= P1_CMOD ? cl + P1_C - P1_CMOD : cl + P1_C;
+                stage_chunk(rec, dr, m + 2, L, lane);
+                stage_trn(cring, dr, m + 2, cs + P1_C >= P1_CMOD ? 0 : cs + P1_C, L, lane);
+                cp_async_commit();
                 __syncwarp();
             }
             cp_async_wait_all();
-            // this strip's maximum: largest score, then smallest row, then smallest column
             {
-                float b = D.best;
-                int rr = (D.best > 0.f) ? r : 0x7fffffff;
-                int cc = (D.best > 0.f) ? D.kbest - lane : 0x7fffffff;
-                if (b > pbest || (b == pbest && (rr < prow || (rr == prow && cc < pcol)))) {
-                    pbest = b; prow = rr; pcol = cc;
+                const int rr = r0 + D.brow, cc = D.kbest - lane;
+                if (D.best > 0.f && (D.best > pbest || (D.best == pbest && (rr < prow || (rr == prow && cc < pcol))))) {
+                    pbest = D.best; prow = rr; pcol = cc;
                 }
             }
             float* t = botr; botr = botw; botw = t;
@@ -869,14 +1041,7 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
         const bool act = r < Lq;
         const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
         RowOps R;
-#pragma unroll
-        for (int i = 0; i < NAA; i++)
-            R.Qt[i] = __fdividef(qr[QR_TRG + i], 0.5f * (qbkg[i] + bd[i]));
-#pragma unroll
-        for (int i = 0; i < NCV; i++) R.qcv[i] = qr[QR_CV + i];
-        R.cq = qr[QR_CN];
-        R.pq = qr[QR_PRIOR];
-        R.hq = qr[QR_HQ];
+        row_ops(R, qr, qbkg, bd);
         __syncwarp();
         {
             // this strip's SS row tables (built once per query, c2_set_query)
@@ -885,7 +1050,9 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
             for (int c = 0; c < card; c++) U[c * 32 + lane] = __ldg(us + c * 32);
         }
         stage_chunk(rec, dr, 0, L, lane);
+        cp_async_commit();
         stage_chunk(rec, dr, 1, L, lane);
+        cp_async_commit();
         // a staged chunk of REC_CHUNK columns at a time: its cells are
         // independent, so their chains overlap
         for (int c0 = 0; c0 < L; c0 += REC_CHUNK) {
@@ -896,9 +1063,8 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
                 const int c = c0 + u;
                 if (c < L) {
                     const float* rc = rec + (c & (REC_SLOTS - 1)) * DR_STRIDE;
-                    float mod;
-                    const float Sc =
-                        cell_score<P1TC_CVREP>(R, reinterpret_cast<const float4*>(rc), U, cvtab, sc, lane, mod);
+                    float mod, Sc;
+                    cell_scores<P1TC_CVREP, 1, 32>(&R, rc, U, lane, cvtab, sc, lane, &Sc, &mod);
                     if (act) {
                         smt[(long long)c * Lq + r] = Sc;
                         mmt[(long long)c * Lq + r] = mod;
@@ -907,6 +1073,7 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
             }
             __syncwarp();
             stage_chunk(rec, dr, (c0 >> REC_CHUNK_LOG) + 2, L, lane);
+            cp_async_commit();
         }
         cp_async_wait_all();
         __syncwarp();
@@ -995,8 +1162,8 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
                     float Sc = act ? __ldcg(smt + (long long)c * Lq + r) : 0.f;
                     if (hasc && (c <= cA || c >= cB)) Sc = -9.f;
                     ring[((c + lane) & (P1C_RING - 1)) * 32 + lane] = Sc;
-                    if (lane < DPT_N)
-                        trn[(c & (P1C_RING - 1)) * P1C_TRS + lane] = __ldg(dr + (long long)c * DR_STRIDE + DR_TRN + dpt_src(lane));
+                    if (lane < 7)
+                        trn[(c & (P1C_RING - 1)) * P1C_TRS + lane] = __ldg(dr + (long long)c * DR_STRIDE + DR_TRN + lane);
                 }
             }
             // the row above for chunk m + 1, loaded while this stage runs
@@ -1199,10 +1366,10 @@ __global__ void __launch_bounds__(128) tc_pack_kernel(const float* __restrict__ 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int L = plen[p];
     const long long off = poff[p];
-    const int ntiles = (L + P1T_C - 1) / P1T_C;
+    const int ntiles = (L + P1_C - 1) / P1_C;
     const int g = lane >> 2, q = lane & 3;
     for (int t = wid; t < ntiles; t += 4) {
-        const int col = P1T_C * t + g;
+        const int col = P1_C * t + g;
         const bool valid = col < L;
         const float* rc = drec + (off + (valid ? col : 0)) * DR_STRIDE;
         const int pk = __float_as_int(rc[DR_SSIDX]);
@@ -1244,7 +1411,7 @@ __global__ void __launch_bounds__(128) tc_pack_kernel(const float* __restrict__ 
         const float* rc = drec + (off + c) * DR_STRIDE;
         float* o = cold + (off + c) * P1C_TRS;
 #pragma unroll
-        for (int i = 0; i < DPT_N; i++) o[i] = rc[DR_TRN + dpt_src(i)];
+        for (int i = 0; i < 7; i++) o[i] = rc[DR_TRN + i];
         o[7] = 0.f;
         o[CO_CD] = rc[DR_CN];
         o[CO_PD2] = 2.f * rc[DR_PRIOR];
@@ -1289,134 +1456,15 @@ __device__ __forceinline__ float tc_cell(float daa, float dot, float ss, float c
     return fmaf(lg2_ftz(daa), C2_LN2, ss + cvm);
 }
 
-// One lane of the wavefront DP with two query rows (2 t and 2 t + 1 of the
-// strip): row 0 takes its "up" states from row 1 of lane t - 1 by shuffle, row
-// 1 from row 0 of this lane at the same step.  Against one row a lane
-// (WfLane), a step's shuffles, record reads and row-above selects serve two
-// cells, and its two chains overlap; each cell's arithmetic is the same.
-struct Wf2 {
-    float MM[2], MI[2], IM[2], DN[2], ND[2];   // states at the previous step (left)
-    float A[2], Y[2], z[2];                    // up-sums of the previous step (WfLane)
-    float qMM[2], qDM[2], qIM[2], qMD[2], qDD[2], qMI[2], qII[2];
-    float best;      // the lane's maximum, its row (0, 1) and step
-    int brow, kbest;
-};
-
-// Diagonal sums and left states of column -1 for the lane's two rows
-struct Wf2Edge {
-    float A[2], Y[2], z[2], IM[2], ND[2];
-};
-
-__device__ __forceinline__ void wf2_init(Wf2& D, const float* __restrict__ qrec, int r0, int Lq)
-{
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-        const int r = r0 + e;
-        const bool act = r < Lq;
-        // rows past the query carry LOG0 transitions and -inf scores: their MM stays 0
-        const float* qr = qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE + QR_TRN;
-        D.qMM[e] = act ? qr[TMM] : LOG0; D.qMI[e] = act ? qr[TMI] : LOG0; D.qMD[e] = act ? qr[TMD] : LOG0;
-        D.qIM[e] = act ? qr[TIM] : LOG0; D.qII[e] = act ? qr[TII] : LOG0; D.qDM[e] = act ? qr[TDM] : LOG0;
-        D.qDD[e] = act ? qr[TDD] : LOG0;
-        D.MM[e] = D.MI[e] = D.IM[e] = D.DN[e] = D.ND[e] = 0.f;
-        D.A[e] = D.Y[e] = D.z[e] = 0.f;
-    }
-    D.best = 0.f;
-    D.brow = D.kbest = 0;
-}
-
-__device__ __forceinline__ void wf2_edge(Wf2Edge& E, const Wf2& D, const float* __restrict__ qrec, int r0, int Lq)
-{
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-        const int r = r0 + e, b = r & 31;
-        const float* qr = qrec + (long long)min(r, Lq - 1) * QR_STRIDE;
-        const bool zl = b == 31, zd = b == 31 || b == 0;
-        E.IM[e] = zl ? 0.f : qr[QR_C + 1];
-        E.ND[e] = zl ? 0.f : LOG0;
-        const float dMI = zd ? 0.f : qr[QR_CP + 0], dIM = zd ? 0.f : qr[QR_CP + 1], dDN = zd ? 0.f : qr[QR_CP + 2];
-        const float dND = zd ? 0.f : LOG0;
-        E.A[e] = max3f(0.f + D.qMM[e], dIM + D.qIM[e], dDN + D.qDM[e]);
-        E.Y[e] = dMI + D.qMM[e];
-        E.z[e] = dND + D.qMM[e];
-    }
-}
-
-// Four wavefront steps: rp the lane's scores (P1T_RLD floats a step), tc its
-// column records, bnd the row above (row: slots u0..), j0 the lane's column at
-// the first step, k0 that step.  HEAD: column 0 may be among the steps (the
-// first P1T_HEAD chunks of a strip).  Cells outside the matrix have scores of
-// -inf, so their MM stays 0, and their other states reach no cell inside.
-template <bool HEAD>
-__device__ __forceinline__ void wf2_steps4(Wf2& D, const Wf2Edge& E, const float* __restrict__ rp,
-                                           const float* __restrict__ tc, float* __restrict__ bnd, int u0, int j0, int k0,
-                                           int lane, bool wr_bot)
-{
-    float m[2][4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const float2 S = *reinterpret_cast<const float2*>(rp + u * P1T_RLD);
-        const float4 ta = *reinterpret_cast<const float4*>(tc + u * P1C_TRS);       // MM IM DM MI
-        const float4 tb = *reinterpret_cast<const float4*>(tc + u * P1C_TRS + 4);   // II MD DD
-        float uMM = __shfl_up_sync(FULL, D.MM[1], 1);
-        float uMI = __shfl_up_sync(FULL, D.MI[1], 1);
-        float uIM = __shfl_up_sync(FULL, D.IM[1], 1);
-        float uDN = __shfl_up_sync(FULL, D.DN[1], 1);
-        float uND = __shfl_up_sync(FULL, D.ND[1], 1);
-        {
-            const float4 ba = *reinterpret_cast<const float4*>(bnd + 4 * (u0 + u));
-            const float b4 = bnd[4 * P1T_C + u0 + u];
-            if (lane == 0) { uMM = ba.x; uMI = ba.y; uIM = ba.z; uDN = ba.w; uND = b4; }
-        }
-        const bool first = HEAD && j0 + u == 0;
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            float Ad = D.A[e], Yd = D.Y[e], zd = D.z[e], lMM = D.MM[e], lIM = D.IM[e], lND = D.ND[e];
-            if (first) { Ad = E.A[e]; Yd = E.Y[e]; zd = E.z[e]; lMM = 0.f; lIM = E.IM[e]; lND = E.ND[e]; }
-            const float X = uMM + D.qMM[e], Y = uMI + D.qMM[e];
-            D.A[e] = max3f(X, uIM + D.qIM[e], uDN + D.qDM[e]);
-            D.Y[e] = Y;
-            D.z[e] = uND + D.qMM[e];
-            const float v = max3f(Ad + ta.x, Yd + ta.y, zd + ta.z);
-            const float nMM = fmaxf(v + (e ? S.y : S.x), 0.f);
-            const float nMI = fmaxf(X + ta.w, Y + tb.x);
-            const float nIM = fmaxf(lMM + D.qMI[e], lIM + D.qII[e]) + ta.x;
-            const float nDN = fmaxf(uMM + D.qMD[e], uDN + D.qDD[e]);
-            const float nND = fmaxf(lMM + tb.y, lND + tb.z);
-            D.MM[e] = nMM; D.MI[e] = nMI; D.IM[e] = nIM; D.DN[e] = nDN; D.ND[e] = nND;
-            m[e][u] = nMM;
-            // row 1's "up" is this cell
-            uMM = nMM; uMI = nMI; uIM = nIM; uDN = nDN; uND = nND;
-        }
-        if (wr_bot) {
-            // lane 31's row 1 (column k0 + u - 31) into the slot lane 0 read at the top of this step
-            *reinterpret_cast<float4*>(bnd + 4 * (u0 + u)) = make_float4(uMM, uMI, uIM, uDN);
-            bnd[4 * P1T_C + u0 + u] = uND;
-        }
-    }
-    // the maximum of the eight cells first (4 three-input maxima); its cell
-    // only when it reaches the lane's maximum, which a lane rarely does
-    // (a compare and two selects per cell otherwise)
-    const float cm = max3f(max3f(m[0][0], m[0][1], m[0][2]), max3f(m[0][3], m[1][0], m[1][1]), fmaxf(m[1][2], m[1][3]));
-    if (cm >= D.best && cm > 0.f) {
-        int row = 1, uu = 0;
-#pragma unroll
-        for (int i = 7; i >= 0; i--)
-            if (m[i >> 2][i & 3] == cm) { row = i >> 2; uu = i & 3; }
-        // a tie goes to the smaller row, then to the earlier column
-        if (cm > D.best || row < D.brow) { D.best = cm; D.brow = row; D.kbest = k0 + uu; }
-    }
-}
-
 // Stage the column records of chunk m (8 columns, ring slots from cs on; the
 // chunk at slot 0 also into the mirror slots after the last chunk)
 __device__ __forceinline__ void stage_cols(float* cring, const float* __restrict__ cold, int m, int cs, int L, int lane)
 {
-    const int n16 = min(P1T_C, L - P1T_C * m) * (P1C_TRS / 4);
+    const int n16 = min(P1_C, L - P1_C * m) * (P1C_TRS / 4);
     if (lane < n16) {
-        const float* src = cold + (long long)(P1T_C * m) * P1C_TRS + 4 * lane;
+        const float* src = cold + (long long)(P1_C * m) * P1C_TRS + 4 * lane;
         cp_async16(cring + cs * P1C_TRS + 4 * lane, src);
-        if (cs == 0) cp_async16(cring + P1T_CMOD * P1C_TRS + 4 * lane, src);
+        if (cs == 0) cp_async16(cring + P1_CMOD * P1C_TRS + 4 * lane, src);
     }
     cp_async_commit();
 }
@@ -1436,11 +1484,11 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
     const int cvcard = a.sc.cvcard;
     float* cvtab = smem;                                      // [cvcard][P1T_CVREP], x CV weight
     float* wb = smem + cvcard * P1T_CVREP + wid * P1T_WARP_FLOATS;
-    float* ring = wb;                                         // [P1T_SLOTS anti-diagonals][P1T_RLD] scores
-    float* cring = ring + P1T_SLOTS * P1T_RLD;                // [P1T_CRING][P1C_TRS] column records
-    float* bnd = cring + P1T_CRING * P1C_TRS;                 // [P1T_BND] row above the strip
-    float* rqt = bnd + P1T_BND;                               // [P1T_ROWS][2] cvnorm, c2 - 2 x CV log prior
-    unsigned* btile = reinterpret_cast<unsigned*>(rqt + 2 * P1T_ROWS);   // [TC_TILE_WORDS] db operand tile
+    float* ring = wb;                                         // [P1_SLOTS anti-diagonals][P1_RLD] scores
+    float* cring = ring + P1_SLOTS * P1_RLD;                // [P1_CRING][P1C_TRS] column records
+    float* bnd = cring + P1_CRING * P1C_TRS;                 // [P1_BND] row above the strip
+    float* rqt = bnd + P1_BND;                               // [P1_ROWS][2] cvnorm, c2 - 2 x CV log prior
+    unsigned* btile = reinterpret_cast<unsigned*>(rqt + 2 * P1_ROWS);   // [TC_TILE_WORDS] db operand tile
     unsigned long long* tbar = reinterpret_cast<unsigned long long*>(btile + TC_TILE_WORDS);
     for (int i = threadIdx.x; i < cvcard * P1T_CVREP; i += blockDim.x)
         cvtab[i] = a.cvvals[i / P1T_CVREP] * a.sc.cvswgt - a.tc.shift;
@@ -1473,7 +1521,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
     const int Lmax = (int)(a.botstride / 10);
     float* bot0 = a.bot + slotw * a.botstride;
     const int Lq = a.Lq;
-    const int nstrips = (Lq + P1T_ROWS - 1) / P1T_ROWS;
+    const int nstrips = (Lq + P1_ROWS - 1) / P1_ROWS;
     const TcConsts tc = a.tc;
     const int g = lane >> 2, q = lane & 3;
     // this lane's CV table replica, offset so that index 0 is the table's key 0
@@ -1486,7 +1534,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int x = 2 * q + (i & 1) + 4 * (i >> 1) + (g >> 1);
-        woff[i] = (x & 7) * P1T_RLD + g + 8 * (i >> 1);
+        woff[i] = (x & 7) * P1_RLD + g + 8 * (i >> 1);
         wnext[i] = x >= 8;
     }
 
@@ -1546,7 +1594,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                 }
                 tmem_wait_st();
             }
-            const int r0 = P1T_ROWS * s + 2 * lane;   // the lane's first row
+            const int r0 = P1_ROWS * s + 2 * lane;   // the lane's first row
             {
                 // the rows' score terms, and scores of -inf for the cells left
                 // of the matrix (step k < lane)
@@ -1557,7 +1605,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
 #pragma unroll 4
                 for (int k = 0; k < 31; k++)
                     if (k < lane)
-                        *reinterpret_cast<float2*>(ring + k * P1T_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
+                        *reinterpret_cast<float2*>(ring + k * P1_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
             }
             Wf2 D;
             wf2_init(D, a.qrec, r0, Lq);
@@ -1566,8 +1614,8 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             const int cB = corner_b(r0, L, edge);
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             stage_cols(cring, cold, 0, 0, L, lane);
-            stage_cols(cring, cold, 1, P1T_C, L, lane);
-            const int nch = (L + P1T_C - 1) / P1T_C;      // chunks holding columns
+            stage_cols(cring, cold, 1, P1_C, L, lane);
+            const int nch = (L + P1_C - 1) / P1_C;      // chunks holding columns
             // db operand tiles stream through the slot, one ahead: tile m + 1
             // loads while tile m's products, epilogue and DP steps run
             if (lane == 0 && !tbroken) {
@@ -1578,12 +1626,12 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             // 0-7, 8-15, ..; the chunk's first record slot; the lane's record slot
             int sg[5];
 #pragma unroll
-            for (int i = 0; i < 5; i++) sg[i] = i * P1T_C * P1T_RLD;
-            int cs = 0, cl = lane == 0 ? 0 : P1T_CMOD - lane;
-            for (int m = 0; P1T_C * m < L + 31; m++) {
-                const int k0 = P1T_C * m;
+            for (int i = 0; i < 5; i++) sg[i] = i * P1_C * P1_RLD;
+            int cs = 0, cl = lane == 0 ? 0 : P1_CMOD - lane;
+            for (int m = 0; P1_C * m < L + 31; m++) {
+                const int k0 = P1_C * m;
                 // the row above for this chunk's steps, copied during the score stage
-                p1_row_async<P1T_C>(a, it, s, bnd, botr, ldb, k0, lane, broken);
+                p1_row_async(a, it, s, bnd, botr, ldb, k0, lane, broken);
                 if (m < nch) {
                     cp_async_wait_2();   // column records of chunk m have landed
                     if (!tbroken && !__all_sync(FULL, mbar_wait(tbar, tph))) {
@@ -1608,7 +1656,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                             asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + TC_TILE_WORDS + lane * 32));
                     }
                     // does any row of the strip have corner cells in this chunk?
-                    const bool hasc = __any_sync(FULL, cA >= k0 || cB < k0 + P1T_C);
+                    const bool hasc = __any_sync(FULL, cA >= k0 || cB < k0 + P1_C);
                     const float* cr = cring + (cs + 2 * q) * P1C_TRS + CO_CD;
                     const float2 cp0 = *reinterpret_cast<const float2*>(cr);
                     const float2 cp1 = *reinterpret_cast<const float2*>(cr + P1C_TRS);
@@ -1648,7 +1696,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                         if (hasc) {
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
-                                const int rr = P1T_ROWS * s + 16 * mt + g + 8 * (i >> 1), cc = k0 + 2 * q + (i & 1);
+                                const int rr = P1_ROWS * s + 16 * mt + g + 8 * (i >> 1), cc = k0 + 2 * q + (i & 1);
                                 // (padding columns past L and rows past the query keep -inf)
                                 if (cc < L && rr < Lq && (cc <= corner_a(rr, Lq, edge) || cc >= corner_b(rr, L, edge)))
                                     S[i] = -9.f;
@@ -1661,11 +1709,11 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                     // past the last column: scores of -inf for the lanes still
                     // to finish the matrix (the lane's rows, anti-diagonals
                     // lane .. lane + 7 past the chunk's first)
-                    int w = sg[0] / P1T_RLD + lane;
+                    int w = sg[0] / P1_RLD + lane;
 #pragma unroll
-                    for (int c = 0; c < P1T_C; c++) {
-                        if (w >= P1T_SLOTS) w -= P1T_SLOTS;
-                        *reinterpret_cast<float2*>(ring + w * P1T_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
+                    for (int c = 0; c < P1_C; c++) {
+                        if (w >= P1_SLOTS) w -= P1_SLOTS;
+                        *reinterpret_cast<float2*>(ring + w * P1_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
                         w++;
                     }
                 }
@@ -1678,21 +1726,21 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                     Wf2Edge E;
                     wf2_edge(E, D, a.qrec, r0, Lq);
 #pragma unroll 1
-                    for (int u0 = 0; u0 < P1T_C; u0 += 4)
-                        wf2_steps4<true>(D, E, rp + u0 * P1T_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
+                    for (int u0 = 0; u0 < P1_C; u0 += 4)
+                        wf2_steps4<true>(D, E, rp + u0 * P1_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
                                          lane, wr_bot);
                 } else {
                     Wf2Edge E;
 #pragma unroll 1
-                    for (int u0 = 0; u0 < P1T_C; u0 += 4)
-                        wf2_steps4<false>(D, E, rp + u0 * P1T_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
+                    for (int u0 = 0; u0 < P1_C; u0 += 4)
+                        wf2_steps4<false>(D, E, rp + u0 * P1_RLD, tcol + u0 * P1C_TRS, bnd, u0, k0 + u0 - lane, k0 + u0,
                                           lane, wr_bot);
                 }
                 __syncwarp();
                 if (s + 1 < nstrips) {
-                    p1_row_flush<P1T_C>(bnd, botw, ldb, k0, L, lane);
+                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
                     // columns up to k0 - 24 are there: published every other chunk
-                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1T_C >= L + 31))
+                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= L + 31))
                         p1_publish(a, it, s, min(k0 - 23, L), lane);
                 }
                 // next chunk: rotate the ring segments and record slots; chunk
@@ -1701,9 +1749,9 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
 #pragma unroll
                 for (int i = 0; i < 4; i++) sg[i] = sg[i + 1];
                 sg[4] = t0;
-                cs = cs + P1T_C >= P1T_CMOD ? 0 : cs + P1T_C;
-                cl = cl + P1T_C >= P1T_CMOD ? cl + P1T_C - P1T_CMOD : cl + P1T_C;
-                stage_cols(cring, cold, m + 2, cs + P1T_C >= P1T_CMOD ? 0 : cs + P1T_C, L, lane);
+                cs = cs + P1_C >= P1_CMOD ? 0 : cs + P1_C;
+                cl = cl + P1_C >= P1_CMOD ? cl + P1_C - P1_CMOD : cl + P1_C;
+                stage_cols(cring, cold, m + 2, cs + P1_C >= P1_CMOD ? 0 : cs + P1_C, L, lane);
                 __syncwarp();
             }
             cp_async_wait_all();
