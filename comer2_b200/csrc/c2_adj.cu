@@ -211,28 +211,29 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// Row buffer of a strip's neighbour, ADJ_RG columns at a time, in the warp's
-// shared buffer rab[32][8] (slot c & 31: column c).  Forward: row 32 s - 1
-// (frow of strip s - 1) at columns c0 + l; backward: row 32 s + 32 (brow of
-// strip s + 1) at mirrored columns c0 + l, i.e. L - 1 - c0 - l.  WAIT: the
-// neighbour strip is being swept now; wait for those columns first (a strip
-// then trails its neighbour by about 32 + ADJ_RG columns).
+// Row of a strip's neighbour, ADJ_RG columns at a time, in the warp's shared
+// buffer rab[32][8] (slot c & 31: column c).  Forward: row 32 s - 1 (frow of
+// strip s - 1) at columns c0 + l; backward: row 32 s + 32 (brow of strip s + 1)
+// at mirrored columns c0 + l.  WAIT: the neighbour strip is being swept now;
+// poll until those columns are there (row hand-off, c2_device.cuh).
 constexpr int ADJ_RG = 8;
-template <bool MIRROR, bool WAIT>
-__device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const float* __restrict__ row, bool have,
-                                             const int* flag, int c0, int L, int lane, bool& broken)
+template <bool WAIT>
+__device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const float* __restrict__ row, int ldr,
+                                             bool have, int c0, int L, int lane, bool& broken)
 {
-    if (WAIT && have) pipe_wait(flag, min(c0 + ADJ_RG, L), lane, a.status, broken, a.spin);
     const int c = c0 + lane;
-    if (lane < ADJ_RG) {
-        const float init[5] = {0.f, XLOG0, XLOG0, XLOG0, XLOG0};
-        float v[5];
-#pragma unroll
-        for (int f = 0; f < 5; f++) {
-            const int col = MIRROR ? L - 1 - c : c;
-            v[f] = (have && c < L) ? (WAIT ? __ldcg(row + (long long)f * L + col) : row[(long long)f * L + col])
-                                   : init[f];
+    float v[5] = {0.f, XLOG0, XLOG0, XLOG0, XLOG0};
+    const bool want = lane < ADJ_RG && c < L;
+    if (have && c0 < L) {
+        if (WAIT) {
+            row_get(row, ldr, c, want, v, lane, a.status, broken, a.spin);
+        } else if (want) {
+            const float4 x = reinterpret_cast<const float4*>(row)[c];
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            v[4] = row[4 * ldr + c];
         }
+    }
+    if (lane < ADJ_RG) {
         float* o = rab + (c & 31) * 8;
         *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
         o[4] = v[4];
@@ -292,9 +293,9 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
     const int L = a.plen[p], Lq = a.pLq[m], ns = (Lq + 31) >> 5;
     const long long cb = a.off[m] + (long long)s * (L + 31) * 32;
     const float* dt0 = a.dtrn + (a.poff[p] + p) * 7;
-    const float* above = a.frow + a.roff[m] + (long long)(s > 0 ? s - 1 : 0) * 5 * L;   // read when s > 0
-    float* mine_row = a.frow + a.roff[m] + (long long)s * 5 * L;
-    const int* pf = a.prog + a.soff[m];
+    const int ldr = row_ld(L);
+    const float* above = a.frow + a.roff[m] + (long long)(s > 0 ? s - 1 : 0) * 5 * ldr;   // read when s > 0
+    float* mine_row = a.frow + a.roff[m] + (long long)s * 5 * ldr;
     const int r = 32 * s + lane;
     const bool act = r < Lq;
     const X5 INIT = {0.f, XLOG0, XLOG0, XLOG0, XLOG0};
@@ -309,11 +310,10 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
     X5 mine = INIT, upp = INIT;
     // the lane's score of the next step, loaded a step ahead
     float scn = (act && lane == 0 && L > 0) ? a.S[cb + lane] : XLOG0;
-    const int* pwait = pf + (s > 0 ? s - 1 : 0);   // strip s - 1's progress (s > 0)
     __syncwarp();
     adj_stage_trn<false>(trs, dt0, 0, L, lane);
     adj_stage_trn<false>(trs, dt0, 32, L, lane);
-    adj_load_row<false, !RECOMP>(a, rab, above, s > 0, pwait, 0, L, lane, broken);
+    adj_load_row<!RECOMP>(a, rab, above, ldr, s > 0, 0, L, lane, broken);
     for (int k = 0; k < L + 31; k++) {
         const int j = k - lane;
         float t7[7];
@@ -331,7 +331,7 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
             if (lane == 0) up = X5{ba.x, ba.y, ba.z, ba.w, b4};
             if ((src & (ADJ_RG - 1)) == ADJ_RG - 1) {
                 __syncwarp();
-                adj_load_row<false, !RECOMP>(a, rab, above, s > 0, pwait, k + 1, L, lane, broken);
+                adj_load_row<!RECOMP>(a, rab, above, ldr, s > 0, k + 1, L, lane, broken);
             }
             if (src == 31) {
                 if (k + 33 <= L) adj_stage_trn<false>(trs, dt0, k + 33, L, lane);
@@ -360,11 +360,7 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
                 if (nw.MM > zm) { zs = zs * xexp(zm - nw.MM) + 1.f; zm = nw.MM; }
                 else zs += xexp(nw.MM - zm);
             }
-            if (wr_row) {
-                mine_row[j] = nw.MM; mine_row[L + j] = nw.MI; mine_row[2 * L + j] = nw.IM;
-                mine_row[3 * L + j] = nw.DN; mine_row[4 * L + j] = nw.ND;
-                pipe_publish(a.prog + a.soff[m] + s, j, L);
-            }
+            if (wr_row) row_put(mine_row, ldr, j, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
         }
         mine = nw;
         upp = up;
@@ -436,6 +432,13 @@ __device__ __forceinline__ X5 fw_ld5(const float* __restrict__ Fw, int k, int l)
     return X5{o[0], o[32], o[64], o[96], o[128]};
 }
 
+// column c of a complete row
+__device__ __forceinline__ X5 row_ld5(const float* __restrict__ row, int ldr, int c)
+{
+    const float4 x = reinterpret_cast<const float4*>(row)[c];
+    return X5{x.x, x.y, x.z, x.w, row[4 * ldr + c]};
+}
+
 __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, int lane, float* rab, float* trs,
                                               const float* __restrict__ Fw, bool& broken)
 {
@@ -446,10 +449,10 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     const float lz = a.logz[m];
     const float* dt0 = a.dtrn + (a.poff[p] + p) * 7;
     const bool has_below = s + 1 < ns;
-    const float* below = a.brow + a.roff[m] + (long long)(has_below ? s + 1 : s) * 5 * L;   // read when has_below
-    float* mine_row = a.brow + a.roff[m] + (long long)s * 5 * L;
-    const float* fab = a.frow + a.roff[m] + (long long)(s > 0 ? s - 1 : 0) * 5 * L;   // row 32 s - 1 (s > 0)
-    const int* pb = a.prog + a.nitems + a.soff[m] + (has_below ? s + 1 : s);
+    const int ldr = row_ld(L);
+    const float* below = a.brow + a.roff[m] + (long long)(has_below ? s + 1 : s) * 5 * ldr;   // read when has_below
+    float* mine_row = a.brow + a.roff[m] + (long long)s * 5 * ldr;
+    const float* fab = a.frow + a.roff[m] + (long long)(s > 0 ? s - 1 : 0) * 5 * ldr;   // row 32 s - 1 (s > 0)
     const int t = lane;
     const int lf = 31 - t;            // the lane's row within the strip
     const int i = 32 * s + lf;
@@ -473,7 +476,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     __syncwarp();
     adj_stage_trn<true>(trs, dt0, 0, L, lane);
     adj_stage_trn<true>(trs, dt0, 32, L, lane);
-    adj_load_row<true, true>(a, rab, below, has_below, pb, 0, L, lane, broken);
+    adj_load_row<true>(a, rab, below, ldr, has_below, 0, L, lane, broken);
     for (int k = 0; k < L + 31; k++) {
         const int jm = k - t;
         const int ca = L - 1 - jm;
@@ -519,7 +522,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
             if (lane == 0) dn = X5{ba.x, ba.y, ba.z, ba.w, b4};
             if ((src & (ADJ_RG - 1)) == ADJ_RG - 1) {
                 __syncwarp();
-                adj_load_row<true, true>(a, rab, below, has_below, pb, k + 1, L, lane, broken);
+                adj_load_row<true>(a, rab, below, ldr, has_below, k + 1, L, lane, broken);
             }
             if (src == 31) {
                 if (k + 33 <= L) adj_stage_trn<true>(trs, dt0, k + 33, L, lane);
@@ -547,7 +550,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
             const X5 own = fw_ld5(Fw, kf, lf);
             X5 up, left, diag;
             if (i == 0) up = INIT;
-            else if (lf == 0) up = X5{fab[ca], fab[L + ca], fab[2 * L + ca], fab[3 * L + ca], fab[4 * L + ca]};
+            else if (lf == 0) up = row_ld5(fab, ldr, ca);
             else up = fw_ld5(Fw, kf - 1, lf - 1);
             if (ca == 0) {
                 left = LB;
@@ -555,8 +558,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
             } else {
                 left = fw_ld5(Fw, kf - 1, lf);
                 if (i == 0) diag = INIT;
-                else if (lf == 0)
-                    diag = X5{fab[ca - 1], fab[L + ca - 1], fab[2 * L + ca - 1], fab[3 * L + ca - 1], fab[4 * L + ca - 1]};
+                else if (lf == 0) diag = row_ld5(fab, ldr, ca - 1);
                 else diag = fw_ld5(Fw, kf - 2, lf - 1);
             }
             const long long kk = cb + (long long)kf * 32 + lf;
@@ -588,11 +590,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
             g[8] += gs * a.pcv[kk];
             a.gS[kk] = gs;
             a.post[kk] = xexp(own.MM + b.MM - lz);
-            if (wr_row) {
-                mine_row[ca] = nw.MM; mine_row[L + ca] = nw.MI; mine_row[2 * L + ca] = nw.IM;
-                mine_row[3 * L + ca] = nw.DN; mine_row[4 * L + ca] = nw.ND;
-                pipe_publish(a.prog + a.nitems + a.soff[m] + s, jm, L);
-            }
+            if (wr_row) row_put(mine_row, ldr, jm, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
         }
         mine = nw;
         upp = dn;

@@ -25,7 +25,7 @@ struct AdjArgs {
     const int2* items_f;    // [nitems] (pair, strip) of the forward sweep
     const int2* items_b;    // [nitems] (pair, strip) of the backward sweep
     const long long* off;   // [npairs] first cell of each pair (nstrips (L + 31) 32 cells a pair)
-    const long long* roff;  // [npairs] first float of each pair's row buffers (nstrips 5 L floats a pair)
+    const long long* roff;  // [npairs] first float of each pair's rows (nstrips x 5 x row_ld(L) floats a pair)
     const int* plen;
     const long long* poff;
     const float* qrec;      // query records (c2_device.cuh layout), queries concatenated
@@ -45,9 +45,8 @@ struct AdjArgs {
     float* pcv;             // [cells] CV term before its weight
     float* gS;              // [cells] dlogZ/dS
     float* post;            // [cells] MM state posterior
-    float* frow;            // forward checkpoint rows: per pair [nstrips][5][L], row 32 s + 31 of strip s
-    float* brow;            // outside values of row 32 s, per pair [nstrips][5][L]
-    int* prog;              // [2][nitems] columns published of frow / brow rows (by soff + strip)
+    float* frow;            // forward checkpoint rows, row 32 s + 31 of strip s (layout of the row hand-off)
+    float* brow;            // outside values of row 32 s by mirrored column, the same layout
     float* zpart;           // [nitems][2] (max, scaled sum) of a strip's exp(F.MM)
     float* gpart;           // [nitems][9] a strip's gradient sums
     float* Fall;            // forward states of every strip, when they fit (else null): strip s of

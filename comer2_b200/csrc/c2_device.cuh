@@ -97,8 +97,8 @@ constexpr int P1C_RING = 64, P1C_TRS = 12;
 constexpr int BND_ND = 32 * 4, BND_FLOATS = 32 * 5;
 // traceback sweep over the stored score matrices: per warp the score ring, the
 // transition ring, the row above and a [32][33]-byte traceback column ring;
-// 17 warps per SM.  P1TC_CVREP: CV table replicas of the phase-2 score kernel
-constexpr int P1TC_WARPS = 17, P1TC_CVREP = 8;
+// 16 warps per SM.  P1TC_CVREP: CV table replicas of the phase-2 score kernel
+constexpr int P1TC_WARPS = 16, P1TC_CVREP = 8;
 constexpr int P1TC_WARP_FLOATS = P1C_RING * 32 + P1C_RING * P1C_TRS + BND_FLOATS;
 // phase-2 score kernel: 8 warps per CTA, per warp the SS row table and the
 // record staging ring; the CV table (P1TC_CVREP replicas) per CTA
@@ -180,8 +180,7 @@ struct P1Args {
     float* mmat;                // [L][Lq] per candidate: modular scores
     int* status;                // device error word (0 = ok)
     // strip pipeline of the traceback variant
-    float* bnd;                 // per candidate at 10 x (cand_off / Lq): two last-row buffers [5][L]
-    int* prog;                  // [ncand][nstrips] finished columns per strip
+    float* bnd;                 // last rows of the strips (row_block)
     unsigned long long* tbkey;  // [ncand] maximum of the traceback sweep and its cell, packed
     const int* worder;          // traceback sweep: rank -> candidate (longest first)
     const int* items;           // traceback sweep: work item -> rank * nstrips + strip
@@ -225,13 +224,21 @@ struct FinArgs {
 // in the order of a host-built table from a global counter.  The table puts
 // (m, s) after (m, s - 1) (ordered by m + K s, K = pairs started per strip
 // lag), so the item a warp waits on was taken earlier by a warp that is
-// running, and strips are handed out about when their predecessor is ready.  Strip s writes its last row (5 states
-// per column) to bnd[m][s & 1][5][L] and publishes the number of finished
-// columns in prog[m * nstrips + s]; strip s+1 waits for the columns it
-// prefetches.  A long pair is thus swept by up to nstrips warps at once
-// instead of one.
+// running, and strips are handed out about when their predecessor is ready.  A long pair
+// is thus swept by up to nstrips warps at once instead of one.
+//
+// Row hand-off.  Strip s writes its last row (5 states per column) to a buffer
+// of its own, filled with ROW_EMPTY words before the sweep; strip s + 1 reads a
+// group of columns ahead of its use and polls until none of their words is
+// empty.  The data is its own flag: no fence, no separate progress word and no
+// cache invalidation stand between the strips, so a hand-off costs one trip
+// through L2 (with progress words, released every 8 columns and acquired by the
+// strip below, the fence and the acquire took longer than the 8 columns' cells).
+// A computed value is never ROW_EMPTY: the device's arithmetic yields only the
+// NaN 0x7fffffff.
+// Layout of a row: [ld][4] states MM MI IM DN, then [ld] ND, ld the length
+// rounded up to 4; the rows of a pair's strips follow one another.
 namespace c2 {
-constexpr int PIPE_G = 8;                 // columns per progress update
 constexpr unsigned PIPE_SPIN = 1u << 22;  // default polls before a wait gives up (c2_set_wait_limit)
 constexpr int PIPE_ERR_TIMEOUT = 3;       // device status of an abandoned wait
 
@@ -272,9 +279,59 @@ __device__ __forceinline__ void pipe_wait(const int* flag, int need, int lane, i
     __syncwarp();
 }
 
-// producer side: lane 31 has stored column c of its strip's last row
-__device__ __forceinline__ void pipe_publish(int* flag, int c, int L)
+constexpr unsigned ROW_EMPTY = 0xffffffffu;
+
+// First column of pair c's rows, pos the sum of the lengths of the pairs before
+// it (each row rounded up to 4 columns fits before the next pair's)
+__host__ __device__ __forceinline__ long long row_start(long long pos, long long c) { return (pos + 8 * c + 3) & ~3LL; }
+__host__ __device__ __forceinline__ int row_ld(int L) { return (L + 3) & ~3; }
+
+// one thread: column c of a row
+__device__ __forceinline__ void row_put(float* row, int ld, int c, float mm, float mi, float im, float dn, float nd)
 {
-    if (((c + 1) % PIPE_G) == 0 || c + 1 == L) pipe_st_release(flag, c + 1);
+    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + 4 * c), "f"(mm), "f"(mi), "f"(im),
+                 "f"(dn)
+                 : "memory");
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(row + 4 * ld + c), "f"(nd) : "memory");
+}
+
+// Warp-uniform wait: poll() (lane predicate, re-reading its words) until it
+// holds for every lane.  After `spin` polls it records PIPE_ERR_TIMEOUT in
+// *status, marks the warp broken (no further waits) and returns; the sweep then
+// finishes with invalid values -- every cell index stays inside its pair, so
+// nothing is read or written out of bounds -- and the host reports the status.
+template <typename F>
+__device__ __forceinline__ void row_poll(F poll, int lane, int* status, bool& broken, unsigned spin)
+{
+    for (unsigned it = 0;;) {
+        if (__all_sync(0xffffffffu, poll()) || broken) return;
+        if (++it >= spin) {
+            if (lane == 0 && status) atomicCAS(status, 0, PIPE_ERR_TIMEOUT);
+            broken = true;
+            return;
+        }
+        // (short sleeps first: the columns are usually a few steps away)
+        __nanosleep(it < 32 ? 20 : 128);
+    }
+}
+
+// The lane's column c of a row another warp writes, for lanes with want
+__device__ __forceinline__ void row_get(const float* row, int ld, int c, bool want, float* v, int lane, int* status,
+                                        bool& broken, unsigned spin)
+{
+    row_poll(
+        [&]() -> bool {
+            if (!want) return true;
+            asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                         : "l"(row + 4 * c)
+                         : "memory");
+            asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v[4]) : "l"(row + 4 * ld + c) : "memory");
+            bool ok = true;
+#pragma unroll
+            for (int f = 0; f < 5; f++) ok = ok && __float_as_uint(v[f]) != ROW_EMPTY;
+            return ok;
+        },
+        lane, status, broken, spin);
 }
 }  // namespace c2

@@ -27,7 +27,7 @@
 
 namespace c2 {
 cudaError_t launch_stats(const StatsArgs& a, cudaStream_t st);
-cudaError_t launch_map(const MapArgs& a, const float* qtrn, const float* dtrn, const float* qcf, int nsm,
+cudaError_t launch_map(MapArgs a, const float* qtrn, const float* dtrn, const float* qcf, int nsm,
                        int* counter, cudaStream_t st, int* nlaunch);
 cudaError_t launch_viterbi_aln(const MapArgs& a, cudaStream_t st);
 size_t p1_smem_bytes(int cvcard);
@@ -156,7 +156,7 @@ struct c2_handle {
     bool adj_fwd_done = false, adj_batch = false;      // adj_batch: the pairs' queries are in d_adjq*
     float adj_theta[7] = {0, 0, 0, 0, 0, 0, 0};
     float adj_wss = 0.f, adj_wcv = 0.f;
-    DevBuf<int> d_adjprof, d_adjprog, d_adjctr, d_adjLq, d_adjqidx;
+    DevBuf<int> d_adjprof, d_adjctr, d_adjLq, d_adjqidx;
     DevBuf<long long> d_adjoff, d_adjroff, d_adjqpos, d_adjsoff;
     DevBuf<int2> d_adjitems;
     DevBuf<float> d_adjbuf, d_adjlogz, d_adjgrad, d_adjpart, d_adjscr;
@@ -190,8 +190,7 @@ struct c2_handle {
     // tensor-core query operands
     DevBuf<unsigned> d_qa;
     DevBuf<float> d_qaaf;
-    DevBuf<int> d_prog;
-    size_t bnd_half = 0, prog_half = 0;   // floats / words of one sweep's strip-pipeline scratch
+    size_t bnd_cols = 0;   // columns of the strips' rows over all candidates (row_start)
     DevBuf<float> d_fscore;
     DevBuf<int> d_fpsts, d_fpassed;
     DevBuf<unsigned> d_fbeg, d_fend;
@@ -1315,12 +1314,13 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
     if (h->ncand == 0) return C2_OK;
     const int nc = h->ncand;
     // strip-pipeline scratch: two halves, the second for the MAP backward sweep
-    h->bnd_half = (size_t)(acc / h->Lq) * 10;
-    h->prog_half = (size_t)nc * ((h->Lq + 31) / 32);
+    const size_t nstrips = (size_t)(h->Lq + 31) / 32;
+    h->bnd_cols = (size_t)row_start(acc / h->Lq, nc);
+    const size_t bnd_half = 5 * nstrips * h->bnd_cols;
     if (h->d_cand_prof.ensure(nc, h->budget) || h->d_cand_off.ensure(nc, h->budget) || h->d_btck.ensure((size_t)acc, h->budget) ||
         h->d_smat.ensure((size_t)acc, h->budget) || h->d_mmat.ensure((size_t)acc, h->budget) || h->d_fscore.ensure(nc, h->budget) || h->d_fpsts.ensure(nc, h->budget) ||
         h->d_fpassed.ensure(nc, h->budget) || h->d_fbeg.ensure(nc, h->budget) || h->d_fend.ensure(nc, h->budget) ||
-        h->d_bnd.ensure(2 * h->bnd_half, h->budget) || h->d_tbkey.ensure(nc, h->budget) || h->d_prog.ensure(2 * h->prog_half, h->budget))
+        h->d_bnd.ensure(2 * bnd_half, h->budget) || h->d_tbkey.ensure(nc, h->budget))
         return fail(h, C2_ERR_NOMEM, "finalisation scratch for %d pairs (%lld cells) failed", nc, acc);
     CK(cudaMemcpyAsync(h->d_cand_prof.p, h->h_cand.data(), (size_t)nc * 4, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_cand_off.p, h->h_cand_off.data(), (size_t)nc * 8, cudaMemcpyHostToDevice, h->stream));
@@ -1348,13 +1348,12 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
     a.smat = h->d_smat.p;
     a.mmat = h->d_mmat.p;
     a.bnd = h->d_bnd.p;
-    a.prog = h->d_prog.p;
     a.tbkey = h->d_tbkey.p;
     a.worder = h->d_worder.p;
     a.items = h->d_tbitems.p;
     const long long nitems = (long long)nc * ((h->Lq + 31) / 32);
     CK(cudaMemsetAsync(h->d_counter.p, 0, 2 * sizeof(int), h->stream));   // the sweep's and the score kernel's
-    CK(cudaMemsetAsync(h->d_prog.p, 0, (size_t)nitems * sizeof(int), h->stream));
+    CK(cudaMemsetAsync(h->d_bnd.p, 0xff, bnd_half * sizeof(float), h->stream));   // the strips' rows: empty
     CK(cudaMemsetAsync(h->d_tbkey.p, 0, (size_t)nc * sizeof(unsigned long long), h->stream));
     // one CTA of P1TC_WARPS warps per SM, one warp per (candidate, strip) work item at most
     const int grid = (int)std::min<long long>(h->nsm, (nitems + P1TC_WARPS - 1) / P1TC_WARPS);
@@ -1650,9 +1649,8 @@ extern "C" c2_status c2_run_map(c2_handle* h, int32_t* nhits)
     a.pairf = h->d_pairf.p;
     a.pairc = h->d_pairc.p;
     a.bnd = h->d_bnd.p;
-    a.prog = h->d_prog.p;
-    a.bnd_b = h->d_bnd.p + h->bnd_half;   // the backward sweep's halves of the scratch
-    a.prog_b = h->d_prog.p + h->prog_half;
+    a.bnd_b = h->d_bnd.p + 5 * (size_t)((h->Lq + 31) / 32) * h->bnd_cols;   // the backward sweep's half
+    a.bnd_cols = h->bnd_cols;
     a.pairk = h->d_pairk.p;
     a.items = h->d_mapitems.p;
     a.status = h->d_status.p;
@@ -1769,7 +1767,7 @@ static void release_phase2(c2_handle* h)
 {
     h->d_cand_prof.release(); h->d_cand_off.release(); h->d_btck.release(); h->d_smat.release();
     h->d_mmat.release(); h->d_fscore.release(); h->d_fpsts.release(); h->d_fpassed.release();
-    h->d_fbeg.release(); h->d_fend.release(); h->d_bnd.release(); h->d_tbkey.release(); h->d_prog.release();
+    h->d_fbeg.release(); h->d_fend.release(); h->d_bnd.release(); h->d_tbkey.release();
     h->d_worder.release(); h->d_tbitems.release(); h->d_mapitems.release(); h->d_p2.release(); h->d_stats.release();
     h->d_mapcand.release(); h->d_mappass.release(); h->d_alninfo.release(); h->d_fb.release(); h->d_bb.release();
     h->d_pairf.release(); h->d_pairc.release(); h->d_pairk.release(); h->d_aln.release(); h->d_alnpack.release();
@@ -1784,7 +1782,7 @@ static void release_phase2(c2_handle* h)
 static size_t pair_scratch_bytes(const c2_handle* h, int L)
 {
     const size_t Lq = (size_t)h->Lq, ns = (Lq + 31) / 32;
-    return 9 * Lq * (size_t)L + 2 * 10 * 4 * (size_t)L + 2 * 4 * ns + 4 * ns * 2 + 2 * 4 * 32 * ns * ((size_t)L + 31) +
+    return 9 * Lq * (size_t)L + 2 * 5 * 4 * ns * ((size_t)L + 12) + 4 * ns * 2 + 2 * 4 * 32 * ns * ((size_t)L + 31) +
            2 * 5 * (Lq + (size_t)h->Lmax + 1) + 512;
 }
 
@@ -2026,7 +2024,6 @@ static void fill_adj(c2_handle* h, AdjArgs& a)
     a.post = b + 4 * NC;
     a.frow = b + 5 * NC;
     a.brow = b + 5 * NC + NR;
-    a.prog = h->d_adjprog.p;
     a.zpart = h->d_adjpart.p;
     a.gpart = h->d_adjpart.p + 2LL * h->adj_nitems;
     a.Fall = h->adj_keepF ? h->d_adjF.p : nullptr;
@@ -2073,7 +2070,7 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
         h->adj_roff[k] = racc;
         soff[k] = sacc;
         acc += (long long)ns * (L + 31) * 32;
-        racc += (long long)ns * 5 * L;
+        racc += (long long)ns * 5 * row_ld(L);
         sacc += ns;
         lmax = std::max(lmax, L);
         nsmax = std::max(nsmax, ns);
@@ -2107,7 +2104,7 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
         h->d_adjsoff.ensure(npairs, h->budget) || h->d_adjitems.ensure((size_t)2 * items, h->budget) ||
         h->d_adjbuf.ensure((size_t)(5 * acc + 2 * racc), h->budget) ||
         h->d_adjlogz.ensure(npairs, h->budget) || h->d_adjgrad.ensure((size_t)npairs * 9, h->budget) ||
-        h->d_adjprog.ensure((size_t)2 * items, h->budget) || h->d_adjpart.ensure((size_t)11 * items, h->budget) ||
+        h->d_adjpart.ensure((size_t)11 * items, h->budget) ||
         h->d_adjctr.ensure(2, h->budget))
         return fail(h, C2_ERR_NOMEM, "logz_fwd: scratch for %d pairs (%lld cells) failed", npairs, acc);
     // persistent grids of the sweeps: as many CTAs as are resident (or as
@@ -2149,7 +2146,7 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
     CK(cudaMemcpyAsync(h->d_adjitems.p, it.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_adjoff.p, h->adj_off.data(), (size_t)npairs * 8, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_adjroff.p, h->adj_roff.data(), (size_t)npairs * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemsetAsync(h->d_adjprog.p, 0, (size_t)items * sizeof(int), h->stream));
+    CK(cudaMemsetAsync(h->d_adjbuf.p + 5 * acc, 0xff, (size_t)racc * sizeof(float), h->stream));   // forward rows: empty
     CK(cudaMemsetAsync(h->d_adjctr.p, 0, 2 * sizeof(int), h->stream));
     CK(cudaMemsetAsync(h->d_status.p, 0, sizeof(int), h->stream));
     AdjArgs a;
@@ -2248,8 +2245,8 @@ extern "C" c2_status c2_logz_bwd(c2_handle* h, float* grad)
     CK(cudaSetDevice(h->device));
     AdjArgs a;
     fill_adj(h, a);
-    const long long items = h->adj_nitems;
-    CK(cudaMemsetAsync(h->d_adjprog.p + items, 0, (size_t)items * sizeof(int), h->stream));
+    // the backward rows empty again (a second call on the same forward sweep)
+    CK(cudaMemsetAsync(h->d_adjbuf.p + 5 * h->adj_cells + h->adj_rows, 0xff, (size_t)h->adj_rows * sizeof(float), h->stream));
     CK(cudaMemsetAsync(h->d_adjctr.p + 1, 0, sizeof(int), h->stream));
     CK(launch_adj_bwd(a, h->adj_bgrid, h->stream));
     h->launches += 2;

@@ -456,7 +456,7 @@ __device__ __forceinline__ void wf_init(WfLane& D, const float* q7, const St5& L
     D.kbest = 0;
 }
 
-// Row above the strip, 32 column slots: states MM, MI, IM, DN as a float4
+// Row above the strip, one slot a column: states MM, MI, IM, DN as a float4
 // per slot ([32][4]), ND after them ([32] at BND_ND)
 __device__ __forceinline__ void bnd_put(float* bnd, int slot, float mm, float mi, float im, float dn, float nd)
 {
@@ -464,22 +464,23 @@ __device__ __forceinline__ void bnd_put(float* bnd, int slot, float mm, float mi
     bnd[BND_ND + slot] = nd;
 }
 
-// Wavefront steps [k0, k0 + nst) of a strip (k0 a multiple of 32, nst <= 32;
-// 32 when !CHECK).  ring: diagonal-indexed scores, 32 floats per slot.  tcol:
-// ring of P1C_RING column records (TMM .. TDD, P1C_TRS floats apart).
-// bnd: row above the strip for columns [k0, k0 + 32).
-// TB (traceback sweep): each cell's traceback code also goes to the warp's
-// column ring btr (column j in slot j & 31, the lane's own row), and column
-// k - 31, complete for every row at step k, is stored to the pair's code
-// matrix bt (column-major, Lq rows; r = this lane's query row).
-template <bool CHECK, bool TB = false>
+// Wavefront steps [k0, k0 + nst) of a strip of the traceback sweep (k0 a multiple
+// of TB_C, nst <= TB_C; TB_C when !CHECK).  ring: diagonal-indexed scores, 32
+// floats per slot.  tcol: ring of P1C_RING column records (TMM .. TDD, P1C_TRS
+// floats apart).  bnd: row above the strip for columns [k0, k0 + TB_C).  Lane 31
+// stores its cells to the strip's row (wr_row).  Each cell's traceback code goes
+// to the warp's column ring btr (column j in slot j & 31, the lane's own row),
+// and column k - 31, complete for every row at step k, is stored to the pair's
+// code matrix bt (column-major, Lq rows; r = this lane's query row).
+constexpr int TB_C = 16;
+template <bool CHECK>
 __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, int L, bool act,
                                          const float* __restrict__ ring, const float* __restrict__ tcol,
-                                         float* __restrict__ bnd, bool wr_bot, signed char (*btr)[33] = nullptr,
-                                         signed char* __restrict__ bt = nullptr, int Lq = 0, int r = 0)
+                                         const float* __restrict__ bnd, bool wr_row, float* row, int ldr,
+                                         signed char (*btr)[33], signed char* __restrict__ bt, int Lq, int r)
 {
     const float* __restrict__ rb = ring + (k0 & (P1C_RING - 1)) * 32 + lane;
-    if (!CHECK) nst = 32;
+    if (!CHECK) nst = TB_C;
     int ub = -1;
     // the instruction cache holds both variants of both kernels at these depths
     constexpr int UNR = CHECK ? 2 : 4;
@@ -518,48 +519,25 @@ __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, i
         // their MM stays 0 and never beats a maximum
         const bool inm = !CHECK || (j >= 0 && j < L);
         if ((!CHECK || act) && inm && nMM > D.best) { D.best = nMM; ub = u; }
-        if (TB) {
-            // ExecDP_Btck's code: DIAG if MM > 0, then the first strictly larger
-            // of MI (UP), IM (LEFT), DN (UP), ND (LEFT)
-            if (act && inm) {
-                int b = BT_STOP;
-                float mx = nMM;
-                if (nMM != 0.f) b = BT_DIAG;
-                if (mx < nMI) { mx = nMI; b = BT_UP; }
-                if (mx < nIM) { mx = nIM; b = BT_LEFT; }
-                if (mx < nDN) { mx = nDN; b = BT_UP; }
-                if (mx < nND) b = BT_LEFT;
-                btr[j & 31][lane] = (signed char)b;
-            }
-            const int cfl = k0 + u - 31;
-            if (act && (!CHECK || (cfl >= 0 && cfl < L))) bt[(long long)cfl * Lq + r] = btr[cfl & 31][lane];
+        // ExecDP_Btck's code: DIAG if MM > 0, then the first strictly larger
+        // of MI (UP), IM (LEFT), DN (UP), ND (LEFT)
+        if (act && inm) {
+            int b = BT_STOP;
+            float mx = nMM;
+            if (nMM != 0.f) b = BT_DIAG;
+            if (mx < nMI) { mx = nMI; b = BT_UP; }
+            if (mx < nIM) { mx = nIM; b = BT_LEFT; }
+            if (mx < nDN) { mx = nDN; b = BT_UP; }
+            if (mx < nND) b = BT_LEFT;
+            btr[j & 31][lane] = (signed char)b;
         }
-        if (wr_bot) {
-            // lane 31's cell (column k0 + u - 31) into the slot lane 0 read at
-            // the top of this step; bot_flush stores the 32 columns per chunk
-            bnd_put(bnd, u, nMM, nMI, nIM, nDN, nND);
-        }
+        const int cfl = k0 + u - 31;
+        if (act && (!CHECK || (cfl >= 0 && cfl < L))) bt[(long long)cfl * Lq + r] = btr[cfl & 31][lane];
+        if (wr_row && (!CHECK || (j >= 0 && j < L))) row_put(row, ldr, j, nMM, nMI, nIM, nDN, nND);
         D.MM = nMM; D.MI = nMI; D.IM = nIM; D.DN = nDN; D.ND = nND;
         D.A = A; D.Y = Y; D.z = z;
     }
     if (ub >= 0) D.kbest = k0 + ub;
-}
-
-// The strip's last row after a DP stage over [k0, k0 + 32): slot l of bnd
-// holds lane 31's states at column k0 - 31 + l; the warp stores the columns
-// inside the matrix to the boundary buffer, one coalesced segment per state
-__device__ __forceinline__ void bot_flush(const float* __restrict__ bnd, float* __restrict__ botw, int k0, int L,
-                                          int Lmax, int lane)
-{
-    const int c = k0 - 31 + lane;
-    if (c >= 0 && c < L) {
-        const float4 a = *reinterpret_cast<const float4*>(bnd + lane * 4);
-        botw[0 * Lmax + c] = a.x;
-        botw[1 * Lmax + c] = a.y;
-        botw[2 * Lmax + c] = a.z;
-        botw[3 * Lmax + c] = a.w;
-        botw[4 * Lmax + c] = bnd[BND_ND + lane];
-    }
 }
 
 // Corner cells (CellYXinCorners): row r keeps S = -9 at columns j <= cA(r)
@@ -991,16 +969,6 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 }
 
 // ---------------------------------------------------------------------------
-// Traceback sweep, chunked: the DP finalisation's FP32 recomputation of the
-// candidates (ExecDP_Btck_Unroll32x, src/libmycu/cudp/CuBatchDP_init_btck.cu:
-// 303-360) with p1c_kernel's schedule -- per 32-column chunk the scores of the
-// strip (also stored to the pair's score and modular-score matrices, column-
-// major, coalesced) and then 32 wavefront steps that also store the traceback
-// codes.  Work items are (candidate, strip) in the strip pipeline of
-// c2_device.cuh: strip s waits, before DP stage m, for the strip above to have
-// published the columns of chunk m + 1 of its last row (loaded into registers
-// during the stage) and publishes its own last row once per chunk.  The
-// arithmetic is p1c_kernel's, so the maxima equal phase 1's in the FP32 form.
 // Phase-2 score matrices: the FP32 scores and modular scores of every cell of
 // the candidate pairs, column-major per pair (the layout of the finalisation,
 // statistics and MAP stages), by cell_score -- the arithmetic of phase 1's
@@ -1081,9 +1049,13 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
 }
 
 // Traceback sweep over the candidate pairs: the FP32 Viterbi DP again, on the
-// score matrices p2s_kernel wrote (read a 32-column chunk at a time into the
-// anti-diagonal ring), with the btck code of every cell stored column-major
-// and the strips of a pair pipelined over warps.
+// score matrices p2s_kernel wrote (ExecDP_Btck_Unroll32x, src/libmycu/cudp/
+// CuBatchDP_init_btck.cu:303-360), with the btck code of every cell stored
+// column-major and the strips of a pair pipelined over warps (c2_device.cuh): a
+// chunk of 16 columns at a time, its scores loaded a chunk ahead into the
+// anti-diagonal ring and the row above fetched just before its steps, so that a
+// strip trails the one above by about 50 steps.  The arithmetic is p1c_kernel's:
+// the maxima equal phase 1's in the FP32 form.
 __global__ void __launch_bounds__(P1TC_WARPS * 32, 1)
 p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
 {
@@ -1118,10 +1090,9 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
         const long long coff = a.cand_off[cand];
         signed char* bt = a.btck + coff;
         const float* smt = a.smat + coff;
-        float* pb = a.bnd + (coff / Lq) * 10;
-        const float* botr = pb + ((s + 1) & 1) * 5 * L;   // last row of strip s-1
-        float* botw = pb + (s & 1) * 5 * L;
-        int* pf = a.prog + (long long)cand * nstrips;
+        const int ldr = row_ld(L);
+        float* rowm = a.bnd + 5 * (nstrips * row_start(coff / Lq, cand) + (long long)s * ldr);   // this strip's last row
+        const float* rowa = rowm - 5 * ldr;                                                      // the one above (s > 0)
         const int r = s * 32 + lane;
         const bool act = r < Lq;
         const float* __restrict__ qr = a.qrec + (long long)(act ? r : Lq - 1) * QR_STRIDE;
@@ -1140,65 +1111,46 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
         }
         const int cA = corner_a(r, Lq, edge);
         const int cB = corner_b(r, L, edge);
-        // columns [0, 32) of the row above, lane i holding column i; bnxt: the next 32
-        float bc[5], bnxt[5];
-        if (s > 0) pipe_wait(pf + s - 1, min(32, L), lane, a.status, broken, a.spin);
-#pragma unroll
-        for (int f = 0; f < 5; f++) bc[f] = (s > 0 && lane < L) ? __ldcg(botr + f * L + lane) : 0.f;
-        const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
-        __syncwarp();
-        bnd_put(bnd, lane, bc[0], bc[1], bc[2], bc[3], bc[4]);
-        const int nch = (L + 31) >> 5;
+        const bool wr_row = (lane == 31) && (s + 1 < nstrips);
         const int kend = L + 31;
-        for (int m = 0; 32 * m < kend; m++) {
-            // ---- score stage: columns [32m, min(32m + 32, L)) from the score
-            // matrix (the lanes' rows of one column: one 128-byte line), and
-            // the columns' transitions
-            if (m < nch) {
-                const int c0 = 32 * m, c1 = min(c0 + 32, L);
-                const bool hasc = __any_sync(FULL, cA >= c0 || cB < c1);
-#pragma unroll 8
-                for (int c = c0; c < c1; c++) {
-                    float Sc = act ? __ldcg(smt + (long long)c * Lq + r) : 0.f;
-                    if (hasc && (c <= cA || c >= cB)) Sc = -9.f;
-                    ring[((c + lane) & (P1C_RING - 1)) * 32 + lane] = Sc;
-                    if (lane < 7)
-                        trn[(c & (P1C_RING - 1)) * P1C_TRS + lane] = __ldg(dr + (long long)c * DR_STRIDE + DR_TRN + lane);
+        // scores of a chunk's columns (the lanes' rows of one column: one
+        // 128-byte line) and the columns' transitions, loaded a chunk ahead
+        float sc[TB_C];
+        float4 tv;
+        auto fetch = [&](int c0) {
+#pragma unroll
+            for (int u = 0; u < TB_C; u++) sc[u] = (act && c0 + u < L) ? __ldcg(smt + (long long)(c0 + u) * Lq + r) : 0.f;
+            const int c = c0 + (lane >> 1);
+            if (c < L) tv = __ldg(reinterpret_cast<const float4*>(dr + (long long)c * DR_STRIDE + DR_TRN) + (lane & 1));
+        };
+        fetch(0);
+        for (int k0 = 0; k0 < kend; k0 += TB_C) {
+            if (k0 < L) {
+                const bool hasc = __any_sync(FULL, cA >= k0 || cB < k0 + TB_C);
+#pragma unroll
+                for (int u = 0; u < TB_C; u++) {
+                    const int c = k0 + u;
+                    if (hasc && (c <= cA || c >= cB)) sc[u] = -9.f;
+                    if (c < L) ring[((c + lane) & (P1C_RING - 1)) * 32 + lane] = sc[u];
                 }
+                const int c = k0 + (lane >> 1);
+                if (c < L) *reinterpret_cast<float4*>(trn + (c & (P1C_RING - 1)) * P1C_TRS + 4 * (lane & 1)) = tv;
+                fetch(k0 + TB_C);
             }
-            // the row above for chunk m + 1, loaded while this stage runs
-            const int k0 = 32 * m, k1 = min(k0 + 32, kend);
-            if (s > 0 && k0 + 32 < L) {
-                pipe_wait(pf + s - 1, min(k0 + 64, L), lane, a.status, broken, a.spin);
-#pragma unroll
-                for (int f = 0; f < 5; f++) {
-                    const int cc = k0 + 32 + lane;
-                    bnxt[f] = (cc < L) ? __ldcg(botr + f * L + cc) : 0.f;
-                }
-            } else {
-#pragma unroll
-                for (int f = 0; f < 5; f++) bnxt[f] = 0.f;
+            // the row above for this chunk's steps
+            {
+                float v[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+                if (s > 0 && k0 < L)
+                    row_get(rowa, ldr, k0 + lane, lane < TB_C && k0 + lane < L, v, lane, a.status, broken, a.spin);
+                if (lane < TB_C) bnd_put(bnd, lane, v[0], v[1], v[2], v[3], v[4]);
             }
             __syncwarp();
-            // ---- DP stage: wavefront steps [32m, 32m + 32), traceback codes stored
-            if (m >= 1 && k0 + 31 < L && k1 == k0 + 32)
-                wf_steps<false, true>(D, k0, 32, lane, L, act, ring, trn, bnd, wr_bot, btr,
-                                                               bt, Lq, r);
+            // ---- DP stage: wavefront steps [k0, k0 + TB_C), traceback codes stored
+            if (k0 >= 32 && k0 + TB_C <= L)
+                wf_steps<false>(D, k0, TB_C, lane, L, act, ring, trn, bnd, wr_row, rowm, ldr, btr, bt, Lq, r);
             else
-                wf_steps<true, true>(D, k0, k1 - k0, lane, L, act, ring, trn, bnd, wr_bot,
-                                                              btr, bt, Lq, r);
-            __syncwarp();
-            if (s + 1 < nstrips) {
-                // last row of columns [k0 - 31, k0] to the pair's buffer, then published
-                bot_flush(bnd, botw, k0, L, L, lane);
-                __syncwarp();
-                if (lane == 0) {
-                    __threadfence();
-                    pipe_st_release(pf + s, min(k1 - 31, L));
-                }
-            }
-            __syncwarp();
-            bnd_put(bnd, lane, bnxt[0], bnxt[1], bnxt[2], bnxt[3], bnxt[4]);
+                wf_steps<true>(D, k0, min(TB_C, kend - k0), lane, L, act, ring, trn, bnd, wr_row, rowm, ldr, btr, bt, Lq,
+                               r);
             __syncwarp();
         }
         // the strip's maximum: largest score, then smallest row, then smallest column

@@ -198,14 +198,20 @@ __device__ __forceinline__ float map_score(const MapArgs& a, const MapPair& P, l
 // consecutive columns c0 + lane of a column-major [L][Lq] matrix: one
 // instruction per lane per 128-byte line, issued a chunk ahead of the
 // sweep's one-step-ahead loads so that those hit L2
-__device__ __forceinline__ void pf_cols(const float* __restrict__ mat, int c, int L, int Lq, int row0)
+// (pf1: into L1 as well, for the few warps per SM whose chunks fit there)
+__device__ __forceinline__ void pf_cols(const float* __restrict__ mat, int c, int L, int Lq, int row0, int pf1)
 {
     if (c < 0 || c >= L) return;
     const int r0 = max(row0, 0), r1 = min(row0 + 31, Lq - 1);
     if (r0 > r1) return;
     const float* p = mat + (long long)c * Lq;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + r0));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + r1));
+    if (pf1) {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p + r0));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p + r1));
+    } else {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + r0));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + r1));
+    }
 }
 
 // L2 prefetch of wavefront row k (32 floats, one 128-byte line) of a strip
@@ -222,8 +228,8 @@ template <bool BWD>
 __device__ __forceinline__ void pf_scores(const MapArgs& a, const MapPair& P, int c0, int Lq, int row0, int lane)
 {
     const int c = BWD ? P.L - 1 - (c0 + lane) : c0 + lane;
-    pf_cols(a.smat + P.base, c, P.L, Lq, row0);
-    if (P.dmul != 0.f && a.modscores) pf_cols(a.mmat + P.base, c, P.L, Lq, row0);
+    pf_cols(a.smat + P.base, c, P.L, Lq, row0, a.pf1);
+    if (P.dmul != 0.f && a.modscores) pf_cols(a.mmat + P.base, c, P.L, Lq, row0, a.pf1);
 }
 
 // ---------------------------------------------------------------------------
@@ -253,10 +259,9 @@ __device__ __forceinline__ void map_fwd_item(const MapArgs& a, const float* __re
             map_trn_col<false>(dt0, 32 + lane, L, tnx);
             __syncwarp();
         }
-        float* bnd = a.bnd + (P.base / Lq) * 10;
-        const float* botr = bnd + ((s + 1) & 1) * 5 * L;   // last row of strip s-1
-        float* botw = bnd + (s & 1) * 5 * L;
-        int* pf = a.prog + (long long)m * nstrips;
+        const int ldr = row_ld(L);
+        float* rowm = a.bnd + 5 * (nstrips * row_start(P.base / Lq, P.c) + (long long)s * ldr);   // this strip's last row
+        const float* rowa = rowm - 5 * ldr;                                                       // strip s - 1's
         float maxF = 0.f;
         {
             const int r = s * 32 + lane;
@@ -275,15 +280,21 @@ __device__ __forceinline__ void map_fwd_item(const MapArgs& a, const float* __re
             // buffer rab[32][8] (slot c & 31: column c), waited for and loaded
             // a group ahead (the strip trails the one above by ~32 + MAP_RG columns)
             const float binit[5] = {0.f, MLOG0, MLOG0, MLOG0, MLOG0};
-            if (s > 0) pipe_wait(pf + s - 1, min(MAP_RG, L), lane, a.status, broken, a.spin);
-            __syncwarp();
-            if (lane < MAP_RG) {
+            auto load_above = [&](int c0) {
                 float v[5];
 #pragma unroll
-                for (int f = 0; f < 5; f++) v[f] = (s > 0 && lane < L) ? __ldcg(botr + f * L + lane) : binit[f];
-                *reinterpret_cast<float4*>(rab + lane * 8) = make_float4(v[0], v[1], v[2], v[3]);
-                rab[lane * 8 + 4] = v[4];
-            }
+                for (int f = 0; f < 5; f++) v[f] = binit[f];
+                const int cc = c0 + lane;
+                if (s > 0 && c0 < L)
+                    row_get(rowa, ldr, cc, lane < MAP_RG && cc < L, v, lane, a.status, broken, a.spin);
+                if (lane < MAP_RG) {
+                    float* o = rab + (cc & 31) * 8;
+                    *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+                    o[4] = v[4];
+                }
+            };
+            __syncwarp();
+            load_above(0);
             __syncwarp();
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             // column k's score is loaded one step ahead, from L2: each chunk's
@@ -308,20 +319,8 @@ __device__ __forceinline__ void map_fwd_item(const MapArgs& a, const float* __re
                     const float4 ba = *reinterpret_cast<const float4*>(rab + src * 8);
                     const float b4 = rab[src * 8 + 4];
                     if (lane == 0) up = S5{ba.x, ba.y, ba.z, ba.w, b4};
-                    if ((src & (MAP_RG - 1)) == MAP_RG - 1) {
-                        // the next group of columns into slots this step does not read
-                        if (s > 0 && k + 1 < L)
-                            pipe_wait(pf + s - 1, min(k + 1 + MAP_RG, L), lane, a.status, broken, a.spin);
-                        if (lane < MAP_RG) {
-                            const int cc = k + 1 + lane;
-                            float v[5];
-#pragma unroll
-                            for (int f = 0; f < 5; f++) v[f] = (s > 0 && cc < L) ? __ldcg(botr + f * L + cc) : binit[f];
-                            float* o = rab + (cc & 31) * 8;
-                            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-                            o[4] = v[4];
-                        }
-                    }
+                    // the next group of columns into slots this step does not read
+                    if ((src & (MAP_RG - 1)) == MAP_RG - 1) load_above(k + 1);
                 }
                 __syncwarp();
                 const int j = k - lane;
@@ -343,11 +342,7 @@ __device__ __forceinline__ void map_fwd_item(const MapArgs& a, const float* __re
                     maxF = hmax(maxF, nw.MM);
                     fs[(long long)k * 32 + lane] = nw.MM;
                 }
-                if (wr_bot && j >= 0 && j < L) {
-                    botw[0 * L + j] = nw.MM; botw[1 * L + j] = nw.MI; botw[2 * L + j] = nw.IM;
-                    botw[3 * L + j] = nw.DN; botw[4 * L + j] = nw.ND;
-                    pipe_publish(pf + s, j, L);
-                }
+                if (wr_bot && j >= 0 && j < L) row_put(rowm, ldr, j, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
                 mine = nw;
                 upp = up;
                 if ((k & 31) == 31) {
@@ -431,10 +426,9 @@ __device__ __forceinline__ void map_bwd_item(const MapArgs& a, const float* __re
             map_trn_col<true>(dt0, 32 + lane, L, tnx);
             __syncwarp();
         }
-        float* bnd = a.bnd_b + (P.base / Lq) * 10;
-        const float* botr = bnd + ((s + 1) & 1) * 5 * L;   // last row of mirrored strip s-1
-        float* botw = bnd + (s & 1) * 5 * L;
-        int* pf = a.prog_b + (long long)m * nstrips;
+        const int ldr = row_ld(L);
+        float* rowm = a.bnd_b + 5 * (nstrips * row_start(P.base / Lq, P.c) + (long long)s * ldr);   // this strip's last row
+        const float* rowa = rowm - 5 * ldr;                                                         // strip s - 1's
         {
             const int rm = s * 32 + lane;       // mirrored row
             const int r = Lq - 1 - rm;          // actual row
@@ -449,15 +443,21 @@ __device__ __forceinline__ void map_bwd_item(const MapArgs& a, const float* __re
             // buffer rab[32][8] (slot c & 31: column c), waited for and loaded
             // a group ahead (the strip trails the one above by ~32 + MAP_RG columns)
             const float binit[5] = {0.f, MLOG0, MLOG0, MLOG0, MLOG0};
-            if (s > 0) pipe_wait(pf + s - 1, min(MAP_RG, L), lane, a.status, broken, a.spin);
-            __syncwarp();
-            if (lane < MAP_RG) {
+            auto load_above = [&](int c0) {
                 float v[5];
 #pragma unroll
-                for (int f = 0; f < 5; f++) v[f] = (s > 0 && lane < L) ? __ldcg(botr + f * L + lane) : binit[f];
-                *reinterpret_cast<float4*>(rab + lane * 8) = make_float4(v[0], v[1], v[2], v[3]);
-                rab[lane * 8 + 4] = v[4];
-            }
+                for (int f = 0; f < 5; f++) v[f] = binit[f];
+                const int cc = c0 + lane;
+                if (s > 0 && c0 < L)
+                    row_get(rowa, ldr, cc, lane < MAP_RG && cc < L, v, lane, a.status, broken, a.spin);
+                if (lane < MAP_RG) {
+                    float* o = rab + (cc & 31) * 8;
+                    *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+                    o[4] = v[4];
+                }
+            };
+            __syncwarp();
+            load_above(0);
             __syncwarp();
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             const bool hasdn = act && r + 1 < Lq;
@@ -494,20 +494,8 @@ __device__ __forceinline__ void map_bwd_item(const MapArgs& a, const float* __re
                     const float4 ba = *reinterpret_cast<const float4*>(rab + src * 8);
                     const float b4 = rab[src * 8 + 4];
                     if (lane == 0) dn = S5{ba.x, ba.y, ba.z, ba.w, b4};
-                    if ((src & (MAP_RG - 1)) == MAP_RG - 1) {
-                        // the next group of columns into slots this step does not read
-                        if (s > 0 && k + 1 < L)
-                            pipe_wait(pf + s - 1, min(k + 1 + MAP_RG, L), lane, a.status, broken, a.spin);
-                        if (lane < MAP_RG) {
-                            const int cc = k + 1 + lane;
-                            float v[5];
-#pragma unroll
-                            for (int f = 0; f < 5; f++) v[f] = (s > 0 && cc < L) ? __ldcg(botr + f * L + cc) : binit[f];
-                            float* o = rab + (cc & 31) * 8;
-                            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-                            o[4] = v[4];
-                        }
-                    }
+                    // the next group of columns into slots this step does not read
+                    if ((src & (MAP_RG - 1)) == MAP_RG - 1) load_above(k + 1);
                 }
                 __syncwarp();
                 S5 rt = mine, dg = upp;         // successor to the right, diagonal successor
@@ -526,11 +514,7 @@ __device__ __forceinline__ void map_bwd_item(const MapArgs& a, const float* __re
                     const int lf = r & 31;
                     bsk[((long long)(r >> 5) * (L + 31) + (L - 1 - j) + lf) * 32 + lf] = nw.MM;
                 }
-                if (wr_bot && j >= 0 && j < L) {
-                    botw[0 * L + j] = nw.MM; botw[1 * L + j] = nw.MI; botw[2 * L + j] = nw.IM;
-                    botw[3 * L + j] = nw.DN; botw[4 * L + j] = nw.ND;
-                    pipe_publish(pf + s, j, L);
-                }
+                if (wr_bot && j >= 0 && j < L) row_put(rowm, ldr, j, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
                 mine = nw;
                 upp = dn;
                 if ((k & 31) == 31) {
@@ -620,10 +604,9 @@ __global__ void __launch_bounds__(MAPW * 32, 8) map_dp_kernel(MapArgs a)
         signed char* bt = a.btck + base;
         const float logZ = a.pairf[m * 4 + 1];
         const int edge = corner_edge_m(Lq, L);
-        float* bnd = a.bnd + (base / Lq) * 10;
-        const float* botr = bnd + ((s + 1) & 1) * 5 * L;   // last row of strip s-1
-        float* botw = bnd + (s & 1) * 5 * L;
-        int* pf = a.prog + (long long)m * nstrips;
+        const int ldr = row_ld(L);
+        float* rowm = a.bnd + nstrips * row_start(base / Lq, c) + (long long)s * ldr;   // this strip's last row
+        const float* rowa = rowm - ldr;                                                 // strip s - 1's
         float best = 0.f;
         int brow = 0x7fffffff, bcol = 0x7fffffff;
         {
@@ -633,8 +616,21 @@ __global__ void __launch_bounds__(MAPW * 32, 8) map_dp_kernel(MapArgs a)
             // row above the strip, one chunk at a time (lane i: column 32 c + i)
             // lane c & 31 holds column c of the row above, MAP_RG columns
             // loaded at a time, a group ahead
-            if (s > 0) pipe_wait(pf + s - 1, min(MAP_RG, L), lane, a.status, broken, a.spin);
-            float bcur = (s > 0 && lane < MAP_RG && lane < L) ? __ldcg(botr + lane) : 0.f;
+            float bcur = 0.f;
+            auto load_above = [&](int c0) {
+                const int d = (lane - c0) & 31;
+                const bool in = d < MAP_RG && c0 + d < L;
+                if (d < MAP_RG) bcur = 0.f;
+                if (s > 0 && c0 < L)
+                    row_poll(
+                        [&]() -> bool {
+                            if (!in) return true;
+                            asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(bcur) : "l"(rowa + c0 + d) : "memory");
+                            return __float_as_uint(bcur) != ROW_EMPTY;
+                        },
+                        lane, a.status, broken, a.spin);
+            };
+            load_above(0);
             const bool wr_bot = (lane == 31) && (s + 1 < nstrips);
             // F + B of the next step's cells is loaded one step ahead, from L2:
             // each chunk of 32 steps (32 lines of 128 bytes) is prefetched a
@@ -668,12 +664,7 @@ __global__ void __launch_bounds__(MAPW * 32, 8) map_dp_kernel(MapArgs a)
                         const int src = k & 31;
                         const float b0 = __shfl_sync(FULL, bcur, src);
                         if (lane == 0) up = b0;
-                        if ((src & (MAP_RG - 1)) == MAP_RG - 1) {
-                            if (s > 0 && k + 1 < L)
-                                pipe_wait(pf + s - 1, min(k + 1 + MAP_RG, L), lane, a.status, broken, a.spin);
-                            const int d = (lane - (k + 1)) & 31;
-                            if (d < MAP_RG) bcur = (s > 0 && k + 1 + d < L) ? __ldcg(botr + k + 1 + d) : 0.f;
-                        }
+                        if ((src & (MAP_RG - 1)) == MAP_RG - 1) load_above(k + 1);
                         if (src == 31) {
                             pf_line(fs, k + 33 + lane, W);
                             pf_line(bs, k + 33 + lane, W);
@@ -696,10 +687,8 @@ __global__ void __launch_bounds__(MAPW * 32, 8) map_dp_kernel(MapArgs a)
                         if (v < left - gap) { v = left - gap; b = BT_LEFT; }
                     }
                     if (valid) bout[j & 31][lane] = (signed char)b;
-                    if (wr_bot && j >= 0 && j < L) {
-                        botw[j] = v;
-                        pipe_publish(pf + s, j, L);
-                    }
+                    if (wr_bot && j >= 0 && j < L)
+                        asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(rowm + j), "f"(v) : "memory");
                     mine = v;
                     upp = up;
                     const int cfl = k - 31;
@@ -890,23 +879,19 @@ cudaError_t launch_viterbi_aln(const MapArgs& a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_map(const MapArgs& a, const float* qtrn, const float* dtrn, const float* qcf, int nsm,
+cudaError_t launch_map(MapArgs a, const float* qtrn, const float* dtrn, const float* qcf, int nsm,
                        int* counter, cudaStream_t st, int* nlaunch)
 {
     if (a.nmap <= 0) return cudaSuccess;
     const int nstrips = (a.Lq + 31) >> 5;
     const long long nitems = (long long)a.nmap * nstrips;
-    const size_t progb = (size_t)nitems * sizeof(int);
+    const size_t rowb = (size_t)nstrips * a.bnd_cols * sizeof(float);   // one float a column of every strip
     cudaError_t e;
-    // per sweep: fresh work counter and strip progress words
-    auto reset = [&]() -> cudaError_t {
-        cudaError_t r = cudaMemsetAsync(counter, 0, sizeof(int), st);
-        if (r == cudaSuccess) r = cudaMemsetAsync(a.prog, 0, progb, st);
-        return r;
-    };
     // grids: persistent CTAs, as many as fit on the SMs at once (the strip
     // pipeline is latency bound: every resident warp adds a wavefront in
     // flight), at most one warp per work item
+    // chunks of at most 6 warps an SM (16 KB each) fit in what the CTAs' shared memory leaves of L1
+    a.pf1 = 2 * nitems <= 6LL * nsm;
     const size_t fbs = (size_t)MAPFBW * MAPFB_WARP_FLOATS * sizeof(float);
     if ((e = cudaFuncSetAttribute(map_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fbs)) != cudaSuccess)
         return e;
@@ -919,11 +904,14 @@ cudaError_t launch_map(const MapArgs& a, const float* qtrn, const float* dtrn, c
     const int g = (int)std::min<long long>((long long)std::max(odp, 1) * nsm, (nitems + MAPW - 1) / MAPW);
     if ((e = cudaMemsetAsync(a.pairf, 0, (size_t)a.nmap * 4 * sizeof(float), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.pairk, 0, (size_t)a.nmap * sizeof(unsigned long long), st)) != cudaSuccess) return e;
-    if ((e = reset()) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(a.prog_b, 0, progb, st)) != cudaSuccess) return e;
+    // per sweep: fresh work counter, empty strip rows
+    if ((e = cudaMemsetAsync(counter, 0, sizeof(int), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.bnd, 0xff, 5 * rowb, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.bnd_b, 0xff, 5 * rowb, st)) != cudaSuccess) return e;
     map_fb_kernel<<<gfb, MAPFBW * 32, fbs, st>>>(a, qtrn, dtrn, qcf);
     map_z_kernel<<<a.nmap, 256, 0, st>>>(a);
-    if ((e = reset()) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(counter, 0, sizeof(int), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.bnd, 0xff, rowb, st)) != cudaSuccess) return e;
     map_dp_kernel<<<g, MAPW * 32, 0, st>>>(a);
     map_tb_kernel<<<(a.nmap + TBW - 1) / TBW, TBW * 32, 0, st>>>(a);
     *nlaunch += 4;

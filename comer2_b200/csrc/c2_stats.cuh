@@ -54,10 +54,10 @@ struct MapArgs {
     signed char* btck;          // [L][Lq] per candidate: MAP traceback codes
     float* pairf;               // [nmap][4]: maxF, logZ, map max, (unused)
     unsigned* pairc;            // [nmap]: MAP end coordinates
-    float* bnd;                 // per candidate at 10 x (cand_off / Lq): two last-row buffers [5][L]
-    int* prog;                  // [ncand][nstrips] finished columns per strip
-    float* bnd_b;               // backward sweep's strip-boundary rows (same layout as bnd)
-    int* prog_b;                // backward sweep's strip progress (same layout as prog)
+    float* bnd;                 // last rows of the strips (c2_device.cuh, row_start)
+    float* bnd_b;               // the backward sweep's
+    size_t bnd_cols;            // columns of a strip's rows over all candidates
+    int pf1;                    // few warps per SM: prefetch the scores into L1, not only L2
     const int* items;           // work item -> m * nstrips + strip (ready-time order)
     unsigned long long* pairk;  // [nmap] MAP DP maximum and end cell, packed for atomicMax
     int* status;
