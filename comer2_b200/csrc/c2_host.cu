@@ -201,6 +201,7 @@ struct c2_handle {
     std::vector<int> h_p2;          // passed pair -> candidate index
     DevBuf<int> d_p2;
     DevBuf<float> d_stats;
+    DevBuf<unsigned> d_hist;
     std::vector<float> h_stats;
     // MAP
     int nmap = 0;
@@ -1484,7 +1485,8 @@ extern "C" c2_status c2_run_stats(c2_handle* h, int32_t* npassed)
     h->npass = (int)h->h_p2.size();
     *npassed = h->npass;
     if (h->npass == 0) return C2_OK;
-    if (h->d_p2.ensure(h->npass, h->budget) || h->d_stats.ensure((size_t)h->npass * STATS_NOUT, h->budget))
+    if (h->d_p2.ensure(h->npass, h->budget) || h->d_stats.ensure((size_t)h->npass * STATS_NOUT, h->budget) ||
+        h->d_hist.ensure((size_t)h->npass * STATS_NBINS, h->budget))
         return fail(h, C2_ERR_NOMEM, "statistics buffers for %d pairs failed", h->npass);
     CK(cudaMemcpyAsync(h->d_p2.p, h->h_p2.data(), (size_t)h->npass * 4, cudaMemcpyHostToDevice, h->stream));
     StatsArgs a;
@@ -1512,9 +1514,12 @@ extern "C" c2_status c2_run_stats(c2_handle* h, int32_t* npassed)
     a.expglambda = h->prm.gapped_lambda;
     a.expgK = h->prm.gapped_K;
     a.out = h->d_stats.p;
+    a.hist = h->d_hist.p;
+    for (int c : h->h_p2) a.maxlen = std::max(a.maxlen, h->h_plen[h->h_cand[c]]);
+    CK(cudaMemsetAsync(h->d_hist.p, 0, (size_t)h->npass * STATS_NBINS * sizeof(unsigned), h->stream));
     if (!a.nnw || h->nnw.size() < 93) return fail(h, C2_ERR_ARG, "SS18 model weights missing (93 values needed)");
     CK(launch_stats(a, h->stream));
-    h->launches++;
+    h->launches += 2;
     return C2_OK;
 }
 
@@ -1526,7 +1531,7 @@ static c2_status viterbi_alignments(c2_handle* h)
 {
     const int nm = h->nmap;
     if (h->d_mapcand.ensure(nm, h->budget) || h->d_mappass.ensure(nm, h->budget) ||
-        h->d_pairf.ensure((size_t)nm * 4, h->budget) || h->d_pairc.ensure(nm, h->budget) ||
+        h->d_pairf.ensure((size_t)nm * 12, h->budget) || h->d_pairc.ensure(nm, h->budget) ||
         h->d_alninfo.ensure((size_t)nm * 8, h->budget) || h->d_aln.ensure((size_t)nm * 5 * h->alnstride, h->budget) ||
         h->d_pairk.ensure(nm, h->budget))
         return fail(h, C2_ERR_NOMEM, "alignment buffers for %d pairs failed", nm);
@@ -1616,7 +1621,7 @@ extern "C" c2_status c2_run_map(c2_handle* h, int32_t* nhits)
     for (int c = 0; c < h->ncand; c++) skl += (long long)h->h_plen[h->h_cand[c]] + 31;
     const size_t fbn = (size_t)32 * ((h->Lq + 31) / 32) * (size_t)skl;
     if (h->d_mapcand.ensure(nm, h->budget) || h->d_mappass.ensure(nm, h->budget) || h->d_fb.ensure(fbn, h->budget) || h->d_bb.ensure(fbn, h->budget) ||
-        h->d_pairf.ensure((size_t)nm * 4, h->budget) ||
+        h->d_pairf.ensure((size_t)nm * 12, h->budget) ||
         h->d_pairc.ensure(nm, h->budget) || h->d_alninfo.ensure((size_t)nm * 8, h->budget) || h->d_aln.ensure((size_t)nm * 5 * h->alnstride, h->budget) ||
         h->d_pairk.ensure(nm, h->budget))
         return fail(h, C2_ERR_NOMEM, "MAP buffers for %d pairs failed", nm);
@@ -1768,7 +1773,7 @@ static void release_phase2(c2_handle* h)
     h->d_cand_prof.release(); h->d_cand_off.release(); h->d_btck.release(); h->d_smat.release();
     h->d_mmat.release(); h->d_fscore.release(); h->d_fpsts.release(); h->d_fpassed.release();
     h->d_fbeg.release(); h->d_fend.release(); h->d_bnd.release(); h->d_tbkey.release();
-    h->d_worder.release(); h->d_tbitems.release(); h->d_mapitems.release(); h->d_p2.release(); h->d_stats.release();
+    h->d_worder.release(); h->d_tbitems.release(); h->d_mapitems.release(); h->d_p2.release(); h->d_stats.release(); h->d_hist.release();
     h->d_mapcand.release(); h->d_mappass.release(); h->d_alninfo.release(); h->d_fb.release(); h->d_bb.release();
     h->d_pairf.release(); h->d_pairc.release(); h->d_pairk.release(); h->d_aln.release(); h->d_alnpack.release();
     h->d_alnoff.release();
@@ -1783,7 +1788,7 @@ static size_t pair_scratch_bytes(const c2_handle* h, int L)
 {
     const size_t Lq = (size_t)h->Lq, ns = (Lq + 31) / 32;
     return 9 * Lq * (size_t)L + 2 * 5 * 4 * ns * ((size_t)L + 12) + 4 * ns * 2 + 2 * 4 * 32 * ns * ((size_t)L + 31) +
-           2 * 5 * (Lq + (size_t)h->Lmax + 1) + 512;
+           2 * 5 * (Lq + (size_t)h->Lmax + 1) + 4 * STATS_NBINS + 512;
 }
 
 // Candidate groups whose phase-2 scratch fits the handle's device memory

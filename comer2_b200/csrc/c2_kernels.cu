@@ -1741,12 +1741,19 @@ __device__ __forceinline__ float warp_butterfly(float v)
 }
 
 // DP finalisation, one warp per candidate pair
-// (src/libmycu/cudp/CuBatchDP_final.cu:170-290).
-__global__ void __launch_bounds__(256) fin_kernel(FinArgs a)
+// (src/libmycu/cudp/CuBatchDP_final.cu:170-290).  The walk from the maximum is a
+// serial chain; the warp stages 32 x 32 windows of the codes and scores in
+// shared memory for it (reading each cell from global memory took 0.3 ms on
+// paths of 300 steps).
+constexpr int FINW = 4;   // warps per CTA
+
+__global__ void __launch_bounds__(FINW * 32) fin_kernel(FinArgs a)
 {
-    __shared__ float cache[8][36];
+    __shared__ float cache[FINW][36];
+    __shared__ signed char wbt[FINW][32][33];
+    __shared__ float wsm[FINW][32][33];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int c = blockIdx.x * 8 + wid;
+    const int c = blockIdx.x * FINW + wid;
     if (c >= a.ncand) return;
     const int p = a.cand_prof[c];
     const int Lq = a.Lq;
@@ -1768,38 +1775,70 @@ __global__ void __launch_bounds__(256) fin_kernel(FinArgs a)
     }
     int x = (int)(xx >> 16), y = (int)(xx & 0xffff);
     int psts = 0;
-    int b = BT_DIAG;
-    int ndx = 0;
+    int ndx = 4;          // next slot of the chunk: slots 4..35, the last four of the chunk before in 0..3
     float sum = 0.f;
-    if (lane < 4) ch[32 + lane] = 0.f;
-    __syncwarp();
+    if (lane < 4) ch[lane] = 0.f;
     // the walk is bounded by the number of cells on any monotone path
     int guard = Lq + L + 2;
-    while (b != BT_STOP) {
-        if (lane < 4) ch[lane] = ch[32 + lane];
+    int stop = 0, x0 = 0, y0 = 0;
+    bool staged = false;
+    while (!stop) {
+        if (!staged && x >= 0 && y >= 0) {
+            x0 = x;
+            y0 = y;
+            const int qy = y0 - lane;
+            __syncwarp();
+#pragma unroll 16
+            for (int i = 0; i < 32; i++) {
+                const int cc = x0 - i;
+                signed char b = (signed char)BT_STOP;
+                float v = 0.f;
+                if (cc >= 0 && qy >= 0) {
+                    const long long k = (long long)cc * Lq + qy;
+                    b = bt[k];
+                    v = sm[k];
+                }
+                wbt[wid][i][lane] = b;
+                wsm[wid][i][lane] = v;
+            }
+            staged = true;
+        }
         __syncwarp();
+        int left = 0;     // the walk left the window
         if (lane == 0) {
-            for (ndx = 4; ndx < 36;) {
-                if (x < 0 || y < 0 || --guard < 0) { b = BT_STOP; break; }
-                const long long qp = (long long)x * Lq + y;
-                b = bt[qp];
-                if (b == BT_STOP) break;
+            while (ndx < 36) {
+                if (x < 0 || y < 0) { stop = 1; break; }
+                const int dx = x0 - x, dy = y0 - y;
+                if (dx >= 32 || dy >= 32) { left = 1; break; }
+                if (--guard < 0) { stop = 1; break; }
+                const int b = wbt[wid][dx][dy];
+                if (b == BT_STOP) { stop = 1; break; }
                 if (b == BT_UP) { y--; continue; }
                 if (b == BT_LEFT) { x--; continue; }
-                ch[ndx] = sm[qp];
-                if (ch[ndx] > 0.f) psts++;
+                const float v = wsm[wid][dx][dy];
+                ch[ndx] = v;
+                if (v > 0.f) psts++;
                 x--; y--;
                 ndx++;
             }
         }
         __syncwarp();
-        b = __shfl_sync(FULL, b, 0);
+        x = __shfl_sync(FULL, x, 0);
+        y = __shfl_sync(FULL, y, 0);
         ndx = __shfl_sync(FULL, ndx, 0);
-        float cs = 0.f;
-        if (!(ndx <= lane + 4))
-            cs = ch[lane + 4] * (((ch[lane] + ch[lane + 1]) + ch[lane + 2]) + ch[lane + 3]);
-        sum += warp_butterfly(cs);
-        __syncwarp();
+        stop = __shfl_sync(FULL, stop, 0);
+        if (__shfl_sync(FULL, left, 0)) staged = false;
+        if (stop || ndx == 36) {
+            float cs = 0.f;
+            if (!(ndx <= lane + 4))
+                cs = ch[lane + 4] * (((ch[lane] + ch[lane + 1]) + ch[lane + 2]) + ch[lane + 3]);
+            sum += warp_butterfly(cs);
+            const float keep = lane < 4 ? ch[32 + lane] : 0.f;
+            __syncwarp();
+            if (lane < 4) ch[lane] = keep;
+            ndx = 4;
+            __syncwarp();
+        }
     }
     if (lane == 0) {
         sum *= 0.5f;
@@ -1810,7 +1849,6 @@ __global__ void __launch_bounds__(256) fin_kernel(FinArgs a)
         a.beg[c] = ((unsigned)(x + 1) << 16) | ((unsigned)(y + 1) & 0xffffu);
         a.endc[c] = xx;
         a.passed[c] = (a.scorethld < maxsc && a.scorethld < sc) ? 1 : 0;
-        (void)L;
     }
 }
 
@@ -1917,8 +1955,7 @@ int p1_blocks_per_sm(int cvcard)
 cudaError_t launch_fin(const FinArgs& a, cudaStream_t st)
 {
     if (a.ncand <= 0) return cudaSuccess;
-    const int grid = (a.ncand + 7) / 8;
-    fin_kernel<<<grid, 256, 0, st>>>(a);
+    fin_kernel<<<(a.ncand + FINW - 1) / FINW, FINW * 32, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -29,6 +29,7 @@ constexpr int MAPDP_Q = 4;
 
 #define FULL 0xffffffffu
 constexpr float MLOG0 = -99.f;
+constexpr int PAIRF = 12, ZPART = 4;   // floats per pair of pairf, its first partial sum
 constexpr int MAPW = 4;     // warps per CTA of the MAP DP sweep
 constexpr int MAPFBW = 3;   // warps per CTA of the forward-backward sweeps (6 CTAs per SM fit)
 
@@ -358,47 +359,58 @@ __device__ __forceinline__ void map_fwd_item(const MapArgs& a, const float* __re
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) maxF = hmax(maxF, __shfl_xor_sync(FULL, maxF, o));
         // maxF >= 0, so its bit pattern orders as an unsigned integer
-        if (lane == 0) atomicMax(reinterpret_cast<unsigned*>(a.pairf + m * 4), __float_as_uint(maxF));
+        if (lane == 0) atomicMax(reinterpret_cast<unsigned*>(a.pairf + m * PAIRF), __float_as_uint(maxF));
         __syncwarp();
     }
 }
 
 // total forward probability: log sum over cells of exp(F.MM - maxF), + maxF
-// (src/libmycu/cumapdp/CuBatchMAPDP_bwd.cuh:185-290)
-__global__ void __launch_bounds__(256) map_z_kernel(MapArgs a)
+// (src/libmycu/cumapdp/CuBatchMAPDP_bwd.cuh:185-290).  Eight partial sums per
+// pair, each by a warp of its own (warp w takes rows w, w + 8, ... of the
+// [strips x W] rows; lane i of row (strip t, step k) is cell (32 t + i, k - i)),
+// eight rows loaded ahead; the MAP DP adds the eight up (map_logz).  With all
+// eight in one CTA a pair and the loads behind the bounds tests, 215 pairs of
+// 3,000 rows took 2.9 ms.
+__global__ void __launch_bounds__(128) map_z_kernel(MapArgs a)
 {
-    // one CTA per pair: per-thread partial sums over a strided range of the
-    // pair's cells, then a CTA reduction
-    __shared__ float part[8];
-    const int m = blockIdx.x;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int m = gw >> 3, wid = gw & 7;
+    if (m >= a.nmap) return;   // whole warp
     const int c = a.map_cand[m];
     const int p = a.cand_prof[c];
     const int Lq = a.Lq, L = a.plen[p], W = L + 31;
     const int nrows = ((Lq + 31) >> 5) * W;   // (strip, step) rows of 32 lanes
-    const float* fs = a.fb + skew_base(a, c);
-    const float maxF = a.pairf[m * 4 + 0];
+    const float* fs = a.fb + skew_base(a, c) + lane;
+    const float maxF = a.pairf[m * PAIRF + 0];
     float s = 0.f;
-    // warp w takes rows w, w + 8, ... of the [strips x W] rows; lane i of row
-    // (strip t, step k) is cell (32 t + i, k - i).  (t, k) advance without a
-    // division: W >= 32 > 8, so k wraps at most once per step.
+    // (t, k) advance without a division: W >= 32 > 8, so k wraps at most once per row
     int t = 0, k = wid;
-#pragma unroll 8
-    for (int rw = wid; rw < nrows; rw += 8) {
-        const int row = 32 * t + lane, col = k - lane;
-        if (row < Lq && col >= 0 && col < L) s += fexp(fs[(long long)rw * 32 + lane] - maxF);
-        k += 8;
-        if (k >= W) { k -= W; t++; }
+    for (int r0 = wid; r0 < nrows; r0 += 64) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = r0 + 8 * u < nrows ? fs[(long long)(r0 + 8 * u) * 32] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int row = 32 * t + lane, col = k - lane;
+            if (r0 + 8 * u < nrows && row < Lq && col >= 0 && col < L) s += fexp(v[u] - maxF);
+            k += 8;
+            if (k >= W) { k -= W; t++; }
+        }
     }
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-    if (lane == 0) part[wid] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int w = 0; w < 8; w++) t += part[w];
-        a.pairf[m * 4 + 1] = flog(t) + maxF;
-    }
+    if (lane == 0) a.pairf[m * PAIRF + ZPART + wid] = s;
+}
+
+// log of the pair's total probability from the eight partial sums
+__device__ __forceinline__ float map_logz(const MapArgs& a, int m)
+{
+    const float* f = a.pairf + m * PAIRF;
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) t += f[ZPART + w];
+    return flog(t) + f[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -602,7 +614,7 @@ __global__ void __launch_bounds__(MAPW * 32, 8) map_dp_kernel(MapArgs a)
         const float* fs = a.fb + sko;
         const float* bs = a.bb + sko;
         signed char* bt = a.btck + base;
-        const float logZ = a.pairf[m * 4 + 1];
+        const float logZ = map_logz(a, m);
         const int edge = corner_edge_m(Lq, L);
         const int ldr = row_ld(L);
         float* rowm = a.bnd + nstrips * row_start(base / Lq, c) + (long long)s * ldr;   // this strip's last row
@@ -729,11 +741,13 @@ __global__ void __launch_bounds__(TBW * 32) map_tb_kernel(MapArgs a)
     // moves by one row and/or column per step; the warp stages 32 x 32 windows
     // of the traceback codes and scores (columns x0 - 31 .. x0, rows
     // y0 - 31 .. y0) and the letters of those rows and columns in shared
-    // memory, lane 0 walks inside the window, and the warp restages where the
-    // walk leaves it.
+    // memory, lane 0 walks inside the window noting each step's code and cell,
+    // the lanes then write the letters of the steps, and the warp restages
+    // where the walk leaves the window.
     __shared__ signed char wbt[TBW][32][33];
     __shared__ float wsm[TBW][32][33];
     __shared__ unsigned char wq[TBW][2][32], wd[TBW][2][32];   // [residue, SS][offset]
+    __shared__ unsigned short wpath[TBW][64];                  // code | dx << 2 | dy << 7
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int m = blockIdx.x * TBW + wid;
     if (m >= a.nmap) return;   // whole warp
@@ -750,32 +764,33 @@ __global__ void __launch_bounds__(TBW * 32) map_tb_kernel(MapArgs a)
     const unsigned cell = 0xffffffffu - (unsigned)(key & 0xffffffffu);
     const unsigned xx = (key != 0ull) ? (((cell & 0xffffu) << 16) | (cell >> 16)) : 0u;
     if (lane == 0) {
-        a.pairf[m * 4 + 2] = mbest;
+        a.pairf[m * PAIRF + 2] = mbest;
         a.pairc[m] = xx;
     }
     int x = (int)(xx >> 16), y = (int)(xx & 0xffff);
     char* o = a.aln + (size_t)m * 5 * a.alnstride;
     char *tq = o, *tm = o + a.alnstride, *tt = o + 2 * a.alnstride, *sq = o + 3 * a.alnstride,
          *st = o + 4 * a.alnstride;
-    int n = 0, idts = 0, psts = 0, gaps = 0;
+    int n = 0, idts = 0, psts = 0, gaps = 0;   // the counts: this lane's steps, added up at the end
     const int cap = a.alnstride - 1;
     int done = 0;
     while (!done && n < cap && x >= 0 && y >= 0) {
         const int x0 = x, y0 = y;
         {
             const int cx = x0 - lane, qy = y0 - lane;
-#pragma unroll 4
-            for (int r = 0; r < 32; r++) {
-                const int ry = y0 - r;
+            // a column's 32 rows are contiguous
+#pragma unroll 16
+            for (int i = 0; i < 32; i++) {
+                const int cc = x0 - i;
                 signed char b = (signed char)BT_STOP;
                 float v = 0.f;
-                if (cx >= 0 && ry >= 0) {
-                    const long long k = (long long)cx * Lq + ry;
+                if (cc >= 0 && qy >= 0) {
+                    const long long k = (long long)cc * Lq + qy;
                     b = bt[k];
                     v = sm[k];
                 }
-                wbt[wid][lane][r] = b;
-                wsm[wid][lane][r] = v;
+                wbt[wid][i][lane] = b;
+                wsm[wid][i][lane] = v;
             }
             wq[wid][0][lane] = qy >= 0 ? a.qaa[qy] : 0;
             wq[wid][1][lane] = (a.qss && qy >= 0) ? a.qss[qy] : ' ';
@@ -783,45 +798,43 @@ __global__ void __launch_bounds__(TBW * 32) map_tb_kernel(MapArgs a)
             wd[wid][1][lane] = (a.dss && cx >= 0) ? a.dss[off + cx] : ' ';
         }
         __syncwarp();
+        int np = 0;
         if (lane == 0) {
-            while (n < cap) {
+            // (a monotone walk inside the window has at most 63 steps)
+            while (n + np < cap && np < 64) {
                 if (x < 0 || y < 0) { done = 1; break; }
                 const int dx = x0 - x, dy = y0 - y;
                 if (dx >= 32 || dy >= 32) break;   // left the window
                 const int b = wbt[wid][dx][dy];
                 if (b == BT_STOP) { done = 1; break; }
-                sq[n] = ' ';
-                st[n] = ' ';
-                if (b == BT_UP) {
-                    gaps++;
-                    tq[n] = (char)wq[wid][0][dy]; tt[n] = '-'; tm[n] = ' ';
-                    if (a.qss) sq[n] = (char)wq[wid][1][dy];
-                    n++; y--;
-                    continue;
-                }
-                if (b == BT_LEFT) {
-                    gaps++;
-                    tq[n] = '-'; tt[n] = (char)wd[wid][0][dx]; tm[n] = ' ';
-                    if (a.dss) st[n] = (char)wd[wid][1][dx];
-                    n++; x--;
-                    continue;
-                }
-                const char cq = (char)wq[wid][0][dy], cd = (char)wd[wid][0][dx];
-                tq[n] = cq;
-                tt[n] = cd;
-                if (a.qss) sq[n] = (char)wq[wid][1][dy];
-                if (a.dss) st[n] = (char)wd[wid][1][dx];
-                if (cq == cd) { tm[n] = cq; idts++; }
-                else if (wsm[wid][dx][dy] > 0.f) { tm[n] = '+'; psts++; }
-                else tm[n] = ' ';
-                n++; x--; y--;
+                wpath[wid][np++] = (unsigned short)(b | (dx << 2) | (dy << 7));
+                if (b != BT_LEFT) y--;
+                if (b != BT_UP) x--;
             }
         }
         x = __shfl_sync(FULL, x, 0);
         y = __shfl_sync(FULL, y, 0);
-        n = __shfl_sync(FULL, n, 0);
+        np = __shfl_sync(FULL, np, 0);
         done = __shfl_sync(FULL, done, 0);
         __syncwarp();
+        for (int i = lane; i < np; i += 32) {
+            const int w = wpath[wid][i], b = w & 3, dx = (w >> 2) & 31, dy = (w >> 7) & 31;
+            const char cq = (char)wq[wid][0][dy], cd = (char)wd[wid][0][dx];
+            char c0 = cq, c1 = ' ', c2 = cd, c3 = (char)wq[wid][1][dy], c4 = (char)wd[wid][1][dx];
+            if (b == BT_UP) { c2 = '-'; c4 = ' '; gaps++; }
+            else if (b == BT_LEFT) { c0 = '-'; c3 = ' '; gaps++; }
+            else if (cq == cd) { c1 = cq; idts++; }
+            else if (wsm[wid][dx][dy] > 0.f) { c1 = '+'; psts++; }
+            tq[n + i] = c0; tm[n + i] = c1; tt[n + i] = c2; sq[n + i] = c3; st[n + i] = c4;
+        }
+        n += np;
+        __syncwarp();
+    }
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+        idts += __shfl_xor_sync(FULL, idts, d);
+        psts += __shfl_xor_sync(FULL, psts, d);
+        gaps += __shfl_xor_sync(FULL, gaps, d);
     }
     // the walk produced the strings back to front: reverse them across the warp
     for (int rr = 0; rr < 5; rr++) {
@@ -902,14 +915,14 @@ cudaError_t launch_map(MapArgs a, const float* qtrn, const float* dtrn, const fl
         return e;
     const int gfb = (int)std::min<long long>((long long)std::max(ofb, 1) * nsm, (2 * nitems + MAPFBW - 1) / MAPFBW);
     const int g = (int)std::min<long long>((long long)std::max(odp, 1) * nsm, (nitems + MAPW - 1) / MAPW);
-    if ((e = cudaMemsetAsync(a.pairf, 0, (size_t)a.nmap * 4 * sizeof(float), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.pairf, 0, (size_t)a.nmap * PAIRF * sizeof(float), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.pairk, 0, (size_t)a.nmap * sizeof(unsigned long long), st)) != cudaSuccess) return e;
     // per sweep: fresh work counter, empty strip rows
     if ((e = cudaMemsetAsync(counter, 0, sizeof(int), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.bnd, 0xff, 5 * rowb, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.bnd_b, 0xff, 5 * rowb, st)) != cudaSuccess) return e;
     map_fb_kernel<<<gfb, MAPFBW * 32, fbs, st>>>(a, qtrn, dtrn, qcf);
-    map_z_kernel<<<a.nmap, 256, 0, st>>>(a);
+    map_z_kernel<<<2 * a.nmap, 128, 0, st>>>(a);
     if ((e = cudaMemsetAsync(counter, 0, sizeof(int), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.bnd, 0xff, rowb, st)) != cudaSuccess) return e;
     map_dp_kernel<<<g, MAPW * 32, 0, st>>>(a);

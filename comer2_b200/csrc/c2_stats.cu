@@ -3,11 +3,11 @@
 // -10..10, threadIdx.x = one of the 32 scaled scores of that unit), the
 // layout of the reference's CalcStatParamsDynPlmProfile
 // (src/libmycu/cuss/CuBatchSS_dynplm.cu:193-430).  The reference spreads
-// this over five dynamic-parallelism launches per pair; here one kernel
-// computes, per pair:
+// this over five dynamic-parallelism launches per pair; here two kernels
+// compute, per pair:
 //  * the histogram of rint(32 s) over the pair's score matrix (cells whose
-//    query or db residue is 'X' skipped when X_UNINF) in shared memory
-//    (_dynplm.cu:80-183);
+//    query or db residue is 'X' skipped when X_UNINF; _dynplm.cu:80-183),
+//    by a kernel of its own before the rest;
 //  * probabilities, expected score, score range, lambda by Newton-Raphson
 //    with bisection, relative entropy and K (_expected.cuh, _minmax.cuh,
 //    _lambda.cuh, _entropy.cuh, _K.cuh);
@@ -321,6 +321,54 @@ __device__ float evalue_ss18(const StatsArgs& a, int nq, int nd, float score, fl
     return lexp;
 }
 
+// ---- score histograms of the passed pairs: counts of rint(32 s), s clamped to
+// [-10, 10].  Blocks of HIST_COLS db columns of a pair are CTAs of their own (a
+// warp takes a column, its lanes the query rows: coalesced reads, eight rows a
+// lane loaded before their counts are added), added to the pair's counts with
+// integer atomics: exact, whatever the order.  Within the statistics kernel, one
+// CTA a pair, the longest pair's 6 million cells took 2.1 ms (1 x 3,000 vs 4,000
+// profiles); read at HBM speed all pairs' cells take 0.15 ms.
+constexpr int HIST_COLS = 32, HIST_WARPS = 8;
+static_assert(STATS_NBINS == NSCALED, "histogram size");
+
+__global__ void __launch_bounds__(HIST_WARPS * 32) hist_kernel(StatsArgs a)
+{
+    __shared__ unsigned hist[NSCALED];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int c = a.p2_cand[blockIdx.x];
+    const int p = a.cand_prof[c];
+    const int Lq = a.Lq, L = a.plen[p];
+    const int x0 = blockIdx.y * HIST_COLS;
+    if (x0 >= L) return;   // whole CTA
+    const long long off = a.poff[p];
+    const float* __restrict__ sm = a.smat + a.cand_off[c];
+    for (int k = threadIdx.x; k < NSCALED; k += HIST_WARPS * 32) hist[k] = 0u;
+    __syncthreads();
+    for (int x = x0 + wid; x < min(x0 + HIST_COLS, L); x += HIST_WARPS) {
+        if (a.xuninf && a.daa[off + x] == 'X') continue;
+        const float* __restrict__ col = sm + (long long)x * Lq;
+        for (int y0 = lane; y0 < Lq; y0 += 8 * 32) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int y = y0 + u * 32;
+                v[u] = y < Lq ? col[y] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int y = y0 + u * 32;
+                if (y >= Lq || (a.xuninf && a.qaa[y] == 'X')) continue;
+                const float s = v[u] < -10.f ? -10.f : (v[u] > 10.f ? 10.f : v[u]);
+                atomicAdd(&hist[(int)rintf(s * SCF) - SMIN], 1u);
+            }
+        }
+    }
+    __syncthreads();
+    unsigned* out = a.hist + (size_t)blockIdx.x * NSCALED;
+    for (int k = threadIdx.x; k < NSCALED; k += HIST_WARPS * 32)
+        if (hist[k]) atomicAdd(out + k, hist[k]);
+}
+
 // ---- the per-pair statistics kernel
 __global__ void __launch_bounds__(SCF * NDS, 2) stats_kernel(StatsArgs a)
 {
@@ -335,36 +383,8 @@ __global__ void __launch_bounds__(SCF * NDS, 2) stats_kernel(StatsArgs a)
     const int c = a.p2_cand[pi];            // candidate index
     const int p = a.cand_prof[c];
     const int Lq = a.Lq, L = a.plen[p];
-    const long long off = a.poff[p];
-    const float* __restrict__ sm = a.smat + a.cand_off[c];
-    __shared__ unsigned hist[NSCALED];
-    for (int k = tid; k < NSCALED + 31; k += SCF * NDS) counts[k] = 0.f;
-    for (int k = tid; k < NSCALED; k += SCF * NDS) hist[k] = 0u;
-    __syncthreads();
-    // histogram of rint(32 s), s clamped to [-10, 10]: warp ty takes db
-    // columns, its lanes the query rows of a column (coalesced reads), eight
-    // rows per lane loaded before their counts are added (loads in flight)
-    for (int x = ty; x < L; x += NDS) {
-        if (a.xuninf && a.daa[off + x] == 'X') continue;
-        const float* __restrict__ col = sm + (long long)x * Lq;
-        for (int y0 = tx; y0 < Lq; y0 += 8 * SCF) {
-            float v[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int y = y0 + u * SCF;
-                v[u] = y < Lq ? col[y] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int y = y0 + u * SCF;
-                if (y >= Lq || (a.xuninf && a.qaa[y] == 'X')) continue;
-                const float s = v[u] < -10.f ? -10.f : (v[u] > 10.f ? 10.f : v[u]);
-                atomicAdd(&hist[(int)rintf(s * SCF) - SMIN], 1u);
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = tid; k < NSCALED; k += SCF * NDS) counts[k] = (float)hist[k];
+    for (int k = tid; k < NSCALED + 31; k += SCF * NDS)
+        counts[k] = k < NSCALED ? (float)a.hist[(size_t)pi * NSCALED + k] : 0.f;
     __syncthreads();
     // probability layout: row ty holds the scaled scores of unscaled score ty-10
     const int u = ty - 10;
@@ -539,6 +559,8 @@ __global__ void __launch_bounds__(SCF * NDS, 2) stats_kernel(StatsArgs a)
 cudaError_t launch_stats(const StatsArgs& a, cudaStream_t st)
 {
     if (a.npass <= 0) return cudaSuccess;
+    const dim3 hg(a.npass, (a.maxlen + HIST_COLS - 1) / HIST_COLS);
+    hist_kernel<<<hg, HIST_WARPS * 32, 0, st>>>(a);
     stats_kernel<<<a.npass, dim3(SCF, NDS), 0, st>>>(a);
     return cudaGetLastError();
 }

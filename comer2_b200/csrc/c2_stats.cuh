@@ -28,8 +28,11 @@ struct StatsArgs {
     const float* nnw;           // SS18 weights and adjustment constants
     int ssemodel, xuninf;
     float qeno, searchspace, reflambda, refK, expglambda, expgK;
+    unsigned* hist;             // [npass][STATS_NBINS] counts of rint(32 s), zeroed before the launch
+    int maxlen;                 // longest profile of the passed pairs
     float* out;                 // [npass][STATS_NOUT]
 };
+constexpr int STATS_NBINS = 641;
 
 // MAP stage: one warp per pair whose log E-value is within the threshold
 struct MapArgs {
@@ -52,7 +55,7 @@ struct MapArgs {
                                 // wavefront order (c2_map.cu, skew_base)
     float* bb;                  // B (backward values), the same layout
     signed char* btck;          // [L][Lq] per candidate: MAP traceback codes
-    float* pairf;               // [nmap][4]: maxF, logZ, map max, (unused)
+    float* pairf;               // [nmap][12]: maxF, (unused), map max, (unused), the 8 partial sums of map_z_kernel
     unsigned* pairc;            // [nmap]: MAP end coordinates
     float* bnd;                 // last rows of the strips (c2_device.cuh, row_start)
     float* bnd_b;               // the backward sweep's
