@@ -66,9 +66,10 @@ constexpr int MAX_CVCARD = 256;
 //     2: cv lo k0-15 (2), cv hi k16-23, cv lo k16-23
 //     3: ss hi k0-15 (2), ss hi k16-31 (2)     4: ss lo, the same
 // query operands (A fragments, strips of 64 rows) per query: context vectors
-// and SS tables qa[strip][mtile 4][7][lane 32][4 words] (cv hi k0-15 (4), hi
-// k16-23 (2), lo k0-15 (4), lo k16-23 (2); ss hi k0-15 (4), hi k16-31 (4), lo
-// k0-15 (4), lo k16-31 (4)) and the unscaled amino-acid rows
+// and SS tables qa[strip][mtile 4][7][lane 32][4 words] (cv hi k0-15, lo k0-15; ss
+// hi k0-15, hi k16-31, lo k0-15, lo k16-31; cv hi k16-23 (2), lo k16-23 (2):
+// groups of 4 words, so that every fragment lands in aligned registers) and the
+// unscaled amino-acid rows
 // qaa[strip][mtile 4][3][lane 32][4 floats] (k0-15: 8, k16-23: 4; scaled per
 // pair by 1 / (0.5 (bq + bd)) and split).
 // The constant parts of the CV and SS terms ride in the spare K columns:

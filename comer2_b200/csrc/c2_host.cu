@@ -930,18 +930,20 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
                         qa[((o + at / 4) * 32 + lane) * 4 + at % 4] = w;
                         at++;
                     };
-                    for (int d = 0; d < 2; d++) {
-                        const int nw = d == 0 ? 6 : 8;
-                        uint32_t lo[8];
-                        for (int w = 0; w < nw; w++) {
+                    uint32_t hi[2][8], lo[2][8];
+                    for (int d = 0; d < 2; d++)
+                        for (int w = 0; w < (d == 0 ? 6 : 8); w++) {
                             const int r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq;
                             const float x0 = aval(d, r, k), x1 = aval(d, r, k + 1);
                             const uint32_t h0 = bf16_rn_bits(x0), h1 = bf16_rn_bits(x1);
-                            lo[w] = bf16_rn_bits(x0 - bf16_to_f(h0)) | (bf16_rn_bits(x1 - bf16_to_f(h1)) << 16);
-                            put(h0 | (h1 << 16));
+                            hi[d][w] = h0 | (h1 << 16);
+                            lo[d][w] = bf16_rn_bits(x0 - bf16_to_f(h0)) | (bf16_rn_bits(x1 - bf16_to_f(h1)) << 16);
                         }
-                        for (int w = 0; w < nw; w++) put(lo[w]);
-                    }
+                    for (int w = 0; w < 4; w++) put(hi[0][w]);
+                    for (int w = 0; w < 4; w++) put(lo[0][w]);
+                    for (int w = 0; w < 8; w++) put(hi[1][w]);
+                    for (int w = 0; w < 8; w++) put(lo[1][w]);
+                    put(hi[0][4]); put(hi[0][5]); put(lo[0][4]); put(lo[0][5]);
                     for (int e = 0; e < 12; e++) {
                         const int w = e >> 1, r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq + (e & 1);
                         qaa[(((size_t)(s * 4 + mt) * 3 + e / 4) * 32 + lane) * 4 + e % 4] =
@@ -1101,6 +1103,7 @@ static void fill_p1(c2_handle* h, P1Args& a)
     a.coords = h->d_coords.p;
     a.status = h->d_status.p;
     a.spin = h->spin;
+    a.tc = tc_consts(h->sc);
 }
 
 // Phase-1 pairs whose strips become work items of their own (p1_take): those
@@ -1108,7 +1111,13 @@ static void fill_p1(c2_handle* h, P1Args& a)
 // time all pairs together take on all warps (both grow with the number of
 // strips alike, so the query length does not enter).  Pairs below that even
 // out over the warps by the longest-first order; pairs above it would be the
-// tail of the search.  0 without the scratch (it is small: the two boundary
+// tail of the search.  Phase-1 times with shares of infinity (none split) / 1 /
+// 0.5 / 0.25 / 0.1: 1 x 3,000 vs 4,000 profiles 41.9 / 23.2 / 23.8 / 26.7 / 25.7
+// ms, 1 x 1,237 vs 4,999 16.2 / 9.7 / 10.4 / 10.8 / 11.3, 1 x 250 vs 3,000 (FP32)
+// 4.5 / 2.3 / 2.1 / 2.3 / 2.3, 7 queries vs 1,000 (FP32) 32 / 11 / 8.4 / 8.6 /
+// 8.6, 1 x 150 vs 2,000 0.70 / 0.66 / 0.60 / 0.57 / 0.55 (with strips of 32 rows);
+// no pair is split, and nothing changes, against 50,000 profiles.  0 without the
+// scratch (it is small: the two boundary
 // rows of the split pairs) -- the pairs then run whole, with the same results.
 constexpr double SPLIT_SHARE = 0.5;
 
@@ -1158,7 +1167,6 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
         a.cold = h->db->d_cold.p;
         a.qa = h->d_qa.p;
         a.qaa = h->d_qaaf.p;
-        a.tc = tc_consts(h->sc);
         cudaError_t oe = cudaSuccess;
         int gt = (h->nsm - h->p1_reserve) * p1t_blocks_per_sm(h->sc.cvcard, &oe);
         if (gt < 1)

@@ -87,11 +87,22 @@ __device__ __forceinline__ void row_ops(RowOps& R, const float* __restrict__ qr,
     R.hq = qr[QR_HQ];
 }
 
+// hardware base-2 logarithm, denormal inputs flushed (the arguments here, an
+// amino-acid odds sum and a CV determinant, are far above the denormal range)
+constexpr float C2_LN2 = 0.693147180559945309f;
+__device__ __forceinline__ float lg2_ftz(float x)
+{
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Scores of NR consecutive rows; the SS row table U has USTR floats a column,
 // the lane's first row at U[urow].  cvtab holds each CV map value CVREP times
 // ([cvcard][CVREP]); a lane reads replica lane % CVREP so that lanes reading
-// different entries rarely share a bank.
-template <int CVREP, int NR, int USTR>
+// different entries rarely share a bank.  CVUNIF: the table's key range
+// coincides with its index clamp (TcConsts).
+template <int CVREP, int NR, int USTR, bool CVUNIF>
 __device__ __forceinline__ void cell_scores(const RowOps* R, const float* __restrict__ rec,
                                             const float* __restrict__ U, int urow, const float* __restrict__ cvtab,
                                             const ScoreConsts& sc, int lane, float* S, float* mod_out)
@@ -133,19 +144,17 @@ __device__ __forceinline__ void cell_scores(const RowOps* R, const float* __rest
     }
 #pragma unroll
     for (int e = 0; e < NR; e++) {
-        const float s0 = __logf(lo2(s[e]) + hi2(s[e])) - sc.shift;
+        const float s0 = lg2_ftz(lo2(s[e]) + hi2(s[e])) * C2_LN2 - sc.shift;
         const float dt = (lo2(dot[e]) + hi2(dot[e])) + sc.lokappa0;
         const float det = R[e].cq * cd - dt * dt;
-        const float cvs = sc.cterm + sc.pownu0 * __logf(det) - R[e].pq - v10.x;
-        float cvm;
-        if (cvs <= sc.cvkey_first) cvm = sc.cvval_first;
-        else if (sc.cvkey_last <= cvs) cvm = sc.cvval_last;
-        else {
-            // clamp keeps the shared-memory read in bounds for any table/argument
-            const int ix = min(max(sc.cvshift + (int)rintf(2.f * cvs), 0), sc.cvcard - 1);
-            cvm = cvtab[ix * CVREP + (lane & (CVREP - 1))];
+        const float cvs = sc.cterm + sc.pownu0 * (lg2_ftz(det) * C2_LN2) - R[e].pq - v10.x;
+        // clamp keeps the shared-memory read in bounds for any table/argument
+        const int ix = min(max(sc.cvshift + __float2int_rn(2.f * cvs), 0), sc.cvcard - 1);
+        float cvm = cvtab[ix * CVREP + (lane & (CVREP - 1))];
+        if (!CVUNIF) {
+            cvm = (sc.cvkey_last <= cvs) ? sc.cvval_last : cvm;
+            cvm = (cvs <= sc.cvkey_first) ? sc.cvval_first : cvm;
         }
-        cvm *= sc.cvswgt;
         // SS term
         float ss = v10.y * w[0][e];
         ss = fmaf(v10.z, w[1][e], ss);
@@ -155,7 +164,7 @@ __device__ __forceinline__ void cell_scores(const RowOps* R, const float* __rest
             ss -= 0.05f;
             ss *= sc.ssswgt;
         }
-        const float add = ss + cvm;
+        const float add = fmaf(cvm, sc.cvswgt, ss);
         mod_out[e] = add - 0.5f * sc.cvswgt;   // modular score of the MAP stage
         S[e] = s0 + add;
     }
@@ -299,7 +308,7 @@ p1_kernel(P1Args a, const float* __restrict__ qbkg)
                 if (k < L) {
                     const float4* rp = reinterpret_cast<const float4*>(rec + (k & (REC_SLOTS - 1)) * DR_STRIDE);
                     float mod, S;
-                    cell_scores<32, 1, 32>(&R, reinterpret_cast<const float*>(rp), U, lane, cvtab, sc, lane, &S, &mod);
+                    cell_scores<32, 1, 32, false>(&R, reinterpret_cast<const float*>(rp), U, lane, cvtab, sc, lane, &S, &mod);
                     if (!act) S = -9.f;
                     ring[(k & 31) * 32 + lane] = S;
                     const float4 ta = rp[12], tb = rp[13];
@@ -810,6 +819,7 @@ __device__ __forceinline__ void wf2_steps4(Wf2& D, const Wf2Edge& E, const float
 // instruction issue: two rows a lane halve the record reads and the DP's
 // shuffles, column and row-above reads per cell, and the packed dot products
 // halve the multiply-adds' issue slots.
+template <bool CVUNIF>
 __global__ void __launch_bounds__(P1C_WARPS * 32, 1)
 p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 {
@@ -856,6 +866,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
         for (int s = it.s0; s < it.s1; s++) {
             __syncwarp();
             const int r0 = P1_ROWS * s + 2 * lane;   // the lane's first row
+            const int kend = L + ((min(P1_ROWS, Lq - P1_ROWS * s) - 1) >> 1);   // wavefront steps
             RowOps R[2];
 #pragma unroll
             for (int e = 0; e < 2; e++) row_ops(R[e], a.qrec + (long long)min(r0 + e, Lq - 1) * QR_STRIDE, qbkg, bd);
@@ -890,7 +901,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
             cp_async_commit();
             int sg = 0;                                 // slot of the chunk's first anti-diagonal
             int cs = 0, cl = lane == 0 ? 0 : P1_CMOD - lane;
-            for (int m = 0; P1_C * m < L + 31; m++) {
+            for (int m = 0; P1_C * m < kend; m++) {
                 const int k0 = P1_C * m;
                 // the row above for this chunk's steps, copied during the score stage
                 p1_row_async(a, it, s, bnd, botr, ldb, k0, lane, broken);
@@ -908,7 +919,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
                         float S[2] = {-INFINITY, -INFINITY};
                         if (k0 + u < L) {
                             float mod[2];
-                            cell_scores<P1C_CVREP, 2, P1_ROWS>(R, rc + u * DR_STRIDE, U, 2 * lane, cvtab, sc, lane, S, mod);
+                            cell_scores<P1C_CVREP, 2, P1_ROWS, CVUNIF>(R, rc + u * DR_STRIDE, U, 2 * lane, cvtab, sc, lane, S, mod);
                             if (hasc) {
                                 const int c = k0 + u;
                                 if (c <= cA0 || c >= cB0) S[0] = -9.f;
@@ -942,7 +953,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
                 if (s + 1 < nstrips) {
                     p1_row_flush(bnd, botw, ldb, k0, L, lane);
                     // columns up to k0 - 24 are there: published every other chunk
-                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= L + 31))
+                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= kend))
                         p1_publish(a, it, s, min(k0 - 23, L), lane);
                 }
                 // next chunk; chunk m + 2's records and transitions into slots no longer read
@@ -975,6 +986,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 // FP32 form.  One warp per (candidate, strip) at a time, lanes own query rows,
 // db records staged in shared memory as in phase 1; no dependencies between
 // work items, so every resident warp works.
+template <bool CVUNIF>
 __global__ void __launch_bounds__(P2S_WARPS * 32)
 p2s_kernel(P1Args a, const float* __restrict__ qbkg)
 {
@@ -1032,7 +1044,7 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
                 if (c < L) {
                     const float* rc = rec + (c & (REC_SLOTS - 1)) * DR_STRIDE;
                     float mod, Sc;
-                    cell_scores<P1TC_CVREP, 1, 32>(&R, rc, U, lane, cvtab, sc, lane, &Sc, &mod);
+                    cell_scores<P1TC_CVREP, 1, 32, CVUNIF>(&R, rc, U, lane, cvtab, sc, lane, &Sc, &mod);
                     if (act) {
                         smt[(long long)c * Lq + r] = Sc;
                         mmt[(long long)c * Lq + r] = mod;
@@ -1253,8 +1265,9 @@ __device__ __forceinline__ void tmem_st40(unsigned taddr, const unsigned* v)
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 40 columns into v; the wait takes v as operands so no use of v can be
-// scheduled before the loads have completed
+// 40 columns into v: the loads, and the wait for them.  The wait takes v as
+// operands, so no use of v can be scheduled before the loads have completed;
+// nothing may touch v in between.
 __device__ __forceinline__ void tmem_ld40(unsigned taddr, unsigned* v)
 {
     asm volatile(
@@ -1267,11 +1280,13 @@ __device__ __forceinline__ void tmem_ld40(unsigned taddr, unsigned* v)
         : "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39])
         : "r"(taddr + 32)
         : "memory");
+}
+__device__ __forceinline__ void tmem_ld40_wait(unsigned* v)
+{
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19])
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]), "+r"(v[32]), "+r"(v[33]), "+r"(v[34]), "+r"(v[35]), "+r"(v[36]), "+r"(v[37]), "+r"(v[38]), "+r"(v[39])
                  :
                  : "memory");
-    asm volatile("" : "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]), "+r"(v[32]), "+r"(v[33]), "+r"(v[34]), "+r"(v[35]), "+r"(v[36]), "+r"(v[37]), "+r"(v[38]), "+r"(v[39]));
 }
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
@@ -1382,15 +1397,6 @@ __global__ void __launch_bounds__(128) tc_pack_kernel(const float* __restrict__ 
 //         the rounding of the split-BF16 products (this form only ranks the
 //         pairs; the candidates are rescored in FP32)
 // (cell_score is the FP32 form; src/libmycu/cusco/CuBatchScoreMatrix_ddms2s_h2.cu)
-constexpr float C2_LN2 = 0.693147180559945309f;
-// hardware base-2 logarithm, denormal inputs flushed (the arguments here, an
-// amino-acid odds sum and a CV determinant, are far above the denormal range)
-__device__ __forceinline__ float lg2_ftz(float x)
-{
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 template <bool CVUNIF>
 __device__ __forceinline__ float tc_cell(float daa, float dot, float ss, float cq, float rq2, float cd, float pd2,
                                          const float* __restrict__ cvl, const TcConsts& tc)
@@ -1509,6 +1515,9 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
 
         for (int s = it.s0; s < it.s1; s++) {
             __syncwarp();
+            const int rows = min(P1_ROWS, Lq - P1_ROWS * s);   // of the query in this strip
+            const int nmt = (rows + 15) >> 4;                  // m-tiles holding any
+            const int kend = L + ((rows - 1) >> 1);            // wavefront steps
             // this strip's query fragments into TMEM, 40 columns per m-tile:
             // the amino-acid rows scaled for the pair (q(a) / (0.5 (bq(a) +
             // bd(a))), as cell_score's Qt) and split, then the CV and SS words
@@ -1520,7 +1529,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                     const int k = 8 * (i >> 1) + 2 * q + (i & 1);
                     w[i] = (k < NAA) ? __fdividef(1.f, 0.5f * (qbkg[k] + bd[k])) : 0.f;
                 }
-                for (int mt = 0; mt < 4; mt++) {
+                for (int mt = 0; mt < nmt; mt++) {
                     unsigned v[40];
                     const float4* sa = reinterpret_cast<const float4*>(a.qaa) + (long long)(s * 4 + mt) * 96 + lane;
                     const uint4* sq = reinterpret_cast<const uint4*>(a.qa) + (long long)(s * 4 + mt) * 224 + lane;
@@ -1532,15 +1541,18 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                         bf16_split(x.y * w[2 * i + 1], h[1], l[1]);
                         bf16_split(x.z * w[2 * i], h[2], l[2]);
                         bf16_split(x.w * w[2 * i + 1], h[3], l[3]);
-                        v[2 * i] = h[0] | (h[1] << 16);
-                        v[2 * i + 1] = h[2] | (h[3] << 16);
-                        v[6 + 2 * i] = l[0] | (l[1] << 16);
-                        v[6 + 2 * i + 1] = l[2] | (l[3] << 16);
+                        const int o = i < 2 ? 2 * i : 32;   // k 0-15; k 16-23
+                        v[o] = h[0] | (h[1] << 16);
+                        v[o + 1] = h[2] | (h[3] << 16);
+                        const int ol = i < 2 ? 4 + 2 * i : 34;
+                        v[ol] = l[0] | (l[1] << 16);
+                        v[ol + 1] = l[2] | (l[3] << 16);
                     }
 #pragma unroll
                     for (int i = 0; i < 7; i++) {
                         const uint4 x = __ldg(sq + i * 32);
-                        v[12 + 4 * i] = x.x; v[13 + 4 * i] = x.y; v[14 + 4 * i] = x.z; v[15 + 4 * i] = x.w;
+                        const int o = i < 6 ? 8 + 4 * i : 36;
+                        v[o] = x.x; v[o + 1] = x.y; v[o + 2] = x.z; v[o + 3] = x.w;
                     }
                     tmem_st40(tq + P1T_TMEM_MT * mt, v);
                 }
@@ -1549,14 +1561,14 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             const int r0 = P1_ROWS * s + 2 * lane;   // the lane's first row
             {
                 // the rows' score terms, and scores of -inf for the cells left
-                // of the matrix (step k < lane)
+                // of the matrix (step k < lane) and the m-tiles past the query
                 const float* qx0 = a.qrec + (long long)min(r0, Lq - 1) * QR_STRIDE;
                 const float* qx1 = a.qrec + (long long)min(r0 + 1, Lq - 1) * QR_STRIDE;
                 *reinterpret_cast<float4*>(rqt + 4 * lane) =
                     make_float4(qx0[QR_CN], tc.c2 - 2.f * qx0[QR_PRIOR], qx1[QR_CN], tc.c2 - 2.f * qx1[QR_PRIOR]);
 #pragma unroll 4
-                for (int k = 0; k < 31; k++)
-                    if (k < lane)
+                for (int k = 0; k < P1_SLOTS; k++)
+                    if (k < lane || lane >= 8 * nmt)
                         *reinterpret_cast<float2*>(ring + k * P1_RLD + 2 * lane) = make_float2(-INFINITY, -INFINITY);
             }
             Wf2 D;
@@ -1580,7 +1592,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
 #pragma unroll
             for (int i = 0; i < 5; i++) sg[i] = i * P1_C * P1_RLD;
             int cs = 0, cl = lane == 0 ? 0 : P1_CMOD - lane;
-            for (int m = 0; P1_C * m < L + 31; m++) {
+            for (int m = 0; P1_C * m < kend; m++) {
                 const int k0 = P1_C * m;
                 // the row above for this chunk's steps, copied during the score stage
                 p1_row_async(a, it, s, bnd, botr, ldb, k0, lane, broken);
@@ -1614,12 +1626,14 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                     const float2 cp1 = *reinterpret_cast<const float2*>(cr + P1C_TRS);
                     const float cd[2] = {cp0.x, cp1.x}, pd[2] = {cp0.y, cp1.y};
                     // ---- score stage: 64 x 8 tile of chunk m on the tensor cores
+                    unsigned Q[40];   // k 0-15: aa hi, lo, cv hi, lo; ss hi 8, lo 8; k 16-23: aa hi 2, lo 2, cv hi 2, lo 2
+                    tmem_ld40(tq, Q);
 #pragma unroll
                     for (int mt = 0; mt < 4; mt++) {
-                        unsigned Q[40];   // aa hi 6, lo 6; cv hi 6, lo 6; ss hi 8, lo 8
-                        tmem_ld40(tq + P1T_TMEM_MT * mt, Q);
+                        if (mt >= nmt) break;
+                        tmem_ld40_wait(Q);
                         float acc[3][4];
-                        const unsigned *Ah = Q, *Al = Q + 6, *Ch = Q + 12, *Cl = Q + 18, *Sh = Q + 24, *Sl = Q + 32;
+                        const unsigned *Ah = Q, *Al = Q + 4, *Ch = Q + 8, *Cl = Q + 12, *Sh = Q + 16, *Sl = Q + 24;
                         mma_bf16_z(acc[0], Al, b0.x, b0.y);
                         mma_bf16_z(acc[1], Cl, b1.z, b1.w);
                         mma_bf16_z(acc[2], Sl, b3.x, b3.y);
@@ -1629,15 +1643,17 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                         mma_bf16(acc[0], Ah, b0.x, b0.y);
                         mma_bf16(acc[1], Ch, b1.z, b1.w);
                         mma_bf16(acc[2], Sh, b3.x, b3.y);
-                        mma_bf16_k8(acc[0], Al[4], Al[5], b0.z);
-                        mma_bf16_k8(acc[1], Cl[4], Cl[5], b2.z);
+                        mma_bf16_k8(acc[0], Q[34], Q[35], b0.z);
+                        mma_bf16_k8(acc[1], Q[38], Q[39], b2.z);
                         mma_bf16(acc[2], Sl + 4, b3.z, b3.w);
-                        mma_bf16_k8(acc[0], Ah[4], Ah[5], b0.w);
-                        mma_bf16_k8(acc[1], Ch[4], Ch[5], b2.w);
+                        mma_bf16_k8(acc[0], Q[32], Q[33], b0.w);
+                        mma_bf16_k8(acc[1], Q[36], Q[37], b2.w);
                         mma_bf16(acc[2], Sh + 4, b4.z, b4.w);
-                        mma_bf16_k8(acc[0], Ah[4], Ah[5], b0.z);
-                        mma_bf16_k8(acc[1], Ch[4], Ch[5], b2.z);
+                        mma_bf16_k8(acc[0], Q[32], Q[33], b0.z);
+                        mma_bf16_k8(acc[1], Q[36], Q[37], b2.z);
                         mma_bf16(acc[2], Sh + 4, b3.z, b3.w);
+                        // the next m-tile's fragments load during the epilogue
+                        if (mt + 1 < nmt) tmem_ld40(tq + P1T_TMEM_MT * (mt + 1), Q);
                         const float2 rq0 = *reinterpret_cast<const float2*>(rqt + 2 * (16 * mt + g));
                         const float2 rq1 = *reinterpret_cast<const float2*>(rqt + 2 * (16 * mt + g + 8));
                         float S[4];
@@ -1692,7 +1708,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                 if (s + 1 < nstrips) {
                     p1_row_flush(bnd, botw, ldb, k0, L, lane);
                     // columns up to k0 - 24 are there: published every other chunk
-                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= L + 31))
+                    if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= kend))
                         p1_publish(a, it, s, min(k0 - 23, L), lane);
                 }
                 // next chunk: rotate the ring segments and record slots; chunk
@@ -1887,8 +1903,9 @@ int p1c_blocks_per_sm(int cvcard)
 {
     int n = 0;
     const size_t sm = p1c_smem_bytes(cvcard);
-    cudaFuncSetAttribute(p1c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, p1c_kernel, P1C_WARPS * 32, sm);
+    cudaFuncSetAttribute(p1c_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(p1c_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, p1c_kernel<false>, P1C_WARPS * 32, sm);
     return n;
 }
 
@@ -1912,8 +1929,9 @@ cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, c
     }
     if (which == P1K_CHUNKED) {
         const size_t sm = p1c_smem_bytes(a.sc.cvcard);
-        cudaFuncSetAttribute(p1c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        p1c_kernel<<<grid, P1C_WARPS * 32, sm, st>>>(a, qbkg);
+        auto* k = a.tc.uniform ? p1c_kernel<true> : p1c_kernel<false>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        k<<<grid, P1C_WARPS * 32, sm, st>>>(a, qbkg);
         return cudaGetLastError();
     }
     const size_t sm = p1_smem_bytes(a.sc.cvcard);
@@ -1921,17 +1939,18 @@ cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, c
         // the score matrices first (their own work counter, a.counter[1]),
         // then the sweep over them
         const size_t sms = (size_t)(a.sc.cvcard * P1TC_CVREP + P2S_WARPS * P2S_WARP_FLOATS) * sizeof(float);
-        cudaError_t e = cudaFuncSetAttribute(p2s_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms);
+        auto* k2 = a.tc.uniform ? p2s_kernel<true> : p2s_kernel<false>;
+        cudaError_t e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms);
         if (e != cudaSuccess) return e;
         int occ = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p2s_kernel, P2S_WARPS * 32, sms)) != cudaSuccess)
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k2, P2S_WARPS * 32, sms)) != cudaSuccess)
             return e;
         int dev = 0, nsm = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         const long long nit = (long long)a.nwork * ((a.Lq + 31) / 32);
         const int gs = (int)std::min<long long>((long long)std::max(occ, 1) * nsm, (nit + P2S_WARPS - 1) / P2S_WARPS);
-        p2s_kernel<<<gs, P2S_WARPS * 32, sms, st>>>(a, qbkg);
+        k2<<<gs, P2S_WARPS * 32, sms, st>>>(a, qbkg);
         const size_t smt = (size_t)P1TC_WARPS * P1TC_WARP_FLOATS * sizeof(float);
         if ((e = cudaFuncSetAttribute(p1tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt)) != cudaSuccess)
             return e;
