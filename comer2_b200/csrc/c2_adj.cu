@@ -7,7 +7,7 @@
 // query and db transition log-probabilities, the column -1 states of its
 // 32-row blocks, a local start term log 1 in the MM state) evaluated with
 // true exponentials and logarithms (the hardware base-2 forms, relative
-// error ~1e-7 at these arguments; the reference's MAP stage uses coarse
+// error ~1e-7 at these arguments, all log values kept in base 2; the reference's MAP stage uses coarse
 // approximations instead) over the score matrix
 //     S = s0 + wss * ss + wcv * cv
 // (amino-acid score, and the SS and context-vector terms before their
@@ -45,26 +45,27 @@
 namespace c2 {
 
 #define FULL 0xffffffffu
-constexpr float XLOG0 = -99.f;   // the MAP model's log 0
-
+// Every log value inside the sweeps is in base 2 (scores, transitions, states,
+// rows): a term of a sum then costs one ex2.approx and a sum one lg2.approx,
+// without the two multiplications that convert e^x and ln x.  (Denormal results
+// and arguments are flushed: the terms they drop are below 2^-126 of the largest
+// term of a sum.)
+constexpr float XLOG2E = 1.4426950408889634f, XLN2 = 0.6931471805599453f;
+constexpr float XLOG0 = -99.f * XLOG2E;   // the MAP model's log 0
 
 struct X5 { float MM, MI, IM, DN, ND; };
 
-// e^x and ln x through the hardware base-2 forms (ex2.approx / lg2.approx,
-// denormal results and arguments flushed: the terms they drop are below
-// e^-87 of the largest term of a sum)
-constexpr float XLOG2E = 1.4426950408889634f, XLN2 = 0.6931471805599453f;
 __device__ __forceinline__ float xexp(float x)
 {
     float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * XLOG2E));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 __device__ __forceinline__ float xlog(float x)
 {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y * XLN2;
+    return y;
 }
 
 // the larger term's exponential is ex2(0) = 1 exactly, the smaller one's
@@ -75,16 +76,16 @@ __device__ __forceinline__ float xlse2(float a, float b)
     return xlog(1.f + xexp(-fabsf(a - b))) + m;
 }
 
-// log(e^v1 + ... + e^v5 + 1): the 1 is the local start (forward) or end (backward)
+// log(2^v1 + ... + 2^v5 + 1): the 1 is the local start (forward) or end (backward)
 __device__ __forceinline__ float xlse5p1(float v1, float v2, float v3, float v4, float v5)
 {
     float m = fmaxf(fmaxf(fmaxf(v1, v2), fmaxf(v3, v4)), fmaxf(v5, 0.f));
-    return xlog(xexp(v1 - m) + xexp(v2 - m) + xexp(v3 - m) + xexp(v4 - m) + xexp(v5 - m) + xexp(-m)) + m;
+    return xlog(((xexp(v1 - m) + xexp(v2 - m)) + (xexp(v3 - m) + xexp(v4 - m))) + (xexp(v5 - m) + xexp(-m))) + m;
 }
 
 // transitions of position i of a profile whose raw rows start at t0: the
 // forward recursion's (MM MD IM DM DD into i, MI II out of i) and the
-// backward's (all out of i); log 0 outside [0, len)
+// backward's (all out of i), in base 2; log 0 outside [0, len)
 __device__ __forceinline__ void xtrn_fwd(const float* __restrict__ t0, int i, int len, float* t7)
 {
     if (i < 0 || i >= len) {
@@ -94,6 +95,7 @@ __device__ __forceinline__ void xtrn_fwd(const float* __restrict__ t0, int i, in
     const float* a = t0 + (long long)i * 7;
     t7[TMM] = a[0]; t7[TMI] = a[7 + 1]; t7[TMD] = a[2];
     t7[TIM] = a[3]; t7[TII] = a[7 + 4]; t7[TDM] = a[5]; t7[TDD] = a[6];
+    for (int k = 0; k < 7; k++) t7[k] *= XLOG2E;
 }
 
 __device__ __forceinline__ void xtrn_bwd(const float* __restrict__ t0, int i, int len, float* t7)
@@ -103,15 +105,7 @@ __device__ __forceinline__ void xtrn_bwd(const float* __restrict__ t0, int i, in
         return;
     }
     const float* b = t0 + (long long)(i + 1) * 7;
-    for (int k = 0; k < 7; k++) t7[k] = b[k];
-}
-
-// ---------------------------------------------------------------------------
-// cell (i, j) of a pair whose wavefront block starts at base
-__device__ __forceinline__ long long fw_cell(long long base, int L, int i, int j)
-{
-    const int l = i & 31;
-    return base + ((long long)(i >> 5) * (L + 31) + j + l) * 32 + l;
+    for (int k = 0; k < 7; k++) t7[k] = b[k] * XLOG2E;
 }
 
 // ---------------------------------------------------------------------------
@@ -196,7 +190,7 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
                 }
                 const long long c = cb + (long long)k * 32 + lane;
                 const float p0 = s0, pss = ss, pcv = cvm;
-                a.S[c] = p0 + a.wss * pss + a.wcv * pcv;
+                a.S[c] = (p0 + a.wss * pss + a.wcv * pcv) * XLOG2E;
                 a.pss[c] = pss;
                 a.pcv[c] = pcv;
             }
@@ -241,7 +235,7 @@ __device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const
     __syncwarp();
 }
 
-// Raw transition rows of a pair's db profile (rows 0..L; row r holds the
+// Transition rows of a pair's db profile, in base 2 (rows 0..L; row r holds the
 // transitions into position r, MI and II of row r + 1 those out of position
 // r) in the warp's shared ring trs[128][7] by sequence index q: q = row in the
 // forward sweep, q = L - row in the mirrored backward sweep.  A step's lanes
@@ -253,7 +247,7 @@ __device__ __forceinline__ void adj_stage_trn(float* trs, const float* __restric
     for (int e = lane; e < nq * 7; e += 32) {
         const int q = q0 + e / 7, f = e % 7;
         const int row = MIRROR ? L - q : q;
-        trs[(q & 127) * 7 + f] = __ldg(dt0 + (long long)row * 7 + f);
+        trs[(q & 127) * 7 + f] = __ldg(dt0 + (long long)row * 7 + f) * XLOG2E;
     }
 }
 
@@ -302,10 +296,10 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
     float q7[7];
     xtrn_fwd(a.qtrn + (a.qpos[m] + a.qidx[m]) * 7, r, Lq, q7);
 #pragma unroll
-    for (int k = 0; k < 7; k++) q7[k] += a.theta[k];
+    for (int k = 0; k < 7; k++) q7[k] += a.theta[k] * XLOG2E;
     const float* cf = a.qcfx + (a.qpos[m] + (act ? r : 0)) * 6;
-    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0], cf[1], cf[2], XLOG0};
-    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3], cf[4], cf[5], XLOG0};
+    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0] * XLOG2E, cf[1] * XLOG2E, cf[2] * XLOG2E, XLOG0};
+    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3] * XLOG2E, cf[4] * XLOG2E, cf[5] * XLOG2E, XLOG0};
     const bool wr_row = !RECOMP && lane == 31 && s + 1 < ns;
     X5 mine = INIT, upp = INIT;
     // the lane's score of the next step, loaded a step ahead
@@ -416,7 +410,8 @@ __global__ void adj_logz_kernel(AdjArgs a)
         zs = (mx == -INFINITY) ? 0.f : zs * xexp(zm - mx) + os * xexp(om - mx);
         zm = mx;
     }
-    a.logz[m] = logf(zs) + zm;
+    a.logz[m] = logf(zs) + zm * XLN2;
+    a.zpart[2 * a.soff[m]] = xlog(zs) + zm;   // base 2, for the backward sweep
 }
 
 // ---------------------------------------------------------------------------
@@ -444,9 +439,8 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
 {
     const int p = a.prof[m];
     const int L = a.plen[p], Lq = a.pLq[m], ns = (Lq + 31) >> 5;
-    const long long base = a.off[m];
-    const long long cb = base + (long long)s * (L + 31) * 32;
-    const float lz = a.logz[m];
+    const long long cb = a.off[m] + (long long)s * (L + 31) * 32;
+    const float lz = a.zpart[2 * a.soff[m]];   // log2 Z
     const float* dt0 = a.dtrn + (a.poff[p] + p) * 7;
     const bool has_below = s + 1 < ns;
     const int ldr = row_ld(L);
@@ -463,11 +457,11 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     xtrn_bwd(qt0, i, Lq, qb);
     xtrn_fwd(qt0, i, Lq, qf);
 #pragma unroll
-    for (int k = 0; k < 7; k++) { qb[k] += a.theta[k]; qf[k] += a.theta[k]; }
+    for (int k = 0; k < 7; k++) { qb[k] += a.theta[k] * XLOG2E; qf[k] += a.theta[k] * XLOG2E; }
     // column -1 states of row i (the forward's left and diagonal at column 0)
     const float* cf = a.qcfx + (a.qpos[m] + (act ? i : 0)) * 6;
-    const X5 LB = (lf == 31) ? INIT : X5{0.f, cf[0], cf[1], cf[2], XLOG0};
-    const X5 DB = (lf == 31 || lf == 0) ? INIT : X5{0.f, cf[3], cf[4], cf[5], XLOG0};
+    const X5 LB = (lf == 31) ? INIT : X5{0.f, cf[0] * XLOG2E, cf[1] * XLOG2E, cf[2] * XLOG2E, XLOG0};
+    const X5 DB = (lf == 31 || lf == 0) ? INIT : X5{0.f, cf[3] * XLOG2E, cf[4] * XLOG2E, cf[5] * XLOG2E, XLOG0};
     const bool wr_row = (t == 31) && s > 0;
     float g[9];
 #pragma unroll
@@ -477,26 +471,53 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     adj_stage_trn<true>(trs, dt0, 0, L, lane);
     adj_stage_trn<true>(trs, dt0, 32, L, lane);
     adj_load_row<true>(a, rab, below, ldr, has_below, 0, L, lane, broken);
+    // Forward states and scores of the lane's own row, one wavefront line a
+    // step: at step k the lane's cell is on line kf = L + 30 - k, its left
+    // neighbour on line kf - 1; the row above (lf - 1) is lane t + 1's, whose
+    // line kf - 2 is the diagonal predecessor now and the one above at the next
+    // step.  So a step loads one line of five states (20 loads a cell when each
+    // neighbour was read from memory) and shuffles it.  Lane 31's row above is
+    // the strip above's last row, the diagonal successor's score of lane 0 the
+    // strip below's first.  Entries of cells outside the matrix are read but not used.
+    const float* Sr = a.S + cb + lf;
+    const float* Sb = a.S + cb + (long long)(L + 31) * 32;   // row 32 s + 32 (has_below), lane 0
+    const int kf0 = L + 30;
+    X5 Ac = fw_ld5(Fw, kf0, lf), Al = fw_ld5(Fw, kf0 - 1, lf), An = fw_ld5(Fw, kf0 - 2, lf), Up = INIT;
+    X5 Ab = INIT;                              // lane 31: row 32 s - 1 at the diagonal column
+    auto load_above = [&](int c) { return (s > 0 && t == 31 && c >= 0 && c < L) ? row_ld5(fab, ldr, c) : INIT; };
+    Ab = load_above(L - 1 + t - 1);            // step 0: ca - 1
+    float sc0 = Sr[(long long)kf0 * 32], sc1 = 0.f, sc2 = 0.f, sb = XLOG0;   // scores at steps k, k - 1, k - 2; row below
     for (int k = 0; k < L + 31; k++) {
         const int jm = k - t;
         const int ca = L - 1 - jm;
+        const int kf = L + 30 - k;
         {
-            // the rows step k + ADJ_PF reads first: forward states of its
-            // diagonal row (5 lines), its own score, SS and CV rows, and lane
-            // 0's diagonal successor in the strip below
-            const int kq = k + ADJ_PF;
-            const int kfq = L + 30 - kq;   // forward step of the lanes' own cells then
-            if (kq < L + 31) {
-                if (lane < 5 && kfq - 2 >= 0) pf_l1(Fw + (long long)(kfq - 2) * 160 + lane * 32);
-                else if (kfq >= 0 && kfq < L + 31) {
-                    if (lane == 5) pf_l1(a.S + cb + (long long)kfq * 32);
-                    else if (lane == 6) pf_l1(a.pss + cb + (long long)kfq * 32);
-                    else if (lane == 7) pf_l1(a.pcv + cb + (long long)kfq * 32);
-                }
-                if (lane == 8 && s + 1 < ns && L - kq >= 0 && L - kq < L)
-                    pf_l1(a.S + cb + (long long)(L + 31) * 32 + (long long)(L - kq) * 32);
+            // lines of the steps to come: forward states (5), scores, SS and CV parts, row below
+            const int kq = kf - ADJ_PF;
+            if (kq >= 0) {
+                if (lane < 5 && kq >= 3) pf_l1(Fw + (long long)(kq - 3) * 160 + lane * 32);
+                else if (lane == 5) pf_l1(a.S + cb + (long long)kq * 32);
+                else if (lane == 6) pf_l1(a.pss + cb + (long long)kq * 32);
+                else if (lane == 7) pf_l1(a.pcv + cb + (long long)kq * 32);
+                else if (lane == 8 && has_below && L - k - ADJ_PF >= 0 && L - k - ADJ_PF < L)
+                    pf_l1(Sb + (long long)(L - k - ADJ_PF) * 32);
             }
         }
+        // loaded now for the next step: line kf - 3, the score, rows above and below
+        X5 Aq = INIT;
+        float scn = 0.f;
+        if (kf >= 3) Aq = fw_ld5(Fw, kf - 3, lf);
+        if (kf >= 1) scn = Sr[(long long)(kf - 1) * 32];
+        const X5 Abn = load_above(ca - 2);
+        const float sbn = (t == 0 && has_below && ca >= 0 && ca < L) ? Sb[(long long)ca * 32] : XLOG0;   // column (ca - 1) + 1
+        X5 dgl;   // diagonal predecessor: lane t + 1's line kf - 2
+        dgl.MM = __shfl_down_sync(FULL, An.MM, 1);
+        dgl.MI = __shfl_down_sync(FULL, An.MI, 1);
+        dgl.IM = __shfl_down_sync(FULL, An.IM, 1);
+        dgl.DN = __shfl_down_sync(FULL, An.DN, 1);
+        dgl.ND = __shfl_down_sync(FULL, An.ND, 1);
+        if (t == 31) dgl = Ab;
+        const float scu = __shfl_up_sync(FULL, sc2, 1);   // score of (i + 1, ca + 1): lane t - 1 two steps ago
         // transitions out of column ca (row ca + 1, sequence index jm) and,
         // for the edge posteriors, into it (rows ca and ca + 1)
         const bool colv = jm >= 0 && jm < L;
@@ -533,7 +554,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         if (jm == 0) { rt = INIT; dg = INIT; }
         const bool valid = act && jm >= 0 && jm < L;
         // score of the diagonal successor (i + 1, ca + 1)
-        const float sco = (valid && i + 1 < Lq && ca + 1 < L) ? a.S[fw_cell(base, L, i + 1, ca + 1)] : XLOG0;
+        const float sco = (valid && i + 1 < Lq && ca + 1 < L) ? (t == 0 ? sb : scu) : XLOG0;
         X5 nw;
         nw.MM = xlse5p1((dn.MI + qb[TMM]) + tb[TMI], (rt.IM + qb[TMI]) + tb[TMM], dn.DN + qb[TMD],
                         rt.ND + tb[TMD], ((dg.MM + qb[TMM]) + tb[TMM]) + sco);
@@ -546,23 +567,14 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         if (!act) nw = INIT;
         if (valid) {
             // edge posteriors of cell (i, ca): its forward predecessors
-            const int kf = ca + lf;
-            const X5 own = fw_ld5(Fw, kf, lf);
-            X5 up, left, diag;
-            if (i == 0) up = INIT;
-            else if (lf == 0) up = row_ld5(fab, ldr, ca);
-            else up = fw_ld5(Fw, kf - 1, lf - 1);
+            const X5 own = Ac, up = Up;
+            X5 left = Al, diag = dgl;
             if (ca == 0) {
                 left = LB;
                 diag = DB;
-            } else {
-                left = fw_ld5(Fw, kf - 1, lf);
-                if (i == 0) diag = INIT;
-                else if (lf == 0) diag = row_ld5(fab, ldr, ca - 1);
-                else diag = fw_ld5(Fw, kf - 2, lf - 1);
             }
             const long long kk = cb + (long long)kf * 32 + lf;
-            const float sc = a.S[kk];
+            const float sc = sc0;
             const X5& b = nw;
             // MM: five emission edges
             const float eMM = b.MM - lz;
@@ -594,6 +606,11 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         }
         mine = nw;
         upp = dn;
+        Up = dgl;
+        Ac = Al; Al = An; An = Aq;
+        Ab = Abn;
+        sc2 = sc1; sc1 = sc0; sc0 = scn;
+        sb = sbn;
     }
     // the strip's gradient sums
 #pragma unroll
@@ -610,7 +627,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     }
 }
 
-__global__ void __launch_bounds__(ADJ_WARPS * 32) adj_bwd_kernel(AdjArgs a)
+__global__ void __launch_bounds__(ADJ_WARPS * 32, 4) adj_bwd_kernel(AdjArgs a)
 {
     __shared__ __align__(16) float rabs[ADJ_WARPS][32 * 8];
     __shared__ float trss[ADJ_WARPS][128 * 7];
