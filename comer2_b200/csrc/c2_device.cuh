@@ -94,13 +94,12 @@ enum : int { P1K_STRIP = 0, P1K_CHUNKED = 1, P1K_TRACEBACK = 2, P1K_TENSOR = 3 }
 // column records in shared memory, 12 floats apart (the two 16-byte reads of 8
 // lanes at consecutive columns cover 32 distinct banks)
 constexpr int P1C_RING = 64, P1C_TRS = 12;
-// row above the strip in the traceback sweep: [32][4] + [32] floats
-constexpr int BND_ND = 32 * 4, BND_FLOATS = 32 * 5;
+constexpr int TB_C = 16;   // columns per chunk of the traceback sweep
 // traceback sweep over the stored score matrices: per warp the score ring, the
 // transition ring, the row above and a [32][33]-byte traceback column ring;
 // 16 warps per SM.  P1TC_CVREP: CV table replicas of the phase-2 score kernel
 constexpr int P1TC_WARPS = 16, P1TC_CVREP = 8;
-constexpr int P1TC_WARP_FLOATS = P1C_RING * 32 + P1C_RING * P1C_TRS + BND_FLOATS;
+constexpr int P1TC_WARP_FLOATS = P1C_RING * 32 + P1C_RING * P1C_TRS + 2 * 5 * TB_C;
 // phase-2 score kernel: 8 warps per CTA, per warp the SS row table and the
 // record staging ring; the CV table (P1TC_CVREP replicas) per CTA
 constexpr int P2S_WARPS = 8;
@@ -184,6 +183,7 @@ struct P1Args {
     float* bnd;                 // last rows of the strips (row_block)
     unsigned long long* tbkey;  // [ncand] maximum of the traceback sweep and its cell, packed
     const int* worder;          // traceback sweep: rank -> candidate (longest first)
+    int p2s_cols, p2s_blocks;   // phase-2 score matrices: columns per work item, items per (candidate, strip)
     const int* items;           // traceback sweep: work item -> rank * nstrips + strip
     unsigned spin;              // polls before a strip wait gives up (pipe_wait)
     // tensor-core operands (P1K_TENSOR)
@@ -242,6 +242,7 @@ struct FinArgs {
 namespace c2 {
 constexpr unsigned PIPE_SPIN = 1u << 22;  // default polls before a wait gives up (c2_set_wait_limit)
 constexpr int PIPE_ERR_TIMEOUT = 3;       // device status of an abandoned wait
+constexpr int PIPE_ERR_TIMEOUT_P1 = 4;    // ... of phase 1
 
 __device__ __forceinline__ int pipe_ld_acquire(const int* p)
 {
@@ -271,7 +272,7 @@ __device__ __forceinline__ void pipe_wait(const int* flag, int need, int lane, i
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (ok) break;
         if (++it >= spin) {
-            if (lane == 0 && status) atomicCAS(status, 0, PIPE_ERR_TIMEOUT);
+            if (lane == 0 && status) atomicCAS(status, 0, PIPE_ERR_TIMEOUT_P1);
             broken = true;
             break;
         }
@@ -316,6 +317,17 @@ __device__ __forceinline__ void row_poll(F poll, int lane, int* status, bool& br
     }
 }
 
+// asynchronous global->shared copies (cp.async, 16 B each, through L2)
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
 // The lane's column c of a row another warp writes, for lanes with want
 __device__ __forceinline__ void row_get(const float* row, int ld, int c, bool want, float* v, int lane, int* status,
                                         bool& broken, unsigned spin)
@@ -334,5 +346,48 @@ __device__ __forceinline__ void row_get(const float* row, int ld, int c, bool wa
             return ok;
         },
         lane, status, broken, spin);
+}
+
+// A group of G columns of the row above in shared memory: [G][4] states, then
+// [G] ND.  row_issue starts its copy a group ahead of its use; row_take, just
+// before the use, looks whether the copy found every column there and polls for
+// the rest only otherwise: a strip that trails far enough never waits for L2.
+// Columns past the matrix stay empty (no cell inside the matrix reads them).
+template <int G> constexpr int ROW_BUF = 5 * G;
+
+template <int G>
+__device__ __forceinline__ void row_issue(float* buf, const float* row, int ld, int c0, int L, int lane)
+{
+    const int c4 = c0 + 4 * (lane - G);
+    if (lane < G) {
+        if (c0 + lane < L) cp_async16(buf + 4 * lane, row + 4 * (c0 + lane));
+    } else if (lane < G + G / 4 && c4 < L) {
+        cp_async16(buf + 4 * G + 4 * (lane - G), row + 4 * ld + c4);
+    }
+    cp_async_commit();
+}
+
+template <int G>
+__device__ __forceinline__ void row_take(float* buf, const float* row, int ld, int c0, int L, int lane, int* status,
+                                         bool& broken, unsigned spin)
+{
+    cp_async_wait_all();
+    __syncwarp();
+    const bool want = lane < G && c0 + lane < L;
+    bool ok = true;
+    if (want) {
+        const uint4 w = *reinterpret_cast<const uint4*>(buf + 4 * lane);
+        ok = w.x != ROW_EMPTY && w.y != ROW_EMPTY && w.z != ROW_EMPTY && w.w != ROW_EMPTY &&
+             __float_as_uint(buf[4 * G + lane]) != ROW_EMPTY;
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+        float v[5];
+        row_get(row, ld, c0 + lane, want, v, lane, status, broken, spin);
+        if (want) {
+            *reinterpret_cast<float4*>(buf + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
+            buf[4 * G + lane] = v[4];
+        }
+    }
+    __syncwarp();
 }
 }  // namespace c2

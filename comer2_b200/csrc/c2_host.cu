@@ -27,7 +27,7 @@
 
 namespace c2 {
 cudaError_t launch_stats(const StatsArgs& a, cudaStream_t st);
-cudaError_t launch_map(MapArgs a, const float* qtrn, const float* dtrn, const float* qcf, int nsm,
+cudaError_t launch_map(const MapArgs& a, const float* qtrn, const float* dtrn, const float* qcf, int nsm,
                        int* counter, cudaStream_t st, int* nlaunch);
 cudaError_t launch_viterbi_aln(const MapArgs& a, cudaStream_t st);
 size_t p1_smem_bytes(int cvcard);
@@ -251,6 +251,7 @@ static const char* status_text(int st)
     switch (st) {
     case 2: return "traceback DP disagrees with phase 1";
     case PIPE_ERR_TIMEOUT: return "a strip wait timed out";
+    case PIPE_ERR_TIMEOUT_P1: return "a wait in phase 1 timed out";
     default: return "unknown device error";
     }
 }
@@ -1360,13 +1361,18 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
     a.tbkey = h->d_tbkey.p;
     a.worder = h->d_worder.p;
     a.items = h->d_tbitems.p;
-    const long long nitems = (long long)nc * ((h->Lq + 31) / 32);
     CK(cudaMemsetAsync(h->d_counter.p, 0, 2 * sizeof(int), h->stream));   // the sweep's and the score kernel's
     CK(cudaMemsetAsync(h->d_bnd.p, 0xff, bnd_half * sizeof(float), h->stream));   // the strips' rows: empty
     CK(cudaMemsetAsync(h->d_tbkey.p, 0, (size_t)nc * sizeof(unsigned long long), h->stream));
-    // one CTA of P1TC_WARPS warps per SM, one warp per (candidate, strip) work item at most
-    const int grid = (int)std::min<long long>(h->nsm, (nitems + P1TC_WARPS - 1) / P1TC_WARPS);
-    CK(launch_p1(a, h->d_qbkg.p, P1K_TRACEBACK, grid, h->stream));   // p2s_kernel, then p1tc_kernel
+    // score matrices: items of p2s_cols columns, about two per resident warp
+    // (8 x 3 an SM) where there are few, at least 32 columns (a row's operands
+    // and the SS table cost about as much as four)
+    const long long scols = (acc / h->Lq) * ((h->Lq + 31) / 32);
+    int lmax = 0;
+    for (int k : h->h_cand) lmax = std::max(lmax, h->h_plen[k]);
+    a.p2s_cols = (int)std::max<long long>(32, (scols / (48LL * h->nsm) + 7) / 8 * 8);
+    a.p2s_blocks = (lmax + a.p2s_cols - 1) / a.p2s_cols;
+    CK(launch_p1(a, h->d_qbkg.p, P1K_TRACEBACK, h->nsm, h->stream));   // p2s_kernel, then p1tc_kernel
     h->launches += 2;
     FinArgs f;
     f.Lq = h->Lq;

@@ -172,17 +172,6 @@ __device__ __forceinline__ void cell_scores(const RowOps* R, const float* __rest
 
 struct St5 { float MM, MI, IM, DN, ND; };
 
-// asynchronous global->shared copies (cp.async, 16 B each)
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
 // Stage the records of columns [REC_CHUNK*m, REC_CHUNK*(m+1)) (clipped to L)
 // into ring slots; records of consecutive columns are contiguous in HBM, so a
 // chunk is one contiguous range copied by all lanes in 16-byte pieces.  The
@@ -465,14 +454,6 @@ __device__ __forceinline__ void wf_init(WfLane& D, const float* q7, const St5& L
     D.kbest = 0;
 }
 
-// Row above the strip, one slot a column: states MM, MI, IM, DN as a float4
-// per slot ([32][4]), ND after them ([32] at BND_ND)
-__device__ __forceinline__ void bnd_put(float* bnd, int slot, float mm, float mi, float im, float dn, float nd)
-{
-    *reinterpret_cast<float4*>(bnd + slot * 4) = make_float4(mm, mi, im, dn);
-    bnd[BND_ND + slot] = nd;
-}
-
 // Wavefront steps [k0, k0 + nst) of a strip of the traceback sweep (k0 a multiple
 // of TB_C, nst <= TB_C; TB_C when !CHECK).  ring: diagonal-indexed scores, 32
 // floats per slot.  tcol: ring of P1C_RING column records (TMM .. TDD, P1C_TRS
@@ -481,7 +462,6 @@ __device__ __forceinline__ void bnd_put(float* bnd, int slot, float mm, float mi
 // to the warp's column ring btr (column j in slot j & 31, the lane's own row),
 // and column k - 31, complete for every row at step k, is stored to the pair's
 // code matrix bt (column-major, Lq rows; r = this lane's query row).
-constexpr int TB_C = 16;
 template <bool CHECK>
 __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, int L, bool act,
                                          const float* __restrict__ ring, const float* __restrict__ tcol,
@@ -507,7 +487,7 @@ __device__ __forceinline__ void wf_steps(WfLane& D, int k0, int nst, int lane, i
         {
             // row above the strip at column k (lane 0's column), broadcast reads
             const float4 ba = *reinterpret_cast<const float4*>(bnd + u * 4);
-            const float b4 = bnd[BND_ND + u];
+            const float b4 = bnd[4 * TB_C + u];
             if (lane == 0) { uMM = ba.x; uMI = ba.y; uIM = ba.z; uDN = ba.w; uND = b4; }
         }
         const int j = k0 + u - lane;
@@ -985,7 +965,8 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 // statistics and MAP stages), by cell_score -- the arithmetic of phase 1's
 // FP32 form.  One warp per (candidate, strip) at a time, lanes own query rows,
 // db records staged in shared memory as in phase 1; no dependencies between
-// work items, so every resident warp works.
+// work items, so every resident warp works.  Where there are few candidates an
+// item is a block of columns (P1Args::p2s_cols).
 template <bool CVUNIF>
 __global__ void __launch_bounds__(P2S_WARPS * 32)
 p2s_kernel(P1Args a, const float* __restrict__ qbkg)
@@ -1001,17 +982,20 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
     __syncthreads();
     const int Lq = a.Lq;
     const int nstrips = (Lq + 31) >> 5;
-    const int nitems = a.nwork * nstrips;
+    const int nsb = nstrips * a.p2s_blocks;
+    const int nitems = a.nwork * nsb;
     const ScoreConsts sc = a.sc;
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(a.counter + 1, 1);
         item = __shfl_sync(FULL, item, 0);
         if (item >= nitems) break;
-        const int cand = a.worder[item / nstrips];
-        const int s = item % nstrips;
+        const int cand = a.worder[item / nsb];
+        const int sb = item % nsb, s = sb / a.p2s_blocks;
         const int p = a.order[cand];
-        const int L = a.plen[p];
+        const int cb = (sb - s * a.p2s_blocks) * a.p2s_cols;   // columns [cb, L)
+        const int L = min(a.plen[p], cb + a.p2s_cols);
+        if (cb >= L) continue;
         const float* __restrict__ dr = a.drec + a.poff[p] * DR_STRIDE;
         const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
         const long long coff = a.cand_off[cand];
@@ -1029,13 +1013,13 @@ p2s_kernel(P1Args a, const float* __restrict__ qbkg)
 #pragma unroll 8
             for (int c = 0; c < card; c++) U[c * 32 + lane] = __ldg(us + c * 32);
         }
-        stage_chunk(rec, dr, 0, L, lane);
+        stage_chunk(rec, dr, cb >> REC_CHUNK_LOG, L, lane);
         cp_async_commit();
-        stage_chunk(rec, dr, 1, L, lane);
+        stage_chunk(rec, dr, (cb >> REC_CHUNK_LOG) + 1, L, lane);
         cp_async_commit();
         // a staged chunk of REC_CHUNK columns at a time: its cells are
         // independent, so their chains overlap
-        for (int c0 = 0; c0 < L; c0 += REC_CHUNK) {
+        for (int c0 = cb; c0 < L; c0 += REC_CHUNK) {
             cp_async_wait_1();
             __syncwarp();
 #pragma unroll
@@ -1078,7 +1062,7 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
     float* wb = smem + wid * P1TC_WARP_FLOATS;
     float* ring = wb;                                         // [P1C_RING][32] scores
     float* trn = ring + P1C_RING * 32;                        // [P1C_RING][P1C_TRS] transitions
-    float* bnd = trn + P1C_RING * P1C_TRS;                    // [BND_FLOATS] row above the strip
+    float* bnd = trn + P1C_RING * P1C_TRS;                    // row above the strip, two chunks
     (void)qbkg;
 
     const int Lq = a.Lq;
@@ -1136,6 +1120,10 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
             if (c < L) tv = __ldg(reinterpret_cast<const float4*>(dr + (long long)c * DR_STRIDE + DR_TRN) + (lane & 1));
         };
         fetch(0);
+        __syncwarp();
+        if (s > 0) row_issue<TB_C>(bnd, rowa, ldr, 0, L, lane);
+        else
+            for (int i = lane; i < 2 * ROW_BUF<TB_C>; i += 32) bnd[i] = 0.f;
         for (int k0 = 0; k0 < kend; k0 += TB_C) {
             if (k0 < L) {
                 const bool hasc = __any_sync(FULL, cA >= k0 || cB < k0 + TB_C);
@@ -1149,19 +1137,18 @@ p1tc_kernel(P1Args a, const float* __restrict__ qbkg)
                 if (c < L) *reinterpret_cast<float4*>(trn + (c & (P1C_RING - 1)) * P1C_TRS + 4 * (lane & 1)) = tv;
                 fetch(k0 + TB_C);
             }
-            // the row above for this chunk's steps
-            {
-                float v[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-                if (s > 0 && k0 < L)
-                    row_get(rowa, ldr, k0 + lane, lane < TB_C && k0 + lane < L, v, lane, a.status, broken, a.spin);
-                if (lane < TB_C) bnd_put(bnd, lane, v[0], v[1], v[2], v[3], v[4]);
+            // the row above for this chunk's steps, the next chunk's on its way
+            float* rb = bnd + (k0 & TB_C ? ROW_BUF<TB_C> : 0);
+            if (s > 0) {
+                if (k0 < L) row_take<TB_C>(rb, rowa, ldr, k0, L, lane, a.status, broken, a.spin);
+                if (k0 + TB_C < L) row_issue<TB_C>(bnd + (k0 & TB_C ? 0 : ROW_BUF<TB_C>), rowa, ldr, k0 + TB_C, L, lane);
             }
             __syncwarp();
             // ---- DP stage: wavefront steps [k0, k0 + TB_C), traceback codes stored
             if (k0 >= 32 && k0 + TB_C <= L)
-                wf_steps<false>(D, k0, TB_C, lane, L, act, ring, trn, bnd, wr_row, rowm, ldr, btr, bt, Lq, r);
+                wf_steps<false>(D, k0, TB_C, lane, L, act, ring, trn, rb, wr_row, rowm, ldr, btr, bt, Lq, r);
             else
-                wf_steps<true>(D, k0, min(TB_C, kend - k0), lane, L, act, ring, trn, bnd, wr_row, rowm, ldr, btr, bt, Lq,
+                wf_steps<true>(D, k0, min(TB_C, kend - k0), lane, L, act, ring, trn, rb, wr_row, rowm, ldr, btr, bt, Lq,
                                r);
             __syncwarp();
         }
@@ -1601,7 +1588,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                     if (!tbroken && !__all_sync(FULL, mbar_wait(tbar, tph))) {
                         tbroken = true;
                         tpend = tph;
-                        if (lane == 0 && a.status) atomicCAS(a.status, 0, PIPE_ERR_TIMEOUT);
+                        if (lane == 0 && a.status) atomicCAS(a.status, 0, PIPE_ERR_TIMEOUT_P1);
                     }
                     tph ^= 1u;
                     const uint4* bt = reinterpret_cast<const uint4*>(btile) + lane;
@@ -1948,13 +1935,17 @@ cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, c
         int dev = 0, nsm = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        const long long nit = (long long)a.nwork * ((a.Lq + 31) / 32);
+        const long long nit2 = (long long)a.nwork * ((a.Lq + 31) / 32), nit = nit2 * a.p2s_blocks;
         const int gs = (int)std::min<long long>((long long)std::max(occ, 1) * nsm, (nit + P2S_WARPS - 1) / P2S_WARPS);
         k2<<<gs, P2S_WARPS * 32, sms, st>>>(a, qbkg);
-        const size_t smt = (size_t)P1TC_WARPS * P1TC_WARP_FLOATS * sizeof(float);
+        // one CTA per SM, of fewer warps where there are few (candidate, strip)
+        // items, so that they spread over all SMs
+        const int wt = (int)std::max<long long>(1, std::min<long long>(P1TC_WARPS, (nit2 + nsm - 1) / nsm));
+        const int gt = (int)std::min<long long>(nsm, (nit2 + wt - 1) / wt);
+        const size_t smt = (size_t)wt * P1TC_WARP_FLOATS * sizeof(float);
         if ((e = cudaFuncSetAttribute(p1tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt)) != cudaSuccess)
             return e;
-        p1tc_kernel<<<grid, P1TC_WARPS * 32, smt, st>>>(a, qbkg);
+        p1tc_kernel<<<gt, wt * 32, smt, st>>>(a, qbkg);
     } else {
         cudaFuncSetAttribute(p1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         p1_kernel<<<grid, P1_WARPS * 32, sm, st>>>(a, qbkg);

@@ -60,7 +60,6 @@ struct MapArgs {
     float* bnd;                 // last rows of the strips (c2_device.cuh, row_start)
     float* bnd_b;               // the backward sweep's
     size_t bnd_cols;            // columns of a strip's rows over all candidates
-    int pf1;                    // few warps per SM: prefetch the scores into L1, not only L2
     const int* items;           // work item -> m * nstrips + strip (ready-time order)
     unsigned long long* pairk;  // [nmap] MAP DP maximum and end cell, packed for atomicMax
     int* status;
