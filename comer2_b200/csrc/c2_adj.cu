@@ -110,26 +110,32 @@ __device__ __forceinline__ void xtrn_bwd(const float* __restrict__ t0, int i, in
 
 // ---------------------------------------------------------------------------
 // score parts per cell: one warp per (pair, strip), lane = query row, the
-// strip's wavefront steps in turn (coalesced stores).  The db records the
-// lanes read (the 46 score fields of 32 consecutive columns per step) are
-// staged per 32-column chunk in a shared ring of 64 columns, ADJ_REC floats
-// apart (odd: the lanes' reads of consecutive columns hit distinct banks).
-constexpr int ADJ_REC = 47, ADJ_RECF = 46;
+// strip's wavefront steps in turn (coalesced stores).  The db records the lanes
+// read (the 46 score fields of 32 consecutive columns per step) are staged per
+// 32-column chunk in a shared ring of 64 columns, ADJ_REC floats apart: an odd
+// number of 16-byte units, so that the lanes' 16-byte reads of consecutive
+// columns share no bank (12 reads a cell instead of 46 single ones), and the SS
+// term reads a table of the strip's rows instead of nine global entries a cell:
+// 0.72 -> 0.54 ms on 256 pairs of 100..600 positions.
+constexpr int ADJ_REC = 52, ADJ_RECF = 48;
+constexpr int ADJ_SCORE_FLOATS = 64 * ADJ_REC + MAX_SSSS_CARD * 32;   // per warp: record ring, SS row table
 
 __device__ __forceinline__ void adj_stage_records(float* ring, const float* __restrict__ d0, int c0, int L, int lane)
 {
     const int nc = min(32, L - c0);
-    for (int e = lane; e < nc * ADJ_RECF; e += 32) {
-        const int c = e / ADJ_RECF, f = e - c * ADJ_RECF;
-        ring[((c0 + c) & 63) * ADJ_REC + f] = __ldg(d0 + (long long)(c0 + c) * DR_STRIDE + f);
+    for (int e = lane; e < nc * (ADJ_RECF / 4); e += 32) {
+        const int c = e / (ADJ_RECF / 4), f = e - c * (ADJ_RECF / 4);
+        *reinterpret_cast<float4*>(ring + ((c0 + c) & 63) * ADJ_REC + 4 * f) =
+            __ldg(reinterpret_cast<const float4*>(d0 + (long long)(c0 + c) * DR_STRIDE) + f);
     }
 }
 
 __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
 {
-    __shared__ float rings[ADJ_WARPS][64 * ADJ_REC];
+    extern __shared__ __align__(16) float adjsm[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* ring = rings[wid];
+    float* ring = adjsm + wid * ADJ_SCORE_FLOATS;
+    float* U = ring + 64 * ADJ_REC;   // [card][32] SS table of the strip's rows
     const int nw = gridDim.x * ADJ_WARPS;
     const ScoreConsts& sc = a.sc;
     const int card = sc.ssss_card;
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
         const float* bd = a.pbkg + (long long)p * NAA;
         const float* qb = a.qbkg + (long long)a.qidx[m] * NAA;
         // the query row's amino-acid odds for this pair, CV vector and SS values
-        float qt[NAA], qc[NCV];
+        float qt[NAA], qc[NCV + 1];
 #pragma unroll
         for (int k = 0; k < NAA; k++) qt[k] = __fdividef(qr[QR_TRG + k], 0.5f * (qb[k] + bd[k]));
 #pragma unroll
@@ -155,37 +161,49 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
         const long long cb = a.off[m] + (long long)s * (L + 31) * 32;
         const float* d0 = a.drec + a.poff[p] * DR_STRIDE;
         __syncwarp();
+        for (int c = 0; c < card; c++)
+            U[c * 32 + lane] = q0 * a.ssss[i0 * card + c] + q1 * a.ssss[i1 * card + c] + q2 * a.ssss[i2 * card + c];
         adj_stage_records(ring, d0, 0, L, lane);
         __syncwarp();
         for (int k = 0; k < L + 31; k++) {
             const int j = k - lane;
             if (act && j >= 0 && j < L) {
-                const float* dr = ring + (j & 63) * ADJ_REC;
+                const float4* dr = reinterpret_cast<const float4*>(ring + (j & 63) * ADJ_REC);
                 float sa = 0.f;
 #pragma unroll
-                for (int t = 0; t < NAA; t++) sa = fmaf(qt[t], dr[DR_TRG + t], sa);
+                for (int t = 0; t < NAA / 4; t++) {
+                    const float4 v = dr[t];
+                    sa = fmaf(qt[4 * t], v.x, sa);
+                    sa = fmaf(qt[4 * t + 1], v.y, sa);
+                    sa = fmaf(qt[4 * t + 2], v.z, sa);
+                    sa = fmaf(qt[4 * t + 3], v.w, sa);
+                }
                 const float s0 = __logf(sa) - sc.shift;
-                float dot = 0.f;
+                float dot = 0.f, dcn = 0.f;
 #pragma unroll
-                for (int t = 0; t < NCV; t++) dot = fmaf(qc[t], dr[DR_CV + t], dot);
+                for (int t = 0; t < 5; t++) {
+                    const float4 v = dr[DR_CV / 4 + t];
+                    dot = fmaf(qc[4 * t], v.x, dot);
+                    dot = fmaf(qc[4 * t + 1], v.y, dot);
+                    dot = fmaf(qc[4 * t + 2], v.z, dot);
+                    if (t < 4) dot = fmaf(qc[4 * t + 3], v.w, dot);
+                    else dcn = v.w;   // DR_CN
+                }
                 dot += sc.lokappa0;
-                const float det = qcn * dr[DR_CN] - dot * dot;
-                const float cvs = sc.cterm + sc.pownu0 * __logf(det) - qpr - dr[DR_PRIOR];
+                const float4 v10 = dr[DR_PRIOR / 4], v11 = dr[DR_SSIDX / 4];   // prior, SS; indices, P(H) + 0.1
+                const float det = qcn * dcn - dot * dot;
+                const float cvs = sc.cterm + sc.pownu0 * __logf(det) - qpr - v10.x;
                 float cvm;
                 if (cvs <= sc.cvkey_first) cvm = sc.cvval_first;
                 else if (sc.cvkey_last <= cvs) cvm = sc.cvval_last;
                 else cvm = a.cvvals[min(max(sc.cvshift + (int)rintf(2.f * cvs), 0), sc.cvcard - 1)];
-                const int pk = __float_as_int(dr[DR_SSIDX]);
-                const int dk[3] = {pk & 0xff, (pk >> 8) & 0xff, (pk >> 16) & 0xff};
+                const int pk = __float_as_int(v11.x);
                 float ss = 0.f;
-#pragma unroll
-                for (int t = 0; t < 3; t++) {
-                    const int cc = dk[t];
-                    const float u = q0 * a.ssss[i0 * card + cc] + q1 * a.ssss[i1 * card + cc] + q2 * a.ssss[i2 * card + cc];
-                    ss = fmaf(dr[DR_SS + t], u, ss);
-                }
+                ss = fmaf(v10.y, U[(pk & 0xff) * 32 + lane], ss);
+                ss = fmaf(v10.z, U[((pk >> 8) & 0xff) * 32 + lane], ss);
+                ss = fmaf(v10.w, U[((pk >> 16) & 0xff) * 32 + lane], ss);
                 if (-99.f < ss) {
-                    ss += qhq * dr[DR_HD] * 0.1111111f;
+                    ss += qhq * v11.y * 0.1111111f;
                     ss -= 0.05f;
                 }
                 const long long c = cb + (long long)k * 32 + lane;
@@ -205,28 +223,57 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// Row of a strip's neighbour, ADJ_RG columns at a time, in the warp's shared
-// buffer rab[32][8] (slot c & 31: column c).  Forward: row 32 s - 1 (frow of
-// strip s - 1) at columns c0 + l; backward: row 32 s + 32 (brow of strip s + 1)
-// at mirrored columns c0 + l.  WAIT: the neighbour strip is being swept now;
-// poll until those columns are there (row hand-off, c2_device.cuh).
+// Row of a strip's neighbour, ADJ_RG columns at a time in two groups of the
+// warp's shared buffer (row hand-off, c2_device.cuh).  Forward: row 32 s - 1
+// (frow of strip s - 1); backward: row 32 s + 32 (brow of strip s + 1) by
+// mirrored column.
 constexpr int ADJ_RG = 8;
-template <bool WAIT>
-__device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const float* __restrict__ row, int ldr,
-                                             bool have, int c0, int L, int lane, bool& broken)
+
+
+// The forward sweep starts a group's copy a group before its use (two buffers;
+// 1.12 -> 0.85 ms on 256 pairs).
+__device__ __forceinline__ void adj_row_init(const AdjArgs& a, float* rab, const float* __restrict__ row, int ldr, bool have,
+                                             int L, int lane, bool& broken)
+{
+    if (have) {
+        row_issue<ADJ_RG>(rab, row, ldr, 0, L, lane);
+        row_take<ADJ_RG>(rab, row, ldr, 0, L, lane, a.status, broken, a.spin);
+        if (ADJ_RG < L) row_issue<ADJ_RG>(rab + ROW_BUF<ADJ_RG>, row, ldr, ADJ_RG, L, lane);
+    } else if (lane < 2 * ADJ_RG) {
+        float* o = rab + (lane < ADJ_RG ? 0 : ROW_BUF<ADJ_RG>);
+        *reinterpret_cast<float4*>(o + 4 * (lane % ADJ_RG)) = make_float4(0.f, XLOG0, XLOG0, XLOG0);
+        o[4 * ADJ_RG + lane % ADJ_RG] = XLOG0;
+    }
+    __syncwarp();
+}
+
+// column k of the row for lane 0; after a group's last column the next group is
+// taken and the one after it started
+__device__ __forceinline__ void adj_row_step(const AdjArgs& a, float* rab, const float* __restrict__ row, int ldr, bool have,
+                                             int k, int L, int lane, bool& broken, X5& up)
+{
+    const float* b = rab + (k & ADJ_RG ? ROW_BUF<ADJ_RG> : 0);
+    const int u = k & (ADJ_RG - 1);
+    const float4 ba = *reinterpret_cast<const float4*>(b + 4 * u);
+    const float b4 = b[4 * ADJ_RG + u];
+    if (lane == 0) up = X5{ba.x, ba.y, ba.z, ba.w, b4};
+    if (u == ADJ_RG - 1 && have) {
+        const int c0 = k + 1;
+        if (c0 < L) row_take<ADJ_RG>(rab + (c0 & ADJ_RG ? ROW_BUF<ADJ_RG> : 0), row, ldr, c0, L, lane, a.status, broken, a.spin);
+        if (c0 + ADJ_RG < L)
+            row_issue<ADJ_RG>(rab + (c0 & ADJ_RG ? 0 : ROW_BUF<ADJ_RG>), row, ldr, c0 + ADJ_RG, L, lane);
+    }
+}
+
+// The backward sweep, whose steps are longer than a trip through L2, fetches a
+// group when it needs it, into rab[32][8] (slot c & 31); started a group earlier,
+// every strip trails 8 columns further (2.0 -> 2.2 ms on 256 pairs).
+__device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const float* __restrict__ row, int ldr, bool have,
+                                             int c0, int L, int lane, bool& broken)
 {
     const int c = c0 + lane;
     float v[5] = {0.f, XLOG0, XLOG0, XLOG0, XLOG0};
-    const bool want = lane < ADJ_RG && c < L;
-    if (have && c0 < L) {
-        if (WAIT) {
-            row_get(row, ldr, c, want, v, lane, a.status, broken, a.spin);
-        } else if (want) {
-            const float4 x = reinterpret_cast<const float4*>(row)[c];
-            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-            v[4] = row[4 * ldr + c];
-        }
-    }
+    if (have && c0 < L) row_get(row, ldr, c, lane < ADJ_RG && c < L, v, lane, a.status, broken, a.spin);
     if (lane < ADJ_RG) {
         float* o = rab + (c & 31) * 8;
         *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
@@ -237,9 +284,13 @@ __device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const
 
 // Transition rows of a pair's db profile, in base 2 (rows 0..L; row r holds the
 // transitions into position r, MI and II of row r + 1 those out of position
-// r) in the warp's shared ring trs[128][7] by sequence index q: q = row in the
+// r) in the warp's shared ring trs[128][TRS] by sequence index q: q = row in the
 // forward sweep, q = L - row in the mirrored backward sweep.  A step's lanes
-// read rows q in [k - 31, k + 1]; chunks of 32 are staged two ahead.
+// read rows q in [k - 31, k + 1]; chunks of 32 are staged two ahead.  Rows are 12
+// floats apart: 16-byte reads of consecutive rows share no bank.  (Rows outside
+// the profile hold what the ring does: only cells outside the matrix read them,
+// and no cell inside reads those.)
+constexpr int TRS = 12;
 template <bool MIRROR>
 __device__ __forceinline__ void adj_stage_trn(float* trs, const float* __restrict__ dt0, int q0, int L, int lane)
 {
@@ -247,22 +298,41 @@ __device__ __forceinline__ void adj_stage_trn(float* trs, const float* __restric
     for (int e = lane; e < nq * 7; e += 32) {
         const int q = q0 + e / 7, f = e % 7;
         const int row = MIRROR ? L - q : q;
-        trs[(q & 127) * 7 + f] = __ldg(dt0 + (long long)row * 7 + f) * XLOG2E;
+        trs[(q & 127) * TRS + f] = __ldg(dt0 + (long long)row * 7 + f) * XLOG2E;
     }
 }
 
-// forward transitions of column j (rows j and j + 1) from the forward ring
-__device__ __forceinline__ void ring_trn_fwd(const float* trs, int j, int L, float* t7)
+// row q of the ring
+__device__ __forceinline__ void ring_row(const float* trs, int q, float* t)
 {
-    if (j < 0 || j >= L) {
-#pragma unroll
-        for (int k = 0; k < 7; k++) t7[k] = XLOG0;
-        return;
-    }
-    const float* a = trs + (j & 127) * 7;
-    const float* b = trs + ((j + 1) & 127) * 7;
-    t7[TMM] = a[0]; t7[TMI] = b[1]; t7[TMD] = a[2];
-    t7[TIM] = a[3]; t7[TII] = b[4]; t7[TDM] = a[5]; t7[TDD] = a[6];
+    const float* o = trs + (q & 127) * TRS;
+    const float4 a = *reinterpret_cast<const float4*>(o);
+    const float4 b = *reinterpret_cast<const float4*>(o + 4);
+    t[0] = a.x; t[1] = a.y; t[2] = a.z; t[3] = a.w; t[4] = b.x; t[5] = b.y; t[6] = b.z;
+}
+
+// forward transitions of column j (rows j and j + 1) from the forward ring
+__device__ __forceinline__ void ring_trn_fwd(const float* trs, int j, float* t7)
+{
+    ring_row(trs, j, t7);
+    const float* b = trs + ((j + 1) & 127) * TRS;
+    t7[TMI] = b[1];
+    t7[TII] = b[4];
+}
+
+// Forward states of a strip's cells: [step][lane][4] MM MI IM DN, then [lane] ND
+// (160 floats a step: two reads or writes a cell)
+__device__ __forceinline__ void fw_st5(float* __restrict__ Fw, int k, int l, const X5& x)
+{
+    float* o = Fw + (long long)k * 160;
+    reinterpret_cast<float4*>(o)[l] = make_float4(x.MM, x.MI, x.IM, x.DN);
+    o[128 + l] = x.ND;
+}
+__device__ __forceinline__ X5 fw_ld5(const float* __restrict__ Fw, int k, int l)
+{
+    const float* o = Fw + (long long)k * 160;
+    const float4 a = reinterpret_cast<const float4*>(o)[l];
+    return X5{a.x, a.y, a.z, a.w, o[128 + l]};
 }
 
 // L1 prefetch of one 128-byte line (the lines a sweep reads a few steps
@@ -278,7 +348,7 @@ __device__ __forceinline__ void pf_l1(const void* p)
 // it is swept; the strip's last row goes to frow (published for the strip
 // below) and the lane's cells into the online log-sum (zm, zs).
 // RECOMP true (backward sweep): the row above from the complete checkpoint,
-// every state into the warp's scratch Fw[(k * 5 + state) * 32 + lane].
+// every state into the warp's scratch Fw (fw_st5).
 template <bool RECOMP>
 __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, int lane, float* rab, float* trs,
                                               float* __restrict__ Fw, bool& broken, float& zm, float& zs)
@@ -307,33 +377,26 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
     __syncwarp();
     adj_stage_trn<false>(trs, dt0, 0, L, lane);
     adj_stage_trn<false>(trs, dt0, 32, L, lane);
-    adj_load_row<!RECOMP>(a, rab, above, ldr, s > 0, 0, L, lane, broken);
+    adj_row_init(a, rab, above, ldr, s > 0, L, lane, broken);
     for (int k = 0; k < L + 31; k++) {
         const int j = k - lane;
         float t7[7];
-        ring_trn_fwd(trs, j, L, t7);
+        ring_trn_fwd(trs, j, t7);
         X5 up;
         up.MM = __shfl_up_sync(FULL, mine.MM, 1);
         up.MI = __shfl_up_sync(FULL, mine.MI, 1);
         up.IM = __shfl_up_sync(FULL, mine.IM, 1);
         up.DN = __shfl_up_sync(FULL, mine.DN, 1);
         up.ND = __shfl_up_sync(FULL, mine.ND, 1);
-        {
-            const int src = k & 31;
-            const float4 ba = *reinterpret_cast<const float4*>(rab + src * 8);
-            const float b4 = rab[src * 8 + 4];
-            if (lane == 0) up = X5{ba.x, ba.y, ba.z, ba.w, b4};
-            if ((src & (ADJ_RG - 1)) == ADJ_RG - 1) {
-                __syncwarp();
-                adj_load_row<!RECOMP>(a, rab, above, ldr, s > 0, k + 1, L, lane, broken);
-            }
-            if (src == 31) {
-                if (k + 33 <= L) adj_stage_trn<false>(trs, dt0, k + 33, L, lane);
-                __syncwarp();
-            }
+        adj_row_step(a, rab, above, ldr, s > 0, k, L, lane, broken, up);
+        if ((k & 31) == 31) {
+            __syncwarp();
+            if (k + 33 <= L) adj_stage_trn<false>(trs, dt0, k + 33, L, lane);
+            __syncwarp();
         }
         X5 left = mine, diag = upp;
         if (j == 0) { left = LB; diag = DB; }
+        if (lane == 0 && k + 2 * ADJ_PF < L + 31) pf_l1(a.S + cb + (long long)(k + 2 * ADJ_PF) * 32);
         const bool valid = act && j >= 0 && j < L;
         const float sc = valid ? scn : XLOG0;
         if (act && j + 1 >= 0 && j + 1 < L) scn = a.S[cb + (long long)(k + 1) * 32 + lane];
@@ -346,13 +409,11 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
         nw.DN = xlse2(up.MM + q7[TMD], up.DN + q7[TDD]);
         nw.ND = xlse2(left.MM + t7[TMD], left.ND + t7[TDD]);
         if (valid) {
-            if (RECOMP || Fw) {
-                float* o = Fw + (long long)k * 160 + lane;
-                o[0] = nw.MM; o[32] = nw.MI; o[64] = nw.IM; o[96] = nw.DN; o[128] = nw.ND;
-            }
+            if (RECOMP || Fw) fw_st5(Fw, k, lane, nw);
             if (!RECOMP) {
-                if (nw.MM > zm) { zs = zs * xexp(zm - nw.MM) + 1.f; zm = nw.MM; }
-                else zs += xexp(nw.MM - zm);
+                const float mx = fmaxf(zm, nw.MM);
+                zs = fmaf(zs, xexp(zm - mx), xexp(nw.MM - mx));
+                zm = mx;
             }
             if (wr_row) row_put(mine_row, ldr, j, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
         }
@@ -364,8 +425,8 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
 // forward sweep: logZ partial sums per strip, checkpoint rows
 __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_fwd_kernel(AdjArgs a)
 {
-    __shared__ __align__(16) float rabs[ADJ_WARPS][32 * 8];
-    __shared__ float trss[ADJ_WARPS][128 * 7];
+    __shared__ __align__(16) float rabs[ADJ_WARPS][2 * ROW_BUF<ADJ_RG>];
+    __shared__ __align__(16) float trss[ADJ_WARPS][128 * TRS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     bool broken = false;
     for (;;) {
@@ -421,12 +482,6 @@ __global__ void adj_logz_kernel(AdjArgs a)
 // follow the transposed recursion; at every cell the posteriors of its
 // incoming edges exp(F(pred) + edge + B(cell) - logZ) come from the
 // recomputed forward states of the strip (and the checkpoint row above it).
-__device__ __forceinline__ X5 fw_ld5(const float* __restrict__ Fw, int k, int l)
-{
-    const float* o = Fw + (long long)k * 160 + l;
-    return X5{o[0], o[32], o[64], o[96], o[128]};
-}
-
 // column c of a complete row
 __device__ __forceinline__ X5 row_ld5(const float* __restrict__ row, int ldr, int c)
 {
@@ -470,7 +525,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     __syncwarp();
     adj_stage_trn<true>(trs, dt0, 0, L, lane);
     adj_stage_trn<true>(trs, dt0, 32, L, lane);
-    adj_load_row<true>(a, rab, below, ldr, has_below, 0, L, lane, broken);
+    adj_load_row(a, rab, below, ldr, has_below, 0, L, lane, broken);
     // Forward states and scores of the lane's own row, one wavefront line a
     // step: at step k the lane's cell is on line kf = L + 30 - k, its left
     // neighbour on line kf - 1; the row above (lf - 1) is lane t + 1's, whose
@@ -520,16 +575,11 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         const float scu = __shfl_up_sync(FULL, sc2, 1);   // score of (i + 1, ca + 1): lane t - 1 two steps ago
         // transitions out of column ca (row ca + 1, sequence index jm) and,
         // for the edge posteriors, into it (rows ca and ca + 1)
-        const bool colv = jm >= 0 && jm < L;
         float tb[7], tf[7];
-        {
-            const float* b = trs + (jm & 127) * 7;         // row ca + 1
-            const float* c = trs + ((jm + 1) & 127) * 7;   // row ca
-#pragma unroll
-            for (int f = 0; f < 7; f++) tb[f] = colv ? b[f] : XLOG0;
-            tf[TMM] = c[0]; tf[TMI] = b[1]; tf[TMD] = c[2];
-            tf[TIM] = c[3]; tf[TII] = b[4]; tf[TDM] = c[5]; tf[TDD] = c[6];
-        }
+        ring_row(trs, jm, tb);          // row ca + 1
+        ring_row(trs, jm + 1, tf);      // row ca
+        tf[TMI] = tb[TMI];
+        tf[TII] = tb[TII];
         X5 dn;
         dn.MM = __shfl_up_sync(FULL, mine.MM, 1);
         dn.MI = __shfl_up_sync(FULL, mine.MI, 1);
@@ -543,7 +593,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
             if (lane == 0) dn = X5{ba.x, ba.y, ba.z, ba.w, b4};
             if ((src & (ADJ_RG - 1)) == ADJ_RG - 1) {
                 __syncwarp();
-                adj_load_row<true>(a, rab, below, ldr, has_below, k + 1, L, lane, broken);
+                adj_load_row(a, rab, below, ldr, has_below, k + 1, L, lane, broken);
             }
             if (src == 31) {
                 if (k + 33 <= L) adj_stage_trn<true>(trs, dt0, k + 33, L, lane);
@@ -627,12 +677,18 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     }
 }
 
-__global__ void __launch_bounds__(ADJ_WARPS * 32, 4) adj_bwd_kernel(AdjArgs a)
+// Bound by the chain of steps (a step of ~350 instructions, ~1,000 steps deep).
+// KEPT: the forward sweep kept its states (Fall), the recomputing sweep and its
+// registers are not in the kernel, and 12 warps an SM at 162 registers beat 16 at
+// 128 (the two in one kernel spilled 4 registers): 2.0 -> 1.72 ms on 256 pairs
+// of 100..600 positions, 0.48 -> 0.43 on 45 of 60..300 (16 warps: 1.88, 0.44).
+template <bool KEPT>
+__global__ void __launch_bounds__(ADJ_WARPS * 32, KEPT ? 3 : 4) adj_bwd_kernel(AdjArgs a)
 {
     __shared__ __align__(16) float rabs[ADJ_WARPS][32 * 8];
-    __shared__ float trss[ADJ_WARPS][128 * 7];
+    __shared__ __align__(16) float trss[ADJ_WARPS][128 * TRS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* const scr = a.Fall ? nullptr : a.scratch + ((long long)blockIdx.x * ADJ_WARPS + wid) * a.scratch_stride;
+    float* const scr = KEPT ? nullptr : a.scratch + ((long long)blockIdx.x * ADJ_WARPS + wid) * a.scratch_stride;
     bool broken = false;
     for (;;) {
         int item = 0;
@@ -642,7 +698,7 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, 4) adj_bwd_kernel(AdjArgs a)
         const int2 ms = a.items_b[item];
         const int m = ms.x, s = ms.y;
         const float* Fw;
-        if (a.Fall) {
+        if (KEPT) {
             // the forward sweep kept the strip's states
             Fw = a.Fall + 5 * a.off[m] + (long long)s * (a.plen[a.prof[m]] + 31) * 160;
         } else {
@@ -673,14 +729,17 @@ cudaError_t adj_occupancy(int* fwd_ctas_per_sm, int* bwd_ctas_per_sm)
 {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(fwd_ctas_per_sm, adj_fwd_kernel, ADJ_WARPS * 32, 0);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bwd_ctas_per_sm, adj_bwd_kernel, ADJ_WARPS * 32, 0);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bwd_ctas_per_sm, adj_bwd_kernel<false>, ADJ_WARPS * 32, 0);
 }
 
 cudaError_t launch_adj_fwd(const AdjArgs& a, int grid, cudaStream_t st)
 {
     if (a.npairs <= 0) return cudaSuccess;
     const int sgrid = std::min((a.nitems + ADJ_WARPS - 1) / ADJ_WARPS, 1184);
-    adj_score_kernel<<<sgrid, 128, 0, st>>>(a);
+    const size_t ssm = (size_t)ADJ_WARPS * ADJ_SCORE_FLOATS * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(adj_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
+    if (e != cudaSuccess) return e;
+    adj_score_kernel<<<sgrid, ADJ_WARPS * 32, ssm, st>>>(a);
     adj_fwd_kernel<<<grid, ADJ_WARPS * 32, 0, st>>>(a);
     adj_logz_kernel<<<(a.npairs + 127) / 128, 128, 0, st>>>(a);
     return cudaGetLastError();
@@ -689,7 +748,10 @@ cudaError_t launch_adj_fwd(const AdjArgs& a, int grid, cudaStream_t st)
 cudaError_t launch_adj_bwd(const AdjArgs& a, int grid, cudaStream_t st)
 {
     if (a.npairs <= 0) return cudaSuccess;
-    adj_bwd_kernel<<<grid, ADJ_WARPS * 32, 0, st>>>(a);
+    if (a.Fall)
+        adj_bwd_kernel<true><<<grid, ADJ_WARPS * 32, 0, st>>>(a);
+    else
+        adj_bwd_kernel<false><<<grid, ADJ_WARPS * 32, 0, st>>>(a);
     adj_gsum_kernel<<<(a.npairs * 9 + 127) / 128, 128, 0, st>>>(a);
     return cudaGetLastError();
 }

@@ -50,7 +50,7 @@ struct AdjArgs {
     float* zpart;           // [nitems][2] (max, scaled sum) of a strip's 2^F.MM; then log2 Z at a pair's first
     float* gpart;           // [nitems][9] a strip's gradient sums
     float* Fall;            // forward states of every strip, when they fit (else null): strip s of
-                            // pair m at Fall + 5 off[m] + s (L + 31) 160, [step][state][lane]
+                            // pair m at Fall + 5 off[m] + s (L + 31) 160 (fw_st5)
     float* scratch;         // per backward warp (Fall null): forward states of its strip, [(Lmax + 31) * 5 * 32]
     long long scratch_stride;
     int* counter;           // [2] work counters of the forward and backward sweeps
