@@ -116,7 +116,28 @@ struct DbStore {
     std::mutex tc_mu;
 };
 
+// Pinned host memory of a handle through which its transfers go: an
+// asynchronous copy from or to pageable memory is staged by the driver piece
+// by piece and returns late.  Space is taken in order; when it runs out, the
+// stream is synchronised (every copy is then done) and it starts over.  It
+// grows to the largest piece taken, at most 2 x STAGE_MAX.
+constexpr size_t STAGE_MIN = size_t(1) << 20, STAGE_MAX = size_t(20) << 20;
+struct HostStage {
+    char* p = nullptr;
+    size_t cap = 0, used = 0;
+    bool pinned = false;
+    ~HostStage() { release(); }
+    void release()
+    {
+        if (p && pinned) cudaFreeHost(p);
+        else free(p);
+        p = nullptr;
+        cap = used = 0;
+    }
+};
+
 struct c2_handle {
+    HostStage stage;
     int device = 0;
     cudaStream_t stream = nullptr;      // stream in use
     cudaStream_t own_stream = nullptr;  // the handle's own stream
@@ -147,6 +168,9 @@ struct c2_handle {
     int Lq = 0;
     float qeno = 0.f;
     std::vector<float> h_qrec;
+    std::vector<float> h_qtrn;        // raw transitions of the query
+    bool qtc_ready = false;           // tensor-core operands of the current query packed
+    bool qcfx_ready = false;          // exact column -1 states of the current query (c2_logz_fwd)
     DevBuf<float> d_qrec, d_qbkg, d_qtrn, d_qcf, d_qcfx, d_qU;
     // differentiable alignment (c2_logz_fwd / c2_logz_bwd)
     std::vector<int> adj_prof, adj_Lq;
@@ -210,6 +234,8 @@ struct c2_handle {
     DevBuf<float> d_fb, d_bb, d_pairf;
     DevBuf<unsigned> d_pairc;
     DevBuf<unsigned long long> d_pairk;
+    bool info_valid = false;          // h_info: the hits' alignment counts, the status checked
+    std::vector<int> h_info;
     DevBuf<char> d_aln, d_alnpack;
     DevBuf<long long> d_alnoff;
     int alnstride = 0;
@@ -244,8 +270,90 @@ static c2_status fail(c2_handle* h, c2_status st, const char* fmt, ...)
                         __FILE__, __LINE__);                                            \
     } while (0)
 
+// `bytes` of the handle's pinned staging memory, valid until the stage starts
+// over (a later stage_take, after a stream synchronisation); null: no memory
+static char* stage_take(c2_handle* h, size_t bytes)
+{
+    HostStage& S = h->stage;
+    bytes = (bytes + 255) & ~size_t(255);
+    if (S.used + bytes > S.cap) {
+        if (cudaStreamSynchronize(h->stream) != cudaSuccess) return nullptr;
+        S.used = 0;
+        if (bytes > S.cap) {
+            const size_t want = std::max(STAGE_MIN, 2 * bytes);
+            S.release();
+            S.pinned = cudaHostAlloc(reinterpret_cast<void**>(&S.p), want, cudaHostAllocDefault) == cudaSuccess;
+            if (!S.pinned) {
+                // pageable memory then: the copies are complete, or taken over, when they return
+                (void)cudaGetLastError();
+                S.p = static_cast<char*>(malloc(want));
+            }
+            if (!S.p) return nullptr;
+            S.cap = want;
+        }
+    }
+    char* r = S.p + S.used;
+    S.used += bytes;
+    return r;
+}
+
+// host -> device through the staging memory; src may be reused at once
+static cudaError_t h2d(c2_handle* h, void* dst, const void* src, size_t bytes)
+{
+    constexpr size_t PIECE = size_t(4) << 20;
+    for (size_t o = 0; o < bytes; o += PIECE) {
+        const size_t n = std::min(PIECE, bytes - o);
+        char* p = stage_take(h, n);
+        if (!p) return cudaErrorMemoryAllocation;
+        memcpy(p, static_cast<const char*>(src) + o, n);
+        const cudaError_t e = cudaMemcpyAsync(static_cast<char*>(dst) + o, p, n, cudaMemcpyHostToDevice, h->stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// device -> host: several arrays with one synchronisation.  get() queues a copy
+// (directly where it is larger than the stage), finish() waits for all of them.
+struct Fetch {
+    c2_handle* h;
+    struct Part { void* dst; const char* p; size_t n; };
+    std::vector<Part> parts;
+    explicit Fetch(c2_handle* hh) : h(hh) {}
+    cudaError_t get(void* dst, const void* src, size_t bytes)
+    {
+        if (bytes == 0) return cudaSuccess;
+        size_t held = 0;
+        for (const Part& q : parts) held += q.n + 256;
+        if (bytes > STAGE_MAX || held + bytes > STAGE_MAX) {
+            const cudaError_t e = finish();
+            if (e != cudaSuccess) return e;
+            if (bytes > STAGE_MAX) {
+                const cudaError_t c = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream);
+                return c != cudaSuccess ? c : cudaStreamSynchronize(h->stream);
+            }
+        }
+        // (taking space may start the stage over: not while parts are in it)
+        if (!parts.empty() && h->stage.used + bytes + 256 > h->stage.cap) {
+            const cudaError_t e = finish();
+            if (e != cudaSuccess) return e;
+        }
+        char* p = stage_take(h, bytes);
+        if (!p) return cudaErrorMemoryAllocation;
+        parts.push_back({dst, p, bytes});
+        return cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, h->stream);
+    }
+    cudaError_t finish()
+    {
+        const cudaError_t e = cudaStreamSynchronize(h->stream);
+        if (e == cudaSuccess)
+            for (const Part& q : parts) memcpy(q.dst, q.p, q.n);
+        parts.clear();
+        return e;
+    }
+};
+
 // device status words: 2 = the traceback DP's maximum differs from phase 1,
-// 3 = a phase-2 sweep gave up waiting for the strip above it
+// 3 = a phase-2 sweep gave up waiting for the strip above it, 4 = phase 1 did
 static const char* status_text(int st)
 {
     switch (st) {
@@ -798,7 +906,11 @@ static void qrec_score_fields(const c2_handle* h, const c2_profiles* q, float* q
 static void colm1_exact(const c2_profiles* q, float* qx)
 {
     const int Lq = q->lengths[0];
-    auto xl2 = [](double a, double b) { const double m = std::max(a, b); return std::log(std::exp(a - m) + std::exp(b - m)) + m; };
+    // (a term below e^-40 of the other does not change the sum in double precision)
+    auto xl2 = [](double a, double b) {
+        const double m = std::max(a, b), d = std::fabs(a - b);
+        return d > 40.0 ? m : std::log(1.0 + std::exp(-d)) + m;
+    };
     double pMI = 0, pIM = 0, pDN = 0;
     for (int r = 0; r < Lq; r++) {
         float t[7];
@@ -843,6 +955,79 @@ static void query_limits(const c2_handle* h, int Lq, unsigned long long* searchs
     }
 }
 
+// SS row table of a query row with SS probabilities s3: U[c] = sum_s p(s) T[idx(s)][c]
+static void ss_row_table(const c2_handle* h, const float* s3, float* U)
+{
+    const int card = h->sc.ssss_card;
+    const float* t0 = &h->ssss[(size_t)(int)(s3[0] * 9.999f) * card];
+    const float* t1 = &h->ssss[(size_t)(10 + (int)(s3[1] * 9.999f)) * card];
+    const float* t2 = &h->ssss[(size_t)(20 + (int)(s3[2] * 9.999f)) * card];
+    for (int c = 0; c < card; c++) U[c] = s3[0] * t0[c] + s3[1] * t1[c] + s3[2] * t2[c];
+}
+
+// Tensor-core operands of the current query (layouts in c2_device.cuh), from
+// its records: context vectors (k = 19: 1, the 1/kappa0 column) and SS row
+// tables (k = 30: P(H) + 0.1, k = 31: 1) as split BF16 A fragments, amino-acid
+// rows unscaled in fragment order.  Packed when the query is set in the
+// tensor-core score mode, or by the first phase 1 after a change to it.
+static c2_status pack_query_operands(c2_handle* h)
+{
+    const int Lq = h->Lq, card = h->sc.ssss_card;
+    const int nt = (Lq + P1_ROWS - 1) / P1_ROWS;
+    // hi and lo parts of a row's operands: CV k 0..23, then SS k 0..31
+    constexpr int KR = 24 + 32;
+    std::vector<uint16_t> hi((size_t)nt * P1_ROWS * KR, 0), lo((size_t)nt * P1_ROWS * KR, 0);
+    for (int r = 0; r < Lq; r++) {
+        const float* rec = h->h_qrec.data() + (size_t)r * QR_STRIDE;
+        float x[KR] = {0.f}, U[MAX_SSSS_CARD];
+        memcpy(x, rec + QR_CV, NCV * 4);
+        x[NCV] = 1.f;
+        ss_row_table(h, rec + QR_SS, U);
+        for (int c = 0; c < std::min(card, TC_SS_KMAX); c++) x[24 + c] = U[c];
+        x[24 + TC_SS_KMAX] = rec[QR_HQ];
+        x[24 + TC_SS_KMAX + 1] = 1.f;
+        uint16_t *ph = &hi[(size_t)r * KR], *pl = &lo[(size_t)r * KR];
+        for (int k = 0; k < KR; k++) {
+            const uint32_t b = bf16_rn_bits(x[k]);
+            ph[k] = (uint16_t)b;
+            pl[k] = (uint16_t)bf16_rn_bits(x[k] - bf16_to_f(b));
+        }
+    }
+    std::vector<uint32_t> qa((size_t)nt * TC_QA_WORDS, 0u);
+    std::vector<float> qaa((size_t)nt * TC_QAA_FLOATS, 0.f);
+    for (int s = 0; s < nt; s++)
+        for (int mt = 0; mt < 4; mt++)
+            for (int lane = 0; lane < 32; lane++) {
+                const int g = lane >> 2, qq = lane & 3;
+                const int r0 = P1_ROWS * s + 16 * mt + g;
+                // word w of an operand: row r0 + 8 (w & 1), k = 8 (w >> 1) + 2 qq, + 1; the
+                // CV operand (first k 0) has words 0..5, the SS operand (24) 0..7
+                const size_t o = (size_t)(s * 4 + mt) * 7;   // 16-byte groups
+                int at = 0;                                  // word of the fragment
+                auto put = [&](const std::vector<uint16_t>& v, int k0, int w) {
+                    const uint16_t* e = &v[(size_t)(r0 + ((w & 1) ? 8 : 0)) * KR + k0 + 8 * (w >> 1) + 2 * qq];
+                    qa[((o + at / 4) * 32 + lane) * 4 + at % 4] = e[0] | ((uint32_t)e[1] << 16);
+                    at++;
+                };
+                for (int w = 0; w < 4; w++) put(hi, 0, w);
+                for (int w = 0; w < 4; w++) put(lo, 0, w);
+                for (int w = 0; w < 8; w++) put(hi, 24, w);
+                for (int w = 0; w < 8; w++) put(lo, 24, w);
+                put(hi, 0, 4); put(hi, 0, 5); put(lo, 0, 4); put(lo, 0, 5);
+                for (int e = 0; e < 12; e++) {
+                    const int w = e >> 1, r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq + (e & 1);
+                    qaa[(((size_t)(s * 4 + mt) * 3 + e / 4) * 32 + lane) * 4 + e % 4] =
+                        (r < Lq && k < NAA) ? h->h_qrec[(size_t)r * QR_STRIDE + QR_TRG + k] : 0.f;
+                }
+            }
+    if (h->d_qa.ensure(qa.size(), h->budget) || h->d_qaaf.ensure(qaa.size(), h->budget))
+        return fail(h, C2_ERR_NOMEM, "query operand allocation failed");
+    CK(h2d(h, h->d_qa.p, qa.data(), qa.size() * 4));
+    CK(h2d(h, h->d_qaaf.p, qaa.data(), qaa.size() * 4));
+    h->qtc_ready = true;
+    return C2_OK;
+}
+
 extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
 {
     if (!h) return C2_ERR_ARG;
@@ -856,9 +1041,12 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
     h->h_cand_off.clear();
     h->ncand = h->npass = h->nmap = 0;
     h->acc_valid = false;
+    h->info_valid = false;
     h->ngroups = 1;
     const int Lq = q->lengths[0];
     h->Lq = Lq;
+    h->qtc_ready = h->qcfx_ready = false;
+    h->h_qtrn.assign(q->trn, q->trn + (size_t)(Lq + 1) * 7);
     h->qeno = q->eno ? q->eno[0] : 0.f;
     h->h_qrec.assign((size_t)Lq * QR_STRIDE, 0.f);
     // column -1 boundary states (see oracle colm1_states; CuBatchDP_init_btck.cu:117-262)
@@ -882,83 +1070,22 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
     }
     if (h->d_qrec.ensure(h->h_qrec.size(), h->budget) || h->d_qbkg.ensure(NAA, h->budget))
         return fail(h, C2_ERR_NOMEM, "query allocation failed");
-    // tensor-core query operands (layouts in c2_device.cuh): context vectors
-    // (k = 19: 1, the 1/kappa0 column) and SS row tables
-    // U[r][c] = sum_s p_q(s) T[idx_q(s)][c] (k = 30: P(H) + 0.1, k = 31: 1) as
-    // split BF16 A fragments, amino-acid rows unscaled in fragment order
+    // the SS row tables per strip of 32 rows, [strip][MAX_SSSS_CARD][32] (lane =
+    // row), for the FP32 kernels
     {
-        const int ns = (Lq + 31) / 32;
-        const int card = h->sc.ssss_card;
-        std::vector<float> U((size_t)Lq * 32, 0.f);
+        const int ns = (Lq + 31) / 32, card = h->sc.ssss_card;
+        std::vector<float> qU((size_t)ns * MAX_SSSS_CARD * 32, 0.f);
         for (int r = 0; r < Lq; r++) {
-            const float* s3 = q->ss + (size_t)r * NSS;
-            const int i0 = (int)(s3[0] * 9.999f), i1 = 10 + (int)(s3[1] * 9.999f), i2 = 20 + (int)(s3[2] * 9.999f);
-            for (int c = 0; c < card; c++)
-                U[(size_t)r * 32 + c] = s3[0] * h->ssss[(size_t)i0 * card + c] + s3[1] * h->ssss[(size_t)i1 * card + c] +
-                                        s3[2] * h->ssss[(size_t)i2 * card + c];
+            float U[MAX_SSSS_CARD];
+            ss_row_table(h, q->ss + (size_t)r * NSS, U);
+            for (int c = 0; c < card; c++) qU[((size_t)(r / 32) * MAX_SSSS_CARD + c) * 32 + (r % 32)] = U[c];
         }
-        // the same tables per strip, [strip][MAX_SSSS_CARD][32] (lane = row), for
-        // the FP32 kernels
-        {
-            std::vector<float> qU((size_t)ns * MAX_SSSS_CARD * 32, 0.f);
-            for (int r = 0; r < Lq; r++)
-                for (int c = 0; c < card; c++)
-                    qU[((size_t)(r / 32) * MAX_SSSS_CARD + c) * 32 + (r % 32)] = U[(size_t)r * 32 + c];
-            if (h->d_qU.ensure(qU.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "query SS table allocation failed");
-            CK(cudaMemcpyAsync(h->d_qU.p, qU.data(), qU.size() * 4, cudaMemcpyHostToDevice, h->stream));
-            CK(cudaStreamSynchronize(h->stream));
-        }
-        auto aval = [&](int d, int r, int k) -> float {
-            if (r >= Lq) return 0.f;
-            if (d == 0) return k < NCV ? q->cv[(size_t)r * NCV + k] : (k == NCV ? 1.f : 0.f);
-            if (k == TC_SS_KMAX) return h->h_qrec[(size_t)r * QR_STRIDE + QR_HQ];
-            if (k == TC_SS_KMAX + 1) return 1.f;
-            return k < card ? U[(size_t)r * 32 + k] : 0.f;
-        };
-        const int nt = (Lq + P1_ROWS - 1) / P1_ROWS;
-        std::vector<uint32_t> qa((size_t)nt * TC_QA_WORDS, 0u);
-        std::vector<float> qaa((size_t)nt * TC_QAA_FLOATS, 0.f);
-        for (int s = 0; s < nt; s++)
-            for (int mt = 0; mt < 4; mt++)
-                for (int lane = 0; lane < 32; lane++) {
-                    const int g = lane >> 2, qq = lane & 3;
-                    const int r0 = P1_ROWS * s + 16 * mt + g;
-                    // word w of operand d: row r0 + 8 (w & 1), k = 8 (w >> 1) + 2 qq, + 1; the
-                    // CV operand has words 0..5 (k < 24), the SS operand 0..7
-                    size_t o = (size_t)(s * 4 + mt) * 7;   // 16-byte groups
-                    int at = 0;                            // word of the fragment
-                    auto put = [&](uint32_t w) {
-                        qa[((o + at / 4) * 32 + lane) * 4 + at % 4] = w;
-                        at++;
-                    };
-                    uint32_t hi[2][8], lo[2][8];
-                    for (int d = 0; d < 2; d++)
-                        for (int w = 0; w < (d == 0 ? 6 : 8); w++) {
-                            const int r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq;
-                            const float x0 = aval(d, r, k), x1 = aval(d, r, k + 1);
-                            const uint32_t h0 = bf16_rn_bits(x0), h1 = bf16_rn_bits(x1);
-                            hi[d][w] = h0 | (h1 << 16);
-                            lo[d][w] = bf16_rn_bits(x0 - bf16_to_f(h0)) | (bf16_rn_bits(x1 - bf16_to_f(h1)) << 16);
-                        }
-                    for (int w = 0; w < 4; w++) put(hi[0][w]);
-                    for (int w = 0; w < 4; w++) put(lo[0][w]);
-                    for (int w = 0; w < 8; w++) put(hi[1][w]);
-                    for (int w = 0; w < 8; w++) put(lo[1][w]);
-                    put(hi[0][4]); put(hi[0][5]); put(lo[0][4]); put(lo[0][5]);
-                    for (int e = 0; e < 12; e++) {
-                        const int w = e >> 1, r = r0 + ((w & 1) ? 8 : 0), k = 8 * (w >> 1) + 2 * qq + (e & 1);
-                        qaa[(((size_t)(s * 4 + mt) * 3 + e / 4) * 32 + lane) * 4 + e % 4] =
-                            (r < Lq && k < NAA) ? q->trg[(size_t)r * NAA + k] : 0.f;
-                    }
-                }
-        if (h->d_qa.ensure(qa.size(), h->budget) || h->d_qaaf.ensure(qaa.size(), h->budget))
-            return fail(h, C2_ERR_NOMEM, "query operand allocation failed");
-        CK(cudaMemcpyAsync(h->d_qa.p, qa.data(), qa.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemcpyAsync(h->d_qaaf.p, qaa.data(), qaa.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        if (h->d_qU.ensure(qU.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "query SS table allocation failed");
+        CK(h2d(h, h->d_qU.p, qU.data(), qU.size() * 4));
     }
-    CK(cudaMemcpyAsync(h->d_qrec.p, h->h_qrec.data(), h->h_qrec.size() * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_qbkg.p, q->bkg, NAA * 4, cudaMemcpyHostToDevice, h->stream));
+    if (h->score_mode == C2_SCORE_BF16_TC && (st = pack_query_operands(h)) != C2_OK) return st;
+    CK(h2d(h, h->d_qrec.p, h->h_qrec.data(), h->h_qrec.size() * 4));
+    CK(h2d(h, h->d_qbkg.p, q->bkg, NAA * 4));
     // MAP forward: column -1 states of the query rows (log-sum-exp form of the
     // Viterbi boundary; src/libmycu/cumapdp/CuBatchMAPDP_fwd.cu:72-478)
     {
@@ -983,20 +1110,13 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
         if (h->d_qcf.ensure(qcf.size(), h->budget) || h->d_qtrn.ensure((size_t)(Lq + 1) * 7, h->budget) || h->d_qaa.ensure(Lq, h->budget) ||
             h->d_qss.ensure(Lq, h->budget))
             return fail(h, C2_ERR_NOMEM, "query side arrays allocation failed");
-        CK(cudaMemcpyAsync(h->d_qcf.p, qcf.data(), qcf.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        // the same column -1 states with exact exp/log, for the log-partition model
-        std::vector<float> qx((size_t)Lq * 6, 0.f);
-        colm1_exact(q, qx.data());
-        if (h->d_qcfx.ensure(qx.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "query side arrays allocation failed");
-        CK(cudaMemcpyAsync(h->d_qcfx.p, qx.data(), qx.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        CK(h2d(h, h->d_qcf.p, qcf.data(), qcf.size() * 4));
         h->adj_fwd_done = false;
-        CK(cudaMemcpyAsync(h->d_qtrn.p, q->trn, (size_t)(Lq + 1) * 7 * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemcpyAsync(h->d_qaa.p, q->aa, (size_t)Lq, cudaMemcpyHostToDevice, h->stream));
-        if (q->ssstate) CK(cudaMemcpyAsync(h->d_qss.p, q->ssstate, (size_t)Lq, cudaMemcpyHostToDevice, h->stream));
+        CK(h2d(h, h->d_qtrn.p, q->trn, (size_t)(Lq + 1) * 7 * 4));
+        CK(h2d(h, h->d_qaa.p, q->aa, (size_t)Lq));
+        if (q->ssstate) CK(h2d(h, h->d_qss.p, q->ssstate, (size_t)Lq));
         else CK(cudaMemsetAsync(h->d_qss.p, ' ', (size_t)Lq, h->stream));
     }
-    CK(cudaStreamSynchronize(h->stream));
     query_limits(h, Lq, &h->searchspace, &h->deltalen, &h->scorethld, &h->logevthld);
     return C2_OK;
 }
@@ -1112,14 +1232,14 @@ static void fill_p1(c2_handle* h, P1Args& a)
 // time all pairs together take on all warps (both grow with the number of
 // strips alike, so the query length does not enter).  Pairs below that even
 // out over the warps by the longest-first order; pairs above it would be the
-// tail of the search.  Phase-1 times with shares of infinity (none split) / 1 /
-// 0.5 / 0.25 / 0.1: 1 x 3,000 vs 4,000 profiles 41.9 / 23.2 / 23.8 / 26.7 / 25.7
-// ms, 1 x 1,237 vs 4,999 16.2 / 9.7 / 10.4 / 10.8 / 11.3, 1 x 250 vs 3,000 (FP32)
-// 4.5 / 2.3 / 2.1 / 2.3 / 2.3, 7 queries vs 1,000 (FP32) 32 / 11 / 8.4 / 8.6 /
-// 8.6, 1 x 150 vs 2,000 0.70 / 0.66 / 0.60 / 0.57 / 0.55 (with strips of 32 rows);
-// no pair is split, and nothing changes, against 50,000 profiles.  0 without the
-// scratch (it is small: the two boundary
-// rows of the split pairs) -- the pairs then run whole, with the same results.
+// tail of the search.  Phase-1 times in ms with shares of 1 / 0.7 / 0.5 / 0.3 /
+// 0.15: 1 x 3,000 vs 4,000 profiles 18.8 / 18.7 / 19.3 / 21.0 / 21.3, 1 x 1,237 vs
+// 4,999 8.2 / 8.2 / 8.7 / 8.8 / 9.4, 1 x 250 vs 3,000 (FP32) 1.36 / 1.47 / 1.40 / 1.44 /
+// 1.54, 7 queries vs 1,000 (FP32) 6.4 / 6.2 / 6.1 / 6.0 / 6.0, 1 x 150 vs 2,000 0.60 /
+// 0.58 / 0.55 / 0.51 / 0.49 (none split, before strips of 64 rows: 41.9, 16.2, 4.5, 32,
+// 0.70); no pair is split, and nothing changes, against 50,000 profiles.  0
+// without the scratch (it is small: the two boundary rows of the split pairs) --
+// the pairs then run whole, with the same results.
 constexpr double SPLIT_SHARE = 0.5;
 
 static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
@@ -1162,6 +1282,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     CK(cudaMemsetAsync(h->d_counter.p, 0, sizeof(int), h->stream));
     if (h->score_mode == C2_SCORE_BF16_TC) {
         c2_status st = tc_prepare_db(h);
+        if (st == C2_OK && !h->qtc_ready) st = pack_query_operands(h);
         if (st != C2_OK) return st;
         a.tcdb = h->db->d_tcdb.p;
         a.ttile = h->db->d_ttile.p;
@@ -1280,11 +1401,15 @@ extern "C" c2_status c2_sync(c2_handle* h)
 extern "C" c2_status c2_get_phase1(c2_handle* h, c2_p1_result* out, int32_t n)
 {
     if (!h || !out || n < h->nprof) return C2_ERR_ARG;
-    CK(cudaStreamSynchronize(h->stream));
     std::vector<float> b(h->nprof);
     std::vector<unsigned> c(h->nprof);
-    CK(cudaMemcpy(b.data(), h->d_best.p, (size_t)h->nprof * 4, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(c.data(), h->d_coords.p, (size_t)h->nprof * 4, cudaMemcpyDeviceToHost));
+    int stw = 0;
+    Fetch F(h);
+    CK(F.get(b.data(), h->d_best.p, (size_t)h->nprof * 4));
+    CK(F.get(c.data(), h->d_coords.p, (size_t)h->nprof * 4));
+    CK(F.get(&stw, h->d_status.p, sizeof(int)));
+    CK(F.finish());
+    if (stw == PIPE_ERR_TIMEOUT_P1) return fail(h, C2_ERR_DEVICE, "device status %d (%s)", stw, status_text(stw));
     for (int k = 0; k < h->nprof; k++) { out[k].best = b[k]; out[k].coords = c[k]; }
     return C2_OK;
 }
@@ -1296,9 +1421,10 @@ extern "C" c2_status c2_get_phase1(c2_handle* h, c2_p1_result* out, int32_t n)
 static c2_status select_candidates(c2_handle* h, std::vector<int>& cand)
 {
     CK(cudaSetDevice(h->device));
-    CK(cudaStreamSynchronize(h->stream));
     std::vector<float> b(h->nprof);
-    CK(cudaMemcpy(b.data(), h->d_best.p, (size_t)h->nprof * 4, cudaMemcpyDeviceToHost));
+    Fetch F(h);
+    CK(F.get(b.data(), h->d_best.p, (size_t)h->nprof * 4));
+    CK(F.finish());
     const float cut = (h->score_mode == C2_SCORE_FP32)
                           ? h->scorethld
                           : h->scorethld - C2_TC_MARGIN * std::max(1.0f, std::fabs(h->scorethld));
@@ -1320,6 +1446,7 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
         acc += (long long)h->Lq * h->h_plen[k];
     }
     h->ncand = (int)h->h_cand.size();
+    h->info_valid = false;
     *ncand = h->ncand;
     if (h->ncand == 0) return C2_OK;
     const int nc = h->ncand;
@@ -1332,8 +1459,8 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
         h->d_fpassed.ensure(nc, h->budget) || h->d_fbeg.ensure(nc, h->budget) || h->d_fend.ensure(nc, h->budget) ||
         h->d_bnd.ensure(2 * bnd_half, h->budget) || h->d_tbkey.ensure(nc, h->budget))
         return fail(h, C2_ERR_NOMEM, "finalisation scratch for %d pairs (%lld cells) failed", nc, acc);
-    CK(cudaMemcpyAsync(h->d_cand_prof.p, h->h_cand.data(), (size_t)nc * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_cand_off.p, h->h_cand_off.data(), (size_t)nc * 8, cudaMemcpyHostToDevice, h->stream));
+    CK(h2d(h, h->d_cand_prof.p, h->h_cand.data(), (size_t)nc * 4));
+    CK(h2d(h, h->d_cand_off.p, h->h_cand_off.data(), (size_t)nc * 8));
     // traceback sweep order: longest candidates first
     {
         std::vector<int> wo(nc);
@@ -1345,9 +1472,8 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
         strip_items(lens, (h->Lq + 31) / 32, h->nsm * P1TC_WARPS, STRIP_LAG_TB, items);
         if (h->d_worder.ensure(nc, h->budget) || h->d_tbitems.ensure(items.size(), h->budget))
             return fail(h, C2_ERR_NOMEM, "candidate order allocation failed");
-        CK(cudaMemcpyAsync(h->d_worder.p, wo.data(), (size_t)nc * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemcpyAsync(h->d_tbitems.p, items.data(), items.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        CK(h2d(h, h->d_worder.p, wo.data(), (size_t)nc * 4));
+        CK(h2d(h, h->d_tbitems.p, items.data(), items.size() * 4));
     }
     P1Args a;
     fill_p1(h, a);
@@ -1482,18 +1608,20 @@ extern "C" c2_status c2_run_stats(c2_handle* h, int32_t* npassed)
 {
     if (!h || !npassed) return C2_ERR_ARG;
     CK(cudaSetDevice(h->device));
-    CK(cudaStreamSynchronize(h->stream));
     int stw = 0;
-    CK(cudaMemcpy(&stw, h->d_status.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (stw != 0) return fail(h, C2_ERR_DEVICE, "device status %d (%s)", stw, status_text(stw));
     const int nc = h->ncand;
     h->h_p2.clear();
+    h->npass = 0;
     h->h_fscore.assign(nc, 0.f);
     h->h_fpassed.assign(nc, 0);
+    Fetch F(h);
+    CK(F.get(&stw, h->d_status.p, sizeof(int)));
     if (nc > 0) {
-        CK(cudaMemcpy(h->h_fpassed.data(), h->d_fpassed.p, (size_t)nc * 4, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(h->h_fscore.data(), h->d_fscore.p, (size_t)nc * 4, cudaMemcpyDeviceToHost));
+        CK(F.get(h->h_fpassed.data(), h->d_fpassed.p, (size_t)nc * 4));
+        CK(F.get(h->h_fscore.data(), h->d_fscore.p, (size_t)nc * 4));
     }
+    CK(F.finish());
+    if (stw != 0) return fail(h, C2_ERR_DEVICE, "device status %d (%s)", stw, status_text(stw));
     for (int c = 0; c < nc; c++)
         if (h->h_fpassed[c]) h->h_p2.push_back(c);
     h->npass = (int)h->h_p2.size();
@@ -1502,7 +1630,7 @@ extern "C" c2_status c2_run_stats(c2_handle* h, int32_t* npassed)
     if (h->d_p2.ensure(h->npass, h->budget) || h->d_stats.ensure((size_t)h->npass * STATS_NOUT, h->budget) ||
         h->d_hist.ensure((size_t)h->npass * STATS_NBINS, h->budget))
         return fail(h, C2_ERR_NOMEM, "statistics buffers for %d pairs failed", h->npass);
-    CK(cudaMemcpyAsync(h->d_p2.p, h->h_p2.data(), (size_t)h->npass * 4, cudaMemcpyHostToDevice, h->stream));
+    CK(h2d(h, h->d_p2.p, h->h_p2.data(), (size_t)h->npass * 4));
     StatsArgs a;
     memset(&a, 0, sizeof a);
     a.Lq = h->Lq;
@@ -1597,10 +1725,13 @@ extern "C" c2_status c2_run_map(c2_handle* h, int32_t* nhits)
 {
     if (!h || !nhits) return C2_ERR_ARG;
     CK(cudaSetDevice(h->device));
-    CK(cudaStreamSynchronize(h->stream));
+    h->info_valid = false;
     h->h_stats.assign((size_t)h->npass * STATS_NOUT, 0.f);
-    if (h->npass > 0)
-        CK(cudaMemcpy(h->h_stats.data(), h->d_stats.p, h->h_stats.size() * 4, cudaMemcpyDeviceToHost));
+    {
+        Fetch F(h);
+        CK(F.get(h->h_stats.data(), h->d_stats.p, h->h_stats.size() * 4));
+        CK(F.finish());
+    }
     h->h_mapcand.clear();
     h->h_mappass.clear();
     for (int i = 0; i < h->npass; i++)
@@ -1644,11 +1775,10 @@ extern "C" c2_status c2_run_map(c2_handle* h, int32_t* nhits)
         for (int i = 0; i < nm; i++) lens[i] = h->h_plen[h->h_cand[h->h_mapcand[i]]];
         strip_items(lens, (h->Lq + 31) / 32, h->grid * P1_WARPS, STRIP_LAG_MAP, items);
         if (h->d_mapitems.ensure(items.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "MAP work table allocation failed");
-        CK(cudaMemcpyAsync(h->d_mapitems.p, items.data(), items.size() * 4, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        CK(h2d(h, h->d_mapitems.p, items.data(), items.size() * 4));
     }
-    CK(cudaMemcpyAsync(h->d_mapcand.p, h->h_mapcand.data(), (size_t)nm * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_mappass.p, h->h_mappass.data(), (size_t)nm * 4, cudaMemcpyHostToDevice, h->stream));
+    CK(h2d(h, h->d_mapcand.p, h->h_mapcand.data(), (size_t)nm * 4));
+    CK(h2d(h, h->d_mappass.p, h->h_mappass.data(), (size_t)nm * 4));
     MapArgs a;
     memset(&a, 0, sizeof a);
     a.Lq = h->Lq;
@@ -1692,14 +1822,19 @@ extern "C" c2_status c2_run_map(c2_handle* h, int32_t* nhits)
 
 static c2_status hits_direct(c2_handle* h, c2_hit* hits, int32_t n, char* alns, size_t* aln_bytes)
 {
-    CK(cudaStreamSynchronize(h->stream));
-    int stw = 0;
-    CK(cudaMemcpy(&stw, h->d_status.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (stw != 0) return fail(h, C2_ERR_DEVICE, "device status %d (%s)", stw, status_text(stw));
     const int nm = h->nmap;
-    const size_t per = (size_t)5 * h->alnstride;
-    std::vector<int> info((size_t)nm * 8);
-    if (nm > 0) CK(cudaMemcpy(info.data(), h->d_alninfo.p, info.size() * 4, cudaMemcpyDeviceToHost));
+    std::vector<int>& info = h->h_info;
+    if (!h->info_valid) {
+        // (once for the call that asks for the sizes and the one that copies)
+        int stw = 0;
+        info.resize((size_t)nm * 8);
+        Fetch F(h);
+        CK(F.get(&stw, h->d_status.p, sizeof(int)));
+        CK(F.get(info.data(), h->d_alninfo.p, info.size() * 4));
+        CK(F.finish());
+        if (stw != 0) return fail(h, C2_ERR_DEVICE, "device status %d (%s)", stw, status_text(stw));
+        h->info_valid = true;
+    }
     size_t need = 0;
     for (int m = 0; m < nm; m++) need += (size_t)5 * (info[(size_t)m * 8] + 1);
     if (!alns || !hits) {
@@ -1707,7 +1842,6 @@ static c2_status hits_direct(c2_handle* h, c2_hit* hits, int32_t n, char* alns, 
         return (hits || alns) ? C2_ERR_ARG : C2_OK;
     }
     if (n < nm || *aln_bytes < need) return fail(h, C2_ERR_ARG, "output buffers too small (%d hits, %zu bytes)", nm, need);
-    (void)per;
     std::vector<int> order(nm);
     std::iota(order.begin(), order.end(), 0);
     auto logE = [&](int m) { return h->h_stats[(size_t)h->h_mappass[m] * STATS_NOUT + ST_LOGE]; };
@@ -1729,11 +1863,12 @@ static c2_status hits_direct(c2_handle* h, c2_hit* hits, int32_t n, char* alns, 
     if (nm > 0) {
         if (h->d_alnoff.ensure((size_t)nm, h->budget) || h->d_alnpack.ensure(need, h->budget))
             return fail(h, C2_ERR_NOMEM, "alignment packing buffers failed");
-        CK(cudaMemcpyAsync(h->d_alnoff.p, off.data(), (size_t)nm * 8, cudaMemcpyHostToDevice, h->stream));
+        CK(h2d(h, h->d_alnoff.p, off.data(), (size_t)nm * 8));
         CK(launch_aln_pack(h->d_aln.p, h->alnstride, h->d_alninfo.p, h->d_alnoff.p, nm, h->d_alnpack.p, h->stream));
         h->launches++;
-        CK(cudaMemcpyAsync(alns, h->d_alnpack.p, need, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        Fetch F(h);
+        CK(F.get(alns, h->d_alnpack.p, need));
+        CK(F.finish());
     }
     size_t pos = 0;
     for (int i = 0; i < nm; i++) {
@@ -2055,13 +2190,17 @@ static void fill_adj(c2_handle* h, AdjArgs& a)
     a.grad = h->d_adjgrad.p;
 }
 
-// device status after a sweep (a strip wait that timed out)
-static c2_status adj_status(c2_handle* h)
+// results of a sweep to the host, and the device status (a strip wait that timed out)
+static c2_status adj_results(c2_handle* h, float* dst, const float* src, size_t n)
 {
     int stw = 0;
-    CK(cudaMemcpyAsync(&stw, h->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    Fetch F(h);
+    CK(F.get(&stw, h->d_status.p, sizeof(int)));
+    std::vector<float> r(n);
+    CK(F.get(r.data(), src, n * sizeof(float)));
+    CK(F.finish());
     if (stw != 0) return fail(h, C2_ERR_DEVICE, "device status %d: %s", stw, status_text(stw));
+    std::copy(r.begin(), r.end(), dst);
     return C2_OK;
 }
 
@@ -2141,8 +2280,12 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
     // columns x 5 floats), its grid halved while that scratch does not fit.
     h->adj_keepF = false;
     {
+        // (asking for the free memory takes longer than a small batch's sweeps: not
+        // for a buffer that is already there)
         size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && (size_t)acc * 5 * sizeof(float) <= fr / 4 &&
+        if (h->d_adjF.p && h->d_adjF.n >= (size_t)acc * 5)
+            h->adj_keepF = true;
+        else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && (size_t)acc * 5 * sizeof(float) <= fr / 4 &&
             h->d_adjF.ensure((size_t)acc * 5, h->budget) == cudaSuccess)
             h->adj_keepF = true;
         (void)cudaGetLastError();   // a refused allocation is not an error of what follows
@@ -2157,14 +2300,14 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
         if (h->adj_bgrid == 0)
             return fail(h, C2_ERR_NOMEM, "logz_fwd: backward sweep scratch (%zu bytes per CTA) failed", per_cta);
     }
-    CK(cudaMemcpyAsync(h->d_adjprof.p, profiles, (size_t)npairs * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjLq.p, Lq, (size_t)npairs * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjqpos.p, qpos, (size_t)npairs * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjqidx.p, qidx, (size_t)npairs * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjsoff.p, soff.data(), (size_t)npairs * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjitems.p, it.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjoff.p, h->adj_off.data(), (size_t)npairs * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjroff.p, h->adj_roff.data(), (size_t)npairs * 8, cudaMemcpyHostToDevice, h->stream));
+    CK(h2d(h, h->d_adjprof.p, profiles, (size_t)npairs * 4));
+    CK(h2d(h, h->d_adjLq.p, Lq, (size_t)npairs * 4));
+    CK(h2d(h, h->d_adjqpos.p, qpos, (size_t)npairs * 8));
+    CK(h2d(h, h->d_adjqidx.p, qidx, (size_t)npairs * 4));
+    CK(h2d(h, h->d_adjsoff.p, soff.data(), (size_t)npairs * 8));
+    CK(h2d(h, h->d_adjitems.p, it.data(), it.size() * sizeof(int2)));
+    CK(h2d(h, h->d_adjoff.p, h->adj_off.data(), (size_t)npairs * 8));
+    CK(h2d(h, h->d_adjroff.p, h->adj_roff.data(), (size_t)npairs * 8));
     CK(cudaMemsetAsync(h->d_adjbuf.p + 5 * acc, 0xff, (size_t)racc * sizeof(float), h->stream));   // forward rows: empty
     CK(cudaMemsetAsync(h->d_adjctr.p, 0, 2 * sizeof(int), h->stream));
     CK(cudaMemsetAsync(h->d_status.p, 0, sizeof(int), h->stream));
@@ -2173,10 +2316,8 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
     const int grid = (int)std::min<long long>((long long)h->nsm * std::max(fwd_occ, 1), (items + ADJ_WARPS - 1) / ADJ_WARPS);
     CK(launch_adj_fwd(a, grid, h->stream));
     h->launches += 3;
-    c2_status st = adj_status(h);
+    const c2_status st = adj_results(h, logz, h->d_adjlogz.p, npairs);
     if (st != C2_OK) return st;
-    CK(cudaMemcpyAsync(logz, h->d_adjlogz.p, (size_t)npairs * 4, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
     h->adj_fwd_done = true;
     return C2_OK;
 }
@@ -2188,6 +2329,22 @@ extern "C" c2_status c2_logz_fwd(c2_handle* h, const int32_t* profiles, int32_t 
     if (h->nprof <= 0 || h->Lq <= 0) return fail(h, C2_ERR_STATE, "logz_fwd needs a database and a query");
     CK(cudaSetDevice(h->device));
     h->adj_batch = false;
+    if (!h->qcfx_ready) {
+        // column -1 states of the current query with exact exp/log
+        const int32_t len = h->Lq;
+        const int64_t zero = 0;
+        c2_profiles v;
+        memset(&v, 0, sizeof v);
+        v.nprofiles = 1;
+        v.lengths = &len;
+        v.offsets = &zero;
+        v.trn = h->h_qtrn.data();
+        std::vector<float> qx((size_t)len * 6, 0.f);
+        colm1_exact(&v, qx.data());
+        if (h->d_qcfx.ensure(qx.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "query side arrays allocation failed");
+        CK(h2d(h, h->d_qcfx.p, qx.data(), qx.size() * 4));
+        h->qcfx_ready = true;
+    }
     const std::vector<int> Lq(npairs, h->Lq), qidx(npairs, 0);
     const std::vector<long long> qpos(npairs, 0);
     return logz_fwd_pairs(h, profiles, Lq.data(), qpos.data(), qidx.data(), npairs, theta, wss, wcv, logz);
@@ -2204,32 +2361,49 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
     // column -1 states), raw transitions and backgrounds, concatenated; the
     // queries packed by up to 16 host threads
     const long long N = queries->npositions;
-    std::vector<float> qrec((size_t)N * QR_STRIDE, 0.f), qcf((size_t)N * 6, 0.f);
-    {
-        std::atomic<int> next(0);
-        auto work = [&]() {
-            const int64_t zero = 0;
-            for (int q; (q = next.fetch_add(1)) < nq;) {
-                const c2_profiles v = query_view(queries, q, &zero);
-                const size_t o = (size_t)queries->offsets[q];
-                qrec_score_fields(h, &v, qrec.data() + o * QR_STRIDE);
-                colm1_exact(&v, qcf.data() + o * 6);
-            }
-        };
-        const int nt = std::max(1, std::min(16, nq / 8));
-        std::vector<std::thread> th;
-        for (int t = 1; t < nt; t++) th.emplace_back(work);
-        work();
-        for (auto& t : th) t.join();
-    }
-    if (h->d_adjqrec.ensure(qrec.size(), h->budget) || h->d_adjqcfx.ensure(qcf.size(), h->budget) ||
+    if (h->d_adjqrec.ensure((size_t)N * QR_STRIDE, h->budget) || h->d_adjqcfx.ensure((size_t)N * 6, h->budget) ||
         h->d_adjqtrn.ensure((size_t)(N + nq) * 7, h->budget) || h->d_adjqbkg.ensure((size_t)nq * NAA, h->budget))
         return fail(h, C2_ERR_NOMEM, "set_query_batch: query arrays for %d queries failed", nq);
-    CK(cudaMemcpyAsync(h->d_adjqrec.p, qrec.data(), qrec.size() * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjqcfx.p, qcf.data(), qcf.size() * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjqtrn.p, queries->trn, (size_t)(N + nq) * 7 * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_adjqbkg.p, queries->bkg, (size_t)nq * NAA * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));   // the host arrays above are freed on return
+    CK(h2d(h, h->d_adjqtrn.p, queries->trn, (size_t)(N + nq) * 7 * 4));
+    CK(h2d(h, h->d_adjqbkg.p, queries->bkg, (size_t)nq * NAA * 4));
+    // pieces of whole queries (a query is at most 65,535 rows), packed by the host
+    // threads straight into the staging memory, each copied while the next is packed
+    constexpr long long ROW_FLOATS = QR_STRIDE + 6;
+    const long long rows_max = std::max<long long>(65535, (long long)(STAGE_MAX / 2 / (ROW_FLOATS * sizeof(float))));
+    for (int q0 = 0; q0 < nq;) {
+        int q1 = q0;
+        long long rows = 0;
+        while (q1 < nq && (q1 == q0 || rows + queries->lengths[q1] <= rows_max / 2)) rows += queries->lengths[q1++];
+        float* buf = reinterpret_cast<float*>(stage_take(h, (size_t)rows * ROW_FLOATS * sizeof(float)));
+        if (!buf) return fail(h, C2_ERR_NOMEM, "set_query_batch: staging memory for %lld rows failed", rows);
+        float *rec = buf, *qcf = buf + rows * QR_STRIDE;
+        const long long r0 = queries->offsets[q0];
+        std::atomic<int> next(q0);
+        auto work = [&]() {
+            const int64_t zero = 0;
+            for (int q; (q = next.fetch_add(1)) < q1;) {
+                const c2_profiles v = query_view(queries, q, &zero);
+                const size_t o = (size_t)(queries->offsets[q] - r0);
+                qrec_score_fields(h, &v, rec + o * QR_STRIDE);
+                colm1_exact(&v, qcf + o * 6);
+            }
+        };
+        const int nt = std::max(1, std::min(16, (q1 - q0) / 8));
+        std::vector<std::thread> th;
+        for (int t = 1; t < nt; t++) {
+            try {
+                th.emplace_back(work);
+            } catch (...) {
+                break;   // no more threads to be had
+            }
+        }
+        work();
+        for (auto& t : th) t.join();
+        CK(cudaMemcpyAsync(h->d_adjqrec.p + (size_t)r0 * QR_STRIDE, rec, (size_t)rows * QR_STRIDE * 4,
+                           cudaMemcpyHostToDevice, h->stream));
+        CK(cudaMemcpyAsync(h->d_adjqcfx.p + (size_t)r0 * 6, qcf, (size_t)rows * 6 * 4, cudaMemcpyHostToDevice, h->stream));
+        q0 = q1;
+    }
     h->adj_qlen.assign(queries->lengths, queries->lengths + nq);
     h->adj_qstart.assign(queries->offsets, queries->offsets + nq);
     h->adj_fwd_done = false;
@@ -2269,11 +2443,7 @@ extern "C" c2_status c2_logz_bwd(c2_handle* h, float* grad)
     CK(cudaMemsetAsync(h->d_adjctr.p + 1, 0, sizeof(int), h->stream));
     CK(launch_adj_bwd(a, h->adj_bgrid, h->stream));
     h->launches += 2;
-    c2_status st = adj_status(h);
-    if (st != C2_OK) return st;
-    CK(cudaMemcpyAsync(grad, h->d_adjgrad.p, (size_t)a.npairs * 9 * 4, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    return C2_OK;
+    return adj_results(h, grad, h->d_adjgrad.p, (size_t)a.npairs * 9);
 }
 
 extern "C" c2_status c2_logz_cells(c2_handle* h, int32_t pair, float* dlogz_ds, float* post)
