@@ -185,7 +185,7 @@ struct P1Args {
     const int* worder;          // traceback sweep: rank -> candidate (longest first)
     int p2s_cols, p2s_blocks;   // phase-2 score matrices: columns per work item, items per (candidate, strip)
     const int* items;           // traceback sweep: work item -> rank * nstrips + strip
-    unsigned spin;              // polls before a strip wait gives up (pipe_wait)
+    unsigned spin;              // polls before a strip wait gives up
     // tensor-core operands (P1K_TENSOR)
     const unsigned* tcdb;       // db B fragments
     const long long* ttile;     // [nprof] first tile of each profile

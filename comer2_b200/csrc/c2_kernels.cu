@@ -5,19 +5,21 @@
 // CalcSM_SSSS_CVS2S_SMEMUnroll2x_2 (src/libmycu/cusco/) and the per-diagonal
 // ExecDP_Btck_Unroll32x launches (src/libmycu/cudp/CuBatchDP.cu:149-320,
 // CuBatchDP_init_btck.cu:65-494).  Instead of materialising the L_q x N score
-// matrix and a traceback byte per cell in HBM, one persistent warp owns one
-// (query, db profile) pair at a time:
-//  * lanes own query rows (a strip of 32 rows at a time); the query-row
-//    operands of the score live in registers for the whole strip;
-//  * each step, the warp reads one db column record with warp-uniform
-//    (broadcast) loads and every lane scores its row against it; the score
-//    goes to a per-lane ring in shared memory;
-//  * the DP runs as an anti-diagonal wavefront: lane t processes column k-t at
-//    step k, taking its "up" states from lane t-1 by __shfl_up_sync, its
-//    "diagonal" states from the previous step's "up", and the column's
-//    transitions passed down the lanes the same way;
-//  * the strip's last row is handed to the next strip through a per-warp
-//    boundary buffer (global memory, L2 resident).
+// matrix and a traceback byte per cell in HBM, one persistent warp sweeps
+// a strip of 64 query rows of one (query, db profile) pair at a time, two rows to
+// a lane, in chunks of 8 db columns:
+//  * the chunk's scores go to a ring in shared memory: from FP32 dot products
+//    against db records staged by cp.async (p1c_kernel), or from split-BF16
+//    tensor-core products of packed db tiles fetched by cp.async.bulk with
+//    query operands held in tensor memory (p1t_kernel);
+//  * the DP then runs 8 steps of an anti-diagonal wavefront: lane t processes
+//    column k - t of rows 2 t, 2 t + 1 at step k, the "up" states of its first row
+//    coming from lane t - 1 by __shfl_up_sync, the "diagonal" states being the
+//    step before's "up", the columns' transitions from a shared-memory ring;
+//  * the strip's last row is handed to the next strip through a boundary
+//    buffer (global memory, L2 resident), the warp's own or, for the longest
+//    pairs of a search, whose strips several warps take, the pair's.
+// p1_kernel (one row a lane, a column a step) serves the allocation-free entry.
 // For the pairs that pass the phase-1 threshold, p2s_kernel stores the FP32
 // scores column-major for the finalisation, statistics and MAP stages, and the
 // traceback sweep (p1tc_kernel) runs the same DP on them again, storing btck
@@ -1943,7 +1945,10 @@ cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, c
         const int wt = (int)std::max<long long>(1, std::min<long long>(P1TC_WARPS, (nit2 + nsm - 1) / nsm));
         const int gt = (int)std::min<long long>(nsm, (nit2 + wt - 1) / wt);
         const size_t smt = (size_t)wt * P1TC_WARP_FLOATS * sizeof(float);
-        if ((e = cudaFuncSetAttribute(p1tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt)) != cudaSuccess)
+        // (the attribute is the kernel's, shared by all threads: always the largest size,
+        // or a thread's launch could find a smaller one set by another in between)
+        constexpr int smtmax = P1TC_WARPS * P1TC_WARP_FLOATS * (int)sizeof(float);
+        if ((e = cudaFuncSetAttribute(p1tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smtmax)) != cudaSuccess)
             return e;
         p1tc_kernel<<<gt, wt * 32, smt, st>>>(a, qbkg);
     } else {

@@ -4,11 +4,11 @@
 //
 // Replaces the reference's ExecMAPDP_Parent_DynPlm and its 3 x nblkdiags
 // device launches plus FinalizeMAPDP_MAP (src/libmycu/cumapdp/).  Here each
-// sweep is one persistent kernel with one warp per pair: lanes own query
+// sweep is one persistent kernel, one warp per strip of 32 query rows of a pair
+// (the strips of a pair hand their last rows on, c2_device.cuh): lanes own query
 // rows, the anti-diagonal wavefront advances one column per step with
-// __shfl_up_sync hand-offs as in the phase-1 kernel, and per-column score
-// and result traffic goes through shared-memory rings so that every global
-// read and write is a coalesced column segment.
+// __shfl_up_sync hand-offs, in groups of 8 steps whose scores, F and B are loaded a
+// group ahead as coalesced lines.
 //
 // Arithmetic follows the reference: Schraudolph's (1999) exponential and its
 // inverse with the reference's adjustment constant
@@ -927,7 +927,10 @@ cudaError_t launch_map(const MapArgs& a, const float* qtrn, const float* dtrn, c
     const int wfb = (int)std::max<long long>(1, std::min<long long>(MAPFBW, (2 * nitems + nsm - 1) / nsm));
     const int wdp = (int)std::max<long long>(1, std::min<long long>(MAPW, (nitems + nsm - 1) / nsm));
     const size_t fbs = (size_t)wfb * MAPFB_WARP_FLOATS * sizeof(float);
-    if ((e = cudaFuncSetAttribute(map_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fbs)) != cudaSuccess)
+    // (the attribute is the kernel's, shared by all threads: always the largest size,
+    // or a thread's launch could find a smaller one set by another in between)
+    constexpr int fbmax = MAPFBW * MAPFB_WARP_FLOATS * (int)sizeof(float);
+    if ((e = cudaFuncSetAttribute(map_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fbmax)) != cudaSuccess)
         return e;
     int ofb = 0, odp = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ofb, map_fb_kernel, wfb * 32, fbs)) != cudaSuccess)

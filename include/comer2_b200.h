@@ -327,11 +327,12 @@ c2_status c2_db_device_bytes(const c2_handle* h, int64_t npositions, int32_t npr
 c2_status c2_get_search_groups(const c2_handle* h, int32_t* ngroups);
 
 /* Bound of the waits between the strips of one pair in the phase-2 sweeps
- * (traceback DP, MAP forward/backward, MAP DP): a strip polls its
- * predecessor's progress at most `polls` times (0 restores the default,
- * 2^22 polls with 128 ns sleeps, about a second), then gives up, the sweep
- * finishes without faulting and c2_get_finalize / c2_run_stats /
- * c2_get_hits return C2_ERR_DEVICE ("a strip wait ... timed out").  The
+ * (traceback DP, MAP forward/backward, MAP DP), the adjoint's sweeps and, for the
+ * longest pairs of a search, phase 1: a strip polls its predecessor's row or
+ * progress at most `polls` times (0 restores the default, 2^22 polls with
+ * 128 ns sleeps, about a second), then gives up, the sweep finishes without
+ * faulting and c2_get_phase1 / c2_get_finalize / c2_run_stats / c2_get_hits /
+ * c2_logz_fwd / c2_logz_bwd return C2_ERR_DEVICE ("a strip wait ... timed out").  The
  * next c2_set_query clears the error.  No counterpart in the reference,
  * whose kernels neither wait on one another nor time out. */
 c2_status c2_set_wait_limit(c2_handle* h, uint32_t polls);
@@ -393,9 +394,9 @@ c2_status c2_db2bin_descriptions(const char* path, char* buf, size_t* bytes, int
  * with theta[7] (MM MI MD IM II DM DD, may be NULL = 0) added to the query's
  * transition log-probabilities in every cell update.  logz[k] receives
  * log sum over cells exp(F.MM) of pair k.  Keeps what c2_logz_bwd needs
- * (the scores and each 32-row strip's last forward row: the backward sweep
- * recomputes a strip's forward states from the row above it); a new query or
- * c2_logz_fwd call replaces them. */
+ * (the scores, each 32-row strip's last forward row and, when they fit, every
+ * forward state: without them the backward sweep recomputes a strip's states
+ * from the row above it); a new query or c2_logz_fwd call replaces them. */
 c2_status c2_logz_fwd(c2_handle* h, const int32_t* profiles, int32_t npairs, const float* theta, float wss,
                       float wcv, float* logz);
 
