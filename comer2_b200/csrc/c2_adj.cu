@@ -33,9 +33,12 @@
 // when they did not fit -- recomputes them from the checkpoint row above into
 // a per-warp scratch (32 rows x (L + 31) x 5 states); it then runs the
 // outside recursion over the same rows (bottom row first) and forms every
-// edge posterior of the strip as it goes.  B is never stored for the matrix,
-// and with checkpointing neither is F: memory per cell is then the 3 score
-// arrays and the 2 outputs.
+// edge posterior of the strip as it goes.  When the states were kept and there is
+// as much room again, the backward sweep only stores its outside values B, and
+// a kernel over all cells forms the posteriors: the chain of steps, which bounds
+// the sweep, is then as short as the forward one's.  With checkpointing neither F
+// nor B is stored for the matrix: memory per cell is then the 3 score arrays and
+// the 2 outputs.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -302,10 +305,11 @@ __device__ __forceinline__ void adj_stage_trn(float* trs, const float* __restric
     }
 }
 
-// row q of the ring
+// row q of a ring of N rows
+template <int N = 128>
 __device__ __forceinline__ void ring_row(const float* trs, int q, float* t)
 {
-    const float* o = trs + (q & 127) * TRS;
+    const float* o = trs + (q & (N - 1)) * TRS;
     const float4 a = *reinterpret_cast<const float4*>(o);
     const float4 b = *reinterpret_cast<const float4*>(o + 4);
     t[0] = a.x; t[1] = a.y; t[2] = a.z; t[3] = a.w; t[4] = b.x; t[5] = b.y; t[6] = b.z;
@@ -476,12 +480,59 @@ __global__ void adj_logz_kernel(AdjArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// backward sweep with the gradients.  Strip s of pair m: lane t holds row
-// i = 32 s + 31 - t (the strip's rows bottom first), mirrored column
-// jm = k - t at step k, actual column ca = L - 1 - jm.  The outside values B
-// follow the transposed recursion; at every cell the posteriors of its
-// incoming edges exp(F(pred) + edge + B(cell) - logZ) come from the
-// recomputed forward states of the strip (and the checkpoint row above it).
+// backward sweep and posteriors
+__device__ __forceinline__ X5 shfl_up5(const X5& x)
+{
+    return X5{__shfl_up_sync(FULL, x.MM, 1), __shfl_up_sync(FULL, x.MI, 1), __shfl_up_sync(FULL, x.IM, 1),
+              __shfl_up_sync(FULL, x.DN, 1), __shfl_up_sync(FULL, x.ND, 1)};
+}
+__device__ __forceinline__ float warp_sum(float v)
+{
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+    return v;
+}
+
+// A strip's lines in up to POST_WARPS equal runs of at least 8 lines; gradient
+// sums are taken over each run from its last line, and over the runs from the
+// last one (in every form, so that they agree bit for bit)
+constexpr int POST_WARPS = 8;
+__device__ __forceinline__ int post_run(int lines) { return max(8, (lines + POST_WARPS - 1) / POST_WARPS); }
+
+// Posteriors of a cell (array index kk) and of its incoming edges, from its
+// outside values b and its forward predecessors; added to the gradient sums g.
+__device__ __forceinline__ void edge_posteriors(const AdjArgs& a, long long kk, const X5& b, float ownMM, const X5& up,
+                                                const X5& left, const X5& diag, const float* qf, const float* tf,
+                                                float sc, float lz, float pss, float pcv, float* g)
+{
+    // MM: five emission edges
+    const float eMM = b.MM - lz;
+    const float m1 = xexp(((diag.MI + qf[TMM]) + tf[TIM]) + sc + eMM);
+    const float m2 = xexp(((diag.IM + qf[TIM]) + tf[TMM]) + sc + eMM);
+    const float m3 = xexp(((diag.DN + qf[TDM]) + tf[TMM]) + sc + eMM);
+    const float m4 = xexp(((diag.ND + qf[TMM]) + tf[TDM]) + sc + eMM);
+    const float m5 = xexp(((diag.MM + qf[TMM]) + tf[TMM]) + sc + eMM);
+    const float gs = (m1 + m2 + m3 + m4) + m5;
+    // MI, IM, DN (ND uses no query transition)
+    const float i1 = xexp((up.MM + qf[TMM]) + tf[TMI] + b.MI - lz);
+    const float i2 = xexp((up.MI + qf[TMM]) + tf[TII] + b.MI - lz);
+    const float l1 = xexp((left.MM + qf[TMI]) + tf[TMM] + b.IM - lz);
+    const float l2 = xexp((left.IM + qf[TII]) + tf[TMM] + b.IM - lz);
+    const float d1 = xexp(up.MM + qf[TMD] + b.DN - lz);
+    const float d2 = xexp(up.DN + qf[TDD] + b.DN - lz);
+    g[TMM] += m1 + m4 + m5 + i1 + i2;
+    g[TIM] += m2;
+    g[TDM] += m3;
+    g[TMI] += l1;
+    g[TII] += l2;
+    g[TMD] += d1;
+    g[TDD] += d2;
+    g[7] += gs * pss;
+    g[8] += gs * pcv;
+    a.gS[kk] = gs;
+    a.post[kk] = xexp(ownMM + b.MM - lz);
+}
+
 // column c of a complete row
 __device__ __forceinline__ X5 row_ld5(const float* __restrict__ row, int ldr, int c)
 {
@@ -489,8 +540,15 @@ __device__ __forceinline__ X5 row_ld5(const float* __restrict__ row, int ldr, in
     return X5{x.x, x.y, x.z, x.w, row[4 * ldr + c]};
 }
 
+// Backward sweep of a strip: lane t holds row i = 32 s + 31 - t (the strip's rows
+// bottom first), mirrored column jm = k - t at step k, actual column
+// ca = L - 1 - jm.  The outside values B follow the transposed recursion.  OUT:
+// they are stored in Bw, in the forward states' layout.  Otherwise the posteriors
+// of a cell's incoming edges exp(F(pred) + edge + B(cell) - logZ) are formed here,
+// from the strip's forward states Fw and the checkpoint row above it.
+template <bool OUT>
 __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, int lane, float* rab, float* trs,
-                                              const float* __restrict__ Fw, bool& broken)
+                                              const float* __restrict__ Fw, float* __restrict__ Bw, bool& broken)
 {
     const int p = a.prof[m];
     const int L = a.plen[p], Lq = a.pLq[m], ns = (Lq + 31) >> 5;
@@ -521,6 +579,8 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     float g[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) g[k] = 0.f;
+    int flush = (L + 30) / post_run(L + 31) * post_run(L + 31);   // first line of the current run
+    float tot = 0.f;                                             // lane f < 9: the complete runs' sum of g[f]
     X5 mine = INIT, upp = INIT;
     __syncwarp();
     adj_stage_trn<true>(trs, dt0, 0, L, lane);
@@ -537,9 +597,14 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     const float* Sr = a.S + cb + lf;
     const float* Sb = a.S + cb + (long long)(L + 31) * 32;   // row 32 s + 32 (has_below), lane 0
     const int kf0 = L + 30;
-    X5 Ac = fw_ld5(Fw, kf0, lf), Al = fw_ld5(Fw, kf0 - 1, lf), An = fw_ld5(Fw, kf0 - 2, lf), Up = INIT;
+    X5 Ac = INIT, Al = INIT, An = INIT, Up = INIT;
+    if (!OUT) {
+        Ac = fw_ld5(Fw, kf0, lf);
+        Al = fw_ld5(Fw, kf0 - 1, lf);
+        An = fw_ld5(Fw, kf0 - 2, lf);
+    }
     X5 Ab = INIT;                              // lane 31: row 32 s - 1 at the diagonal column
-    auto load_above = [&](int c) { return (s > 0 && t == 31 && c >= 0 && c < L) ? row_ld5(fab, ldr, c) : INIT; };
+    auto load_above = [&](int c) { return (!OUT && s > 0 && t == 31 && c >= 0 && c < L) ? row_ld5(fab, ldr, c) : INIT; };
     Ab = load_above(L - 1 + t - 1);            // step 0: ca - 1
     float sc0 = Sr[(long long)kf0 * 32], sc1 = 0.f, sc2 = 0.f, sb = XLOG0;   // scores at steps k, k - 1, k - 2; row below
     for (int k = 0; k < L + 31; k++) {
@@ -550,10 +615,10 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
             // lines of the steps to come: forward states (5), scores, SS and CV parts, row below
             const int kq = kf - ADJ_PF;
             if (kq >= 0) {
-                if (lane < 5 && kq >= 3) pf_l1(Fw + (long long)(kq - 3) * 160 + lane * 32);
+                if (!OUT && lane < 5 && kq >= 3) pf_l1(Fw + (long long)(kq - 3) * 160 + lane * 32);
                 else if (lane == 5) pf_l1(a.S + cb + (long long)kq * 32);
-                else if (lane == 6) pf_l1(a.pss + cb + (long long)kq * 32);
-                else if (lane == 7) pf_l1(a.pcv + cb + (long long)kq * 32);
+                else if (!OUT && lane == 6) pf_l1(a.pss + cb + (long long)kq * 32);
+                else if (!OUT && lane == 7) pf_l1(a.pcv + cb + (long long)kq * 32);
                 else if (lane == 8 && has_below && L - k - ADJ_PF >= 0 && L - k - ADJ_PF < L)
                     pf_l1(Sb + (long long)(L - k - ADJ_PF) * 32);
             }
@@ -561,7 +626,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         // loaded now for the next step: line kf - 3, the score, rows above and below
         X5 Aq = INIT;
         float scn = 0.f;
-        if (kf >= 3) Aq = fw_ld5(Fw, kf - 3, lf);
+        if (!OUT && kf >= 3) Aq = fw_ld5(Fw, kf - 3, lf);
         if (kf >= 1) scn = Sr[(long long)(kf - 1) * 32];
         const X5 Abn = load_above(ca - 2);
         const float sbn = (t == 0 && has_below && ca >= 0 && ca < L) ? Sb[(long long)ca * 32] : XLOG0;   // column (ca - 1) + 1
@@ -577,7 +642,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         // for the edge posteriors, into it (rows ca and ca + 1)
         float tb[7], tf[7];
         ring_row(trs, jm, tb);          // row ca + 1
-        ring_row(trs, jm + 1, tf);      // row ca
+        if (!OUT) ring_row(trs, jm + 1, tf);   // row ca
         tf[TMI] = tb[TMI];
         tf[TII] = tb[TII];
         X5 dn;
@@ -615,7 +680,11 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         // rows past the query (the last strip's first lanes) are the matrix
         // edge for the rows above them
         if (!act) nw = INIT;
-        if (valid) {
+        if (OUT && valid) {
+            fw_st5(Bw, kf, lf, nw);
+            if (wr_row) row_put(mine_row, ldr, jm, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
+        }
+        if (!OUT && valid) {
             // edge posteriors of cell (i, ca): its forward predecessors
             const X5 own = Ac, up = Up;
             X5 left = Al, diag = dgl;
@@ -624,35 +693,18 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
                 diag = DB;
             }
             const long long kk = cb + (long long)kf * 32 + lf;
-            const float sc = sc0;
-            const X5& b = nw;
-            // MM: five emission edges
-            const float eMM = b.MM - lz;
-            const float m1 = xexp(((diag.MI + qf[TMM]) + tf[TIM]) + sc + eMM);
-            const float m2 = xexp(((diag.IM + qf[TIM]) + tf[TMM]) + sc + eMM);
-            const float m3 = xexp(((diag.DN + qf[TDM]) + tf[TMM]) + sc + eMM);
-            const float m4 = xexp(((diag.ND + qf[TMM]) + tf[TDM]) + sc + eMM);
-            const float m5 = xexp(((diag.MM + qf[TMM]) + tf[TMM]) + sc + eMM);
-            const float gs = (m1 + m2 + m3 + m4) + m5;
-            // MI, IM, DN (ND uses no query transition)
-            const float i1 = xexp((up.MM + qf[TMM]) + tf[TMI] + b.MI - lz);
-            const float i2 = xexp((up.MI + qf[TMM]) + tf[TII] + b.MI - lz);
-            const float l1 = xexp((left.MM + qf[TMI]) + tf[TMM] + b.IM - lz);
-            const float l2 = xexp((left.IM + qf[TII]) + tf[TMM] + b.IM - lz);
-            const float d1 = xexp(up.MM + qf[TMD] + b.DN - lz);
-            const float d2 = xexp(up.DN + qf[TDD] + b.DN - lz);
-            g[TMM] += m1 + m4 + m5 + i1 + i2;
-            g[TIM] += m2;
-            g[TDM] += m3;
-            g[TMI] += l1;
-            g[TII] += l2;
-            g[TMD] += d1;
-            g[TDD] += d2;
-            g[7] += gs * a.pss[kk];
-            g[8] += gs * a.pcv[kk];
-            a.gS[kk] = gs;
-            a.post[kk] = xexp(own.MM + b.MM - lz);
+            edge_posteriors(a, kk, nw, own.MM, up, left, diag, qf, tf, sc0, lz, a.pss[kk], a.pcv[kk], g);
             if (wr_row) row_put(mine_row, ldr, jm, nw.MM, nw.MI, nw.IM, nw.DN, nw.ND);
+        }
+        if (!OUT && kf == flush) {
+            // a run of lines is complete (adj_post_kernel's order of summation)
+#pragma unroll
+            for (int f = 0; f < 9; f++) {
+                const float v = warp_sum(g[f]);
+                if (lane == f) tot += v;
+                g[f] = 0.f;
+            }
+            flush -= post_run(L + 31);
         }
         mine = nw;
         upp = dn;
@@ -662,33 +714,25 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         sc2 = sc1; sc1 = sc0; sc0 = scn;
         sb = sbn;
     }
-    // the strip's gradient sums
-#pragma unroll
-    for (int f = 0; f < 9; f++) {
-        float v = g[f];
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-        g[f] = v;
-    }
-    if (lane == 0) {
-        float* o = a.gpart + (a.soff[m] + s) * 9;
-#pragma unroll
-        for (int f = 0; f < 9; f++) o[f] = g[f];
-    }
+    if (!OUT && lane < 9) a.gpart[(a.soff[m] + s) * 9 + lane] = tot;
 }
 
-// Bound by the chain of steps (a step of ~350 instructions, ~1,000 steps deep).
-// KEPT: the forward sweep kept its states (Fall), the recomputing sweep and its
-// registers are not in the kernel, and 12 warps an SM at 162 registers beat 16 at
-// 128 (the two in one kernel spilled 4 registers): 2.0 -> 1.72 ms on 256 pairs
-// of 100..600 positions, 0.48 -> 0.43 on 45 of 60..300 (16 warps: 1.88, 0.44).
-template <bool KEPT>
-__global__ void __launch_bounds__(ADJ_WARPS * 32, KEPT ? 3 : 4) adj_bwd_kernel(AdjArgs a)
+// Bound by the chain of steps.  Three forms:
+//  ADJ_OUT: the forward sweep kept its states (Fall) and there is room for the
+//    outside values too (Ball): this sweep stores B, adj_post_kernel then forms the
+//    posteriors of all cells at once.  The chain's step is ~110 instructions
+//    instead of ~350.
+//  ADJ_KEPT: room for Fall only.  Posteriors in the sweep, 12 warps an SM at 162
+//    registers (16 at 128 were slower: 1.88 against 1.72 ms on 256 pairs of 100..600).
+//  ADJ_RECOMP: Fall did not fit; the strip's forward states are computed again.
+constexpr int ADJ_RECOMP = 0, ADJ_KEPT = 1, ADJ_OUT = 2;
+template <int MODE>
+__global__ void __launch_bounds__(ADJ_WARPS * 32, MODE == ADJ_OUT ? 5 : MODE == ADJ_KEPT ? 3 : 4) adj_bwd_kernel(AdjArgs a)
 {
     __shared__ __align__(16) float rabs[ADJ_WARPS][32 * 8];
     __shared__ __align__(16) float trss[ADJ_WARPS][128 * TRS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* const scr = KEPT ? nullptr : a.scratch + ((long long)blockIdx.x * ADJ_WARPS + wid) * a.scratch_stride;
+    float* const scr = MODE == ADJ_RECOMP ? a.scratch + ((long long)blockIdx.x * ADJ_WARPS + wid) * a.scratch_stride : nullptr;
     bool broken = false;
     for (;;) {
         int item = 0;
@@ -697,10 +741,13 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, KEPT ? 3 : 4) adj_bwd_kernel(A
         if (item >= a.nitems) break;
         const int2 ms = a.items_b[item];
         const int m = ms.x, s = ms.y;
-        const float* Fw;
-        if (KEPT) {
-            // the forward sweep kept the strip's states
-            Fw = a.Fall + 5 * a.off[m] + (long long)s * (a.plen[a.prof[m]] + 31) * 160;
+        const long long st5 = 5 * a.off[m] + (long long)s * (a.plen[a.prof[m]] + 31) * 160;   // the strip's states
+        const float* Fw = nullptr;
+        float* Bw = nullptr;
+        if (MODE == ADJ_OUT) {
+            Bw = a.Ball + st5;
+        } else if (MODE == ADJ_KEPT) {
+            Fw = a.Fall + st5;
         } else {
             // checkpointing: the strip's states again, from the row above
             float zm = 0.f, zs = 0.f;
@@ -708,8 +755,97 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, KEPT ? 3 : 4) adj_bwd_kernel(A
             Fw = scr;
         }
         __syncwarp();
-        adj_bwd_strip(a, m, s, lane, rabs[wid], trss[wid], Fw, broken);
+        adj_bwd_strip<MODE == ADJ_OUT>(a, m, s, lane, rabs[wid], trss[wid], Fw, Bw, broken);
         __syncwarp();
+    }
+}
+
+// Posteriors and gradient sums from stored F and B: one CTA per strip, one warp per
+// run of its lines, from the last line of the run.  A line's cells lie on
+// consecutive lanes; the left, upper and diagonal neighbours are on the two lines
+// below it, kept in registers, the row above by shuffle.  Every line of F, B and the
+// three score arrays is read once (the first two of a run twice) and the two
+// outputs written: 60 bytes a cell, bound by DRAM on large batches.
+__global__ void __launch_bounds__(POST_WARPS * 32) adj_post_kernel(AdjArgs a)
+{
+    __shared__ __align__(16) float trss[POST_WARPS][64 * TRS];
+    __shared__ float gsh[POST_WARPS][9];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float* trs = trss[wid];
+    const int2 ms = a.items_b[blockIdx.x];
+    const int m = ms.x, s = ms.y;
+    const int p = a.prof[m];
+    const int L = a.plen[p], Lq = a.pLq[m];
+    const long long cb = a.off[m] + (long long)s * (L + 31) * 32;
+    const float* Fw = a.Fall + 5 * a.off[m] + (long long)s * (L + 31) * 160;
+    const float* Bw = a.Ball + 5 * a.off[m] + (long long)s * (L + 31) * 160;
+    const float lz = a.zpart[2 * a.soff[m]];
+    const float* dt0 = a.dtrn + (a.poff[p] + p) * 7;
+    const int ldr = row_ld(L);
+    const float* fab = a.frow + a.roff[m] + (long long)(s > 0 ? s - 1 : 0) * 5 * ldr;
+    const int i = 32 * s + lane;
+    const bool act = i < Lq;
+    const X5 INIT = {0.f, XLOG0, XLOG0, XLOG0, XLOG0};
+    float qf[7];
+    xtrn_fwd(a.qtrn + (a.qpos[m] + a.qidx[m]) * 7, i, Lq, qf);
+#pragma unroll
+    for (int k = 0; k < 7; k++) qf[k] += a.theta[k] * XLOG2E;
+    const float* cf = a.qcfx + (a.qpos[m] + (act ? i : 0)) * 6;
+    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0] * XLOG2E, cf[1] * XLOG2E, cf[2] * XLOG2E, XLOG0};
+    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3] * XLOG2E, cf[4] * XLOG2E, cf[5] * XLOG2E, XLOG0};
+    const int nl = L + 31, run = post_run(nl);
+    const int k0 = wid * run, k1 = min(nl, k0 + run);
+    float g[9];
+#pragma unroll
+    for (int f = 0; f < 9; f++) g[f] = 0.f;
+    if (k0 < k1) {
+        auto row_above = [&](int c) { return (s > 0 && lane == 0 && c >= 0 && c < L) ? row_ld5(fab, ldr, c) : INIT; };
+        // lines k (own), k - 1 (left), and the row above at columns c and c - 1
+        X5 own = fw_ld5(Fw, k1 - 1, lane);
+        X5 left = k1 >= 2 ? fw_ld5(Fw, k1 - 2, lane) : INIT;
+        X5 up = shfl_up5(left);
+        if (lane == 0) up = row_above(k1 - 1);
+        for (int ke = k1; ke > k0; ke -= 32) {
+            // transition rows ke - 63 .. ke of the next 32 lines, in base 2 (row r at r & 63)
+            __syncwarp();
+            for (int e = lane; e < 64 * 7; e += 32) {
+                const int row = ke - 63 + e / 7, f = e % 7;
+                if (row >= 0 && row <= L) trs[(row & 63) * TRS + f] = __ldg(dt0 + (long long)row * 7 + f) * XLOG2E;
+            }
+            __syncwarp();
+#pragma unroll 2
+            for (int k = ke - 1; k >= max(k0, ke - 32); k--) {
+                const int c = k - lane;
+                const bool valid = act && c >= 0 && c < L;
+                const long long kk = cb + (long long)k * 32 + lane;
+                const X5 nx = k >= 2 ? fw_ld5(Fw, k - 2, lane) : INIT;
+                const X5 b = fw_ld5(Bw, k, lane);
+                const float sc = a.S[kk], ps = a.pss[kk], pc = a.pcv[kk];
+                X5 dg = shfl_up5(nx);
+                if (lane == 0) dg = row_above(c - 1);
+                float tf[7], tn[7];
+                ring_row<64>(trs, c, tf);
+                ring_row<64>(trs, c + 1, tn);
+                tf[TMI] = tn[TMI];
+                tf[TII] = tn[TII];
+                if (valid)
+                    edge_posteriors(a, kk, b, own.MM, up, c == 0 ? LB : left, c == 0 ? DB : dg, qf, tf, sc, lz, ps, pc, g);
+                up = dg;
+                own = left;
+                left = nx;
+            }
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < 9; f++) {
+        const float v = warp_sum(g[f]);
+        if (lane == 0) gsh[wid][f] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 9) {
+        float v = 0.f;
+        for (int w = POST_WARPS - 1; w >= 0; w--) v += gsh[w][threadIdx.x];
+        a.gpart[(a.soff[m] + s) * 9 + threadIdx.x] = v;
     }
 }
 
@@ -729,7 +865,7 @@ cudaError_t adj_occupancy(int* fwd_ctas_per_sm, int* bwd_ctas_per_sm)
 {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(fwd_ctas_per_sm, adj_fwd_kernel, ADJ_WARPS * 32, 0);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bwd_ctas_per_sm, adj_bwd_kernel<false>, ADJ_WARPS * 32, 0);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bwd_ctas_per_sm, adj_bwd_kernel<ADJ_RECOMP>, ADJ_WARPS * 32, 0);
 }
 
 cudaError_t launch_adj_fwd(const AdjArgs& a, int grid, cudaStream_t st)
@@ -748,10 +884,20 @@ cudaError_t launch_adj_fwd(const AdjArgs& a, int grid, cudaStream_t st)
 cudaError_t launch_adj_bwd(const AdjArgs& a, int grid, cudaStream_t st)
 {
     if (a.npairs <= 0) return cudaSuccess;
-    if (a.Fall)
-        adj_bwd_kernel<true><<<grid, ADJ_WARPS * 32, 0, st>>>(a);
-    else
-        adj_bwd_kernel<false><<<grid, ADJ_WARPS * 32, 0, st>>>(a);
+    if (a.Ball) {
+        int occ = 0, dev = 0, nsm = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, adj_bwd_kernel<ADJ_OUT>, ADJ_WARPS * 32, 0);
+        if (e == cudaSuccess) e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        const int g = std::min(nsm * std::max(occ, 1), (a.nitems + ADJ_WARPS - 1) / ADJ_WARPS);
+        adj_bwd_kernel<ADJ_OUT><<<g, ADJ_WARPS * 32, 0, st>>>(a);
+        adj_post_kernel<<<a.nitems, POST_WARPS * 32, 0, st>>>(a);
+    } else if (a.Fall) {
+        adj_bwd_kernel<ADJ_KEPT><<<grid, ADJ_WARPS * 32, 0, st>>>(a);
+    } else {
+        adj_bwd_kernel<ADJ_RECOMP><<<grid, ADJ_WARPS * 32, 0, st>>>(a);
+    }
     adj_gsum_kernel<<<(a.npairs * 9 + 127) / 128, 128, 0, st>>>(a);
     return cudaGetLastError();
 }

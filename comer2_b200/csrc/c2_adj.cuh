@@ -51,6 +51,7 @@ struct AdjArgs {
     float* gpart;           // [nitems][9] a strip's gradient sums
     float* Fall;            // forward states of every strip, when they fit (else null): strip s of
                             // pair m at Fall + 5 off[m] + s (L + 31) 160 (fw_st5)
+    float* Ball;            // outside values of every strip, like Fall, when they fit too (else null)
     float* scratch;         // per backward warp (Fall null): forward states of its strip, [(Lmax + 31) * 5 * 32]
     long long scratch_stride;
     int* counter;           // [2] work counters of the forward and backward sweeps

@@ -116,23 +116,110 @@ struct DbStore {
     std::mutex tc_mu;
 };
 
-// Pinned host memory of a handle through which its transfers go: an
-// asynchronous copy from or to pageable memory is staged by the driver piece
-// by piece and returns late.  Space is taken in order; when it runs out, the
-// stream is synchronised (every copy is then done) and it starts over.  It
-// grows to the largest piece taken, at most 2 x STAGE_MAX.
-constexpr size_t STAGE_MIN = size_t(1) << 20, STAGE_MAX = size_t(20) << 20;
+// Pinned host memory of the process, lent to its handles.  Allocating it takes
+// milliseconds, more than a small search, so a handle borrows one of PIN_SLOTS
+// slots for its life and a query batch's packing borrows the block for a call;
+// both are given back, and the memory (at most PIN_SLOTS x PIN_SLOT +
+// PIN_BLOCK_MAX = 28 MiB) serves the next borrower.  Any thread may borrow.  Who
+// gets nothing (all slots out, block lent, no memory) uses pageable memory.
+constexpr size_t PIN_SLOT = size_t(256) << 10, PIN_BLOCK_MAX = size_t(24) << 20;
+constexpr int PIN_SLOTS = 16;
+class PinnedPool {
+public:
+    static PinnedPool& get()
+    {
+        static PinnedPool* p = new PinnedPool;   // not destroyed: the CUDA runtime may be gone by then
+        return *p;
+    }
+    // a slot (and the generation to give it back with), or null
+    char* take_slot(unsigned& gen)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (slots_ && !alive(slots_)) slots_ = nullptr;   // the device was reset
+        if (!slots_) {
+            slots_ = alloc(PIN_SLOTS * PIN_SLOT);
+            taken_ = 0;
+            gen_++;
+        }
+        for (int i = 0; slots_ && i < PIN_SLOTS; i++)
+            if (!(taken_ >> i & 1u)) {
+                taken_ |= 1u << i;
+                gen = gen_;
+                return slots_ + (size_t)i * PIN_SLOT;
+            }
+        return nullptr;
+    }
+    void give_slot(char* p, unsigned gen)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (gen == gen_ && slots_) taken_ &= ~(1u << ((p - slots_) / PIN_SLOT));
+    }
+    // the block, at least `bytes` (<= PIN_BLOCK_MAX) large, or null
+    char* lend_block(size_t bytes)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (lent_ || bytes > PIN_BLOCK_MAX) return nullptr;
+        if (block_ && !alive(block_)) block_ = nullptr;
+        if (!block_ || block_bytes_ < bytes) {
+            if (block_) cudaFreeHost(block_);
+            block_bytes_ = std::min(PIN_BLOCK_MAX, (bytes + (size_t(4) << 20) - 1) & ~((size_t(4) << 20) - 1));
+            block_ = alloc(block_bytes_);
+        }
+        lent_ = block_ != nullptr;
+        return block_;
+    }
+    void return_block()
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        lent_ = false;
+    }
+
+private:
+    static char* alloc(size_t bytes)
+    {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return static_cast<char*>(p);
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    static bool alive(const char* p)
+    {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost) return true;
+        (void)cudaGetLastError();
+        return false;
+    }
+    std::mutex mu_;
+    char *slots_ = nullptr, *block_ = nullptr;
+    unsigned taken_ = 0, gen_ = 0;
+    size_t block_bytes_ = 0;
+    bool lent_ = false;
+};
+
+// A handle's slot (or pageable memory of that size).  Space is taken in order and
+// free again once the handle's stream has been synchronised.
 struct HostStage {
     char* p = nullptr;
-    size_t cap = 0, used = 0;
+    size_t used = 0;
+    unsigned gen = 0;
     bool pinned = false;
-    ~HostStage() { release(); }
-    void release()
+    ~HostStage()
     {
-        if (p && pinned) cudaFreeHost(p);
+        if (p && pinned) PinnedPool::get().give_slot(p, gen);
         else free(p);
-        p = nullptr;
-        cap = used = 0;
+    }
+    char* take(size_t bytes)   // null: no room now
+    {
+        if (!p) {
+            p = PinnedPool::get().take_slot(gen);
+            pinned = p != nullptr;
+            if (!p) p = static_cast<char*>(malloc(PIN_SLOT));
+        }
+        bytes = (bytes + 255) & ~size_t(255);
+        if (!p || used + bytes > PIN_SLOT) return nullptr;
+        char* r = p + used;
+        used += bytes;
+        return r;
     }
 };
 
@@ -184,8 +271,8 @@ struct c2_handle {
     DevBuf<long long> d_adjoff, d_adjroff, d_adjqpos, d_adjsoff;
     DevBuf<int2> d_adjitems;
     DevBuf<float> d_adjbuf, d_adjlogz, d_adjgrad, d_adjpart, d_adjscr;
-    DevBuf<float> d_adjF;            // all forward states, when they fit (no recompute in the backward sweep)
-    bool adj_keepF = false;
+    // (d_adjbuf: per-cell arrays, strip rows, then, when they fit, every forward state and outside value)
+    bool adj_keepF = false, adj_keepB = false;
     DevBuf<float> d_adjqrec, d_adjqtrn, d_adjqcfx, d_adjqbkg;   // queries of c2_set_query_batch
     std::vector<int> adj_qlen;                                   // their lengths
     std::vector<long long> adj_qstart;                           // and first rows
@@ -270,50 +357,22 @@ static c2_status fail(c2_handle* h, c2_status st, const char* fmt, ...)
                         __FILE__, __LINE__);                                            \
     } while (0)
 
-// `bytes` of the handle's pinned staging memory, valid until the stage starts
-// over (a later stage_take, after a stream synchronisation); null: no memory
-static char* stage_take(c2_handle* h, size_t bytes)
-{
-    HostStage& S = h->stage;
-    bytes = (bytes + 255) & ~size_t(255);
-    if (S.used + bytes > S.cap) {
-        if (cudaStreamSynchronize(h->stream) != cudaSuccess) return nullptr;
-        S.used = 0;
-        if (bytes > S.cap) {
-            const size_t want = std::max(STAGE_MIN, 2 * bytes);
-            S.release();
-            S.pinned = cudaHostAlloc(reinterpret_cast<void**>(&S.p), want, cudaHostAllocDefault) == cudaSuccess;
-            if (!S.pinned) {
-                // pageable memory then: the copies are complete, or taken over, when they return
-                (void)cudaGetLastError();
-                S.p = static_cast<char*>(malloc(want));
-            }
-            if (!S.p) return nullptr;
-            S.cap = want;
-        }
-    }
-    char* r = S.p + S.used;
-    S.used += bytes;
-    return r;
-}
-
-// host -> device through the staging memory; src may be reused at once
+// host -> device; src may be reused at once.  What fits goes through the handle's
+// staging memory; a larger copy straight from pageable memory, which the driver
+// takes over before the call returns.
 static cudaError_t h2d(c2_handle* h, void* dst, const void* src, size_t bytes)
 {
-    constexpr size_t PIECE = size_t(4) << 20;
-    for (size_t o = 0; o < bytes; o += PIECE) {
-        const size_t n = std::min(PIECE, bytes - o);
-        char* p = stage_take(h, n);
-        if (!p) return cudaErrorMemoryAllocation;
-        memcpy(p, static_cast<const char*>(src) + o, n);
-        const cudaError_t e = cudaMemcpyAsync(static_cast<char*>(dst) + o, p, n, cudaMemcpyHostToDevice, h->stream);
-        if (e != cudaSuccess) return e;
+    if (bytes == 0) return cudaSuccess;
+    if (char* p = h->stage.take(bytes)) {
+        memcpy(p, src, bytes);
+        src = p;
     }
-    return cudaSuccess;
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
 }
 
 // device -> host: several arrays with one synchronisation.  get() queues a copy
-// (directly where it is larger than the stage), finish() waits for all of them.
+// (straight to its destination where it is larger than the stage), finish()
+// waits for all of them.
 struct Fetch {
     c2_handle* h;
     struct Part { void* dst; const char* p; size_t n; };
@@ -322,23 +381,13 @@ struct Fetch {
     cudaError_t get(void* dst, const void* src, size_t bytes)
     {
         if (bytes == 0) return cudaSuccess;
-        size_t held = 0;
-        for (const Part& q : parts) held += q.n + 256;
-        if (bytes > STAGE_MAX || held + bytes > STAGE_MAX) {
-            const cudaError_t e = finish();
+        char* p = h->stage.take(bytes);
+        if (!p && bytes <= PIN_SLOT) {
+            const cudaError_t e = finish();   // frees the stage
             if (e != cudaSuccess) return e;
-            if (bytes > STAGE_MAX) {
-                const cudaError_t c = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream);
-                return c != cudaSuccess ? c : cudaStreamSynchronize(h->stream);
-            }
+            p = h->stage.take(bytes);
         }
-        // (taking space may start the stage over: not while parts are in it)
-        if (!parts.empty() && h->stage.used + bytes + 256 > h->stage.cap) {
-            const cudaError_t e = finish();
-            if (e != cudaSuccess) return e;
-        }
-        char* p = stage_take(h, bytes);
-        if (!p) return cudaErrorMemoryAllocation;
+        if (!p) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream);
         parts.push_back({dst, p, bytes});
         return cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, h->stream);
     }
@@ -348,6 +397,7 @@ struct Fetch {
         if (e == cudaSuccess)
             for (const Part& q : parts) memcpy(q.dst, q.p, q.n);
         parts.clear();
+        h->stage.used = 0;
         return e;
     }
 };
@@ -2133,6 +2183,9 @@ extern "C" c2_status c2_run_phase1_static(c2_handle* h, float* d_best, uint32_t*
 
 static c2_profiles query_view(const c2_profiles* qs, int k, const int64_t* zero);
 
+// floats of the adjoint's per-cell arrays and strip rows; the kept states follow
+static size_t adj_base(long long cells, long long rows) { return (size_t)((5 * cells + 2 * rows + 31) / 32 * 32); }
+
 static void fill_adj(c2_handle* h, AdjArgs& a)
 {
     memset(&a, 0, sizeof a);
@@ -2180,7 +2233,8 @@ static void fill_adj(c2_handle* h, AdjArgs& a)
     a.brow = b + 5 * NC + NR;
     a.zpart = h->d_adjpart.p;
     a.gpart = h->d_adjpart.p + 2LL * h->adj_nitems;
-    a.Fall = h->adj_keepF ? h->d_adjF.p : nullptr;
+    a.Fall = h->adj_keepF ? h->d_adjbuf.p + adj_base(h->adj_cells, h->adj_rows) : nullptr;
+    a.Ball = h->adj_keepB ? a.Fall + 5 * h->adj_cells : nullptr;
     a.scratch = h->d_adjscr.p;
     a.scratch_stride = (long long)(h->adj_Lmax + 31) * 160;
     a.counter = h->d_adjctr.p;
@@ -2260,7 +2314,6 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
         h->d_adjroff.ensure(npairs, h->budget) || h->d_adjLq.ensure(npairs, h->budget) ||
         h->d_adjqpos.ensure(npairs, h->budget) || h->d_adjqidx.ensure(npairs, h->budget) ||
         h->d_adjsoff.ensure(npairs, h->budget) || h->d_adjitems.ensure((size_t)2 * items, h->budget) ||
-        h->d_adjbuf.ensure((size_t)(5 * acc + 2 * racc), h->budget) ||
         h->d_adjlogz.ensure(npairs, h->budget) || h->d_adjgrad.ensure((size_t)npairs * 9, h->budget) ||
         h->d_adjpart.ensure((size_t)11 * items, h->budget) ||
         h->d_adjctr.ensure(2, h->budget))
@@ -2278,20 +2331,40 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
     // otherwise the backward sweep recomputes each strip's states from the
     // checkpoint row above into per-warp scratch (32 rows x (Lmax + 31)
     // columns x 5 floats), its grid halved while that scratch does not fit.
-    h->adj_keepF = false;
+    // Where both fit the quarter, there is room for the backward sweep's outside
+    // values too, and the posteriors get a kernel of their own (c2_adj.cu).  Not
+    // under a memory limit: that is for the buffers a call cannot do without.
+    h->adj_keepF = h->adj_keepB = false;
     {
+        const size_t base = adj_base(acc, racc), nF = (size_t)acc * 5;
+        const size_t have = h->d_adjbuf.p ? h->d_adjbuf.n : 0;
+        bool limited;
+        {
+            std::lock_guard<std::mutex> lk(h->budget->mu);
+            limited = h->budget->limit != 0;
+        }
         // (asking for the free memory takes longer than a small batch's sweeps: not
         // for a buffer that is already there)
         size_t fr = 0, tot = 0;
-        if (h->d_adjF.p && h->d_adjF.n >= (size_t)acc * 5)
+        if (have >= base + (limited ? 1 : 2) * nF) {
             h->adj_keepF = true;
-        else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && (size_t)acc * 5 * sizeof(float) <= fr / 4 &&
-            h->d_adjF.ensure((size_t)acc * 5, h->budget) == cudaSuccess)
-            h->adj_keepF = true;
+            h->adj_keepB = !limited;
+        } else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
+            const size_t room = (fr / sizeof(float) + have) / 4;
+            for (int n = limited ? 1 : 2; n >= 1 && !h->adj_keepF; n--)
+                if (n * nF <= room && h->d_adjbuf.ensure(base + n * nF, h->budget) == cudaSuccess) {
+                    h->adj_keepF = true;
+                    h->adj_keepB = n == 2;
+                }
+        }
+        if (!h->adj_keepF) {
+            if (h->d_adjbuf.n > base) h->d_adjbuf.release();   // what it holds beyond goes to the scratch below
+            if (h->d_adjbuf.ensure(base, h->budget) != cudaSuccess)
+                return fail(h, C2_ERR_NOMEM, "logz_fwd: scratch for %d pairs (%lld cells) failed", npairs, acc);
+        }
         (void)cudaGetLastError();   // a refused allocation is not an error of what follows
     }
     if (!h->adj_keepF) {
-        h->d_adjF.release();
         const size_t per_cta = (size_t)ADJ_WARPS * (lmax + 31) * 160 * sizeof(float);
         h->adj_bgrid = 0;
         for (long long g = want; g >= 1 && h->adj_bgrid == 0; g /= 2)
@@ -2366,17 +2439,41 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
         return fail(h, C2_ERR_NOMEM, "set_query_batch: query arrays for %d queries failed", nq);
     CK(h2d(h, h->d_adjqtrn.p, queries->trn, (size_t)(N + nq) * 7 * 4));
     CK(h2d(h, h->d_adjqbkg.p, queries->bkg, (size_t)nq * NAA * 4));
-    // pieces of whole queries (a query is at most 65,535 rows), packed by the host
-    // threads straight into the staging memory, each copied while the next is packed
-    constexpr long long ROW_FLOATS = QR_STRIDE + 6;
-    const long long rows_max = std::max<long long>(65535, (long long)(STAGE_MAX / 2 / (ROW_FLOATS * sizeof(float))));
-    for (int q0 = 0; q0 < nq;) {
+    // pieces of whole queries, packed by the host threads straight into pinned
+    // memory, each copied while the next is packed.  (A query of 65,535 rows, the
+    // longest, fits the block.)
+    constexpr size_t ROW_BYTES = (QR_STRIDE + 6) * sizeof(float);
+    static_assert(65535 * ROW_BYTES <= PIN_BLOCK_MAX, "the longest query must fit the pinned block");
+    struct Loan {
+        char* p = nullptr;
+        ~Loan() { if (p) PinnedPool::get().return_block(); }
+    } loan;
+    std::vector<char> heap;
+    const size_t need = (size_t)N * ROW_BYTES;
+    size_t cap = need, used = 0;
+    char* base = h->stage.take(need);
+    if (!base) {
+        cap = std::min(need, PIN_BLOCK_MAX);
+        base = loan.p = PinnedPool::get().lend_block(cap);
+        if (!base) {
+            heap.resize(cap);
+            base = heap.data();
+        }
+    }
+    c2_status rc = C2_OK;
+    for (int q0 = 0; q0 < nq && rc == C2_OK;) {
         int q1 = q0;
-        long long rows = 0;
-        while (q1 < nq && (q1 == q0 || rows + queries->lengths[q1] <= rows_max / 2)) rows += queries->lengths[q1++];
-        float* buf = reinterpret_cast<float*>(stage_take(h, (size_t)rows * ROW_FLOATS * sizeof(float)));
-        if (!buf) return fail(h, C2_ERR_NOMEM, "set_query_batch: staging memory for %lld rows failed", rows);
-        float *rec = buf, *qcf = buf + rows * QR_STRIDE;
+        size_t rows = 0;
+        while (q1 < nq && (q1 == q0 || (rows + queries->lengths[q1]) * ROW_BYTES <= PIN_BLOCK_MAX / 3))
+            rows += queries->lengths[q1++];
+        if (used + rows * ROW_BYTES > cap) {
+            const cudaError_t e = cudaStreamSynchronize(h->stream);
+            if (e != cudaSuccess) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
+            used = 0;
+        }
+        float* rec = reinterpret_cast<float*>(base + used);
+        float* qcf = rec + rows * QR_STRIDE;
+        used += rows * ROW_BYTES;
         const long long r0 = queries->offsets[q0];
         std::atomic<int> next(q0);
         auto work = [&]() {
@@ -2399,11 +2496,20 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
         }
         work();
         for (auto& t : th) t.join();
-        CK(cudaMemcpyAsync(h->d_adjqrec.p + (size_t)r0 * QR_STRIDE, rec, (size_t)rows * QR_STRIDE * 4,
-                           cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemcpyAsync(h->d_adjqcfx.p + (size_t)r0 * 6, qcf, (size_t)rows * 6 * 4, cudaMemcpyHostToDevice, h->stream));
+        cudaError_t e = cudaMemcpyAsync(h->d_adjqrec.p + (size_t)r0 * QR_STRIDE, rec, rows * QR_STRIDE * 4,
+                                        cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(h->d_adjqcfx.p + (size_t)r0 * 6, qcf, rows * 6 * 4, cudaMemcpyHostToDevice, h->stream);
+        if (e != cudaSuccess && rc == C2_OK) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
         q0 = q1;
     }
+    if (loan.p || !heap.empty()) {
+        // before the block goes back
+        const cudaError_t e = cudaStreamSynchronize(h->stream);
+        if (e != cudaSuccess && rc == C2_OK) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
+        h->stage.used = 0;
+    }
+    if (rc != C2_OK) return rc;
     h->adj_qlen.assign(queries->lengths, queries->lengths + nq);
     h->adj_qstart.assign(queries->offsets, queries->offsets + nq);
     h->adj_fwd_done = false;
@@ -2442,7 +2548,7 @@ extern "C" c2_status c2_logz_bwd(c2_handle* h, float* grad)
     CK(cudaMemsetAsync(h->d_adjbuf.p + 5 * h->adj_cells + h->adj_rows, 0xff, (size_t)h->adj_rows * sizeof(float), h->stream));
     CK(cudaMemsetAsync(h->d_adjctr.p + 1, 0, sizeof(int), h->stream));
     CK(launch_adj_bwd(a, h->adj_bgrid, h->stream));
-    h->launches += 2;
+    h->launches += a.Ball ? 3 : 2;
     return adj_results(h, grad, h->d_adjgrad.p, (size_t)a.npairs * 9);
 }
 
