@@ -1278,19 +1278,23 @@ static void fill_p1(c2_handle* h, P1Args& a)
 }
 
 // Phase-1 pairs whose strips become work items of their own (p1_take): those
-// that one of the nwarps warps would sweep in more than SPLIT_SHARE of the
-// time all pairs together take on all warps (both grow with the number of
-// strips alike, so the query length does not enter).  Pairs below that even
-// out over the warps by the longest-first order; pairs above it would be the
-// tail of the search.  Phase-1 times in ms with shares of 1 / 0.7 / 0.5 / 0.3 /
-// 0.15: 1 x 3,000 vs 4,000 profiles 18.8 / 18.7 / 19.3 / 21.0 / 21.3, 1 x 1,237 vs
-// 4,999 8.2 / 8.2 / 8.7 / 8.8 / 9.4, 1 x 250 vs 3,000 (FP32) 1.36 / 1.47 / 1.40 / 1.44 /
-// 1.54, 7 queries vs 1,000 (FP32) 6.4 / 6.2 / 6.1 / 6.0 / 6.0, 1 x 150 vs 2,000 0.60 /
-// 0.58 / 0.55 / 0.51 / 0.49 (none split, before strips of 64 rows: 41.9, 16.2, 4.5, 32,
-// 0.70); no pair is split, and nothing changes, against 50,000 profiles.  0
+// that one of the nwarps warps would sweep in more than a share of the time all
+// pairs together take on all warps (both grow with the number of strips alike, so
+// the query length does not enter).  A strip handed from warp to warp costs more
+// than one of a whole pair, so the share is as large as the end of the search
+// allows.  The whole pairs come last, longest first: where a last one per warp
+// is short (the nwarps-th shortest pair at most SPLIT_EVEN of the mean time), they
+// even out what the longer ones leave, and only pairs above SPLIT_MANY would be the
+// tail; where not (few pairs a warp), a pair above SPLIT_FEW is.  Phase-1
+// times in ms with shares of 1 / 0.7 / 0.5 / 0.3 / 0.15: 1 x 3,000 vs 4,000 profiles
+// 18.8 / 18.7 / 19.3 / 21.0 / 21.3, 1 x 1,237 vs 4,999 8.2 / 8.2 / 8.7 / 8.8 / 9.4, 1 x 250
+// vs 3,000 (FP32) 1.36 / 1.47 / 1.40 / 1.44 / 1.54; with few pairs a warp, 7 queries
+// vs 1,000 (FP32) 6.4 / 6.2 / 6.1 / 6.0 / 6.0, 1 x 150 vs 2,000 0.60 / 0.58 / 0.55 / 0.51 /
+// 0.49 (none split, before strips of 64 rows: 41.9, 16.2, 4.5, 32, 0.70); no pair
+// is split, and nothing changes, against 50,000 profiles.  0
 // without the scratch (it is small: the two boundary rows of the split pairs) --
 // the pairs then run whole, with the same results.
-constexpr double SPLIT_SHARE = 0.5;
+constexpr double SPLIT_MANY = 0.8, SPLIT_FEW = 0.15, SPLIT_EVEN = 0.4;
 
 static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
 {
@@ -1298,9 +1302,11 @@ static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
     a.nsplit = 0;
     if (ns < 2) return 0;
     const double mean = ((double)h->npos + 31.0 * P) / std::max(1, nwarps);
-    const std::vector<int>& sl = h->db->slen;
+    const std::vector<int>& sl = h->db->slen;   // longest first
+    const bool even = P > nwarps && (double)sl[P - nwarps] + 31.0 <= SPLIT_EVEN * mean;
+    const double share = even ? SPLIT_MANY : SPLIT_FEW;
     const int n = (int)(std::partition_point(sl.begin(), sl.end(),
-                                             [&](int L) { return (double)L + 31.0 > SPLIT_SHARE * mean; }) - sl.begin());
+                                             [&](int L) { return (double)L + 31.0 > share * mean; }) - sl.begin());
     if (n == 0 || (long long)n * ns > 0x7fffffff) return 0;
     const size_t words = (size_t)n * 8 + (size_t)n * 4 + (size_t)n * ns * 4;
     if (h->d_splitbnd.ensure((size_t)h->db->soff[n] * 10, h->budget) != cudaSuccess ||
