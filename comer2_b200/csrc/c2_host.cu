@@ -1982,6 +1982,7 @@ static void release_phase2(c2_handle* h)
     h->d_mapcand.release(); h->d_mappass.release(); h->d_alninfo.release(); h->d_fb.release(); h->d_bb.release();
     h->d_pairf.release(); h->d_pairc.release(); h->d_pairk.release(); h->d_aln.release(); h->d_alnpack.release();
     h->d_alnoff.release();
+    h->d_splitbnd.release(); h->d_splitsync.release();   // (phase 1 is done by then)
 }
 
 // Device bytes phase 2 takes for one candidate pair of db length L: score,
@@ -2020,7 +2021,9 @@ static c2_status plan_groups(c2_handle* h, const std::vector<int>& cand, std::ve
     if (used + margin >= limit)
         return fail(h, C2_ERR_NOMEM, "device memory budget of %zu bytes leaves nothing for phase 2 (%zu in use)", limit,
                     used);
-    const size_t avail = (limit - used - margin) / 10 * 9;
+    // (the estimate counts every array; 3 % for what else may come.  A pair's strip
+    // rows take 7 % of its scratch: a pair that fits 90 % without them fits 97 % with.)
+    const size_t avail = (limit - used - margin) / 100 * 97;
     std::vector<int> g;
     size_t gb = 0;
     for (int k : cand) {

@@ -1,6 +1,7 @@
 """Phase 1 with the longest pairs split into strip items: a database of many
 short profiles and a few much longer than the mean (split pairs and whole pairs
-in one launch), of few profiles (all split), and of equal ones (none split).
+in one launch), of few profiles (all split), and of equal ones (none split, or, with fewer pairs
+a warp in the tensor-core form, all).
 The strip kernel of the allocation-free entry point never splits and scores
 with the same FP32 arithmetic, so the FP32 maxima and cells must be its bits;
 the tensor-core form's maxima must lie within its rounding of them (1e-4
