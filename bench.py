@@ -554,7 +554,7 @@ def main():
                         "achieved_tflops": 40.0 * cells / (bf["p1ms"] * 1e-3) / 1e12,
                         "peak_tflops": _bf16_peak(), "frac": 40.0 * cells / (bf["p1ms"] * 1e-3) / 1e12 / _bf16_peak(),
                         "note": "40 flops/cell = the amino-acid contraction (20 multiply-adds); executed tensor "
-                                "work is 3 split products x 3 contractions x K 32"},
+                                "work is 3 split products x 3 contractions of K 24, 24 and 32"},
         "roofline": {"kernel": ("p1t_kernel" if args.score_mode == "bf16" else "p1c_kernel")
                                + " (fused score + Viterbi DP)", "bound": "hbm",
                      "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
