@@ -405,11 +405,13 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
         const float sc = valid ? scn : XLOG0;
         if (act && j + 1 >= 0 && j + 1 < L) scn = a.S[cb + (long long)(k + 1) * 32 + lane];
         X5 nw;
-        nw.MM = xlse5p1(((diag.MI + q7[TMM]) + t7[TIM]) + sc, ((diag.IM + q7[TIM]) + t7[TMM]) + sc,
-                        ((diag.DN + q7[TDM]) + t7[TMM]) + sc, ((diag.ND + q7[TMM]) + t7[TDM]) + sc,
-                        ((diag.MM + q7[TMM]) + t7[TMM]) + sc);
-        nw.MI = xlse2((up.MM + q7[TMM]) + t7[TMI], (up.MI + q7[TMM]) + t7[TII]);
-        nw.IM = xlse2((left.MM + q7[TMI]) + t7[TMM], (left.IM + q7[TII]) + t7[TMM]);
+        // (a state is added last, to the sum of the step's own terms: one rounding
+        // at the state's magnitude, and one addition in the chain of steps)
+        nw.MM = xlse5p1(diag.MI + ((q7[TMM] + t7[TIM]) + sc), diag.IM + ((q7[TIM] + t7[TMM]) + sc),
+                        diag.DN + ((q7[TDM] + t7[TMM]) + sc), diag.ND + ((q7[TMM] + t7[TDM]) + sc),
+                        diag.MM + ((q7[TMM] + t7[TMM]) + sc));
+        nw.MI = xlse2(up.MM + (q7[TMM] + t7[TMI]), up.MI + (q7[TMM] + t7[TII]));
+        nw.IM = xlse2(left.MM + (q7[TMI] + t7[TMM]), left.IM + (q7[TII] + t7[TMM]));
         nw.DN = xlse2(up.MM + q7[TMD], up.DN + q7[TDD]);
         nw.ND = xlse2(left.MM + t7[TMD], left.ND + t7[TDD]);
         if (valid) {
@@ -476,7 +478,7 @@ __global__ void adj_logz_kernel(AdjArgs a)
         zm = mx;
     }
     a.logz[m] = logf(zs) + zm * XLN2;
-    a.zpart[2 * a.soff[m]] = xlog(zs) + zm;   // base 2, for the backward sweep
+    a.zpart[2 * a.soff[m]] = log2f(zs) + zm;   // base 2, for the backward sweep (its error scales every posterior: not xlog)
 }
 
 // ---------------------------------------------------------------------------
@@ -505,21 +507,22 @@ __device__ __forceinline__ void edge_posteriors(const AdjArgs& a, long long kk, 
                                                 const X5& left, const X5& diag, const float* qf, const float* tf,
                                                 float sc, float lz, float pss, float pcv, float* g)
 {
+    // (the predecessor's and the cell's states first: they nearly cancel)
     // MM: five emission edges
-    const float eMM = b.MM - lz;
-    const float m1 = xexp(((diag.MI + qf[TMM]) + tf[TIM]) + sc + eMM);
-    const float m2 = xexp(((diag.IM + qf[TIM]) + tf[TMM]) + sc + eMM);
-    const float m3 = xexp(((diag.DN + qf[TDM]) + tf[TMM]) + sc + eMM);
-    const float m4 = xexp(((diag.ND + qf[TMM]) + tf[TDM]) + sc + eMM);
-    const float m5 = xexp(((diag.MM + qf[TMM]) + tf[TMM]) + sc + eMM);
+    const float eMM = b.MM - lz, eMI = b.MI - lz, eIM = b.IM - lz, eDN = b.DN - lz;
+    const float m1 = xexp((diag.MI + eMM) + ((qf[TMM] + tf[TIM]) + sc));
+    const float m2 = xexp((diag.IM + eMM) + ((qf[TIM] + tf[TMM]) + sc));
+    const float m3 = xexp((diag.DN + eMM) + ((qf[TDM] + tf[TMM]) + sc));
+    const float m4 = xexp((diag.ND + eMM) + ((qf[TMM] + tf[TDM]) + sc));
+    const float m5 = xexp((diag.MM + eMM) + ((qf[TMM] + tf[TMM]) + sc));
     const float gs = (m1 + m2 + m3 + m4) + m5;
     // MI, IM, DN (ND uses no query transition)
-    const float i1 = xexp((up.MM + qf[TMM]) + tf[TMI] + b.MI - lz);
-    const float i2 = xexp((up.MI + qf[TMM]) + tf[TII] + b.MI - lz);
-    const float l1 = xexp((left.MM + qf[TMI]) + tf[TMM] + b.IM - lz);
-    const float l2 = xexp((left.IM + qf[TII]) + tf[TMM] + b.IM - lz);
-    const float d1 = xexp(up.MM + qf[TMD] + b.DN - lz);
-    const float d2 = xexp(up.DN + qf[TDD] + b.DN - lz);
+    const float i1 = xexp((up.MM + eMI) + (qf[TMM] + tf[TMI]));
+    const float i2 = xexp((up.MI + eMI) + (qf[TMM] + tf[TII]));
+    const float l1 = xexp((left.MM + eIM) + (qf[TMI] + tf[TMM]));
+    const float l2 = xexp((left.IM + eIM) + (qf[TII] + tf[TMM]));
+    const float d1 = xexp((up.MM + eDN) + qf[TMD]);
+    const float d2 = xexp((up.DN + eDN) + qf[TDD]);
     g[TMM] += m1 + m4 + m5 + i1 + i2;
     g[TIM] += m2;
     g[TDM] += m3;
@@ -530,7 +533,7 @@ __device__ __forceinline__ void edge_posteriors(const AdjArgs& a, long long kk, 
     g[7] += gs * pss;
     g[8] += gs * pcv;
     a.gS[kk] = gs;
-    a.post[kk] = xexp(ownMM + b.MM - lz);
+    a.post[kk] = xexp(ownMM + eMM);
 }
 
 // column c of a complete row
@@ -671,12 +674,12 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
         // score of the diagonal successor (i + 1, ca + 1)
         const float sco = (valid && i + 1 < Lq && ca + 1 < L) ? (t == 0 ? sb : scu) : XLOG0;
         X5 nw;
-        nw.MM = xlse5p1((dn.MI + qb[TMM]) + tb[TMI], (rt.IM + qb[TMI]) + tb[TMM], dn.DN + qb[TMD],
-                        rt.ND + tb[TMD], ((dg.MM + qb[TMM]) + tb[TMM]) + sco);
-        nw.MI = xlse2(((dg.MM + qb[TMM]) + tb[TIM]) + sco, (dn.MI + qb[TMM]) + tb[TII]);
-        nw.IM = xlse2(((dg.MM + qb[TIM]) + tb[TMM]) + sco, (rt.IM + qb[TII]) + tb[TMM]);
-        nw.DN = xlse2(((dg.MM + qb[TDM]) + tb[TMM]) + sco, dn.DN + qb[TDD]);
-        nw.ND = xlse2(((dg.MM + qb[TMM]) + tb[TDM]) + sco, rt.ND + tb[TDD]);
+        nw.MM = xlse5p1(dn.MI + (qb[TMM] + tb[TMI]), rt.IM + (qb[TMI] + tb[TMM]), dn.DN + qb[TMD],
+                        rt.ND + tb[TMD], dg.MM + ((qb[TMM] + tb[TMM]) + sco));
+        nw.MI = xlse2(dg.MM + ((qb[TMM] + tb[TIM]) + sco), dn.MI + (qb[TMM] + tb[TII]));
+        nw.IM = xlse2(dg.MM + ((qb[TIM] + tb[TMM]) + sco), rt.IM + (qb[TII] + tb[TMM]));
+        nw.DN = xlse2(dg.MM + ((qb[TDM] + tb[TMM]) + sco), dn.DN + qb[TDD]);
+        nw.ND = xlse2(dg.MM + ((qb[TMM] + tb[TDM]) + sco), rt.ND + tb[TDD]);
         // rows past the query (the last strip's first lanes) are the matrix
         // edge for the rows above them
         if (!act) nw = INIT;
