@@ -7,7 +7,7 @@
 // query and db transition log-probabilities, the column -1 states of its
 // 32-row blocks, a local start term log 1 in the MM state) evaluated with
 // true exponentials and logarithms (the hardware base-2 forms, relative
-// error ~1e-7 at these arguments, all log values kept in base 2; the reference's MAP stage uses coarse
+// error ~1e-7 at these arguments; the reference's MAP stage uses coarse
 // approximations instead) over the score matrix
 //     S = s0 + wss * ss + wcv * cv
 // (amino-acid score, and the SS and context-vector terms before their
@@ -48,23 +48,23 @@
 namespace c2 {
 
 #define FULL 0xffffffffu
-// Every log value inside the sweeps is in base 2 (scores, transitions, states,
-// rows): a term of a sum then costs one ex2.approx and a sum one lg2.approx,
-// without the two multiplications that convert e^x and ln x.  (Denormal results
-// and arguments are flushed: the terms they drop are below 2^-126 of the largest
-// term of a sum.)
-constexpr float XLOG2E = 1.4426950408889634f, XLN2 = 0.6931471805599453f;
-constexpr float XLOG0 = -99.f * XLOG2E;   // the MAP model's log 0
+constexpr float XLOG0 = -99.f;   // the MAP model's log 0
 
 struct X5 { float MM, MI, IM, DN, ND; };
 
+// e^x through the hardware base-2 form (denormal results and arguments flushed:
+// the terms they drop are below e^-87 of the largest term of a sum); log2 x, whose
+// factor ln 2 goes into the addition of the maximum.  (States kept in base 2
+// need neither factor, but are 1.44 times as large: the same time, and gradients
+// up to 1.2 times as far from the 64-bit ones.)
+constexpr float XLOG2E = 1.4426950408889634f, XLN2 = 0.6931471805599453f;
 __device__ __forceinline__ float xexp(float x)
 {
     float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * XLOG2E));
     return y;
 }
-__device__ __forceinline__ float xlog(float x)
+__device__ __forceinline__ float xlog2(float x)
 {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -76,19 +76,19 @@ __device__ __forceinline__ float xlog(float x)
 __device__ __forceinline__ float xlse2(float a, float b)
 {
     const float m = fmaxf(a, b);
-    return xlog(1.f + xexp(-fabsf(a - b))) + m;
+    return fmaf(xlog2(1.f + xexp(-fabsf(a - b))), XLN2, m);
 }
 
-// log(2^v1 + ... + 2^v5 + 1): the 1 is the local start (forward) or end (backward)
+// log(e^v1 + ... + e^v5 + 1): the 1 is the local start (forward) or end (backward)
 __device__ __forceinline__ float xlse5p1(float v1, float v2, float v3, float v4, float v5)
 {
     float m = fmaxf(fmaxf(fmaxf(v1, v2), fmaxf(v3, v4)), fmaxf(v5, 0.f));
-    return xlog(((xexp(v1 - m) + xexp(v2 - m)) + (xexp(v3 - m) + xexp(v4 - m))) + (xexp(v5 - m) + xexp(-m))) + m;
+    return fmaf(xlog2(((xexp(v1 - m) + xexp(v2 - m)) + (xexp(v3 - m) + xexp(v4 - m))) + (xexp(v5 - m) + xexp(-m))), XLN2, m);
 }
 
 // transitions of position i of a profile whose raw rows start at t0: the
 // forward recursion's (MM MD IM DM DD into i, MI II out of i) and the
-// backward's (all out of i), in base 2; log 0 outside [0, len)
+// backward's (all out of i); log 0 outside [0, len)
 __device__ __forceinline__ void xtrn_fwd(const float* __restrict__ t0, int i, int len, float* t7)
 {
     if (i < 0 || i >= len) {
@@ -98,7 +98,6 @@ __device__ __forceinline__ void xtrn_fwd(const float* __restrict__ t0, int i, in
     const float* a = t0 + (long long)i * 7;
     t7[TMM] = a[0]; t7[TMI] = a[7 + 1]; t7[TMD] = a[2];
     t7[TIM] = a[3]; t7[TII] = a[7 + 4]; t7[TDM] = a[5]; t7[TDD] = a[6];
-    for (int k = 0; k < 7; k++) t7[k] *= XLOG2E;
 }
 
 __device__ __forceinline__ void xtrn_bwd(const float* __restrict__ t0, int i, int len, float* t7)
@@ -108,7 +107,7 @@ __device__ __forceinline__ void xtrn_bwd(const float* __restrict__ t0, int i, in
         return;
     }
     const float* b = t0 + (long long)(i + 1) * 7;
-    for (int k = 0; k < 7; k++) t7[k] = b[k] * XLOG2E;
+    for (int k = 0; k < 7; k++) t7[k] = b[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -211,7 +210,7 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32) adj_score_kernel(AdjArgs a)
                 }
                 const long long c = cb + (long long)k * 32 + lane;
                 const float p0 = s0, pss = ss, pcv = cvm;
-                a.S[c] = (p0 + a.wss * pss + a.wcv * pcv) * XLOG2E;
+                a.S[c] = (p0 + a.wss * pss + a.wcv * pcv);
                 a.pss[c] = pss;
                 a.pcv[c] = pcv;
             }
@@ -285,7 +284,7 @@ __device__ __forceinline__ void adj_load_row(const AdjArgs& a, float* rab, const
     __syncwarp();
 }
 
-// Transition rows of a pair's db profile, in base 2 (rows 0..L; row r holds the
+// Transition rows of a pair's db profile (rows 0..L; row r holds the
 // transitions into position r, MI and II of row r + 1 those out of position
 // r) in the warp's shared ring trs[128][TRS] by sequence index q: q = row in the
 // forward sweep, q = L - row in the mirrored backward sweep.  A step's lanes
@@ -301,7 +300,7 @@ __device__ __forceinline__ void adj_stage_trn(float* trs, const float* __restric
     for (int e = lane; e < nq * 7; e += 32) {
         const int q = q0 + e / 7, f = e % 7;
         const int row = MIRROR ? L - q : q;
-        trs[(q & 127) * TRS + f] = __ldg(dt0 + (long long)row * 7 + f) * XLOG2E;
+        trs[(q & 127) * TRS + f] = __ldg(dt0 + (long long)row * 7 + f);
     }
 }
 
@@ -370,10 +369,10 @@ __device__ __forceinline__ void adj_fwd_strip(const AdjArgs& a, int m, int s, in
     float q7[7];
     xtrn_fwd(a.qtrn + (a.qpos[m] + a.qidx[m]) * 7, r, Lq, q7);
 #pragma unroll
-    for (int k = 0; k < 7; k++) q7[k] += a.theta[k] * XLOG2E;
+    for (int k = 0; k < 7; k++) q7[k] += a.theta[k];
     const float* cf = a.qcfx + (a.qpos[m] + (act ? r : 0)) * 6;
-    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0] * XLOG2E, cf[1] * XLOG2E, cf[2] * XLOG2E, XLOG0};
-    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3] * XLOG2E, cf[4] * XLOG2E, cf[5] * XLOG2E, XLOG0};
+    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0], cf[1], cf[2], XLOG0};
+    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3], cf[4], cf[5], XLOG0};
     const bool wr_row = !RECOMP && lane == 31 && s + 1 < ns;
     X5 mine = INIT, upp = INIT;
     // the lane's score of the next step, loaded a step ahead
@@ -477,8 +476,9 @@ __global__ void adj_logz_kernel(AdjArgs a)
         zs = (mx == -INFINITY) ? 0.f : zs * xexp(zm - mx) + os * xexp(om - mx);
         zm = mx;
     }
-    a.logz[m] = logf(zs) + zm * XLN2;
-    a.zpart[2 * a.soff[m]] = log2f(zs) + zm;   // base 2, for the backward sweep (its error scales every posterior: not xlog)
+    const float lz = logf(zs) + zm;
+    a.logz[m] = lz;
+    a.zpart[2 * a.soff[m]] = lz;   // for the backward sweep
 }
 
 // ---------------------------------------------------------------------------
@@ -556,7 +556,7 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     const int p = a.prof[m];
     const int L = a.plen[p], Lq = a.pLq[m], ns = (Lq + 31) >> 5;
     const long long cb = a.off[m] + (long long)s * (L + 31) * 32;
-    const float lz = a.zpart[2 * a.soff[m]];   // log2 Z
+    const float lz = a.zpart[2 * a.soff[m]];   // log Z
     const float* dt0 = a.dtrn + (a.poff[p] + p) * 7;
     const bool has_below = s + 1 < ns;
     const int ldr = row_ld(L);
@@ -573,11 +573,11 @@ __device__ __forceinline__ void adj_bwd_strip(const AdjArgs& a, int m, int s, in
     xtrn_bwd(qt0, i, Lq, qb);
     xtrn_fwd(qt0, i, Lq, qf);
 #pragma unroll
-    for (int k = 0; k < 7; k++) { qb[k] += a.theta[k] * XLOG2E; qf[k] += a.theta[k] * XLOG2E; }
+    for (int k = 0; k < 7; k++) { qb[k] += a.theta[k]; qf[k] += a.theta[k]; }
     // column -1 states of row i (the forward's left and diagonal at column 0)
     const float* cf = a.qcfx + (a.qpos[m] + (act ? i : 0)) * 6;
-    const X5 LB = (lf == 31) ? INIT : X5{0.f, cf[0] * XLOG2E, cf[1] * XLOG2E, cf[2] * XLOG2E, XLOG0};
-    const X5 DB = (lf == 31 || lf == 0) ? INIT : X5{0.f, cf[3] * XLOG2E, cf[4] * XLOG2E, cf[5] * XLOG2E, XLOG0};
+    const X5 LB = (lf == 31) ? INIT : X5{0.f, cf[0], cf[1], cf[2], XLOG0};
+    const X5 DB = (lf == 31 || lf == 0) ? INIT : X5{0.f, cf[3], cf[4], cf[5], XLOG0};
     const bool wr_row = (t == 31) && s > 0;
     float g[9];
 #pragma unroll
@@ -792,10 +792,10 @@ __global__ void __launch_bounds__(POST_WARPS * 32) adj_post_kernel(AdjArgs a)
     float qf[7];
     xtrn_fwd(a.qtrn + (a.qpos[m] + a.qidx[m]) * 7, i, Lq, qf);
 #pragma unroll
-    for (int k = 0; k < 7; k++) qf[k] += a.theta[k] * XLOG2E;
+    for (int k = 0; k < 7; k++) qf[k] += a.theta[k];
     const float* cf = a.qcfx + (a.qpos[m] + (act ? i : 0)) * 6;
-    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0] * XLOG2E, cf[1] * XLOG2E, cf[2] * XLOG2E, XLOG0};
-    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3] * XLOG2E, cf[4] * XLOG2E, cf[5] * XLOG2E, XLOG0};
+    const X5 LB = (lane == 31) ? INIT : X5{0.f, cf[0], cf[1], cf[2], XLOG0};
+    const X5 DB = (lane == 31 || lane == 0) ? INIT : X5{0.f, cf[3], cf[4], cf[5], XLOG0};
     const int nl = L + 31, run = post_run(nl);
     const int k0 = wid * run, k1 = min(nl, k0 + run);
     float g[9];
@@ -809,11 +809,11 @@ __global__ void __launch_bounds__(POST_WARPS * 32) adj_post_kernel(AdjArgs a)
         X5 up = shfl_up5(left);
         if (lane == 0) up = row_above(k1 - 1);
         for (int ke = k1; ke > k0; ke -= 32) {
-            // transition rows ke - 63 .. ke of the next 32 lines, in base 2 (row r at r & 63)
+            // transition rows ke - 63 .. ke of the next 32 lines (row r at r & 63)
             __syncwarp();
             for (int e = lane; e < 64 * 7; e += 32) {
                 const int row = ke - 63 + e / 7, f = e % 7;
-                if (row >= 0 && row <= L) trs[(row & 63) * TRS + f] = __ldg(dt0 + (long long)row * 7 + f) * XLOG2E;
+                if (row >= 0 && row <= L) trs[(row & 63) * TRS + f] = __ldg(dt0 + (long long)row * 7 + f);
             }
             __syncwarp();
 #pragma unroll 2

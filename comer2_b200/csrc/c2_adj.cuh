@@ -40,14 +40,14 @@ struct AdjArgs {
     const float* qcfx;      // [rows][6] exact column -1 states: MI IM DN of row r, of row r - 1
     float theta[7];
     float wss, wcv;
-    float* S;               // [cells] score (s0 + wss ss + wcv cv) log2 e
+    float* S;               // [cells] score s0 + wss ss + wcv cv
     float* pss;             // [cells] SS term before its weight
     float* pcv;             // [cells] CV term before its weight
     float* gS;              // [cells] dlogZ/dS
     float* post;            // [cells] MM state posterior
     float* frow;            // forward checkpoint rows, row 32 s + 31 of strip s (layout of the row hand-off)
     float* brow;            // outside values of row 32 s by mirrored column, the same layout
-    float* zpart;           // [nitems][2] (max, scaled sum) of a strip's 2^F.MM; then log2 Z at a pair's first
+    float* zpart;           // [nitems][2] (max, scaled sum) of a strip's e^F.MM; then log Z at a pair's first
     float* gpart;           // [nitems][9] a strip's gradient sums
     float* Fall;            // forward states of every strip, when they fit (else null): strip s of
                             // pair m at Fall + 5 off[m] + s (L + 31) 160 (fw_st5)
