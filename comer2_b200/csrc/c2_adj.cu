@@ -25,7 +25,7 @@
 // order of their dependencies (all pairs' strip 0, then strip 1, ...; the
 // backward sweep from the last strip up), so a pair is swept by up to
 // nstrips warps at once, each trailing the strip it depends on by about 40
-// columns (bounded waits on published progress, as the phase-2 sweeps).
+// columns (row hand-off with bounded waits, c2_device.cuh).
 // Memory: the forward sweep keeps the last row of every strip (5 states x L
 // per strip, the rows the next strip reads) and each strip's partial log-sum,
 // and, when they fit (20 bytes a cell), every forward state.  The backward

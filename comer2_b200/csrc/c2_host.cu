@@ -295,7 +295,7 @@ struct c2_handle {
     DevBuf<long long> d_cand_off;
     DevBuf<signed char> d_btck;
     DevBuf<float> d_smat, d_mmat;
-    // strip pipeline of the phase-2 sweeps: last-row buffers, progress words
+    // strip pipeline of the phase-2 sweeps: last-row buffers
     DevBuf<float> d_bnd;
     DevBuf<unsigned long long> d_tbkey;
     // tensor-core query operands
@@ -620,13 +620,12 @@ static inline void trn_of(const c2_profiles* d, int k, int i, float* t7)
 
 // Dispatch lag of the sweeps' work-item order, in wavefront steps: strip s of
 // a pair is handed out about `lag` steps' worth of work after strip s - 1.
-// The physical lag is about 96 steps for the traceback sweep (the row above
-// is loaded a 32-column chunk ahead and published once per chunk) and about
-// 48 for the MAP sweeps (8 columns at a time); handing strips out later than
-// that leaves fewer warps polling for their predecessor, and the values below
-// were chosen by measurement (kernel times on configs 1 and 4 with lags of
-// 64 / 96 / 128 / 160-192 / 256-320: traceback sweep 21.4 -> 16.3 ms, MAP DP
-// 22.4 -> 17.5-18.0 ms and MAP forward-backward 74.4 -> 72.3 ms on config 4).
+// The physical lag is about 50 steps (the row above is taken 16 columns at a
+// time by the traceback sweep, 8 by the MAP sweeps); handing strips out later
+// than that leaves fewer warps polling for their predecessor.  With the rows as
+// their own flags the values hardly matter (48 to 640: within the runs'
+// differences on 1 x 3,000 vs 4,000 profiles); with progress words 64 -> 320 took
+// the traceback sweep 21.4 -> 16.3 ms on 1 x 3,000 vs 50,000.
 constexpr int STRIP_LAG_TB = 320, STRIP_LAG_MAP = 192;
 
 // Work-item table of a strip-pipelined sweep over np pairs (in processing

@@ -540,7 +540,7 @@ __device__ __forceinline__ int corner_b(int r, int L, int edge) { return (r < ed
 // the rows between the strips in the warp's own boundary buffer -- except the
 // nsplit longest pairs, whose strips are items of their own (any warp may take
 // them): those hand the rows on through per-pair buffers with published
-// progress, as the phase-2 sweeps do (c2_device.cuh).  Without that a search
+// progress (pipe_wait, c2_device.cuh).  Without that a search
 // with few pairs, or with pairs much longer than the mean, ends in a tail where
 // a few warps walk all strips of a long pair alone: 1 x 1,237 against 4,999
 // profiles took 16.3 ms, the time of its longest pair (39 strips x 2,031 steps).
