@@ -197,7 +197,7 @@ private:
 };
 
 // A handle's slot (or pageable memory of that size).  Space is taken in order and
-// free again once the handle's stream has been synchronised.
+// free again once the handle's stream has been synchronised (sync_stream).
 struct HostStage {
     char* p = nullptr;
     size_t used = 0;
@@ -357,18 +357,44 @@ static c2_status fail(c2_handle* h, c2_status st, const char* fmt, ...)
                         __FILE__, __LINE__);                                            \
     } while (0)
 
-// host -> device; src may be reused at once.  What fits goes through the handle's
-// staging memory; a larger copy straight from pageable memory, which the driver
-// takes over before the call returns.
-static cudaError_t h2d(c2_handle* h, void* dst, const void* src, size_t bytes)
+// wait for the handle's stream, after which all of its staging memory is free
+static cudaError_t sync_stream(c2_handle* h)
 {
-    if (bytes == 0) return cudaSuccess;
-    if (char* p = h->stage.take(bytes)) {
-        memcpy(p, src, bytes);
-        src = p;
-    }
-    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
+    h->stage.used = 0;
+    return e;
 }
+
+// host -> device.  What fits goes through the handle's staging memory and needs
+// no wait; where it does not, the copy reads the source itself, asynchronously if
+// that is page-locked (a caller's array may be), and the stream is waited for
+// before the source may change: by finish(), or when the Upload goes out of scope,
+// so declare it after the arrays it copies from.
+struct Upload {
+    c2_handle* h;
+    bool direct = false;
+    explicit Upload(c2_handle* hh) : h(hh) {}
+    Upload(const Upload&) = delete;
+    Upload& operator=(const Upload&) = delete;
+    ~Upload() { (void)finish(); }
+    cudaError_t put(void* dst, const void* src, size_t bytes)
+    {
+        if (bytes == 0) return cudaSuccess;
+        if (char* p = h->stage.take(bytes)) {
+            memcpy(p, src, bytes);
+            src = p;
+        } else {
+            direct = true;
+        }
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
+    }
+    cudaError_t finish()
+    {
+        if (!direct) return cudaSuccess;
+        direct = false;
+        return sync_stream(h);
+    }
+};
 
 // device -> host: several arrays with one synchronisation.  get() queues a copy
 // (straight to its destination where it is larger than the stage), finish()
@@ -393,11 +419,10 @@ struct Fetch {
     }
     cudaError_t finish()
     {
-        const cudaError_t e = cudaStreamSynchronize(h->stream);
+        const cudaError_t e = sync_stream(h);
         if (e == cudaSuccess)
             for (const Part& q : parts) memcpy(q.dst, q.p, q.n);
         parts.clear();
-        h->stage.used = 0;
         return e;
     }
 };
@@ -1018,8 +1043,9 @@ static void ss_row_table(const c2_handle* h, const float* s3, float* U)
 // its records: context vectors (k = 19: 1, the 1/kappa0 column) and SS row
 // tables (k = 30: P(H) + 0.1, k = 31: 1) as split BF16 A fragments, amino-acid
 // rows unscaled in fragment order.  Packed when the query is set in the
-// tensor-core score mode, or by the first phase 1 after a change to it.
-static c2_status pack_query_operands(c2_handle* h)
+// tensor-core score mode, or by the first phase 1 after a change to it.  The
+// arrays they are packed in are the caller's, declared before its Upload.
+static c2_status pack_query_operands(c2_handle* h, std::vector<uint32_t>& qa, std::vector<float>& qaa, Upload& up)
 {
     const int Lq = h->Lq, card = h->sc.ssss_card;
     const int nt = (Lq + P1_ROWS - 1) / P1_ROWS;
@@ -1042,8 +1068,8 @@ static c2_status pack_query_operands(c2_handle* h)
             pl[k] = (uint16_t)bf16_rn_bits(x[k] - bf16_to_f(b));
         }
     }
-    std::vector<uint32_t> qa((size_t)nt * TC_QA_WORDS, 0u);
-    std::vector<float> qaa((size_t)nt * TC_QAA_FLOATS, 0.f);
+    qa.assign((size_t)nt * TC_QA_WORDS, 0u);
+    qaa.assign((size_t)nt * TC_QAA_FLOATS, 0.f);
     for (int s = 0; s < nt; s++)
         for (int mt = 0; mt < 4; mt++)
             for (int lane = 0; lane < 32; lane++) {
@@ -1071,8 +1097,8 @@ static c2_status pack_query_operands(c2_handle* h)
             }
     if (h->d_qa.ensure(qa.size(), h->budget) || h->d_qaaf.ensure(qaa.size(), h->budget))
         return fail(h, C2_ERR_NOMEM, "query operand allocation failed");
-    CK(h2d(h, h->d_qa.p, qa.data(), qa.size() * 4));
-    CK(h2d(h, h->d_qaaf.p, qaa.data(), qaa.size() * 4));
+    CK(up.put(h->d_qa.p, qa.data(), qa.size() * 4));
+    CK(up.put(h->d_qaaf.p, qaa.data(), qaa.size() * 4));
     h->qtc_ready = true;
     return C2_OK;
 }
@@ -1119,26 +1145,29 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
     }
     if (h->d_qrec.ensure(h->h_qrec.size(), h->budget) || h->d_qbkg.ensure(NAA, h->budget))
         return fail(h, C2_ERR_NOMEM, "query allocation failed");
+    std::vector<float> qU, qcf, qaa;   // (before the Upload that reads them)
+    std::vector<uint32_t> qa;
+    Upload up(h);
     // the SS row tables per strip of 32 rows, [strip][MAX_SSSS_CARD][32] (lane =
     // row), for the FP32 kernels
     {
         const int ns = (Lq + 31) / 32, card = h->sc.ssss_card;
-        std::vector<float> qU((size_t)ns * MAX_SSSS_CARD * 32, 0.f);
+        qU.assign((size_t)ns * MAX_SSSS_CARD * 32, 0.f);
         for (int r = 0; r < Lq; r++) {
             float U[MAX_SSSS_CARD];
             ss_row_table(h, q->ss + (size_t)r * NSS, U);
             for (int c = 0; c < card; c++) qU[((size_t)(r / 32) * MAX_SSSS_CARD + c) * 32 + (r % 32)] = U[c];
         }
         if (h->d_qU.ensure(qU.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "query SS table allocation failed");
-        CK(h2d(h, h->d_qU.p, qU.data(), qU.size() * 4));
+        CK(up.put(h->d_qU.p, qU.data(), qU.size() * 4));
     }
-    if (h->score_mode == C2_SCORE_BF16_TC && (st = pack_query_operands(h)) != C2_OK) return st;
-    CK(h2d(h, h->d_qrec.p, h->h_qrec.data(), h->h_qrec.size() * 4));
-    CK(h2d(h, h->d_qbkg.p, q->bkg, NAA * 4));
+    if (h->score_mode == C2_SCORE_BF16_TC && (st = pack_query_operands(h, qa, qaa, up)) != C2_OK) return st;
+    CK(up.put(h->d_qrec.p, h->h_qrec.data(), h->h_qrec.size() * 4));
+    CK(up.put(h->d_qbkg.p, q->bkg, NAA * 4));
     // MAP forward: column -1 states of the query rows (log-sum-exp form of the
     // Viterbi boundary; src/libmycu/cumapdp/CuBatchMAPDP_fwd.cu:72-478)
     {
-        std::vector<float> qcf((size_t)Lq * 6, 0.f);
+        qcf.assign((size_t)Lq * 6, 0.f);
         float pMI = 0.f, pIM = 0.f, pDN = 0.f;
         for (int r = 0; r < Lq; r++) {
             float t[7];
@@ -1159,13 +1188,14 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
         if (h->d_qcf.ensure(qcf.size(), h->budget) || h->d_qtrn.ensure((size_t)(Lq + 1) * 7, h->budget) || h->d_qaa.ensure(Lq, h->budget) ||
             h->d_qss.ensure(Lq, h->budget))
             return fail(h, C2_ERR_NOMEM, "query side arrays allocation failed");
-        CK(h2d(h, h->d_qcf.p, qcf.data(), qcf.size() * 4));
+        CK(up.put(h->d_qcf.p, qcf.data(), qcf.size() * 4));
         h->adj_fwd_done = false;
-        CK(h2d(h, h->d_qtrn.p, q->trn, (size_t)(Lq + 1) * 7 * 4));
-        CK(h2d(h, h->d_qaa.p, q->aa, (size_t)Lq));
-        if (q->ssstate) CK(h2d(h, h->d_qss.p, q->ssstate, (size_t)Lq));
+        CK(up.put(h->d_qtrn.p, q->trn, (size_t)(Lq + 1) * 7 * 4));
+        CK(up.put(h->d_qaa.p, q->aa, (size_t)Lq));
+        if (q->ssstate) CK(up.put(h->d_qss.p, q->ssstate, (size_t)Lq));
         else CK(cudaMemsetAsync(h->d_qss.p, ' ', (size_t)Lq, h->stream));
     }
+    CK(up.finish());
     query_limits(h, Lq, &h->searchspace, &h->deltalen, &h->scorethld, &h->logevthld);
     return C2_OK;
 }
@@ -1337,8 +1367,14 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     CK(cudaMemsetAsync(h->d_counter.p, 0, sizeof(int), h->stream));
     if (h->score_mode == C2_SCORE_BF16_TC) {
         c2_status st = tc_prepare_db(h);
-        if (st == C2_OK && !h->qtc_ready) st = pack_query_operands(h);
         if (st != C2_OK) return st;
+        if (!h->qtc_ready) {
+            std::vector<uint32_t> qa;
+            std::vector<float> qaa;
+            Upload up(h);
+            if ((st = pack_query_operands(h, qa, qaa, up)) != C2_OK) return st;
+            CK(up.finish());
+        }
         a.tcdb = h->db->d_tcdb.p;
         a.ttile = h->db->d_ttile.p;
         a.cold = h->db->d_cold.p;
@@ -1369,7 +1405,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
 extern "C" c2_status c2_set_stream(c2_handle* h, void* stream)
 {
     if (!h) return C2_ERR_ARG;
-    CK(cudaStreamSynchronize(h->stream));
+    CK(sync_stream(h));
     h->stream = stream ? (cudaStream_t)stream : h->own_stream;
     return C2_OK;
 }
@@ -1449,7 +1485,7 @@ extern "C" c2_status c2_set_wait_limit(c2_handle* h, uint32_t polls)
 extern "C" c2_status c2_sync(c2_handle* h)
 {
     if (!h) return C2_ERR_ARG;
-    CK(cudaStreamSynchronize(h->stream));
+    CK(sync_stream(h));
     return C2_OK;
 }
 
@@ -1514,22 +1550,24 @@ static c2_status finalize_set(c2_handle* h, const std::vector<int>& cand, int32_
         h->d_fpassed.ensure(nc, h->budget) || h->d_fbeg.ensure(nc, h->budget) || h->d_fend.ensure(nc, h->budget) ||
         h->d_bnd.ensure(2 * bnd_half, h->budget) || h->d_tbkey.ensure(nc, h->budget))
         return fail(h, C2_ERR_NOMEM, "finalisation scratch for %d pairs (%lld cells) failed", nc, acc);
-    CK(h2d(h, h->d_cand_prof.p, h->h_cand.data(), (size_t)nc * 4));
-    CK(h2d(h, h->d_cand_off.p, h->h_cand_off.data(), (size_t)nc * 8));
+    std::vector<int> wo(nc), items;
+    Upload up(h);
+    CK(up.put(h->d_cand_prof.p, h->h_cand.data(), (size_t)nc * 4));
+    CK(up.put(h->d_cand_off.p, h->h_cand_off.data(), (size_t)nc * 8));
     // traceback sweep order: longest candidates first
     {
-        std::vector<int> wo(nc);
         std::iota(wo.begin(), wo.end(), 0);
         std::stable_sort(wo.begin(), wo.end(),
                          [&](int x, int y) { return h->h_plen[h->h_cand[x]] > h->h_plen[h->h_cand[y]]; });
-        std::vector<int> lens(nc), items;
+        std::vector<int> lens(nc);
         for (int i = 0; i < nc; i++) lens[i] = h->h_plen[h->h_cand[wo[i]]];
         strip_items(lens, (h->Lq + 31) / 32, h->nsm * P1TC_WARPS, STRIP_LAG_TB, items);
         if (h->d_worder.ensure(nc, h->budget) || h->d_tbitems.ensure(items.size(), h->budget))
             return fail(h, C2_ERR_NOMEM, "candidate order allocation failed");
-        CK(h2d(h, h->d_worder.p, wo.data(), (size_t)nc * 4));
-        CK(h2d(h, h->d_tbitems.p, items.data(), items.size() * 4));
+        CK(up.put(h->d_worder.p, wo.data(), (size_t)nc * 4));
+        CK(up.put(h->d_tbitems.p, items.data(), items.size() * 4));
     }
+    CK(up.finish());
     P1Args a;
     fill_p1(h, a);
     a.nwork = nc;
@@ -1685,7 +1723,9 @@ extern "C" c2_status c2_run_stats(c2_handle* h, int32_t* npassed)
     if (h->d_p2.ensure(h->npass, h->budget) || h->d_stats.ensure((size_t)h->npass * STATS_NOUT, h->budget) ||
         h->d_hist.ensure((size_t)h->npass * STATS_NBINS, h->budget))
         return fail(h, C2_ERR_NOMEM, "statistics buffers for %d pairs failed", h->npass);
-    CK(h2d(h, h->d_p2.p, h->h_p2.data(), (size_t)h->npass * 4));
+    Upload up(h);
+    CK(up.put(h->d_p2.p, h->h_p2.data(), (size_t)h->npass * 4));
+    CK(up.finish());
     StatsArgs a;
     memset(&a, 0, sizeof a);
     a.Lq = h->Lq;
@@ -1745,9 +1785,11 @@ static c2_status viterbi_alignments(c2_handle* h)
         memcpy(&bits, &sc, 4);
         key[m] = ((unsigned long long)bits << 32) | (unsigned long long)(0xffffffffu - cell);
     }
-    CK(cudaMemcpyAsync(h->d_pairk.p, key.data(), (size_t)nm * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_mapcand.p, h->h_mapcand.data(), (size_t)nm * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_mappass.p, h->h_mappass.data(), (size_t)nm * 4, cudaMemcpyHostToDevice, h->stream));
+    Upload up(h);
+    CK(up.put(h->d_pairk.p, key.data(), (size_t)nm * 8));
+    CK(up.put(h->d_mapcand.p, h->h_mapcand.data(), (size_t)nm * 4));
+    CK(up.put(h->d_mappass.p, h->h_mappass.data(), (size_t)nm * 4));
+    CK(up.finish());
     MapArgs a;
     memset(&a, 0, sizeof a);
     a.Lq = h->Lq;
@@ -1825,15 +1867,18 @@ extern "C" c2_status c2_run_map(c2_handle* h, int32_t* nhits)
         h->d_pairc.ensure(nm, h->budget) || h->d_alninfo.ensure((size_t)nm * 8, h->budget) || h->d_aln.ensure((size_t)nm * 5 * h->alnstride, h->budget) ||
         h->d_pairk.ensure(nm, h->budget))
         return fail(h, C2_ERR_NOMEM, "MAP buffers for %d pairs failed", nm);
+    std::vector<int> items;
+    Upload up(h);
     {
-        std::vector<int> lens(nm), items;
+        std::vector<int> lens(nm);
         for (int i = 0; i < nm; i++) lens[i] = h->h_plen[h->h_cand[h->h_mapcand[i]]];
         strip_items(lens, (h->Lq + 31) / 32, h->grid * P1_WARPS, STRIP_LAG_MAP, items);
         if (h->d_mapitems.ensure(items.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "MAP work table allocation failed");
-        CK(h2d(h, h->d_mapitems.p, items.data(), items.size() * 4));
+        CK(up.put(h->d_mapitems.p, items.data(), items.size() * 4));
     }
-    CK(h2d(h, h->d_mapcand.p, h->h_mapcand.data(), (size_t)nm * 4));
-    CK(h2d(h, h->d_mappass.p, h->h_mappass.data(), (size_t)nm * 4));
+    CK(up.put(h->d_mapcand.p, h->h_mapcand.data(), (size_t)nm * 4));
+    CK(up.put(h->d_mappass.p, h->h_mappass.data(), (size_t)nm * 4));
+    CK(up.finish());
     MapArgs a;
     memset(&a, 0, sizeof a);
     a.Lq = h->Lq;
@@ -1918,7 +1963,9 @@ static c2_status hits_direct(c2_handle* h, c2_hit* hits, int32_t n, char* alns, 
     if (nm > 0) {
         if (h->d_alnoff.ensure((size_t)nm, h->budget) || h->d_alnpack.ensure(need, h->budget))
             return fail(h, C2_ERR_NOMEM, "alignment packing buffers failed");
-        CK(h2d(h, h->d_alnoff.p, off.data(), (size_t)nm * 8));
+        Upload up(h);
+        CK(up.put(h->d_alnoff.p, off.data(), (size_t)nm * 8));
+        CK(up.finish());
         CK(launch_aln_pack(h->d_aln.p, h->alnstride, h->d_alninfo.p, h->d_alnoff.p, nm, h->d_alnpack.p, h->stream));
         h->launches++;
         Fetch F(h);
@@ -2381,14 +2428,16 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
         if (h->adj_bgrid == 0)
             return fail(h, C2_ERR_NOMEM, "logz_fwd: backward sweep scratch (%zu bytes per CTA) failed", per_cta);
     }
-    CK(h2d(h, h->d_adjprof.p, profiles, (size_t)npairs * 4));
-    CK(h2d(h, h->d_adjLq.p, Lq, (size_t)npairs * 4));
-    CK(h2d(h, h->d_adjqpos.p, qpos, (size_t)npairs * 8));
-    CK(h2d(h, h->d_adjqidx.p, qidx, (size_t)npairs * 4));
-    CK(h2d(h, h->d_adjsoff.p, soff.data(), (size_t)npairs * 8));
-    CK(h2d(h, h->d_adjitems.p, it.data(), it.size() * sizeof(int2)));
-    CK(h2d(h, h->d_adjoff.p, h->adj_off.data(), (size_t)npairs * 8));
-    CK(h2d(h, h->d_adjroff.p, h->adj_roff.data(), (size_t)npairs * 8));
+    Upload up(h);
+    CK(up.put(h->d_adjprof.p, profiles, (size_t)npairs * 4));
+    CK(up.put(h->d_adjLq.p, Lq, (size_t)npairs * 4));
+    CK(up.put(h->d_adjqpos.p, qpos, (size_t)npairs * 8));
+    CK(up.put(h->d_adjqidx.p, qidx, (size_t)npairs * 4));
+    CK(up.put(h->d_adjsoff.p, soff.data(), (size_t)npairs * 8));
+    CK(up.put(h->d_adjitems.p, it.data(), it.size() * sizeof(int2)));
+    CK(up.put(h->d_adjoff.p, h->adj_off.data(), (size_t)npairs * 8));
+    CK(up.put(h->d_adjroff.p, h->adj_roff.data(), (size_t)npairs * 8));
+    CK(up.finish());
     CK(cudaMemsetAsync(h->d_adjbuf.p + 5 * acc, 0xff, (size_t)racc * sizeof(float), h->stream));   // forward rows: empty
     CK(cudaMemsetAsync(h->d_adjctr.p, 0, 2 * sizeof(int), h->stream));
     CK(cudaMemsetAsync(h->d_status.p, 0, sizeof(int), h->stream));
@@ -2423,7 +2472,9 @@ extern "C" c2_status c2_logz_fwd(c2_handle* h, const int32_t* profiles, int32_t 
         std::vector<float> qx((size_t)len * 6, 0.f);
         colm1_exact(&v, qx.data());
         if (h->d_qcfx.ensure(qx.size(), h->budget)) return fail(h, C2_ERR_NOMEM, "query side arrays allocation failed");
-        CK(h2d(h, h->d_qcfx.p, qx.data(), qx.size() * 4));
+        Upload up(h);
+        CK(up.put(h->d_qcfx.p, qx.data(), qx.size() * 4));
+        CK(up.finish());
         h->qcfx_ready = true;
     }
     const std::vector<int> Lq(npairs, h->Lq), qidx(npairs, 0);
@@ -2445,8 +2496,9 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
     if (h->d_adjqrec.ensure((size_t)N * QR_STRIDE, h->budget) || h->d_adjqcfx.ensure((size_t)N * 6, h->budget) ||
         h->d_adjqtrn.ensure((size_t)(N + nq) * 7, h->budget) || h->d_adjqbkg.ensure((size_t)nq * NAA, h->budget))
         return fail(h, C2_ERR_NOMEM, "set_query_batch: query arrays for %d queries failed", nq);
-    CK(h2d(h, h->d_adjqtrn.p, queries->trn, (size_t)(N + nq) * 7 * 4));
-    CK(h2d(h, h->d_adjqbkg.p, queries->bkg, (size_t)nq * NAA * 4));
+    Upload up(h);
+    CK(up.put(h->d_adjqtrn.p, queries->trn, (size_t)(N + nq) * 7 * 4));
+    CK(up.put(h->d_adjqbkg.p, queries->bkg, (size_t)nq * NAA * 4));
     // pieces of whole queries, packed by the host threads straight into pinned
     // memory, each copied while the next is packed.  (A query of 65,535 rows, the
     // longest, fits the block.)
@@ -2475,7 +2527,7 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
         while (q1 < nq && (q1 == q0 || (rows + queries->lengths[q1]) * ROW_BYTES <= PIN_BLOCK_MAX / 3))
             rows += queries->lengths[q1++];
         if (used + rows * ROW_BYTES > cap) {
-            const cudaError_t e = cudaStreamSynchronize(h->stream);
+            const cudaError_t e = sync_stream(h);
             if (e != cudaSuccess) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
             used = 0;
         }
@@ -2511,12 +2563,10 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
         if (e != cudaSuccess && rc == C2_OK) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
         q0 = q1;
     }
-    if (loan.p || !heap.empty()) {
-        // before the block goes back
-        const cudaError_t e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess && rc == C2_OK) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
-        h->stage.used = 0;
-    }
+    // before the block goes back, and the caller has its arrays again
+    if (loan.p || !heap.empty()) up.direct = true;
+    const cudaError_t e = up.finish();
+    if (e != cudaSuccess && rc == C2_OK) rc = fail(h, C2_ERR_CUDA, "set_query_batch: %s", cudaGetErrorString(e));
     if (rc != C2_OK) return rc;
     h->adj_qlen.assign(queries->lengths, queries->lengths + nq);
     h->adj_qstart.assign(queries->offsets, queries->offsets + nq);
@@ -2700,14 +2750,14 @@ extern "C" c2_status c2_search_batch(c2_handle* h, const c2_profiles* queries, i
             if (s == C2_OK) {
                 std::lock_guard<std::mutex> g(p1_mu);
                 s = c2_run_phase1(w);
-                if (s == C2_OK && cudaStreamSynchronize(w->stream) != cudaSuccess) s = C2_ERR_CUDA;
+                if (s == C2_OK && sync_stream(w) != cudaSuccess) s = C2_ERR_CUDA;
             }
             if (s == C2_OK) {
                 int32_t n = 0;
                 if (s == C2_OK) s = c2_run_finalize(w, &n);
                 if (s == C2_OK) s = c2_run_stats(w, &n);
                 if (s == C2_OK) s = c2_run_map(w, &nh);
-                if (s == C2_OK && cudaStreamSynchronize(w->stream) != cudaSuccess) s = C2_ERR_CUDA;
+                if (s == C2_OK && sync_stream(w) != cudaSuccess) s = C2_ERR_CUDA;
             }
             if (s == C2_OK) s = c2_get_hits(w, nullptr, 0, nullptr, &nb);
             if (s == C2_OK) {

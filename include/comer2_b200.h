@@ -150,7 +150,9 @@ c2_status c2_upload_db(c2_handle* h, const c2_profiles* db,
 /* Set the query profile (profile 0 of q); replaces SetQueryLen and the query
  * part of ProcessScoreMatrix (CuBatchProcessing.cuh:87-99).  Computes the
  * score threshold and log E threshold as JobDispatcher::CalculateScoreThreshold
- * (src/libmycu/cualn/JobDispatcher.cpp:809-860). */
+ * (src/libmycu/cualn/JobDispatcher.cpp:809-860).  The caller's arrays, page-
+ * locked ones too, are free to change once the call has returned (so with every
+ * call here that takes host arrays). */
 c2_status c2_set_query(c2_handle* h, const c2_profiles* q);
 
 /* Run phase 1 (fused score matrix + Viterbi DP max) of the current query over
