@@ -43,6 +43,7 @@ struct ScoreConsts {
     float lokappa0, pownu0, cterm;        // context-vector constants
     float cvkey_first, cvkey_last, cvval_first, cvval_last;
     int cvcard, cvshift, ssss_card;
+    int cvhi;                             // cvcard - 1 - cvshift: largest table index before its shift
 };
 
 constexpr int P1_WARPS = 8;               // warps per CTA of the DP kernels

@@ -570,6 +570,7 @@ extern "C" c2_status c2_create(int device, const c2_params* p, c2_handle** out)
     sc.cvval_last = h->cvvals.back();
     sc.cvcard = p->cvs2s_card;
     sc.cvshift = p->cvs2s_shift;
+    sc.cvhi = sc.cvcard - 1 - sc.cvshift;
     sc.ssss_card = p->ssss_card;
     c2_status st = C2_OK;
     do {
@@ -1233,7 +1234,7 @@ static TcConsts tc_consts(const ScoreConsts& sc)
     t.vfw = sc.cvval_first * sc.cvswgt;
     t.vlw = sc.cvval_last * sc.cvswgt;
     t.ilo = -sc.cvshift;
-    t.ihi = sc.cvcard - 1 - sc.cvshift;
+    t.ihi = sc.cvhi;
     // x <= 2 key_first gives index <= 0 and x >= 2 key_last index >= card - 1
     // when the keys sit at the table's ends: the clamp alone is exact then
     t.uniform = (sc.cvshift + (int)rintf(t.kf2) <= 0 && sc.cvshift + (int)rintf(t.kl2) >= sc.cvcard - 1) ? 1 : 0;

@@ -150,8 +150,10 @@ __device__ __forceinline__ void cell_scores(const RowOps* R, const float* __rest
         const float dt = (lo2(dot[e]) + hi2(dot[e])) + sc.lokappa0;
         const float det = R[e].cq * cd - dt * dt;
         const float cvs = sc.cterm + sc.pownu0 * (lg2_ftz(det) * C2_LN2) - R[e].pq - v10.x;
-        // clamp keeps the shared-memory read in bounds for any table/argument
-        const int ix = min(max(sc.cvshift + __float2int_rn(2.f * cvs), 0), sc.cvcard - 1);
+        // the clamp keeps the shared-memory read in bounds for any table and argument;
+        // from above before the shift is added, since the conversion saturates (a
+        // determinant of 0 makes the score +inf, and 2^31 - 1 + shift is negative)
+        const int ix = max(min(__float2int_rn(2.f * cvs), sc.cvhi) + sc.cvshift, 0);
         float cvm = cvtab[ix * CVREP + (lane & (CVREP - 1))];
         if (!CVUNIF) {
             cvm = (sc.cvkey_last <= cvs) ? sc.cvval_last : cvm;
