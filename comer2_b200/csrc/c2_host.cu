@@ -365,6 +365,16 @@ static cudaError_t sync_stream(c2_handle* h)
     return e;
 }
 
+// Is the handle's stream being captured into a graph?  (Then nothing may be
+// allocated or waited for, and nothing copied from host memory that is used again.)
+static bool capturing(const c2_handle* h)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+    return true;
+}
+
 // host -> device.  What fits goes through the handle's staging memory and needs
 // no wait; where it does not, the copy reads the source itself, asynchronously if
 // that is page-locked (a caller's array may be), and the stream is waited for
@@ -1044,8 +1054,8 @@ static void ss_row_table(const c2_handle* h, const float* s3, float* U)
 // its records: context vectors (k = 19: 1, the 1/kappa0 column) and SS row
 // tables (k = 30: P(H) + 0.1, k = 31: 1) as split BF16 A fragments, amino-acid
 // rows unscaled in fragment order.  Packed when the query is set in the
-// tensor-core score mode, or by the first phase 1 after a change to it.  The
-// arrays they are packed in are the caller's, declared before its Upload.
+// tensor-core score mode, or by a change to it.  The arrays they are packed in are
+// the caller's, declared before its Upload.
 static c2_status pack_query_operands(c2_handle* h, std::vector<uint32_t>& qa, std::vector<float>& qaa, Upload& up)
 {
     const int Lq = h->Lq, card = h->sc.ssss_card;
@@ -1279,6 +1289,17 @@ extern "C" c2_status c2_set_score_mode(c2_handle* h, int32_t mode)
         if (h->sc.cvcard > P1T_MAX_CVCARD)
             return fail(h, C2_ERR_ARG, "tensor-core score form holds CV maps of at most %d entries (this one: %d)",
                         P1T_MAX_CVCARD, h->sc.cvcard);
+        if (h->Lq > 0 && !h->qtc_ready) {
+            // the current query was set in the other mode
+            CK(cudaSetDevice(h->device));
+            if (capturing(h)) return fail(h, C2_ERR_CUDA, "set_score_mode: the handle's stream is in a stream capture");
+            std::vector<uint32_t> qa;
+            std::vector<float> qaa;
+            Upload up(h);
+            const c2_status st = pack_query_operands(h, qa, qaa, up);
+            if (st != C2_OK) return st;
+            CK(up.finish());
+        }
     }
     h->score_mode = mode;
     return C2_OK;
@@ -1330,7 +1351,8 @@ static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
 {
     const int P = h->nprof, ns = (h->Lq + P1_ROWS - 1) / P1_ROWS;
     a.nsplit = 0;
-    if (ns < 2) return 0;
+    // (a graph would outlive the scratch, and allocating it is not allowed there)
+    if (ns < 2 || capturing(h)) return 0;
     const double mean = ((double)h->npos + 31.0 * P) / std::max(1, nwarps);
     const std::vector<int>& sl = h->db->slen;   // longest first
     const bool even = P > nwarps && (double)sl[P - nwarps] + 31.0 <= SPLIT_EVEN * mean;
@@ -1369,13 +1391,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     if (h->score_mode == C2_SCORE_BF16_TC) {
         c2_status st = tc_prepare_db(h);
         if (st != C2_OK) return st;
-        if (!h->qtc_ready) {
-            std::vector<uint32_t> qa;
-            std::vector<float> qaa;
-            Upload up(h);
-            if ((st = pack_query_operands(h, qa, qaa, up)) != C2_OK) return st;
-            CK(up.finish());
-        }
+        if (!h->qtc_ready) return fail(h, C2_ERR_STATE, "run_phase1: the query's tensor-core operands are missing");
         a.tcdb = h->db->d_tcdb.p;
         a.ttile = h->db->d_ttile.p;
         a.cold = h->db->d_cold.p;

@@ -158,7 +158,9 @@ c2_status c2_set_query(c2_handle* h, const c2_profiles* q);
 /* Run phase 1 (fused score matrix + Viterbi DP max) of the current query over
  * the uploaded database on the device, asynchronously on the handle's stream;
  * results stay on the device.  Replaces ComputeScoreMatrixDevice +
- * PerformCompleteDynProgDevice's DP launches (CuBatchProcessing.cu:324-372). */
+ * PerformCompleteDynProgDevice's DP launches (CuBatchProcessing.cu:324-372).
+ * May be captured into a graph (in the BF16 mode after a first call for the
+ * database, which packs its operands); pairs are not split then. */
 c2_status c2_run_phase1(c2_handle* h);
 
 /* Wait for the handle's stream and copy phase-1 results, one per db profile. */
@@ -350,7 +352,8 @@ c2_status c2_launch_count(const c2_handle* h, uint64_t* n);
  * In BF16 mode the phase-1 maxima (c2_get_phase1) carry the BF16 rounding;
  * pairs within a 2e-3 relative margin of the score threshold are recomputed
  * in FP32 (traceback sweep), so the finalised scores, hits, E-values and
- * alignments are those of the FP32 mode.  Default: C2_SCORE_FP32. */
+ * alignments are those of the FP32 mode.  Default: C2_SCORE_FP32.  A query
+ * set in the other mode gets its tensor-core operands packed by the change. */
 #define C2_SCORE_FP32 0
 #define C2_SCORE_BF16_TC 1
 c2_status c2_set_score_mode(c2_handle* h, int32_t mode);
