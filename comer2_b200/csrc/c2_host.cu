@@ -1119,6 +1119,7 @@ extern "C" c2_status c2_set_query(c2_handle* h, const c2_profiles* q)
     if (!h) return C2_ERR_ARG;
     c2_status st = check_profiles(h, q);
     if (st != C2_OK) return st;
+    if (capturing(h)) return fail(h, C2_ERR_CUDA, "set_query: the handle's stream is in a stream capture");
     if (h->nprof <= 0) return fail(h, C2_ERR_STATE, "set_query before upload_db");
     CK(cudaSetDevice(h->device));
     // a new search starts with a clear device status word and no results
@@ -2504,6 +2505,7 @@ extern "C" c2_status c2_set_query_batch(c2_handle* h, const c2_profiles* queries
     if (!h || !queries) return C2_ERR_ARG;
     c2_status st = check_profiles(h, queries);
     if (st != C2_OK) return st;
+    if (capturing(h)) return fail(h, C2_ERR_CUDA, "set_query_batch: the handle's stream is in a stream capture");
     CK(cudaSetDevice(h->device));
     const int nq = queries->nprofiles;
     // the queries' rows as c2_set_query packs them (score fields, exact

@@ -152,7 +152,8 @@ c2_status c2_upload_db(c2_handle* h, const c2_profiles* db,
  * score threshold and log E threshold as JobDispatcher::CalculateScoreThreshold
  * (src/libmycu/cualn/JobDispatcher.cpp:809-860).  The caller's arrays, page-
  * locked ones too, are free to change once the call has returned (so with every
- * call here that takes host arrays). */
+ * call here that takes host arrays).  Refused (C2_ERR_CUDA) while the handle's
+ * stream is being captured, as is c2_set_query_batch. */
 c2_status c2_set_query(c2_handle* h, const c2_profiles* q);
 
 /* Run phase 1 (fused score matrix + Viterbi DP max) of the current query over

@@ -1,6 +1,7 @@
 """Stream capture.  Phase 1 allocates nothing and waits for nothing once its
 operands are there, so it can be captured into a CUDA graph, on a handle's
-first phase 1 of a query too."""
+first phase 1 of a query too; c2_set_query and c2_set_query_batch copy from
+host memory that later calls use again, and refuse."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode", [0, 1])
 def test_phase1_captured(params, mode):
     import torch
-    from comer2_b200.native import Handle
+    from comer2_b200.native import C2Error, Handle
     rng = np.random.default_rng(8)
     db = S.random_profiles(rng, [20, 64, 300, 1001])     # few pairs: split where nothing forbids it
     short, q, q2 = (S.random_profiles(rng, [n]) for n in (20, 200, 200))
@@ -44,7 +45,16 @@ def test_phase1_captured(params, mode):
             g.replay()
         b, c = h.phase1()
         assert np.array_equal(b.view(np.uint32), best.view(np.uint32)) and np.array_equal(c, coords)
+    g2 = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g2, stream=stream):
+        with pytest.raises(C2Error, match="capture"):
+            h.set_query(q)
+        with pytest.raises(C2Error, match="capture"):
+            h.set_query_batch(q)
+    h.set_query(q)
+    h.run_phase1()
+    assert np.array_equal(h.phase1()[0].view(np.uint32), want[0][0].view(np.uint32))
     h.set_stream(0)
-    del g
+    del g, g2
     h.close()
     ref.close()
