@@ -1531,9 +1531,13 @@ static c2_status select_candidates(c2_handle* h, std::vector<int>& cand)
 {
     CK(cudaSetDevice(h->device));
     std::vector<float> b(h->nprof);
+    int stw = 0;
     Fetch F(h);
     CK(F.get(b.data(), h->d_best.p, (size_t)h->nprof * 4));
+    CK(F.get(&stw, h->d_status.p, sizeof(int)));
     CK(F.finish());
+    // (the maxima of a phase 1 whose wait gave up mean nothing)
+    if (stw == PIPE_ERR_TIMEOUT_P1) return fail(h, C2_ERR_DEVICE, "device status %d (%s)", stw, status_text(stw));
     const float cut = (h->score_mode == C2_SCORE_FP32)
                           ? h->scorethld
                           : h->scorethld - C2_TC_MARGIN * std::max(1.0f, std::fabs(h->scorethld));

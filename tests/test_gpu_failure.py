@@ -51,3 +51,19 @@ def test_map_sweep_wait_timeout(params):
     h.set_wait_limit(0)
     assert len(h.search(w.queries[0])) == n
     h.close()
+
+
+def test_candidates_of_a_timed_out_phase1_are_refused(params):
+    """The maxima of a phase 1 whose wait gave up are no candidates: the
+    finalisation reports the wait instead of working on them.  (With 300
+    profiles, fewer than the warps, the strips of every pair are split.)"""
+    from comer2_b200.native import C2Error, Handle
+    w = S.config(1, seed=2, scale=0.003)
+    h = Handle(params, 0)
+    h.upload_db(w.db)
+    h.set_query(w.queries[0])
+    h.set_wait_limit(1)
+    h.run_phase1()
+    with pytest.raises(C2Error, match="a wait in phase 1 timed out"):
+        h.run_finalize()
+    h.close()
