@@ -242,7 +242,7 @@ struct c2_handle {
     std::vector<float> ssss, cvkeys, cvvals, nnw;
     ScoreConsts sc{};
     DevBuf<float> d_ssss, d_cvvals, d_nnw;
-    DevBuf<int> d_status;
+    DevBuf<int> d_status;             // device status of the search, and of the adjoint
     // database
     int nprof = 0;
     int64_t npos = 0;
@@ -591,10 +591,10 @@ extern "C" c2_status c2_create(int device, const c2_params* p, c2_handle** out)
         h->nsm = prop.multiProcessorCount;
         h->grid = h->nsm * p1_blocks_per_sm(sc.cvcard);
         if (h->d_ssss.ensure(h->ssss.size(), h->budget) || h->d_cvvals.ensure(h->cvvals.size(), h->budget) ||
-            h->d_status.ensure(1, h->budget) || h->d_counter.ensure(4, h->budget)) { st = C2_ERR_NOMEM; break; }
+            h->d_status.ensure(2, h->budget) || h->d_counter.ensure(4, h->budget)) { st = C2_ERR_NOMEM; break; }
         if (cudaMemcpy(h->d_ssss.p, h->ssss.data(), h->ssss.size() * 4, cudaMemcpyHostToDevice) ||
             cudaMemcpy(h->d_cvvals.p, h->cvvals.data(), h->cvvals.size() * 4, cudaMemcpyHostToDevice) ||
-            cudaMemset(h->d_status.p, 0, sizeof(int))) { st = C2_ERR_CUDA; break; }
+            cudaMemset(h->d_status.p, 0, 2 * sizeof(int))) { st = C2_ERR_CUDA; break; }
         if (!h->nnw.empty()) {
             if (h->d_nnw.ensure(h->nnw.size(), h->budget) ||
                 cudaMemcpy(h->d_nnw.p, h->nnw.data(), h->nnw.size() * 4, cudaMemcpyHostToDevice)) { st = C2_ERR_CUDA; break; }
@@ -2315,7 +2315,7 @@ static void fill_adj(c2_handle* h, AdjArgs& a)
     a.scratch = h->d_adjscr.p;
     a.scratch_stride = (long long)(h->adj_Lmax + 31) * 160;
     a.counter = h->d_adjctr.p;
-    a.status = h->d_status.p;
+    a.status = h->d_status.p + 1;
     a.spin = h->spin;
     a.logz = h->d_adjlogz.p;
     a.grad = h->d_adjgrad.p;
@@ -2326,7 +2326,7 @@ static c2_status adj_results(c2_handle* h, float* dst, const float* src, size_t 
 {
     int stw = 0;
     Fetch F(h);
-    CK(F.get(&stw, h->d_status.p, sizeof(int)));
+    CK(F.get(&stw, h->d_status.p + 1, sizeof(int)));
     std::vector<float> r(n);
     CK(F.get(r.data(), src, n * sizeof(float)));
     CK(F.finish());
@@ -2462,7 +2462,7 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
     CK(up.finish());
     CK(cudaMemsetAsync(h->d_adjbuf.p + 5 * acc, 0xff, (size_t)racc * sizeof(float), h->stream));   // forward rows: empty
     CK(cudaMemsetAsync(h->d_adjctr.p, 0, 2 * sizeof(int), h->stream));
-    CK(cudaMemsetAsync(h->d_status.p, 0, sizeof(int), h->stream));
+    CK(cudaMemsetAsync(h->d_status.p + 1, 0, sizeof(int), h->stream));
     AdjArgs a;
     fill_adj(h, a);
     const int grid = (int)std::min<long long>((long long)h->nsm * std::max(fwd_occ, 1), (items + ADJ_WARPS - 1) / ADJ_WARPS);

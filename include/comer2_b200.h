@@ -336,10 +336,13 @@ c2_status c2_get_search_groups(const c2_handle* h, int32_t* ngroups);
  * longest pairs of a search, phase 1: a strip polls its predecessor's row or
  * progress at most `polls` times (0 restores the default, 2^22 polls with
  * 128 ns sleeps, about a second), then gives up, the sweep finishes without
- * faulting and c2_get_phase1 / c2_get_finalize / c2_run_stats / c2_get_hits /
- * c2_logz_fwd / c2_logz_bwd return C2_ERR_DEVICE ("a strip wait ... timed out").  The
- * next c2_set_query clears the error.  No counterpart in the reference,
- * whose kernels neither wait on one another nor time out. */
+ * faulting and the next call that reads its results returns C2_ERR_DEVICE:
+ * c2_get_phase1, c2_run_finalize and c2_search after phase 1 ("a wait in phase 1
+ * timed out"), c2_get_finalize / c2_run_stats / c2_get_hits after a phase-2 sweep
+ * and c2_logz_fwd / c2_logz_bwd themselves ("a strip wait timed out").  The next
+ * c2_set_query clears a search's error, the next c2_logz_fwd the adjoint's.  No
+ * counterpart in the reference, whose kernels neither wait on one another nor
+ * time out. */
 c2_status c2_set_wait_limit(c2_handle* h, uint32_t polls);
 
 /* Number of kernel launches issued by the handle since creation. */

@@ -2,6 +2,7 @@
 phase-2 strip pipelines give up after the poll limit set with
 c2_set_wait_limit, the sweep returns, and the call reports the device status
 (C2_ERR_DEVICE) instead of hanging; the handle then serves the next search."""
+import numpy as np
 import pytest
 
 from comer2_b200 import synth as S
@@ -66,4 +67,25 @@ def test_candidates_of_a_timed_out_phase1_are_refused(params):
     h.run_phase1()
     with pytest.raises(C2Error, match="a wait in phase 1 timed out"):
         h.run_finalize()
+    h.close()
+
+
+def test_adjoint_leaves_the_search_status(params):
+    """A forward call of the adjoint between a timed-out phase 1 and its fetch
+    does not clear phase 1's status; nor does a search's status fail it."""
+    from comer2_b200.native import C2Error, Handle
+    w = S.config(1, seed=2, scale=0.003)
+    h = Handle(params, 0)
+    h.upload_db(w.db)
+    h.set_query(w.queries[0])
+    pr = np.arange(4, dtype=np.int32)
+    z = h.logz_fwd(pr, None, 1.0, 1.0)
+    h.set_wait_limit(1)
+    h.run_phase1()
+    h.sync()
+    h.set_wait_limit(0)
+    assert np.array_equal(h.logz_fwd(pr, None, 1.0, 1.0), z)
+    h.logz_bwd()
+    with pytest.raises(C2Error, match="a wait in phase 1 timed out"):
+        h.phase1()
     h.close()
