@@ -1861,6 +1861,16 @@ __global__ void __launch_bounds__(FINW * 32) fin_kernel(FinArgs a)
 
 // ---------------------------------------------------------------------------
 // launchers (host)
+// A kernel's largest dynamic shared memory.  The attribute is the kernel's, shared
+// by all threads: set to the size at the largest CV map the layout takes, whatever
+// the call's own, or a thread's launch could find a smaller one set by another in
+// between.
+template <typename K>
+static cudaError_t set_smem_max(K* kernel, size_t bytes)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 size_t p1t_smem_bytes(int cvcard)
 {
     return (size_t)(cvcard * P1T_CVREP + P1T_WARPS * P1T_WARP_FLOATS) * sizeof(float);
@@ -1870,8 +1880,7 @@ int p1t_blocks_per_sm(int cvcard, cudaError_t* err)
 {
     int n = 0;
     const size_t sm = p1t_smem_bytes(cvcard);
-    cudaError_t e = cudaFuncSetAttribute(p1t_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(p1t_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = set_smem_max(p1t_kernel<true>, p1t_smem_bytes(P1T_MAX_CVCARD));
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, p1t_kernel<true>, P1T_WARPS * 32, sm);
     if (err) *err = e;
     return n;
@@ -1894,8 +1903,7 @@ int p1c_blocks_per_sm(int cvcard)
 {
     int n = 0;
     const size_t sm = p1c_smem_bytes(cvcard);
-    cudaFuncSetAttribute(p1c_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(p1c_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (set_smem_max(p1c_kernel<false>, p1c_smem_bytes(MAX_CVCARD)) != cudaSuccess) return 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, p1c_kernel<false>, P1C_WARPS * 32, sm);
     return n;
 }
@@ -1905,23 +1913,25 @@ size_t p1_smem_bytes(int cvcard)
     return (size_t)(cvcard * 32 + P1_WARPS * P1_WARP_FLOATS) * sizeof(float);
 }
 
+size_t p2s_smem_bytes(int cvcard)
+{
+    return (size_t)(cvcard * P1TC_CVREP + P2S_WARPS * P2S_WARP_FLOATS) * sizeof(float);
+}
+
 cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, cudaStream_t st)
 {
+    cudaError_t e;
     if (which == P1K_TENSOR) {
         const size_t sm = p1t_smem_bytes(a.sc.cvcard);
-        if (a.tc.uniform) {
-            cudaFuncSetAttribute(p1t_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            p1t_kernel<true><<<grid, P1T_WARPS * 32, sm, st>>>(a, qbkg);
-        } else {
-            cudaFuncSetAttribute(p1t_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            p1t_kernel<false><<<grid, P1T_WARPS * 32, sm, st>>>(a, qbkg);
-        }
+        auto* k = a.tc.uniform ? p1t_kernel<true> : p1t_kernel<false>;
+        if ((e = set_smem_max(k, p1t_smem_bytes(P1T_MAX_CVCARD))) != cudaSuccess) return e;
+        k<<<grid, P1T_WARPS * 32, sm, st>>>(a, qbkg);
         return cudaGetLastError();
     }
     if (which == P1K_CHUNKED) {
         const size_t sm = p1c_smem_bytes(a.sc.cvcard);
         auto* k = a.tc.uniform ? p1c_kernel<true> : p1c_kernel<false>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if ((e = set_smem_max(k, p1c_smem_bytes(MAX_CVCARD))) != cudaSuccess) return e;
         k<<<grid, P1C_WARPS * 32, sm, st>>>(a, qbkg);
         return cudaGetLastError();
     }
@@ -1929,10 +1939,9 @@ cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, c
     if (which == P1K_TRACEBACK) {
         // the score matrices first (their own work counter, a.counter[1]),
         // then the sweep over them
-        const size_t sms = (size_t)(a.sc.cvcard * P1TC_CVREP + P2S_WARPS * P2S_WARP_FLOATS) * sizeof(float);
+        const size_t sms = p2s_smem_bytes(a.sc.cvcard);
         auto* k2 = a.tc.uniform ? p2s_kernel<true> : p2s_kernel<false>;
-        cudaError_t e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms);
-        if (e != cudaSuccess) return e;
+        if ((e = set_smem_max(k2, p2s_smem_bytes(std::min(MAX_CVCARD, P1TC_MAX_CVCARD)))) != cudaSuccess) return e;
         int occ = 0;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k2, P2S_WARPS * 32, sms)) != cudaSuccess)
             return e;
@@ -1947,14 +1956,10 @@ cudaError_t launch_p1(const P1Args& a, const float* qbkg, int which, int grid, c
         const int wt = (int)std::max<long long>(1, std::min<long long>(P1TC_WARPS, (nit2 + nsm - 1) / nsm));
         const int gt = (int)std::min<long long>(nsm, (nit2 + wt - 1) / wt);
         const size_t smt = (size_t)wt * P1TC_WARP_FLOATS * sizeof(float);
-        // (the attribute is the kernel's, shared by all threads: always the largest size,
-        // or a thread's launch could find a smaller one set by another in between)
-        constexpr int smtmax = P1TC_WARPS * P1TC_WARP_FLOATS * (int)sizeof(float);
-        if ((e = cudaFuncSetAttribute(p1tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smtmax)) != cudaSuccess)
-            return e;
+        if ((e = set_smem_max(p1tc_kernel, P1TC_WARPS * P1TC_WARP_FLOATS * sizeof(float))) != cudaSuccess) return e;
         p1tc_kernel<<<gt, wt * 32, smt, st>>>(a, qbkg);
     } else {
-        cudaFuncSetAttribute(p1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if ((e = set_smem_max(p1_kernel, p1_smem_bytes(MAX_CVCARD))) != cudaSuccess) return e;
         p1_kernel<<<grid, P1_WARPS * 32, sm, st>>>(a, qbkg);
     }
     return cudaGetLastError();
@@ -1964,7 +1969,7 @@ int p1_blocks_per_sm(int cvcard)
 {
     int n = 0;
     const size_t sm = p1_smem_bytes(cvcard);
-    cudaFuncSetAttribute(p1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (set_smem_max(p1_kernel, p1_smem_bytes(MAX_CVCARD)) != cudaSuccess) return 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, p1_kernel, P1_WARPS * 32, sm);
     return n > 0 ? n : 1;
 }

@@ -1,6 +1,7 @@
 """Handles of one process used from several threads at once: what they share
 (the kernels' attributes, the pinned memory that handles borrow) must not let one
 thread's call disturb another's.  Each result equals the same call's alone."""
+import copy
 import threading
 
 import numpy as np
@@ -89,5 +90,43 @@ def test_query_batches_and_many_handles(params):
     for i, runs in enumerate(got):
         for z, g in runs:
             assert np.array_equal(z, want[i % 2][0]) and np.array_equal(g, want[i % 2][1])
+    for h in hs:
+        h.close()
+
+
+@pytest.mark.parametrize("mode,cards", [(0, (93, 250)), (1, (93, 106))])
+def test_context_vector_maps_of_different_sizes(params, mode, cards):
+    """Handles whose kernels want different amounts of shared memory (the CV
+    map's size), over and over in two threads."""
+    from comer2_b200.native import Handle
+    rng = np.random.default_rng(12)
+    q = S.random_profiles(rng, [70])
+    db = S.concat([S.planted_homolog(rng, q, 90, seg_lo=50, seg_hi=68), S.random_profiles(rng, [60] * 20)])
+    hs, alone = [], []
+    for card in cards:
+        p = copy.deepcopy(params)
+        n = card - len(p.cvs2s_keys)
+        p.cvs2s_keys = np.concatenate([p.cvs2s_keys, p.cvs2s_keys[-1] + 0.5 * np.arange(1, n + 1)])
+        p.cvs2s_values = np.concatenate([p.cvs2s_values, np.full(n, p.cvs2s_values[-1])])
+        h = Handle(p, 0)
+        h.set_score_mode(mode)
+        h.upload_db(db)
+        hs.append(h)
+        alone.append(h.search(q, arrays=True))
+        assert len(alone[-1][0]) >= 1
+
+    def body(h):
+        def run():
+            h.set_query(q)
+            for _ in range(20):
+                h.run_phase1()
+            h.phase1()
+            return h.search(q, arrays=True)
+        return run
+
+    got = _in_threads([body(h) for h in hs], 150)
+    for (ra, ba), runs in zip(alone, got):
+        for rb, bb in runs:
+            assert ra.tobytes() == rb.tobytes() and bytes(ba) == bytes(bb)
     for h in hs:
         h.close()
