@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <atomic>
@@ -52,6 +53,19 @@ struct Budget {
     size_t limit = 0;
     size_t used = 0;
     std::mutex mu;
+    // Spare memory: scratch that its handle can do without (phase 1's split pairs).
+    // Where an allocation would fail, all of it is given back first.  A handle
+    // holds spare_mu while it takes such scratch and launches what uses it.
+    struct Spare { const void* owner; std::function<bool()> give_back; };
+    std::mutex spare_mu;
+    std::vector<Spare> spare;
+    bool reclaim()
+    {
+        std::lock_guard<std::mutex> lk(spare_mu);
+        bool any = false;
+        for (const Spare& s : spare) any = s.give_back() || any;
+        return any;
+    }
 };
 
 template <typename T>
@@ -73,9 +87,18 @@ struct DevBuf {
         bud.reset();
     }
     // at least cnt elements; a request beyond the budget fails as an
-    // allocation failure would, before cudaMalloc
-    cudaError_t ensure(size_t cnt, const std::shared_ptr<Budget>& b = nullptr) {
+    // allocation failure would, before cudaMalloc.  Spare memory gives way first
+    // (not to a request for spare memory: reclaim false).
+    cudaError_t ensure(size_t cnt, const std::shared_ptr<Budget>& b = nullptr, bool reclaim = true) {
         if (cnt <= n && p) return cudaSuccess;
+        cudaError_t e = take(cnt, b);
+        if (e == cudaErrorMemoryAllocation && b && reclaim && b->reclaim()) {
+            (void)cudaGetLastError();
+            e = take(cnt, b);
+        }
+        return e;
+    }
+    cudaError_t take(size_t cnt, const std::shared_ptr<Budget>& b) {
         release();
         if (cnt == 0) cnt = 1;
         const size_t bytes = cnt * sizeof(T);
@@ -285,8 +308,9 @@ struct c2_handle {
     DevBuf<int> d_counter;
     DevBuf<float> d_bot;
     long long botstride = 0;
-    DevBuf<float> d_splitbnd;                  // phase-1 pairs split into strip items (split_pairs)
+    DevBuf<float> d_splitbnd;                  // phase-1 pairs split into strip items (split_pairs): spare memory
     DevBuf<unsigned long long> d_splitsync;    // their maxima, done counts and strip progress
+    bool spare_known = false;                  // the budget knows of it
     // finalisation
     int ncand = 0;
     std::vector<int> h_cand;
@@ -617,6 +641,12 @@ extern "C" c2_status c2_destroy(c2_handle* h)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
+    if (h->spare_known) {
+        Budget& b = *h->budget;   // (other handles may draw on it further)
+        std::lock_guard<std::mutex> lk(b.spare_mu);
+        b.spare.erase(std::remove_if(b.spare.begin(), b.spare.end(), [h](const Budget::Spare& s) { return s.owner == h; }),
+                      b.spare.end());
+    }
     delete h;
     return C2_OK;
 }
@@ -1329,6 +1359,16 @@ static void fill_p1(c2_handle* h, P1Args& a)
     a.tc = tc_consts(h->sc);
 }
 
+// Scratch of the split pairs given back (the caller holds the budget's spare_mu)
+static bool release_split(c2_handle* h)
+{
+    if (!h->d_splitbnd.p && !h->d_splitsync.p) return false;
+    (void)cudaDeviceSynchronize();   // a phase 1 in flight uses it
+    h->d_splitbnd.release();
+    h->d_splitsync.release();
+    return true;
+}
+
 // Phase-1 pairs whose strips become work items of their own (p1_take): those
 // that one of the nwarps warps would sweep in more than a share of the time all
 // pairs together take on all warps (both grow with the number of strips alike, so
@@ -1344,8 +1384,10 @@ static void fill_p1(c2_handle* h, P1Args& a)
 // vs 1,000 (FP32) 6.4 / 6.2 / 6.1 / 6.0 / 6.0, 1 x 150 vs 2,000 0.60 / 0.58 / 0.55 / 0.51 /
 // 0.49 (none split, before strips of 64 rows: 41.9, 16.2, 4.5, 32, 0.70); no pair
 // is split, and nothing changes, against 50,000 profiles.  0
-// without the scratch (it is small: the two boundary rows of the split pairs) --
-// the pairs then run whole, with the same results.
+// without the scratch -- the pairs then run whole, with the same results.  It is
+// the two boundary rows of the split pairs, 40 bytes a column (where few pairs come
+// to a warp all are split: 240 MB for 3,000 profiles of 2,000 columns), and spare
+// memory; the caller holds the budget's spare_mu until phase 1 is launched.
 constexpr double SPLIT_MANY = 0.8, SPLIT_FEW = 0.15, SPLIT_EVEN = 0.4;
 
 static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
@@ -1362,12 +1404,15 @@ static int split_pairs(c2_handle* h, int nwarps, P1Args& a)
                                              [&](int L) { return (double)L + 31.0 > share * mean; }) - sl.begin());
     if (n == 0 || (long long)n * ns > 0x7fffffff) return 0;
     const size_t words = (size_t)n * 8 + (size_t)n * 4 + (size_t)n * ns * 4;
-    if (h->d_splitbnd.ensure((size_t)h->db->soff[n] * 10, h->budget) != cudaSuccess ||
-        h->d_splitsync.ensure((words + 7) / 8, h->budget) != cudaSuccess ||
+    if (!h->spare_known) {
+        h->budget->spare.push_back({h, [h]() { return release_split(h); }});
+        h->spare_known = true;
+    }
+    if (h->d_splitbnd.ensure((size_t)h->db->soff[n] * 10, h->budget, false) != cudaSuccess ||
+        h->d_splitsync.ensure((words + 7) / 8, h->budget, false) != cudaSuccess ||
         cudaMemsetAsync(h->d_splitsync.p, 0, words, h->stream) != cudaSuccess) {
         (void)cudaGetLastError();
-        h->d_splitbnd.release();
-        h->d_splitsync.release();
+        release_split(h);
         return 0;
     }
     a.nsplit = n;
@@ -1404,6 +1449,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
             return fail(h, C2_ERR_CUDA, "tensor-core phase-1 kernel does not fit on an SM (%s)",
                         cudaGetErrorString(oe));
         gt = std::min(gt, h->grid * P1_WARPS / P1T_WARPS);
+        std::lock_guard<std::mutex> lk(h->budget->spare_mu);
         split_pairs(h, gt * P1T_WARPS, a);
         CK(launch_p1(a, h->d_qbkg.p, P1K_TENSOR, gt, h->stream));
         h->launches++;
@@ -1414,6 +1460,7 @@ extern "C" c2_status c2_run_phase1(c2_handle* h)
     int gc = (h->nsm - h->p1_reserve) * p1c_blocks_per_sm(h->sc.cvcard);
     if (gc < 1) return fail(h, C2_ERR_CUDA, "phase-1 kernel does not fit on an SM");
     gc = std::min(gc, h->grid * P1_WARPS / P1C_WARPS);
+    std::lock_guard<std::mutex> lk(h->budget->spare_mu);
     split_pairs(h, gc * P1C_WARPS, a);
     CK(launch_p1(a, h->d_qbkg.p, P1K_CHUNKED, gc, h->stream));
     h->launches++;
@@ -2050,7 +2097,8 @@ static void release_phase2(c2_handle* h)
     h->d_mapcand.release(); h->d_mappass.release(); h->d_alninfo.release(); h->d_fb.release(); h->d_bb.release();
     h->d_pairf.release(); h->d_pairc.release(); h->d_pairk.release(); h->d_aln.release(); h->d_alnpack.release();
     h->d_alnoff.release();
-    h->d_splitbnd.release(); h->d_splitsync.release();   // (phase 1 is done by then)
+    std::lock_guard<std::mutex> lk(h->budget->spare_mu);
+    release_split(h);
 }
 
 // Device bytes phase 2 takes for one candidate pair of db length L: score,

@@ -73,3 +73,49 @@ def test_budget_below_the_database_is_refused(params):
     h.upload_db(w.db)
     assert len(h.search(w.queries[0])) >= 1
     h.close()
+
+
+@pytest.mark.parametrize("staged", [True, False])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_split_scratch_gives_way(params, mode, staged):
+    """The boundary rows of phase 1's split pairs (40 bytes a db column; with
+    few pairs all are split) are not needed after it: under a limit that leaves
+    phase 2 what it needs without them, the stages run, one by one and in a
+    batch, within the limit and with the same hits."""
+    from comer2_b200.native import Handle
+    rng = np.random.default_rng(21)
+    q = S.random_profiles(rng, [300])
+    db = S.concat([S.planted_homolog(rng, q, 400, seg_lo=90, seg_hi=140) for _ in range(4)] +
+                  [S.random_profiles(rng, [400] * 40)])
+    rows = 40 * db.npositions
+
+    def handle():
+        h = Handle(params, 0)
+        h.set_score_mode(mode)
+        h.upload_db(db)
+        return h
+
+    def stages(h):
+        h.set_query(q)
+        h.run_phase1()
+        use = h.memory_use()
+        h.run_finalize()
+        h.run_stats()
+        return use, h.hits_arrays(h.run_map())
+
+    h = handle()
+    after1, (rec, buf) = stages(h)
+    full = h.memory_use()
+    assert len(rec) >= 4
+    h.close()
+    limit = full - rows + (64 << 10)
+    h = handle()
+    h.set_memory_limit(limit)
+    if staged:
+        use, got = stages(h)
+        assert use == after1                   # the rows were there, and in phase 2's way
+    else:
+        got = h.search_batch(q, 1)[0]
+    assert got[0].tobytes() == rec.tobytes() and np.array_equal(got[1], buf)
+    assert h.memory_use() <= limit
+    h.close()
