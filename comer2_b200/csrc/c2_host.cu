@@ -389,6 +389,12 @@ static cudaError_t sync_stream(c2_handle* h)
     return e;
 }
 
+static bool memory_limited(const c2_handle* h)
+{
+    std::lock_guard<std::mutex> lk(h->budget->mu);
+    return h->budget->limit != 0;
+}
+
 // Is the handle's stream being captured into a graph?  (Then nothing may be
 // allocated or waited for, and nothing copied from host memory that is used again.)
 static bool capturing(const c2_handle* h)
@@ -2161,13 +2167,11 @@ static c2_status plan_groups(c2_handle* h, const std::vector<int>& cand, std::ve
     return C2_OK;
 }
 
-extern "C" c2_status c2_search(c2_handle* h, const c2_profiles* q, int32_t* nhits)
+// Phase 2 of the current query in candidate groups that fit the memory budget
+static c2_status search_groups(c2_handle* h, int32_t* nhits)
 {
-    if (!h || !q || !nhits) return C2_ERR_ARG;
     c2_status st;
     int32_t n = 0;
-    if ((st = c2_set_query(h, q)) != C2_OK) return st;
-    if ((st = c2_run_phase1(h)) != C2_OK) return st;
     std::vector<int> cand;
     if ((st = select_candidates(h, cand)) != C2_OK) return st;
     std::vector<std::vector<int>> groups;
@@ -2219,6 +2223,15 @@ extern "C" c2_status c2_search(c2_handle* h, const c2_profiles* q, int32_t* nhit
     h->acc_valid = true;
     *nhits = (int32_t)h->acc_hits.size();
     return C2_OK;
+}
+
+extern "C" c2_status c2_search(c2_handle* h, const c2_profiles* q, int32_t* nhits)
+{
+    if (!h || !q || !nhits) return C2_ERR_ARG;
+    c2_status st;
+    if ((st = c2_set_query(h, q)) != C2_OK) return st;
+    if ((st = c2_run_phase1(h)) != C2_OK) return st;
+    return search_groups(h, nhits);
 }
 
 extern "C" c2_status c2_get_search_groups(const c2_handle* h, int32_t* ngroups)
@@ -2463,11 +2476,7 @@ static c2_status logz_fwd_pairs(c2_handle* h, const int32_t* profiles, const int
     {
         const size_t base = adj_base(acc, racc), nF = (size_t)acc * 5;
         const size_t have = h->d_adjbuf.p ? h->d_adjbuf.n : 0;
-        bool limited;
-        {
-            std::lock_guard<std::mutex> lk(h->budget->mu);
-            limited = h->budget->limit != 0;
-        }
+        const bool limited = memory_limited(h);
         // (asking for the free memory takes longer than a small batch's sweeps: not
         // for a buffer that is already there)
         size_t fr = 0, tot = 0;
@@ -2828,6 +2837,8 @@ extern "C" c2_status c2_search_batch(c2_handle* h, const c2_profiles* queries, i
                 if (s == C2_OK) s = c2_run_finalize(w, &n);
                 if (s == C2_OK) s = c2_run_stats(w, &n);
                 if (s == C2_OK) s = c2_run_map(w, &nh);
+                // all candidates at once beyond the memory limit: in groups
+                if (s == C2_ERR_NOMEM && memory_limited(w)) s = search_groups(w, &nh);
                 if (s == C2_OK && sync_stream(w) != cudaSuccess) s = C2_ERR_CUDA;
             }
             if (s == C2_OK) s = c2_get_hits(w, nullptr, 0, nullptr, &nb);

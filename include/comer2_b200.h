@@ -299,8 +299,9 @@ c2_status c2_sync(c2_handle* h);
 
 /* Device memory budget of the handle, in bytes (0: none): a buffer that
  * would take the handle's device memory beyond it is refused with
- * C2_ERR_NOMEM before cudaMalloc; c2_search then processes its candidate
- * pairs in groups whose phase-2 scratch fits.  Replaces the reference's
+ * C2_ERR_NOMEM before cudaMalloc; c2_search, and c2_search_batch for a query
+ * whose candidate pairs do not fit at once, then process them in groups whose
+ * phase-2 scratch fits (c2_run_finalize takes all at once).  Replaces the reference's
  * --dev-mem limit on its device heap (CuDeviceMemory, src/comer/comer.h
  * usage: "Maximum amount of GPU memory (MB) that can be used").  Worker
  * handles of c2_search_batch draw on the same budget. */

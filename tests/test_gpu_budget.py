@@ -119,3 +119,39 @@ def test_split_scratch_gives_way(params, mode, staged):
     assert got[0].tobytes() == rec.tobytes() and np.array_equal(got[1], buf)
     assert h.memory_use() <= limit
     h.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_batch_under_a_limit_goes_in_groups(params, mode):
+    """c2_search_batch runs a query whose candidates do not fit the limit at
+    once in groups, as c2_search does, and the others as before."""
+    from comer2_b200.native import Handle
+    rng = np.random.default_rng(22)
+    qs = S.random_profiles(rng, [300, 40])
+    db = S.concat([S.planted_homolog(rng, qs.profile(0), 400, seg_lo=90, seg_hi=140) for _ in range(12)] +
+                  [S.random_profiles(rng, [300] * 20)])
+
+    def handle(limit):
+        h = Handle(params, 0)
+        h.set_score_mode(mode)
+        h.upload_db(db)
+        h.set_memory_limit(limit)
+        return h
+
+    h = handle(0)
+    h.set_query(qs.profile(0))
+    h.run_phase1()
+    h.sync()
+    base = h.memory_use()
+    want = [_key(*h.search(qs.profile(k), arrays=True)) for k in range(2)]
+    full = h.memory_use()
+    assert len(want[0]) >= 12
+    h.close()
+    limit = base + (full - base) // 2
+    h = handle(limit)
+    got = [_key(*r) for r in h.search_batch(qs, 1)]
+    assert got == want
+    assert h.memory_use() <= limit
+    got = h.search_batch(qs.profile(0), 1)
+    assert h.search_groups() >= 2 and _key(*got[0]) == want[0]
+    h.close()
