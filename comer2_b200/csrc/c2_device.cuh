@@ -120,11 +120,15 @@ constexpr int P1T_MAX_CVCARD = 106;
 // rows, or the tensor fragments) and the wavefront's 8-byte reads are free of
 // bank conflicts; column-record ring of 7 chunks and a mirror of its first
 // chunk, so that the 8 records a lane reads in one DP stage never wrap; the row
-// above the strip for one chunk.
+// above the strip for one chunk and the strip's own last row (not in its place:
+// nothing orders lane 31's write of a step before lane 0's read of it).
 constexpr int P1_C = 8;
 constexpr int P1_SLOTS = 40, P1_RLD = 68, P1_CMOD = 56, P1_CRING = 64;
 constexpr int P1_BND = 5 * P1_C;
-constexpr int P1_WF_FLOATS = P1_SLOTS * P1_RLD + P1_CRING * P1C_TRS + P1_BND;
+// (the two rows, and a gap that leaves the arrays after them where the FP32 kernel
+// runs best: 14.08 ms on 1 x 400 vs 20,000 profiles, without it 14.27)
+constexpr int P1_BNDS = 2 * P1_BND + 24;
+constexpr int P1_WF_FLOATS = P1_SLOTS * P1_RLD + P1_CRING * P1C_TRS + P1_BNDS;
 // FP32 kernel: also the SS row table of the strip and the record staging ring
 constexpr int P1C_WARPS = 8, P1C_CVREP = 16;
 constexpr int P1C_WARP_FLOATS = P1_WF_FLOATS + MAX_SSSS_CARD * P1_ROWS + REC_SLOTS * DR_STRIDE;

@@ -616,15 +616,15 @@ __device__ __forceinline__ void p1_row_async(const P1Args& a, const P1Item& it, 
     cp_async_commit();
 }
 
-// The strip's last row after a DP stage over [k0, k0 + P1_C): slot l of bnd holds
+// The strip's last row after a DP stage over [k0, k0 + P1_C): slot l of own holds
 // lane 31's states at column k0 - 31 + l
-__device__ __forceinline__ void p1_row_flush(const float* __restrict__ bnd, float* __restrict__ botw, int ldb, int k0,
+__device__ __forceinline__ void p1_row_flush(const float* __restrict__ own, float* __restrict__ botw, int ldb, int k0,
                                              int L, int lane)
 {
     const int c = k0 - 31 + lane;
     if (lane < P1_C && c >= 0 && c < L) {
-        reinterpret_cast<float4*>(botw)[c] = *reinterpret_cast<const float4*>(bnd + lane * 4);
-        botw[4 * ldb + c] = bnd[4 * P1_C + lane];
+        reinterpret_cast<float4*>(botw)[c] = *reinterpret_cast<const float4*>(own + lane * 4);
+        botw[4 * ldb + c] = own[4 * P1_C + lane];
     }
 }
 
@@ -731,9 +731,9 @@ __device__ __forceinline__ void wf2_edge(Wf2Edge& E, const Wf2& D, const float* 
 }
 
 // Four wavefront steps: rp the lane's scores (P1_RLD floats a step), tc its
-// column records, bnd the row above (row: slots u0..), j0 the lane's column at
-// the first step, k0 that step.  HEAD: column 0 may be among the steps (the
-// first P1T_HEAD chunks of a strip).  Cells outside the matrix have scores of
+// column records, bnd the row above (slots u0..) and P1_BND on the strip's own, j0 the lane's column at
+// the first step, k0 that step.  HEAD: column 0 may be among the steps (steps
+// below 32 of a strip).  Cells outside the matrix have scores of
 // -inf, so their MM stays 0, and their other states reach no cell inside.
 template <bool HEAD>
 __device__ __forceinline__ void wf2_steps4(Wf2& D, const Wf2Edge& E, const float* __restrict__ rp,
@@ -777,9 +777,9 @@ __device__ __forceinline__ void wf2_steps4(Wf2& D, const Wf2Edge& E, const float
             uMM = nMM; uMI = nMI; uIM = nIM; uDN = nDN; uND = nND;
         }
         if (wr_bot) {
-            // lane 31's row 1 (column k0 + u - 31) into the slot lane 0 read at the top of this step
-            *reinterpret_cast<float4*>(bnd + 4 * (u0 + u)) = make_float4(uMM, uMI, uIM, uDN);
-            bnd[4 * P1_C + u0 + u] = uND;
+            // lane 31's row 1 (column k0 + u - 31) into the strip's last row
+            *reinterpret_cast<float4*>(bnd + P1_BND + 4 * (u0 + u)) = make_float4(uMM, uMI, uIM, uDN);
+            bnd[P1_BND + 4 * P1_C + u0 + u] = uND;
         }
     }
     // the maximum of the eight cells first (4 three-input maxima); its cell
@@ -815,8 +815,8 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
     float* wb = smem + cvcard * P1C_CVREP + wid * P1C_WARP_FLOATS;
     float* ring = wb;                                         // [P1_SLOTS anti-diagonals][P1_RLD] scores
     float* cring = ring + P1_SLOTS * P1_RLD;                  // [P1_CRING][P1C_TRS] column transitions
-    float* bnd = cring + P1_CRING * P1C_TRS;                  // [P1_BND] row above the strip
-    float* U = bnd + P1_BND;                                  // [card][P1_ROWS] SS row table
+    float* bnd = cring + P1_CRING * P1C_TRS;                  // [2][P1_BND] row above the strip, its last row
+    float* U = bnd + P1_BNDS;                                  // [card][P1_ROWS] SS row table
     float* rec = U + MAX_SSSS_CARD * P1_ROWS;                 // [REC_SLOTS][DR_STRIDE] db records
     for (int i = threadIdx.x; i < cvcard * P1C_CVREP; i += blockDim.x) cvtab[i] = a.cvvals[i / P1C_CVREP];
     // (a lane may read a score slot or record that no chunk has filled yet;
@@ -935,7 +935,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
                 }
                 __syncwarp();
                 if (s + 1 < nstrips) {
-                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
+                    p1_row_flush(bnd + P1_BND, botw, ldb, k0, L, lane);
                     // columns up to k0 - 24 are there: published every other chunk
                     if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= kend))
                         p1_publish(a, it, s, min(k0 - 23, L), lane);
@@ -1435,8 +1435,8 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
     float* wb = smem + cvcard * P1T_CVREP + wid * P1T_WARP_FLOATS;
     float* ring = wb;                                         // [P1_SLOTS anti-diagonals][P1_RLD] scores
     float* cring = ring + P1_SLOTS * P1_RLD;                // [P1_CRING][P1C_TRS] column records
-    float* bnd = cring + P1_CRING * P1C_TRS;                 // [P1_BND] row above the strip
-    float* rqt = bnd + P1_BND;                               // [P1_ROWS][2] cvnorm, c2 - 2 x CV log prior
+    float* bnd = cring + P1_CRING * P1C_TRS;                 // [2][P1_BND] row above the strip, its last row
+    float* rqt = bnd + P1_BNDS;                               // [P1_ROWS][2] cvnorm, c2 - 2 x CV log prior
     unsigned* btile = reinterpret_cast<unsigned*>(rqt + 2 * P1_ROWS);   // [TC_TILE_WORDS] db operand tile
     unsigned long long* tbar = reinterpret_cast<unsigned long long*>(btile + TC_TILE_WORDS);
     for (int i = threadIdx.x; i < cvcard * P1T_CVREP; i += blockDim.x)
@@ -1697,7 +1697,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
                 }
                 __syncwarp();
                 if (s + 1 < nstrips) {
-                    p1_row_flush(bnd, botw, ldb, k0, L, lane);
+                    p1_row_flush(bnd + P1_BND, botw, ldb, k0, L, lane);
                     // columns up to k0 - 24 are there: published every other chunk
                     if (it.pi >= 0 && k0 >= 24 && ((m & 1) || k0 + P1_C >= kend))
                         p1_publish(a, it, s, min(k0 - 23, L), lane);
