@@ -17,8 +17,8 @@ def _pair_scratch_bytes(Lq, L, Lmax):
     """The library's estimate of one candidate pair's phase-2 device bytes
     (pair_scratch_bytes in c2_host.cu)."""
     ns = (Lq + 31) // 32
-    return (9 * Lq * L + 2 * 10 * 4 * L + 2 * 4 * ns + 4 * ns * 2 + 2 * 4 * 32 * ns * (L + 31)
-            + 2 * 5 * (Lq + Lmax + 1) + 512)
+    return (9 * Lq * L + 2 * 5 * 4 * ns * (L + 12) + 4 * ns * 2 + 2 * 4 * 32 * ns * (L + 31)
+            + 2 * 5 * (Lq + Lmax + 1) + 4 * 641 + 512)
 
 
 def _key(rec, buf):
@@ -52,7 +52,7 @@ def test_budget_groups_give_the_same_hits(params, mode):
     # more, so that the candidates go in several groups
     Lq = int(w.queries[0].lengths[0])
     longest = max(int(w.db.lengths[x[0]]) for x in ref)
-    limit = base + (2 << 20) + int(1.3 * _pair_scratch_bytes(Lq, longest, int(w.db.lengths.max())) / 0.9)
+    limit = base + (2 << 20) + int(1.3 * _pair_scratch_bytes(Lq, longest, int(w.db.lengths.max())) / 0.97)
     h.set_memory_limit(limit)
     got = _key(*h.search(w.queries[0], arrays=True))
     assert h.search_groups() >= 2

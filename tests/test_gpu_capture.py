@@ -10,6 +10,7 @@ from comer2_b200 import synth as S
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
 @pytest.mark.parametrize("mode", [0, 1])
 def test_phase1_captured(params, mode):
     import torch

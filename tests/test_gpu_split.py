@@ -7,7 +7,9 @@ with the same FP32 arithmetic, so the FP32 maxima and cells must be its bits;
 the tensor-core form's maxima must lie within its rounding of them (1e-4
 relative; a context-vector value at a bin edge moves one cell by one table
 step, 0.05 allows for that in at most 2 % of the pairs, which needs sets of many
-pairs: test_gpu_phase1.py has the tensor-core form on a dozen pairs)."""
+pairs: test_gpu_phase1.py has the tensor-core form on a dozen pairs).  That pairs
+were split shows in the handle's device memory: their boundary rows, 40 bytes a
+column, are allocated by the first phase 1 that splits any."""
 import ctypes as C
 
 import numpy as np
@@ -42,11 +44,15 @@ def test_split_pairs_match_whole_pairs(params, which, lq):
     h._ck(h.lib.c2_run_phase1_static(h._h, C.c_void_p(d_best.data_ptr()), C.c_void_p(d_coords.data_ptr())), "static")
     h.sync()
     ref = d_best.cpu().numpy()
+    use = h.memory_use()
+    # (of the mixed set the three pairs above the mean time per warp)
+    split = {"mixed": 700 + 1999 + 2000, "few": sum(LENGTHS["few"]), "equal": 0}[which] if lq > 64 else 0
     for _ in range(2):   # the second run reuses the split pairs' scratch
         h.run_phase1()
         best, coords = h.phase1()
         assert np.array_equal(best.view(np.uint32), ref.view(np.uint32))
         assert np.array_equal(coords, d_coords.cpu().numpy().view(np.uint32))
+        assert (h.memory_use() > use) == (split > 0) and h.memory_use() - use >= 40 * split
     if n >= 1000:
         h.set_score_mode(1)
         for _ in range(2):
