@@ -241,7 +241,10 @@ struct FinArgs {
 // through L2 (with progress words, released every 8 columns and acquired by the
 // strip below, the fence and the acquire took longer than the 8 columns' cells).
 // A computed value is never ROW_EMPTY: the device's arithmetic yields only the
-// NaN 0x7fffffff.
+// NaN 0x7fffffff.  The copies (16 bytes each) may read words that another SM is
+// writing.  What is relied on is that an aligned 4-byte word arrives whole, old or
+// new; nothing is assumed about the order in which a row's words arrive: every one
+// is tested, and one found empty is read again (ld.relaxed.gpu).
 // Layout of a row: [ld][4] states MM MI IM DN, then [ld] ND, ld the length
 // rounded up to 4; the rows of a pair's strips follow one another.
 namespace c2 {

@@ -1383,14 +1383,23 @@ static bool release_split(c2_handle* h)
 // allows.  The whole pairs come last, longest first: where a last one per warp
 // is short (the nwarps-th shortest pair at most SPLIT_EVEN of the mean time), they
 // even out what the longer ones leave, and only pairs above SPLIT_MANY would be the
-// tail; where not (few pairs a warp), a pair above SPLIT_FEW is.  Phase-1
-// times in ms with shares of 1 / 0.7 / 0.5 / 0.3 / 0.15: 1 x 3,000 vs 4,000 profiles
-// 18.8 / 18.7 / 19.3 / 21.0 / 21.3, 1 x 1,237 vs 4,999 8.2 / 8.2 / 8.7 / 8.8 / 9.4, 1 x 250
-// vs 3,000 (FP32) 1.36 / 1.47 / 1.40 / 1.44 / 1.54; with few pairs a warp, 7 queries
-// vs 1,000 (FP32) 6.4 / 6.2 / 6.1 / 6.0 / 6.0, 1 x 150 vs 2,000 0.60 / 0.58 / 0.55 / 0.51 /
-// 0.49 (none split, before strips of 64 rows: 41.9, 16.2, 4.5, 32, 0.70); no pair
-// is split, and nothing changes, against 50,000 profiles.  0
-// without the scratch -- the pairs then run whole, with the same results.  It is
+// tail; where not (few pairs a warp), a pair above SPLIT_FEW is.
+// Phase-1 times in ms (medians of three processes, which differ by up to 0.5 %; r the
+// nwarps-th shortest pair over the mean time) with shares of
+//                                       1     0.9   0.8   0.7   0.5   0.3   0.15  0.08
+//   1 x 3,000 vs 4,000, r 0.35          18.8  18.9  19.0  18.7  19.3  20.9  21.2  20.3
+//   1 x 1,237 vs 4,999, r 0.25          8.12  8.08  8.12  8.17  8.73  8.77  9.37  9.02
+//   16 queries vs 5,000, r 0.25         27.4  27.9  28.5  29.3  30.1  30.7  32.5  32.8
+//   1 x 250 vs 3,000, r 0.29 (FP32)     1.35  1.35  1.39  1.45  1.39  1.42  1.54  1.55
+//   1 x 150 vs 2,000, r 1.39            0.597 0.581 0.587 0.579 0.535 0.518 0.488 0.489
+//   7 queries vs 1,000 (FP32, fewer
+//   pairs than warps)                   6.36  6.22  6.09  5.95  5.81  5.79  5.81  5.80
+// (none split, before strips of 64 rows: 41.9, 16.2, 59, 4.5, 0.70, 32).  Between
+// the two groups, 1 x 400 with r of 0.44 / 0.57 / 0.83 (1,776 warps), shares of 1, 0.8
+// and 0.15 take 1.67, 1.69, 1.94 / 1.53, 1.54, 1.75 / 1.35, 1.38, 1.54 ms: SPLIT_EVEN
+// could lie at 0.9 and SPLIT_MANY at 1.  No pair is split, and nothing changes,
+// against 50,000 profiles.
+// 0 without the scratch -- the pairs then run whole, with the same results.  It is
 // the two boundary rows of the split pairs, 40 bytes a column (where few pairs come
 // to a warp all are split: 240 MB for 3,000 profiles of 2,000 columns), and spare
 // memory; the caller holds the budget's spare_mu until phase 1 is launched.
@@ -2108,8 +2117,8 @@ static void release_phase2(c2_handle* h)
 }
 
 // Device bytes phase 2 takes for one candidate pair of db length L: score,
-// modular-score and traceback matrices, strip-boundary rows and progress
-// words, the MAP sweeps' F and B in wavefront order, the alignment rows, and
+// modular-score and traceback matrices, the strips' last rows (forward and
+// backward), the MAP sweeps' F and B in wavefront order, the alignment rows, and
 // the per-pair records (an upper estimate of the buffers finalize_set,
 // c2_run_stats, c2_run_map and c2_get_hits size by the pairs).
 static size_t pair_scratch_bytes(const c2_handle* h, int L)

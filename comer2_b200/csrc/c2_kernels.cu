@@ -581,9 +581,9 @@ __device__ __forceinline__ bool p1_take(const P1Args& a, int nstrips, int lane, 
 }
 
 // The rows between the strips of a pair, in the layout of the shared-memory
-// row (bnd_put): states MM MI IM DN per column, then the ND values from
-// 4 ldb on; ldb a multiple of 4 columns, the buffer 16-byte aligned.  Each
-// half is thus one wide store or asynchronous copy per chunk.
+// row: states MM MI IM DN per column, then the ND values from 4 ldb on; ldb a
+// multiple of 4 columns, the buffer 16-byte aligned.  Each half is thus one wide
+// store or asynchronous copy per chunk.
 
 // Wait (split pairs only) until columns [c0, c0 + P1_C) of the row above strip s
 // are there; false: no such row
@@ -966,7 +966,7 @@ p1c_kernel(P1Args a, const float* __restrict__ qbkg)
 // ---------------------------------------------------------------------------
 // Phase-2 score matrices: the FP32 scores and modular scores of every cell of
 // the candidate pairs, column-major per pair (the layout of the finalisation,
-// statistics and MAP stages), by cell_score -- the arithmetic of phase 1's
+// statistics and MAP stages), by cell_scores -- the arithmetic of phase 1's
 // FP32 form.  One warp per (candidate, strip) at a time, lanes own query rows,
 // db records staged in shared memory as in phase 1; no dependencies between
 // work items, so every resident warp works.  Where there are few candidates an
@@ -1387,7 +1387,7 @@ __global__ void __launch_bounds__(128) tc_pack_kernel(const float* __restrict__ 
 //         (cvm - shift)) with the table pre-shifted: a reassociation within
 //         the rounding of the split-BF16 products (this form only ranks the
 //         pairs; the candidates are rescored in FP32)
-// (cell_score is the FP32 form; src/libmycu/cusco/CuBatchScoreMatrix_ddms2s_h2.cu)
+// (cell_scores is the FP32 form; src/libmycu/cusco/CuBatchScoreMatrix_ddms2s_h2.cu)
 template <bool CVUNIF>
 __device__ __forceinline__ float tc_cell(float daa, float dot, float ss, float cq, float rq2, float cd, float pd2,
                                          const float* __restrict__ cvl, const TcConsts& tc)
@@ -1511,7 +1511,7 @@ p1t_kernel(P1Args a, const float* __restrict__ qbkg)
             const int kend = L + ((rows - 1) >> 1);            // wavefront steps
             // this strip's query fragments into TMEM, 40 columns per m-tile:
             // the amino-acid rows scaled for the pair (q(a) / (0.5 (bq(a) +
-            // bd(a))), as cell_score's Qt) and split, then the CV and SS words
+            // bd(a))), as row_ops' Qt) and split, then the CV and SS words
             {
                 const float* __restrict__ bd = a.pbkg + (long long)p * NAA;
                 float w[6];
