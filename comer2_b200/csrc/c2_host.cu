@@ -385,7 +385,7 @@ static c2_status fail(c2_handle* h, c2_status st, const char* fmt, ...)
 static cudaError_t sync_stream(c2_handle* h)
 {
     const cudaError_t e = cudaStreamSynchronize(h->stream);
-    h->stage.used = 0;
+    if (e == cudaSuccess) h->stage.used = 0;   // (refused on a capturing stream: copies may be in flight)
     return e;
 }
 
